@@ -108,7 +108,7 @@ __device__ __forceinline__ void m2l_field(float dx, float dy, float dz, float d2
                                           float& fx, float& fy, float& fz) {
     // polesitter.h:1065-1092 with rsqrt: 1/r^3 and 1/r^5 of the softened distance
     const float soft = d2 + 0.1f;
-    const float inv = rsqrtf(soft);
+    const float inv = rsqrt_soft(soft);
     const float inv2 = inv * inv;
     const float ir3 = inv2 * inv;
     const float ir5 = ir3 * inv2;
@@ -126,7 +126,7 @@ __device__ __forceinline__ void m2l_field_grad(float dx, float dy, float dz, flo
                                                float& fx, float& fy, float& fz, float& g3,
                                                float& gi) {
     const float soft = d2 + 0.1f;
-    const float inv = rsqrtf(soft);
+    const float inv = rsqrt_soft(soft);
     const float inv2 = inv * inv;
     const float ir3 = inv2 * inv;
     const float ir5 = ir3 * inv2;
@@ -214,7 +214,7 @@ __device__ __forceinline__ void p2p_range(const float4* __restrict__ xyzm, uint2
         const float4 p = xyzm[r.x + j];
         const float dx = p.x - t.x, dy = p.y - t.y, dz = p.z - t.z;
         const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) + 0.1f;
-        const float inv = rsqrtf(r2);
+        const float inv = rsqrt_soft(r2);
         const float f = p.w * (inv * inv * inv);
         if (kahan) {
             const float yx = __fsub_rn(__fmul_rn(dx, f), cx);
@@ -841,7 +841,7 @@ __global__ void __launch_bounds__(
                         // pairs add (x * 1 + acc = x + acc, x * 0 + acc = acc)
                         const float2 on = make_float2(s0 ? 1.f : 0.f, s1 ? 1.f : 0.f);
                         const float2 soft = __fadd2_rn(d2, make_float2(0.1f, 0.1f));
-                        const float2 inv = make_float2(rsqrtf(soft.x), rsqrtf(soft.y));
+                        const float2 inv = make_float2(rsqrt_soft(soft.x), rsqrt_soft(soft.y));
                         const float2 inv2 = __fmul2_rn(inv, inv);
                         const float2 ir3 = __fmul2_rn(inv2, inv);
                         const float2 ir5 = __fmul2_rn(ir3, inv2);
@@ -1131,7 +1131,7 @@ __device__ __forceinline__ void dense_tile(const DenseTile& tile, uint32_t m0, u
                             pw = h ? b.w : b.z;
                 const float dx = px - t.x, dy = py - t.y, dz = pz - t.z;
                 const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) + 0.1f;
-                const float inv = rsqrtf(r2);
+                const float inv = rsqrt_soft(r2);
                 const float f = pw * (inv * inv * inv);
                 const float yx = __fsub_rn(__fmul_rn(dx, f), cx);
                 const float yy = __fsub_rn(__fmul_rn(dy, f), cy);
@@ -1160,7 +1160,7 @@ __device__ __forceinline__ void dense_tile(const DenseTile& tile, uint32_t m0, u
             float2 r = __ffma2_rn(dz, dz, eps);
             r = __ffma2_rn(dy, dy, r);
             r = __ffma2_rn(dx, dx, r);
-            const float2 i = make_float2(rsqrtf(r.x), rsqrtf(r.y));
+            const float2 i = make_float2(rsqrt_soft(r.x), rsqrt_soft(r.y));
             const float2 f = __fmul2_rn(make_float2(b.z, b.w), __fmul2_rn(__fmul2_rn(i, i), i));
             sx = __ffma2_rn(dx, f, sx);
             sy = __ffma2_rn(dy, f, sy);
@@ -1229,7 +1229,7 @@ __device__ __forceinline__ void walk_leaf(const float4* __restrict__ xyzm, uint3
         for (uint32_t j = slice; j < cnt; j += S) {
             const float4 p = xyzm[first + j];
             const float dx = p.x - t.x, dy = p.y - t.y, dz = p.z - t.z;
-            const float inv = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 0.1f))));
+            const float inv = rsqrt_soft(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 0.1f))));
             const float f = p.w * (inv * inv * inv);
             const float yx = __fsub_rn(__fmul_rn(dx, f), cx);
             const float yy = __fsub_rn(__fmul_rn(dy, f), cy);
@@ -1251,8 +1251,8 @@ __device__ __forceinline__ void walk_leaf(const float4* __restrict__ xyzm, uint3
             const float4 p0 = xyzm[first + j], p1 = xyzm[first + j + S];
             const float dx0 = p0.x - t.x, dy0 = p0.y - t.y, dz0 = p0.z - t.z;
             const float dx1 = p1.x - t.x, dy1 = p1.y - t.y, dz1 = p1.z - t.z;
-            const float i0 = rsqrtf(fmaf(dx0, dx0, fmaf(dy0, dy0, fmaf(dz0, dz0, 0.1f))));
-            const float i1 = rsqrtf(fmaf(dx1, dx1, fmaf(dy1, dy1, fmaf(dz1, dz1, 0.1f))));
+            const float i0 = rsqrt_soft(fmaf(dx0, dx0, fmaf(dy0, dy0, fmaf(dz0, dz0, 0.1f))));
+            const float i1 = rsqrt_soft(fmaf(dx1, dx1, fmaf(dy1, dy1, fmaf(dz1, dz1, 0.1f))));
             const float f0 = p0.w * (i0 * i0 * i0), f1 = p1.w * (i1 * i1 * i1);
             ax = fmaf(dx0, f0, ax);
             ay = fmaf(dy0, f0, ay);
@@ -1264,7 +1264,7 @@ __device__ __forceinline__ void walk_leaf(const float4* __restrict__ xyzm, uint3
         if (j < cnt) {
             const float4 p = xyzm[first + j];
             const float dx = p.x - t.x, dy = p.y - t.y, dz = p.z - t.z;
-            const float inv = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 0.1f))));
+            const float inv = rsqrt_soft(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 0.1f))));
             const float f = p.w * (inv * inv * inv);
             ax = fmaf(dx, f, ax);
             ay = fmaf(dy, f, ay);
@@ -1866,7 +1866,7 @@ __global__ void __launch_bounds__(kHeavyThreads, 2) k_heavy_leaf(TravArgs A) {
                                     float2 r = __ffma2_rn(dz, dz, eps);
                                     r = __ffma2_rn(dy, dy, r);
                                     r = __ffma2_rn(dx, dx, r);
-                                    const float2 i = make_float2(rsqrtf(r.x), rsqrtf(r.y));
+                                    const float2 i = make_float2(rsqrt_soft(r.x), rsqrt_soft(r.y));
                                     const float2 fw =
                                         __fmul2_rn(pw, __fmul2_rn(__fmul2_rn(i, i), i));
                                     sx[k] = __ffma2_rn(dx, fw, sx[k]);

@@ -116,6 +116,16 @@ __device__ __forceinline__ bool mac_separated(float tx, float ty, float tz, floa
     return d2 > __fmul_rn(theta2, __fmul_rn(hs, hs));
 }
 
+// 1/sqrt of a softened squared distance (x >= 0.1f, inf or NaN).  The same
+// hardware approximation as rsqrtf; without -ftz=true rsqrtf also guards
+// against subnormal arguments and results, which cannot occur here, with
+// extra instructions around it.
+__device__ __forceinline__ float rsqrt_soft(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 __device__ __forceinline__ uint32_t lane_id() {
     uint32_t l;
     asm volatile("mov.u32 %0, %%laneid;" : "=r"(l));
