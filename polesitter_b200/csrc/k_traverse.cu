@@ -47,6 +47,8 @@
 // (mac_separated), so the interaction set is identical, ties included.
 // Bound: FP32 pipe (M2L ~35 flop + 1 MUFU per pair; P2P ~20 flop + 1 MUFU
 // per particle pair) and the latency of the candidate loads.
+#include <type_traits>
+
 #include "psg_common.cuh"
 #include "psg_kernels.h"
 
@@ -54,14 +56,13 @@ namespace psg {
 
 constexpr int kTravWarps = 4;
 constexpr int kTravThreads = kTravWarps * 32;
-static_assert(kTravWarps == kDenseWarpsPerBlock, "k_dense_p2p runs kTravThreads a block");
 constexpr int kCandBuf = 256;             // children of 32 opened entries
 constexpr int kStackCap = 384;            // DFS stack (node, child mask)
 constexpr int kStackSlack = 72;           // 9 levels x 7: growth of a single-entry descent
 constexpr int kP2PCap = 128;              // staged P2P sources of a group
 constexpr uint32_t kNsPool = 4096;        // near-list entries a warp reserves at once
 constexpr uint32_t kChunkPool = 16;       // P2P spill chunks a warp reserves at once
-constexpr uint32_t kDenseChunk = 32;      // target particles per dense work record
+constexpr uint32_t kSegChunks = 32;       // chunks of source list per dense work record
 constexpr uint32_t kDenseSwitch = 32;     // fullest leaf from which the DENSE leaf pass runs
 constexpr uint32_t kDenseCap = 8;         // ... or leaf capacity (leaves of many particles)
 
@@ -90,6 +91,9 @@ struct SmemLeaf {
     uint32_t stk_node[kStackCap];
     uint32_t p2p_node[kP2PCap];
     uint32_t chunk_next, chunk_end;
+    // DENSE: the group's source list so far -- chunks in the open segment,
+    // segments recorded, the first and the latest recorded segment's slots
+    uint32_t seg_chunks, seg_cnt, seg_first, seg_prev;
     uint32_t dbg_m2l[8];
     uint32_t dbg_p2p[8];
     uint8_t cand_mask[kCandBuf];
@@ -164,13 +168,98 @@ __device__ __forceinline__ void cgp_put(float4 (*cgp)[2], const float4* cgeo, ui
     __syncwarp();
 }
 
+// k_dense_p2p work records for the leaf children in mask of the group whose
+// children start at node fc, over the source chain phead: each run of
+// consecutive children (their particles are contiguous) is cut into records
+// of up to kDenseTargets particles.  A long source list is recorded in
+// segments of kSegChunks chunks (last: the group's last segment), so that the
+// records of a shallow leaf, whose list reaches most of the tree, are shared
+// out over many warps; the segments' sums meet in slots (DenseStore).  One
+// warp per whole list took 7.7 of a 131K closure tick's 9.9 ms, as segments
+// 0.9 ms; 32 chunks (at most 1,024 source leaves) keep a record to tens of
+// microseconds while most lists of a 1M tick stay whole.
+// Records: {fc, phead, first particle, count | run's child mask << 8},
+// {slot or kNone, the same targets' slot of the first segment, 0, 0}.
+__device__ __noinline__ void record_dense(SmemLeaf& sm, const DenseStore& ds, uint32_t mask,
+                                          uint32_t fc, uint32_t phead, bool last,
+                                          Status* status) {
+    const uint32_t lane = lane_id();
+    const uint32_t segs = sm.seg_cnt;
+    const bool split = !last || segs != 0;
+    uint32_t nall = 0;
+    for (uint32_t m = mask; m;) {
+        const uint32_t q0 = __ffs(m) - 1;
+        uint32_t q1 = q0, count = sm.cpart[q0].y;
+        while (q1 + 1 < 8 && ((m >> (q1 + 1)) & 1u)) count += sm.cpart[++q1].y;
+        m &= ~((2u << q1) - 1u);
+        nall += (count + kDenseTargets - 1) / kDenseTargets;
+    }
+    uint32_t r0 = 0, s0 = kNone;
+    if (lane == 0) {
+        r0 = atomicAdd(&status->dense_count, nall);
+        if (split) s0 = atomicAdd(&status->dense_slots, nall);
+    }
+    r0 = __shfl_sync(0xFFFFFFFFu, r0, 0);
+    s0 = __shfl_sync(0xFFFFFFFFu, s0, 0);
+    const uint32_t first_slot = segs ? sm.seg_first : s0;
+    const uint32_t prev_slot = segs ? sm.seg_prev : kNone;
+    uint32_t ord = 0;
+    for (uint32_t m = mask; m;) {
+        const uint32_t q0 = __ffs(m) - 1;
+        uint32_t q1 = q0, count = sm.cpart[q0].y;
+        while (q1 + 1 < 8 && ((m >> (q1 + 1)) & 1u)) count += sm.cpart[++q1].y;
+        const uint32_t run = ((2u << q1) - 1u) & ~((1u << q0) - 1u);
+        m &= ~((2u << q1) - 1u);
+        const uint32_t first = sm.cpart[q0].x;
+        const uint32_t nrec = (count + kDenseTargets - 1) / kDenseTargets;
+        for (uint32_t k = lane; k < nrec; k += 32) {
+            const uint32_t r = r0 + ord + k, sl = s0 + ord + k, f = first_slot + ord + k;
+            if (r < ds.rec_cap) {
+                const uint32_t c0 = k * kDenseTargets;
+                ds.rec[2 * (size_t)r] = make_uint4(fc, phead, first + c0,
+                                                   min(kDenseTargets, count - c0) | (run << 8));
+                ds.rec[2 * (size_t)r + 1] = make_uint4(split ? sl : kNone, f, 0u, 0u);
+            }
+            if (split && sl < ds.slot_cap) {
+                ds.meta[sl] = make_uint4(prev_slot == kNone ? kNone : prev_slot + ord + k,
+                                         kNone, 0u, 0u);
+                if (last) {
+                    ds.meta[f].y = sl;
+                    ds.meta[f].z = segs + 1;
+                }
+            }
+        }
+        ord += nrec;
+    }
+    if (lane == 0 && (r0 + nall > ds.rec_cap || (split && s0 + nall > ds.slot_cap)))
+        set_err(status, PSG_ERR_DENSE_OVERFLOW);
+    __syncwarp();
+    if (lane == 0) {
+        sm.seg_first = first_slot;
+        sm.seg_prev = s0;
+        sm.seg_cnt = segs + 1;
+        sm.seg_chunks = 0;
+    }
+    __syncwarp();
+}
+
 // Spill the group's staged P2P sources [0, fill) to HBM chunks of
 // kP2PChunk (node, child mask) entries, chained to the group's earlier
 // chunks.  Warp-collective; chunk ids come from a per-warp pool.  Returns the
-// new chain head.
+// new chain head.  DENSE: a segment of kSegChunks chunks is recorded for
+// k_dense_p2p and the chain starts over.
+template <bool DENSE>
 __device__ __noinline__ uint32_t spill_p2p(SmemLeaf& sm, uint32_t fill, uint32_t head,
-                                           P2PStore st, Status* status) {
+                                           const TravArgs& A, uint32_t tgt_mask, uint32_t fc) {
     const uint32_t lane = lane_id();
+    const P2PStore& st = A.p2p;
+    Status* status = A.status;
+    if constexpr (DENSE) {
+        if (sm.seg_chunks >= kSegChunks) {
+            record_dense(sm, A.dense, tgt_mask, fc, head, false, status);
+            head = kNone;
+        }
+    }
     for (uint32_t e0 = 0; e0 < fill; e0 += kP2PChunk) {
         if (sm.chunk_next >= sm.chunk_end) {
             uint32_t c = 0;
@@ -200,6 +289,10 @@ __device__ __noinline__ uint32_t spill_p2p(SmemLeaf& sm, uint32_t fill, uint32_t
         }
         __syncwarp();
         if (lane == 0) sm.chunk_next = c + 1;
+        __syncwarp();
+    }
+    if constexpr (DENSE) {
+        if (lane == 0) sm.seg_chunks += (fill + kP2PChunk - 1) / kP2PChunk;
         __syncwarp();
     }
     return head;
@@ -237,53 +330,6 @@ __device__ __forceinline__ void p2p_range(const float4* __restrict__ xyzm, uint2
     }
 }
 
-// k_dense_p2p work records for the leaf children in mask of the group whose
-// children start at node fc: each run of consecutive children (their
-// particles are contiguous) is cut into records of up to kDenseChunk
-// particles; phead is the group's complete P2P source chain.
-// Record: fc, phead, first particle, count | run's child mask << 8.
-__device__ __noinline__ void record_dense(const SmemLeaf& sm, uint32_t mask, uint32_t fc,
-                                          uint32_t phead, uint4* rec, uint32_t cap,
-                                          Status* status) {
-    const uint32_t lane = lane_id();
-    while (mask) {
-        const uint32_t q0 = __ffs(mask) - 1;
-        uint32_t q1 = q0;
-        while (q1 + 1 < 8 && ((mask >> (q1 + 1)) & 1u)) ++q1;
-        const uint32_t run = ((2u << q1) - 1u) & ~((1u << q0) - 1u);
-        mask &= ~run;
-        const uint32_t first = sm.cpart[q0].x;
-        uint32_t count = 0;
-        for (uint32_t q = q0; q <= q1; ++q) count += sm.cpart[q].y;
-        const uint32_t nrec = (count + kDenseChunk - 1) / kDenseChunk;
-        uint32_t r0 = 0;
-        if (lane == 0) r0 = atomicAdd(&status->dense_count, nrec);
-        r0 = __shfl_sync(0xFFFFFFFFu, r0, 0);
-        for (uint32_t k = lane; k < nrec; k += 32) {
-            if (r0 + k < cap) {
-                const uint32_t c0 = k * kDenseChunk;
-                rec[r0 + k] = make_uint4(fc, phead, first + c0,
-                                         min(kDenseChunk, count - c0) | (run << 8));
-            }
-        }
-        if (lane == 0 && r0 + nrec > cap) set_err(status, PSG_ERR_DENSE_OVERFLOW);
-    }
-}
-
-struct LeafOut {
-    const float4* xyzm;
-    const uint4* info;
-    P2PStore p2p;
-    float* fx;
-    float* fy;
-    float* fz;
-    uint32_t* leaf_of;
-    uint32_t* dbg_p2p;
-    uint4* dense_rec;
-    uint32_t dense_cap;
-    int kahan;
-};
-
 // STREAM: the P2P sums of the staged sources [0, pfill) for every target
 // particle of the work item's leaf children (tgt_mask), computed where they
 // are found instead of spilled to HBM, so that no store grows with the size
@@ -295,12 +341,12 @@ struct LeafOut {
 // left there).  fin: the item's last flush, which also applies L2P,
 // F = m (L + all P2P sums), with order 1's shift to the particle.
 template <bool DEBUG, bool GRAD>
-__device__ __noinline__ void stream_p2p(SmemLeaf& sm, const LeafOut& o, uint32_t tgt_mask,
+__device__ __noinline__ void stream_p2p(SmemLeaf& sm, const TravArgs& o, uint32_t tgt_mask,
                                         uint32_t fc, uint32_t pfill, bool accum, bool fin,
                                         unsigned long long& inter) {
     const uint32_t lane = lane_id();
     for (uint32_t e = lane; e < pfill; e += 32) {
-        const uint4 si = o.info[sm.p2p_node[e]];
+        const uint4 si = o.tv.info[sm.p2p_node[e]];
         sm.p2p_range[e] = make_uint2(si.x, si.y);
     }
     __syncwarp();
@@ -379,11 +425,12 @@ __device__ __noinline__ void stream_p2p(SmemLeaf& sm, const LeafOut& o, uint32_t
 // otherwise F = m (L + P2P sum) here, one target particle at a time with the
 // lanes over its sources.
 template <bool DEBUG, bool GRAD, bool DENSE>
-__device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const LeafOut o, uint32_t tgt_mask,
+__device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const TravArgs& o, uint32_t tgt_mask,
                                            uint32_t fc, uint32_t pfill, uint32_t phead,
                                            bool stream, bool flushed,
-                                           unsigned long long inter0, Status* status) {
+                                           unsigned long long inter0) {
     const uint32_t lane = lane_id();
+    Status* status = o.status;
     if (stream) {
         // the staged remainder, then L2P, in the warp (no spill, no records)
         unsigned long long inter = inter0;
@@ -392,7 +439,7 @@ __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const LeafOut o, uin
             if (lane == 0) {
                 for (uint32_t m = tgt_mask; m; m &= m - 1) {
                     const uint32_t q = __ffs(m) - 1;
-                    o.dbg_p2p[fc + q] = sm.dbg_p2p[q];
+                    o.tv.dbg_p2p[fc + q] = sm.dbg_p2p[q];
                     atomicAdd(&status->stat[PSG_STAT_P2P_PAIRS],
                               (unsigned long long)sm.dbg_p2p[q]);
                 }
@@ -405,13 +452,13 @@ __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const LeafOut o, uin
     }
     if constexpr (DENSE) {
         // the group's whole source list to HBM chunks, then k_dense_p2p work
-        // records of up to 32 target particles
-        if (pfill) phead = spill_p2p(sm, pfill, phead, o.p2p, status);
-        record_dense(sm, tgt_mask, fc, phead, o.dense_rec, o.dense_cap, status);
+        // records of up to kDenseTargets target particles
+        if (pfill) phead = spill_p2p<true>(sm, pfill, phead, o, tgt_mask, fc);
+        record_dense(sm, o.dense, tgt_mask, fc, phead, true, status);
         if (DEBUG && lane == 0) {
             for (uint32_t m = tgt_mask; m; m &= m - 1) {
                 const uint32_t q = __ffs(m) - 1;
-                o.dbg_p2p[fc + q] = sm.dbg_p2p[q];
+                o.tv.dbg_p2p[fc + q] = sm.dbg_p2p[q];
                 atomicAdd(&status->stat[PSG_STAT_P2P_PAIRS], (unsigned long long)sm.dbg_p2p[q]);
             }
         }
@@ -420,7 +467,7 @@ __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const LeafOut o, uin
     }
     // ---- L2P + P2P: F = m * (L(u) + sum of u's P2P sources) ----
     for (uint32_t e = lane; e < pfill; e += 32) {
-        const uint4 si = o.info[sm.p2p_node[e]];
+        const uint4 si = o.tv.info[sm.p2p_node[e]];
         sm.p2p_range[e] = make_uint2(si.x, si.y);
     }
     __syncwarp();
@@ -443,7 +490,7 @@ __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const LeafOut o, uin
             for (uint32_t c = phead; c != kNone; c = o.p2p.next[c]) {
                 if (lane < o.p2p.cnt[c] &&
                     ((o.p2p.mask[(size_t)c * kP2PChunk + lane] >> q) & 1u)) {
-                    const uint4 si = o.info[o.p2p.src[(size_t)c * kP2PChunk + lane]];
+                    const uint4 si = o.tv.info[o.p2p.src[(size_t)c * kP2PChunk + lane]];
                     p2p_range(o.xyzm, make_uint2(si.x, si.y), t, o.kahan, bx, by, bz,
                               cx, cy, cz);
                     if (DEBUG) inter += si.y;
@@ -473,7 +520,7 @@ __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const LeafOut o, uin
             }
         }
         if (DEBUG && lane == 0) {
-            o.dbg_p2p[fc + q] = sm.dbg_p2p[q];
+            o.tv.dbg_p2p[fc + q] = sm.dbg_p2p[q];
             atomicAdd(&status->stat[PSG_STAT_P2P_PAIRS],
                       (unsigned long long)sm.dbg_p2p[q]);
         }
@@ -497,7 +544,7 @@ __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const LeafOut o, uin
 template <int MODE, bool DEBUG, bool GRAD, bool DENSE, bool XL>
 __global__ void __launch_bounds__(
     kTravThreads, (MODE == MODE_LEAF && !DEBUG && !XL) ? (GRAD ? 4 : (DENSE ? 1 : 7)) : 1)
-    k_trav(TravArgs A) {
+    k_trav(const __grid_constant__ TravArgs A) {
     using Smem = typename SmemOf<MODE>::T;
     __shared__ Smem smem[kTravWarps];
     const uint32_t lane = lane_id();
@@ -623,6 +670,7 @@ __global__ void __launch_bounds__(
                     sm.ns_cnt[lane] = 0;
                 } else {
                     if (DEBUG) sm.dbg_p2p[lane] = 0;
+                    if (DENSE && lane == 0) sm.seg_chunks = sm.seg_cnt = 0;
                 }
             }
             // chain group (leaf pass, parent deeper than the near lists
@@ -935,15 +983,11 @@ __global__ void __launch_bounds__(
                         if (pb) {
                             if (pfill + __popc(pb) > (uint32_t)kP2PCap) {
                                 if (XL && A.stream) {
-                                    stream_p2p<DEBUG, GRAD>(
-                                        sm,
-                                        LeafOut{A.xyzm, tv.info, A.p2p, A.fx, A.fy, A.fz,
-                                                A.leaf_of, tv.dbg_p2p, A.dense_rec, A.dense_cap,
-                                                A.kahan},
-                                        tgt_mask, fc, pfill, flushed, false, sinter);
+                                    stream_p2p<DEBUG, GRAD>(sm, A, tgt_mask, fc, pfill,
+                                                            flushed, false, sinter);
                                     flushed = true;
                                 } else {
-                                    phead = spill_p2p(sm, pfill, phead, A.p2p, status);
+                                    phead = spill_p2p<DENSE>(sm, pfill, phead, A, tgt_mask, fc);
                                 }
                                 pfill = 0;
                             }
@@ -1058,11 +1102,8 @@ __global__ void __launch_bounds__(
             __syncwarp();
 
             if constexpr (MODE == MODE_LEAF) {
-                leaf_epilogue<DEBUG, GRAD, DENSE>(
-                    sm,
-                    LeafOut{A.xyzm, tv.info, A.p2p, A.fx, A.fy, A.fz, A.leaf_of, tv.dbg_p2p,
-                            A.dense_rec, A.dense_cap, A.kahan},
-                    tgt_mask, fc, pfill, phead, XL && A.stream != 0, flushed, sinter, status);
+                leaf_epilogue<DEBUG, GRAD, DENSE>(sm, A, tgt_mask, fc, pfill, phead,
+                                                  XL && A.stream != 0, flushed, sinter);
                 if (DEBUG && lane == 0) {
                     const unsigned long long cyc = (unsigned long long)(clock64() - t_group);
                     atomicMax(&status->stat[PSG_STAT_SLOWEST_GROUP],
@@ -1074,207 +1115,31 @@ __global__ void __launch_bounds__(
 }
 
 // L2P + P2P of the full leaves recorded by the leaf pass.  A warp takes one
-// record (a run of leaves, up to 32 of their particles, the group's source
-// chain) at a time from a shared counter.  The chain's entries (source
-// leaves) are split by the leaves of the record they serve:
-//  * an entry that serves every leaf of the record is summed by all lanes:
-//    T lanes own the record's target particles (T the smallest power of two
-//    >= their count) and the 32 / T slices of lanes split the entry's
-//    particles;
-//  * an entry that serves only some of its leaves is summed per leaf q, in
-//    another walk of the chain, with the lanes dealt over q's targets alone
-//    (T_q lanes, 32 / T_q slices),
-// so no lane computes a pair its target does not want.  A chunk's taken
-// entries go through the warp's shared tile (sum_tiles); with 8 or more
-// slices (4 or fewer targets) the slices instead walk whole source leaves
-// from global memory (walk_leaf), as the tile's search would cost more than
-// its reuse saves.  The per-leaf sums reach the target's lane through
-// shared memory (a target belongs to one leaf, so its slot is written once).
-// Sums are taken in chain order, so the result does not depend on
-// scheduling.
-
-// A tile of 32 source particles, pair-packed: pair m holds particles 2m and
-// 2m + 1 as a = {x, x', y, y'} and b = {z, z', w, w'}, so one 128-bit
-// shared load gives two sources' coordinates as the float2 operands of
-// sm_100's paired FP32 instructions (__fadd2_rn, __ffma2_rn, __fmul2_rn):
-// one issued instruction does a step of two pairs.
-struct DenseTile {
-    float4 a[16];
-    float4 b[16];
-};
-
-__device__ __forceinline__ void tile_put(DenseTile& tile, uint32_t lane, float4 p) {
-    float* a = reinterpret_cast<float*>(&tile.a[lane >> 1]);
-    float* b = reinterpret_cast<float*>(&tile.b[lane >> 1]);
-    const uint32_t h = lane & 1u;
-    a[h] = p.x;
-    a[2 + h] = p.y;
-    b[h] = p.z;
-    b[2 + h] = p.w;
-}
-
-// one target against the tile's source pairs m = m0, m0 + S, ... (sources
-// 2m and 2m + 1, fewer than nt real ones; the slot past an odd nt holds a
-// zero mass, which adds exactly zero).  Plain sums keep the two sources of
-// a pair in the two halves of float2 accumulators (two FMA chains in one
-// instruction); Kahan sums go source by source.
-template <bool KAHAN>
-__device__ __forceinline__ void dense_tile(const DenseTile& tile, uint32_t m0, uint32_t S,
-                                           uint32_t nt, float4 t, float2& sx, float2& sy,
-                                           float2& sz, float& ax, float& ay, float& az,
-                                           float& cx, float& cy, float& cz) {
-    if constexpr (KAHAN) {
-        for (uint32_t m = m0; 2 * m < nt; m += S) {
-            const float4 a = tile.a[m], b = tile.b[m];
-            for (uint32_t h = 0; h < 2 && 2 * m + h < nt; ++h) {
-                const float px = h ? a.y : a.x, py = h ? a.w : a.z, pz = h ? b.y : b.x,
-                            pw = h ? b.w : b.z;
-                const float dx = px - t.x, dy = py - t.y, dz = pz - t.z;
-                const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) + 0.1f;
-                const float inv = rsqrt_soft(r2);
-                const float f = pw * (inv * inv * inv);
-                const float yx = __fsub_rn(__fmul_rn(dx, f), cx);
-                const float yy = __fsub_rn(__fmul_rn(dy, f), cy);
-                const float yz = __fsub_rn(__fmul_rn(dz, f), cz);
-                const float tx = __fadd_rn(ax, yx);
-                const float ty = __fadd_rn(ay, yy);
-                const float tz = __fadd_rn(az, yz);
-                cx = __fsub_rn(__fsub_rn(tx, ax), yx);
-                cy = __fsub_rn(__fsub_rn(ty, ay), yy);
-                cz = __fsub_rn(__fsub_rn(tz, az), yz);
-                ax = tx;
-                ay = ty;
-                az = tz;
-            }
-        }
-    } else {
-        const float2 ntx = make_float2(-t.x, -t.x), nty = make_float2(-t.y, -t.y),
-                     ntz = make_float2(-t.z, -t.z), eps = make_float2(0.1f, 0.1f);
-        const uint32_t np = (nt + 1u) >> 1;
-#pragma unroll 2
-        for (uint32_t m = m0; m < np; m += S) {
-            const float4 a = tile.a[m], b = tile.b[m];
-            const float2 dx = __fadd2_rn(make_float2(a.x, a.y), ntx);
-            const float2 dy = __fadd2_rn(make_float2(a.z, a.w), nty);
-            const float2 dz = __fadd2_rn(make_float2(b.x, b.y), ntz);
-            float2 r = __ffma2_rn(dz, dz, eps);
-            r = __ffma2_rn(dy, dy, r);
-            r = __ffma2_rn(dx, dx, r);
-            const float2 i = make_float2(rsqrt_soft(r.x), rsqrt_soft(r.y));
-            const float2 f = __fmul2_rn(make_float2(b.z, b.w), __fmul2_rn(__fmul2_rn(i, i), i));
-            sx = __ffma2_rn(dx, f, sx);
-            sy = __ffma2_rn(dy, f, sy);
-            sz = __ffma2_rn(dz, f, sz);
-        }
-    }
-}
-
-// The particles of the chunk entries the lanes hold (entry start es, count
-// en; en = 0 for an entry not taken) against target t: laid end to end by a
-// warp prefix sum, they pass through the warp's shared tile 32 at a time --
-// lane j finds the entry of flat particle b + j by a binary search over the
-// prefix sums and stages it (coalesced within a leaf) -- and every lane runs
-// its target against the tile's source pairs m = slice, slice + S, ...
-// Returns the particles summed (the same on every lane).
-template <bool KAHAN>
-__device__ __forceinline__ uint32_t sum_tiles(DenseTile& tile, const float4* __restrict__ xyzm,
-                                              uint32_t es, uint32_t en, uint32_t slice,
-                                              uint32_t S, float4 t, float& ax, float& ay,
-                                              float& az, float& cx, float& cy, float& cz) {
-    const uint32_t lane = lane_id();
-    const uint32_t incl = warp_incl_scan(en);
-    const uint32_t ptot = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    const uint32_t excl = incl - en;
-    // lane j's particle of the tile starting at flat index b (warp-collective)
-    auto fetch = [&](uint32_t b) -> float4 {
-        const uint32_t f = b + lane;
-        uint32_t e = 0;
-#pragma unroll
-        for (uint32_t step = 16; step > 0; step >>= 1) {
-            const uint32_t v = __shfl_sync(0xFFFFFFFFu, incl, e + step - 1);
-            if (v <= f) e += step;
-        }
-        const uint32_t e_start = __shfl_sync(0xFFFFFFFFu, es, e);
-        const uint32_t e_excl = __shfl_sync(0xFFFFFFFFu, excl, e);
-        return f < ptot ? xyzm[e_start + (f - e_excl)] : make_float4(0.f, 0.f, 0.f, 0.f);
-    };
-    float2 sx = make_float2(0.f, 0.f), sy = sx, sz = sx;
-    float4 pcur = ptot ? fetch(0u) : make_float4(0.f, 0.f, 0.f, 0.f);
-    for (uint32_t b = 0; b < ptot; b += 32) {
-        __syncwarp();
-        tile_put(tile, lane, pcur);
-        __syncwarp();
-        // the next tile's particle is in flight while this tile is summed
-        if (b + 32 < ptot) pcur = fetch(b + 32);
-        const uint32_t nt = min(32u, ptot - b);
-        dense_tile<KAHAN>(tile, slice, S, nt, t, sx, sy, sz, ax, ay, az, cx, cy, cz);
-    }
-    __syncwarp();
-    if constexpr (!KAHAN) {
-        ax += sx.x + sx.y;
-        ay += sy.x + sy.y;
-        az += sz.x + sz.y;
-    }
-    return ptot;
-}
-
-// target t against the particles first + slice, first + slice + S, ... <
-// first + cnt (polesitter.h:1424-1444, rsqrt), optionally Kahan-compensated
-template <bool KAHAN>
-__device__ __forceinline__ void walk_leaf(const float4* __restrict__ xyzm, uint32_t first,
-                                          uint32_t cnt, uint32_t slice, uint32_t S, float4 t,
-                                          float& ax, float& ay, float& az, float& cx,
-                                          float& cy, float& cz) {
-    if constexpr (KAHAN) {
-        for (uint32_t j = slice; j < cnt; j += S) {
-            const float4 p = xyzm[first + j];
-            const float dx = p.x - t.x, dy = p.y - t.y, dz = p.z - t.z;
-            const float inv = rsqrt_soft(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 0.1f))));
-            const float f = p.w * (inv * inv * inv);
-            const float yx = __fsub_rn(__fmul_rn(dx, f), cx);
-            const float yy = __fsub_rn(__fmul_rn(dy, f), cy);
-            const float yz = __fsub_rn(__fmul_rn(dz, f), cz);
-            const float tx = __fadd_rn(ax, yx);
-            const float ty = __fadd_rn(ay, yy);
-            const float tz = __fadd_rn(az, yz);
-            cx = __fsub_rn(__fsub_rn(tx, ax), yx);
-            cy = __fsub_rn(__fsub_rn(ty, ay), yy);
-            cz = __fsub_rn(__fsub_rn(tz, az), yz);
-            ax = tx;
-            ay = ty;
-            az = tz;
-        }
-    } else {
-        float ex = 0.f, ey = 0.f, ez = 0.f;
-        uint32_t j = slice;
-        for (; j + S < cnt; j += 2 * S) {
-            const float4 p0 = xyzm[first + j], p1 = xyzm[first + j + S];
-            const float dx0 = p0.x - t.x, dy0 = p0.y - t.y, dz0 = p0.z - t.z;
-            const float dx1 = p1.x - t.x, dy1 = p1.y - t.y, dz1 = p1.z - t.z;
-            const float i0 = rsqrt_soft(fmaf(dx0, dx0, fmaf(dy0, dy0, fmaf(dz0, dz0, 0.1f))));
-            const float i1 = rsqrt_soft(fmaf(dx1, dx1, fmaf(dy1, dy1, fmaf(dz1, dz1, 0.1f))));
-            const float f0 = p0.w * (i0 * i0 * i0), f1 = p1.w * (i1 * i1 * i1);
-            ax = fmaf(dx0, f0, ax);
-            ay = fmaf(dy0, f0, ay);
-            az = fmaf(dz0, f0, az);
-            ex = fmaf(dx1, f1, ex);
-            ey = fmaf(dy1, f1, ey);
-            ez = fmaf(dz1, f1, ez);
-        }
-        if (j < cnt) {
-            const float4 p = xyzm[first + j];
-            const float dx = p.x - t.x, dy = p.y - t.y, dz = p.z - t.z;
-            const float inv = rsqrt_soft(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, 0.1f))));
-            const float f = p.w * (inv * inv * inv);
-            ax = fmaf(dx, f, ax);
-            ay = fmaf(dy, f, ay);
-            az = fmaf(dz, f, az);
-        }
-        ax += ex;
-        ay += ey;
-        az += ez;
-    }
-}
+// record at a time from a shared counter: up to 16 target particles of a run
+// of leaves, and the chain of source leaves (or a segment of it) that their
+// group found.  The lanes own sources: the source leaves' particles are laid
+// end to end over the lanes, and each lane sums its particle into its own
+// accumulators of every target, two targets at a time in the paired FP32
+// instructions (__fadd2_rn, __ffma2_rn, __fmul2_rn; one issued instruction
+// does a step of two pairs).  At the record's end the lanes' sums are added.
+// So targets are padded to the pair only, sources not at all, a source's
+// load and lookup serve all targets, and no source passes through shared
+// memory.  A source that serves only some leaves of the record (its child
+// mask) has its mass zeroed for the other targets; steps whose sources serve
+// all of them skip that.
+//
+// Bound: the FP32 pipe.  A step on a pair of targets is 12 paired FP32
+// instructions of two cycles and 2 MUFU; alone in a loop that takes 32 cycles
+// per scheduler (2.3e12 particle pairs/s on 148 SMs).  16 targets a record
+// and 4 blocks per SM (128 registers) is the best of 8-24 targets and 2-6
+// blocks measured: the accumulators' registers trade against the warps that
+// hide the chain's latency.  Measured at 1M clumpy, theta 6.25, leaf capacity
+// 16 (8.2 G pairs): closure tick 14.2 -> 13.0 ms against lanes that owned
+// targets, with sources staged in shared-memory tiles and a second walk per
+// leaf for partly wanted sources.
+//
+// Sums are taken in chain order, the lanes and the segments added in a fixed
+// order, so the result does not depend on scheduling.
 
 // a spilled chunk as one lane sees it: the chunk's entry count and link,
 // and the lane's entry (its source leaf and child mask; slots past the count
@@ -1294,209 +1159,300 @@ __device__ __forceinline__ ChunkHead load_chunk(const P2PStore& st, uint32_t c, 
     return h;
 }
 
-template <bool DEBUG, bool GRAD, bool KAHAN>
-__global__ void __launch_bounds__(kTravThreads, kDenseBlocksPerSm) k_dense_p2p(TravArgs A) {
-    __shared__ float4 s_part[kTravWarps][32];  // per-leaf sums of the record's targets
-    __shared__ DenseTile tiles[kTravWarps];
-    __shared__ uint2 s_ent[kTravWarps][32];  // pass 2: a leaf's entries, 32 at a time
-    float4* part = s_part[threadIdx.x >> 5];
-    DenseTile& tile = tiles[threadIdx.x >> 5];
-    uint2* ent = s_ent[threadIdx.x >> 5];
-    // this warp's list of partial entries (source start, count | mask << 16)
-    const uint32_t wslot = blockIdx.x * kTravWarps + (threadIdx.x >> 5);
-    if (wslot >= A.dense_part_warps) return;  // (no list: the other warps take the records)
-    uint2* const plist = A.dense_part + (size_t)wslot * kDensePartCap;
-    Status* status = A.status;
-    if (status->err & (PSG_ERR_NODES | PSG_ERR_SORT_SPIN | PSG_ERR_DENSE_OVERFLOW)) return;
+// Two of a record's targets (negated, one in each half of a float2) and this
+// lane's sums for them.
+template <bool KAHAN>
+struct DensePair {
+    float2 sx, sy, sz;
+};
+template <>
+struct DensePair<true> {
+    float2 sx, sy, sz, cx, cy, cz;
+};
+
+struct DenseSmem {
+    uint2 ent[32];
+    float4 txy[kDenseTargets / 2];  // a pair's targets, negated: x, x', y, y'
+    float2 tz[kDenseTargets / 2];
+};
+
+__device__ __forceinline__ void kahan_add(float2& s, float2& c, float2 v) {
+    const float2 y = __fadd2_rn(v, make_float2(-c.x, -c.y));
+    const float2 t = __fadd2_rn(s, y);
+    const float2 d = __fadd2_rn(t, make_float2(-s.x, -s.y));
+    c = __fadd2_rn(d, make_float2(-y.x, -y.y));
+    s = t;
+}
+
+// source particle p on target pair k, where the set tm holds the targets that
+// want it (polesitter.h:1424-1444 with rsqrt)
+template <bool KAHAN, bool MASKED>
+__device__ __forceinline__ void dense_pair(DensePair<KAHAN>& a, const DenseSmem& sm, float4 p,
+                                           uint32_t tm, int k) {
+    const float4 txy = sm.txy[k];
+    const float2 tz = sm.tz[k];
+    float2 pw = make_float2(p.w, p.w);
+    if constexpr (MASKED) {
+        if (!(tm & (1u << (2 * k)))) pw.x = 0.f;
+        if (!(tm & (2u << (2 * k)))) pw.y = 0.f;
+    }
+    const float2 dx = __fadd2_rn(make_float2(p.x, p.x), make_float2(txy.x, txy.y));
+    const float2 dy = __fadd2_rn(make_float2(p.y, p.y), make_float2(txy.z, txy.w));
+    const float2 dz = __fadd2_rn(make_float2(p.z, p.z), tz);
+    float2 r = __ffma2_rn(dz, dz, make_float2(0.1f, 0.1f));
+    r = __ffma2_rn(dy, dy, r);
+    r = __ffma2_rn(dx, dx, r);
+    const float2 i = make_float2(rsqrt_soft(r.x), rsqrt_soft(r.y));
+    const float2 f = __fmul2_rn(pw, __fmul2_rn(__fmul2_rn(i, i), i));
+    if constexpr (KAHAN) {
+        kahan_add(a.sx, a.cx, __fmul2_rn(dx, f));
+        kahan_add(a.sy, a.cy, __fmul2_rn(dy, f));
+        kahan_add(a.sz, a.cz, __fmul2_rn(dz, f));
+    } else {
+        a.sx = __ffma2_rn(dx, f, a.sx);
+        a.sy = __ffma2_rn(dy, f, a.sy);
+        a.sz = __ffma2_rn(dz, f, a.sz);
+    }
+}
+
+constexpr int kDensePairs = (int)kDenseTargets / 2;
+constexpr int kDenseBlock = 4;
+
+// one step: a lane's source p on the record's np target pairs, kDenseBlock
+// pairs at a time (their chains of dependent instructions overlap)
+template <bool KAHAN, bool MASKED>
+__device__ __forceinline__ void dense_step(DensePair<KAHAN> (&a)[kDensePairs],
+                                           const DenseSmem& sm, float4 p, uint32_t tm,
+                                           uint32_t np) {
+#pragma unroll
+    for (int k = 0; k < kDensePairs; k += kDenseBlock) {
+        if (k == 0 || np > (uint32_t)k) {
+#pragma unroll
+            for (int j = 0; j < kDenseBlock; ++j)
+                dense_pair<KAHAN, MASKED>(a[k + j], sm, p, tm, k + j);
+        }
+    }
+}
+
+// one record
+template <bool KAHAN>
+__device__ __forceinline__ void dense_record(const TravArgs& A, DenseSmem& sm, uint4 rec, uint4 rec2,
+                                             unsigned long long& inter) {
     const TreeView& tv = A.tv;
     const float4* __restrict__ xyzm = A.xyzm;
+    const uint32_t lane = lane_id(), le_mask = lanemask_lt() | (1u << lane);
+    const uint32_t fc = rec.x, run = rec.w >> 8, cnt = rec.w & 0xFFu, first = rec.z;
+    const uint32_t np = (cnt + 1u) >> 1;
+    // lane k < cnt: target k, its leaf (the child of the run that holds it)
+    const uint32_t ti = first + min(lane, cnt - 1u);
+    uint32_t q = __ffs(run) - 1;
+    for (uint32_t m = run & (run - 1u); m; m &= m - 1) {
+        const uint32_t qq = __ffs(m) - 1;
+        if (tv.info[fc + qq].x <= ti) q = qq;
+    }
+    const float4 t = xyzm[ti];
+    // the record's leaves, and per leaf (in lane q) the set of its targets
+    const uint32_t leaves = __reduce_or_sync(0xFFFFFFFFu, 1u << q);
+    uint32_t tset = 0;
+    for (uint32_t m = leaves; m; m &= m - 1) {
+        const uint32_t qq = __ffs(m) - 1;
+        const uint32_t b = __ballot_sync(0xFFFFFFFFu, lane < cnt && q == qq);
+        if (lane == qq) tset = b;
+    }
+    DensePair<KAHAN> a[kDensePairs];
+#pragma unroll
+    for (int k = 0; k < kDensePairs; ++k) {
+        a[k].sx = a[k].sy = a[k].sz = make_float2(0.f, 0.f);
+        if constexpr (KAHAN) a[k].cx = a[k].cy = a[k].cz = make_float2(0.f, 0.f);
+    }
+    __syncwarp();
+    if (lane < kDenseTargets) {  // (slots past cnt: the last target again, not used)
+        float* xy = reinterpret_cast<float*>(&sm.txy[lane >> 1]);
+        xy[lane & 1u] = -t.x;
+        xy[2 + (lane & 1u)] = -t.y;
+        reinterpret_cast<float*>(&sm.tz[lane >> 1])[lane & 1u] = -t.z;
+    }
+    __syncwarp();
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    // chunks one ahead: the next chunk's source ranges and the header after
+    // it are in flight while a chunk is summed
+    auto src_range = [&](const ChunkHead& hh) -> uint2 {
+        if (lane < hh.cnt && (hh.mask & leaves) != 0u) {
+            const uint4 si = tv.info[hh.src];
+            return make_uint2(si.x, si.y);
+        }
+        return make_uint2(0u, 0u);
+    };
+    ChunkHead h = load_chunk(A.p2p, rec.y, lane);
+    uint2 hr = src_range(h);
+    ChunkHead hn = load_chunk(A.p2p, h.next, lane);
+    uint32_t c = rec.y;
+    // positions left over from a chunk (fewer than 32) are carried into the
+    // next, and the particle loaded in one step is summed in the next one
+    uint32_t carry = 0, carry_idx = 0, carry_tm = 0;
+    const uint32_t all = (1u << cnt) - 1u;
+    float4 p = none;
+    uint32_t ptm = all;
+    for (bool more = true; more;) {
+        uint32_t en = 0, tm = 0, es = 0;
+        more = c != kNone;
+        if (more) {
+            const uint32_t em = lane < h.cnt ? (h.mask & leaves) : 0u;
+            es = hr.x;
+            en = hr.y;
+            for (uint32_t m = leaves; m; m &= m - 1) {
+                const uint32_t qq = __ffs(m) - 1;
+                const uint32_t v = __shfl_sync(0xFFFFFFFFu, tset, qq);
+                tm |= ((em >> qq) & 1u) ? v : 0u;
+            }
+            c = h.next;
+            h = hn;
+            hr = src_range(h);
+            hn = load_chunk(A.p2p, h.next, lane);
+        }
+        // the entries' particles laid end to end after the carried ones: entry
+        // e starts at position start; its (particle - position, targets) in
+        // ent, compacted past empty entries
+        const uint32_t incl = warp_incl_scan(en);
+        const uint32_t ptot = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        const uint32_t start = carry + incl - en;
+        const uint32_t full = __ballot_sync(0xFFFFFFFFu, en != 0u);
+        __syncwarp();
+        if (en) sm.ent[__popc(full & lanemask_lt())] = make_uint2(es - start, tm);
+        __syncwarp();
+        if (A.debug) inter += (unsigned long long)en * __popc(tm);
+        const uint32_t total = carry + ptot;
+        // at the chain's end: the remainder, and the step that sums it
+        const uint32_t steps = more ? total >> 5 : ((total + 31u) >> 5) + 1u;
+        uint32_t before = 0;  // entries that start before the step's positions
+        uint32_t b = 0;
+        // lane's source at position b + lane: its entry is the last to start
+        // at or before it
+        auto locate = [&](uint32_t& idx, uint32_t& mask) {
+            const uint32_t d = start - b;
+            const uint32_t bits =
+                __reduce_or_sync(0xFFFFFFFFu, (en != 0u && d < 32u) ? 1u << d : 0u);
+            const uint32_t f = b + lane;
+            const uint32_t e = before + __popc(bits & le_mask);
+            const uint2 v = sm.ent[e ? e - 1u : 0u];
+            before += __popc(bits);
+            idx = f < carry ? carry_idx : v.x + f;
+            mask = f < carry ? carry_tm : v.y;
+        };
+#pragma unroll 1
+        for (uint32_t st = 0; st < steps; ++st, b += 32) {
+            uint32_t idx, mask;
+            locate(idx, mask);
+            const bool in = b + lane < total;
+            const float4 pn = in ? xyzm[idx] : none;
+            // most steps' sources serve every leaf of the record
+            if (__all_sync(0xFFFFFFFFu, ptm == all))
+                dense_step<KAHAN, false>(a, sm, p, ptm, np);
+            else
+                dense_step<KAHAN, true>(a, sm, p, ptm, np);
+            p = pn;
+            ptm = in ? mask : all;  // (no source: no mass)
+        }
+        if (more && b < total) {
+            uint32_t idx, mask;
+            locate(idx, mask);  // (lanes past the remainder are not used)
+            carry_idx = idx;
+            carry_tm = mask;
+        }
+        carry = more ? total - b : 0u;
+    }
+    // the lanes' sums; lane k keeps target k's
+    double bx = 0.0, by = 0.0, bz = 0.0;
+#pragma unroll
+    for (int k = 0; k < kDensePairs; ++k) {
+        if (k > 0 && np <= (uint32_t)k) continue;
+        using Sum = typename std::conditional<KAHAN, double, float>::type;
+        Sum v[6] = {a[k].sx.x, a[k].sx.y, a[k].sy.x, a[k].sy.y, a[k].sz.x, a[k].sz.y};
+        if constexpr (KAHAN) {
+            v[0] -= a[k].cx.x;
+            v[1] -= a[k].cx.y;
+            v[2] -= a[k].cy.x;
+            v[3] -= a[k].cy.y;
+            v[4] -= a[k].cz.x;
+            v[5] -= a[k].cz.y;
+        }
+#pragma unroll
+        for (int j = 0; j < 6; ++j) v[j] = warp_sum(v[j]);
+        if ((lane >> 1) == (uint32_t)k) {
+            bx = (lane & 1u) ? v[1] : v[0];
+            by = (lane & 1u) ? v[3] : v[2];
+            bz = (lane & 1u) ? v[5] : v[4];
+        }
+    }
+    // a segment of a longer list: its sums go to its slot, and the segment
+    // that comes last adds them all, from the list's end
+    const uint32_t slot = rec2.x;
+    if (slot != kNone) {
+        const DenseStore& ds = A.dense;
+        double* own = ds.sums + (size_t)slot * kDenseTargets * 3;
+        if (lane < cnt) {
+            __stcg(own + 3 * lane, bx);
+            __stcg(own + 3 * lane + 1, by);
+            __stcg(own + 3 * lane + 2, bz);
+        }
+        __threadfence();
+        __syncwarp();
+        const uint32_t item = rec2.y;
+        uint32_t done = 0;
+        if (lane == 0) done = atomicAdd(&ds.meta[item].w, 1u);
+        done = __shfl_sync(0xFFFFFFFFu, done, 0);
+        if (done + 1u != ds.meta[item].z) return;
+        __threadfence();
+        bx = by = bz = 0.0;
+        for (uint32_t sl = ds.meta[item].y; sl != kNone; sl = ds.meta[sl].x) {
+            if (lane < cnt) {
+                const double* v = ds.sums + (size_t)sl * kDenseTargets * 3 + 3 * lane;
+                bx += __ldcg(v);
+                by += __ldcg(v + 1);
+                bz += __ldcg(v + 2);
+            }
+        }
+    }
+    if (lane < cnt) {
+        const uint32_t u = fc + q;
+        const float4 L = tv.lt[u];
+        float lx = L.y, ly = L.z, lz = L.w;
+        if (A.order >= 1) {
+            const float4 cu = tv.geo[u];
+            const float3 sh = grad_apply(tv.lg0[u], tv.lg1[u], t.x - cu.x, t.y - cu.y,
+                                         t.z - cu.z);
+            lx += sh.x;
+            ly += sh.y;
+            lz += sh.z;
+            if (A.leaf_of) A.leaf_of[ti] = u;
+        }
+        const double mm = (double)t.w;
+        A.fx[ti] = (float)(mm * ((double)lx + bx));
+        A.fy[ti] = (float)(mm * ((double)ly + by));
+        A.fz[ti] = (float)(mm * ((double)lz + bz));
+    }
+}
+
+template <bool KAHAN>
+__global__ void __launch_bounds__(kDenseThreads, KAHAN ? 2 : kDenseBlocksPerSm)
+    k_dense_p2p(const __grid_constant__ TravArgs A) {
+    __shared__ DenseSmem smem[kDenseWarpsPerBlock];
+    DenseSmem& sm = smem[threadIdx.x >> 5];
+    Status* status = A.status;
+    if (status->err & (PSG_ERR_NODES | PSG_ERR_SORT_SPIN | PSG_ERR_DENSE_OVERFLOW)) return;
     const uint32_t lane = lane_id();
-    const uint32_t total = min(status->dense_count, A.dense_cap);
-    if (total == 0) return;
+    const uint32_t total = min(status->dense_count, A.dense.rec_cap);
     unsigned long long inter = 0;
     for (;;) {
         uint32_t r = 0;
         if (lane == 0) r = atomicAdd(&status->dense_work, 1u);
         r = __shfl_sync(0xFFFFFFFFu, r, 0);
         if (r >= total) break;
-        const uint4 rec = A.dense_rec[r];
-        const uint32_t fc = rec.x, run = rec.w >> 8, cnt_t = rec.w & 0xFFu, first = rec.z;
-        uint32_t T = 1;
-        while (T < cnt_t) T <<= 1;
-        const uint32_t S = 32u / T;
-        const uint32_t tl = lane & (T - 1u), slice = lane / T;
-        const bool active = tl < cnt_t;
-        const uint32_t i = first + (active ? tl : 0u);
-        // this lane's leaf: the child of the run whose particles hold i
-        uint32_t q = __ffs(run) - 1;
-        for (uint32_t m = run; m; m &= m - 1) {
-            const uint32_t qq = __ffs(m) - 1;
-            if (tv.info[fc + qq].x <= i) q = qq;
-        }
-        const uint32_t u = fc + q;
-        const float4 t = xyzm[i];
-        part[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-        __syncwarp();
-        float bx = 0.f, by = 0.f, bz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-        uint32_t used = 0;
-        // The chain is walked once, in segments.  Pass 1 sums the entries
-        // that serve every leaf of the record and keeps the others (partial
-        // entries) in the warp's list, in chain order; when the list could
-        // not take another chunk, or at the chain's end, pass 2 sums the
-        // listed entries leaf by leaf and the list starts over.  While a
-        // chunk is summed, the next chunk's source ranges and the header
-        // after it are in flight.
-        auto src_range = [&](const ChunkHead& hh) -> uint2 {
-            if (lane < hh.cnt && (hh.mask & run) != 0u) {
-                const uint4 si = tv.info[hh.src];
-                return make_uint2(si.x, si.y);
-            }
-            return make_uint2(0u, 0u);
-        };
-        ChunkHead h = load_chunk(A.p2p, rec.y, lane);
-        uint2 hr = src_range(h);
-        ChunkHead hn = load_chunk(A.p2p, h.next, lane);
-        uint32_t c = rec.y;
-        for (;;) {
-            uint32_t npart = 0, partial_q = 0;
-            while (c != kNone && npart + 32u <= kDensePartCap) {
-                const uint32_t em = lane < h.cnt ? (h.mask & run) : 0u;
-                const uint32_t es = hr.x, en = hr.y;
-                c = h.next;
-                h = hn;
-                hr = src_range(h);
-                hn = load_chunk(A.p2p, h.next, lane);
-                const bool partial = em != 0u && em != run;
-                partial_q |= __reduce_or_sync(0xFFFFFFFFu, partial ? em : 0u);
-                const uint32_t pb = __ballot_sync(0xFFFFFFFFu, partial);
-                if (partial)
-                    plist[npart + __popc(pb & ((1u << lane) - 1u))] =
-                        make_uint2(es, en | (em << 16));
-                npart += __popc(pb);
-                if (S >= 8u) {
-                    for (uint32_t full = __ballot_sync(0xFFFFFFFFu, em == run); full;
-                         full &= full - 1) {
-                        const uint32_t e = __ffs(full) - 1;
-                        const uint32_t s0 = __shfl_sync(0xFFFFFFFFu, es, e);
-                        const uint32_t n0 = __shfl_sync(0xFFFFFFFFu, en, e);
-                        walk_leaf<KAHAN>(xyzm, s0, n0, slice, S, t, bx, by, bz, cx, cy, cz);
-                        if (DEBUG) used += n0;
-                    }
-                } else {
-                    const uint32_t got = sum_tiles<KAHAN>(tile, xyzm, es, em == run ? en : 0u,
-                                                          slice, S, t, bx, by, bz, cx, cy, cz);
-                    if (DEBUG) used += got;
-                }
-            }
-            // pass 2: per leaf q of the record, its listed entries, gathered
-            // 32 at a time in shared memory so that the tiles run full; the
-            // lanes are dealt over q's targets alone (T_q lanes, 32 / T_q
-            // slices)
-            __syncwarp();
-            for (uint32_t m = partial_q; m; m &= m - 1) {
-                const uint32_t qq = __ffs(m) - 1;
-                const uint4 ci = tv.info[fc + qq];
-                const uint32_t lo = max(ci.x, first), hi = min(ci.x + ci.y, first + cnt_t);
-                if (hi <= lo) continue;
-                const uint32_t nq = hi - lo;
-                uint32_t Tq = 1;
-                while (Tq < nq) Tq <<= 1;
-                const uint32_t Sq = 32u / Tq, tq = lane & (Tq - 1u), sq = lane / Tq;
-                const bool actq = tq < nq;
-                const uint32_t iq = lo + (actq ? tq : 0u);
-                const float4 tp = xyzm[iq];
-                float px = 0.f, py = 0.f, pz = 0.f, kx = 0.f, ky = 0.f, kz = 0.f;
-                uint32_t usedq = 0, kept = 0;
-                for (uint32_t b = 0;; b += 32) {
-                    // take the next 32 listed entries' share for q; sum the
-                    // gathered ones when 32 are in (or at the list's end)
-                    const bool more = b < npart;
-                    uint2 v = make_uint2(0u, 0u);
-                    if (more && b + lane < npart) v = plist[b + lane];
-                    const bool mine = (v.y >> (16 + qq)) & 1u;
-                    const uint32_t mb = __ballot_sync(0xFFFFFFFFu, mine);
-                    const uint32_t pos = kept + __popc(mb & ((1u << lane) - 1u));
-                    const uint2 e2 = make_uint2(v.x, v.y & 0xFFFFu);
-                    if (mine && pos < 32u) ent[pos] = e2;
-                    kept += __popc(mb);
-                    if (kept >= 32u || (!more && kept > 0u)) {
-                        const uint32_t k = min(kept, 32u);
-                        __syncwarp();
-                        const uint2 g = lane < k ? ent[lane] : make_uint2(0u, 0u);
-                        __syncwarp();
-                        if (mine && pos >= 32u) ent[pos - 32u] = e2;
-                        kept -= k;
-                        if (Sq >= 8u) {
-                            for (uint32_t pm = __ballot_sync(0xFFFFFFFFu, lane < k); pm;
-                                 pm &= pm - 1) {
-                                const uint32_t e = __ffs(pm) - 1;
-                                const uint32_t s0 = __shfl_sync(0xFFFFFFFFu, g.x, e);
-                                const uint32_t n0 = __shfl_sync(0xFFFFFFFFu, g.y, e);
-                                walk_leaf<KAHAN>(xyzm, s0, n0, sq, Sq, tp, px, py, pz, kx, ky, kz);
-                                if (DEBUG) usedq += n0;
-                            }
-                        } else {
-                            const uint32_t got = sum_tiles<KAHAN>(tile, xyzm, g.x, g.y, sq, Sq, tp,
-                                                                  px, py, pz, kx, ky, kz);
-                            if (DEBUG) usedq += got;
-                        }
-                    }
-                    if (!more) break;
-                }
-                px -= kx;
-                py -= ky;
-                pz -= kz;
-                for (uint32_t o = Tq; o < 32u; o <<= 1) {
-                    px += __shfl_xor_sync(0xFFFFFFFFu, px, o);
-                    py += __shfl_xor_sync(0xFFFFFFFFu, py, o);
-                    pz += __shfl_xor_sync(0xFFFFFFFFu, pz, o);
-                }
-                if (actq && sq == 0) {
-                    float4& pp = part[iq - first];
-                    pp.x += px;
-                    pp.y += py;
-                    pp.z += pz;
-                }
-                if (DEBUG) inter += (actq && sq == 0) ? usedq : 0u;
-                __syncwarp();
-            }
-            if (c == kNone) break;
-        }
-        __syncwarp();
-        if (DEBUG) inter += (active && slice == 0) ? used : 0u;
-        // sum the slices' partial sums (fixed order)
-        bx -= cx;
-        by -= cy;
-        bz -= cz;
-        for (uint32_t o = T; o < 32u; o <<= 1) {
-            bx += __shfl_xor_sync(0xFFFFFFFFu, bx, o);
-            by += __shfl_xor_sync(0xFFFFFFFFu, by, o);
-            bz += __shfl_xor_sync(0xFFFFFFFFu, bz, o);
-        }
-        if (active && slice == 0) {
-            const float4 pp = part[tl];
-            bx += pp.x;
-            by += pp.y;
-            bz += pp.z;
-            const float4 L = tv.lt[u];
-            float lx = L.y, ly = L.z, lz = L.w;
-            if constexpr (GRAD) {
-                const float4 cu = tv.geo[u];
-                const float3 sh = grad_apply(tv.lg0[u], tv.lg1[u], t.x - cu.x, t.y - cu.y,
-                                             t.z - cu.z);
-                lx += sh.x;
-                ly += sh.y;
-                lz += sh.z;
-                if (A.leaf_of) A.leaf_of[i] = u;
-            }
-            const double mm = (double)t.w;
-            A.fx[i] = (float)(mm * ((double)lx + (double)bx));
-            A.fy[i] = (float)(mm * ((double)ly + (double)by));
-            A.fz[i] = (float)(mm * ((double)lz + (double)bz));
-        }
+        const uint4 rec = A.dense.rec[2 * (size_t)r], rec2 = A.dense.rec[2 * (size_t)r + 1];
+        dense_record<KAHAN>(A, sm, rec, rec2, inter);
         __syncwarp();
     }
-    if (DEBUG) {
+    if (A.debug) {
         inter = warp_sum(inter);
         if (lane == 0 && inter) {
             atomicAdd(&status->stat[PSG_STAT_P2P_INTER], inter);
@@ -1538,7 +1494,7 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t& excl, uint3
 }
 
 template <bool DEBUG, bool GRAD>
-__global__ void __launch_bounds__(kHeavyThreads, 2) k_heavy_leaf(TravArgs A) {
+__global__ void __launch_bounds__(kHeavyThreads, 2) k_heavy_leaf(const __grid_constant__ TravArgs A) {
     __shared__ uint32_t s_w[kHeavyWarps];
     __shared__ uint32_t s_rec;
     __shared__ float s_red[kHeavyWarps][12];
@@ -1947,20 +1903,9 @@ void launch_heavy_leaf(const TravArgs& A, int grid, cudaStream_t st) {
     }
 }
 
-template <bool DEBUG, bool GRAD>
-static void launch_dense_kahan(const TravArgs& A, int grid, cudaStream_t st) {
-    if (A.kahan) k_dense_p2p<DEBUG, GRAD, true><<<grid, kTravThreads, 0, st>>>(A);
-    else k_dense_p2p<DEBUG, GRAD, false><<<grid, kTravThreads, 0, st>>>(A);
-}
-
 void launch_dense_p2p(const TravArgs& A, int grid, cudaStream_t st) {
-    if (A.order >= 1) {
-        if (A.debug) launch_dense_kahan<true, true>(A, grid, st);
-        else launch_dense_kahan<false, true>(A, grid, st);
-    } else {
-        if (A.debug) launch_dense_kahan<true, false>(A, grid, st);
-        else launch_dense_kahan<false, false>(A, grid, st);
-    }
+    if (A.kahan) k_dense_p2p<true><<<grid, kDenseThreads, 0, st>>>(A);
+    else k_dense_p2p<false><<<grid, kDenseThreads, 0, st>>>(A);
 }
 
 template <int MODE, bool DENSE, bool XL>

@@ -85,6 +85,7 @@ struct Status {
     uint32_t sort_tiles[6];                // onesweep tile tickets (code + system passes)
     uint32_t dense_count;                  // full-leaf P2P records written
     uint32_t dense_work;                   // ... and taken by k_dense_p2p
+    uint32_t dense_slots;                  // slots taken by records of split source lists
     uint32_t max_leaf;                     // particles in the fullest leaf
     uint32_t heavy_work;                   // groups taken by k_heavy_leaf
     uint32_t ns_fail;                      // bit k: level k's near lists did not fit

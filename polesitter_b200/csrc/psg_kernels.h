@@ -141,12 +141,22 @@ void launch_direct_f64(const float4* xyzm, size_t n, const uint32_t* targets, si
 #include "psg_common.cuh"
 
 namespace psg {
-// k_dense_p2p: blocks per SM, warps per block, and the partial entries
-// (source leaves that serve only some leaves of a record) a warp keeps for
-// its record's second pass
-constexpr int kDenseBlocksPerSm = 8;
+// k_dense_p2p: blocks per SM, warps per block, target particles of a record
+constexpr int kDenseBlocksPerSm = 4;
 constexpr int kDenseWarpsPerBlock = 4;
-constexpr uint32_t kDensePartCap = 2048;
+constexpr int kDenseThreads = 32 * kDenseWarpsPerBlock;
+constexpr uint32_t kDenseTargets = 16;
+
+// work records of k_dense_p2p and, where a group's source list is recorded in
+// several segments, the slots their sums meet in
+struct DenseStore {
+    uint4* rec;         // two words per record (record_dense)
+    uint4* meta;        // per slot: the previous segment's slot; and in a target
+                        // chunk's first slot: its last slot, segments, segments done
+    double* sums;       // per slot: kDenseTargets x 3
+    uint32_t rec_cap;
+    uint32_t slot_cap;
+};
 }  // namespace psg
 
 namespace psg {
@@ -166,10 +176,7 @@ struct TravArgs {
     int kahan;          // compensated FP32 sums in P2P
     int order;          // closure: 0 = the reference's order-0 local, 1 = order-1
     uint32_t* leaf_of;  // closure: leaf node of each sorted particle (order 1)
-    uint4* dense_rec;   // full-leaf P2P work records: leaf | q << 28, chain, first, count
-    uint32_t dense_cap;
-    uint2* dense_part;  // per warp of k_dense_p2p: kDensePartCap partial entries
-    uint32_t dense_part_warps;
+    DenseStore dense;   // full-leaf P2P work records
     int heavy_depth;    // leaf children of nodes above this depth go to k_heavy_leaf
     uint32_t* heavy_frontier;  // per block: 2 x heavy_fcap candidate slots
     uint32_t heavy_fcap;

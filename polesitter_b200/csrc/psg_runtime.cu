@@ -104,10 +104,7 @@ struct State {
     uint32_t* ns;
     unsigned long long ns_cap;
     P2PStore p2p;
-    uint4* dense_rec;      // full-leaf P2P work records
-    uint32_t dense_cap;
-    uint2* dense_part;     // per warp of k_dense_p2p: its record's partial entries
-    uint32_t dense_part_warps;
+    DenseStore dense;      // full-leaf P2P work records
     uint32_t* heavy_frontier;
     uint32_t heavy_fcap;
     int heavy_slots;       // blocks of k_heavy_leaf
@@ -194,12 +191,17 @@ static int alloc_p2p(State* s, uint32_t chunks) {
     return PSG_OK;
 }
 
-static int alloc_dense(State* s, uint32_t cap) {
-    if (s->dense_rec) cudaFree(s->dense_rec);
-    s->dense_rec = nullptr;
-    s->dense_cap = 0;
-    PSG_ALLOC(s->dense_rec, (size_t)cap * sizeof(uint4));
-    s->dense_cap = cap;
+static int alloc_dense(State* s, uint32_t recs, uint32_t slots) {
+    DenseStore& d = s->dense;
+    void* ps[3] = {d.rec, d.meta, d.sums};
+    for (void* p : ps)
+        if (p) cudaFree(p);
+    d = DenseStore{};
+    PSG_ALLOC(d.rec, (size_t)recs * 2 * sizeof(uint4));
+    PSG_ALLOC(d.meta, (size_t)slots * sizeof(uint4));
+    PSG_ALLOC(d.sums, (size_t)slots * kDenseTargets * 3 * sizeof(double));
+    d.rec_cap = recs;
+    d.slot_cap = slots;
     return PSG_OK;
 }
 
@@ -271,7 +273,7 @@ static void free_state(State* s) {
                   s->tv.mp, s->tv.lt, s->tv.info, s->tv.parent, s->tv.arrive, s->tv.cbase,
                   s->tv.ns_off, s->tv.ns_cnt, s->tv.dbg_m2l, s->tv.dbg_p2p, s->tv.link,
                   s->tv.p2p_head, s->ns, s->p2p.src, s->p2p.mask, s->p2p.next, s->p2p.cnt,
-                  s->d_status, s->dense_rec, s->dense_part, s->heavy_frontier, s->tk_partial, s->tk_bbox, s->tk_v[0], s->tk_v[1], s->tk_v[2],
+                  s->d_status, s->dense.rec, s->dense.meta, s->dense.sums, s->heavy_frontier, s->tk_partial, s->tk_bbox, s->tk_v[0], s->tk_v[1], s->tk_v[2],
                   s->tk_vmir[0], s->tk_vmir[1], s->tk_vmir[2], s->cl.lg0, s->cl.lg1,
                   s->cl.leaf_of, s->cl.dF, s->cl.params, s->cl.packed, s->cl.judge_tg,
                   s->cl.judge_f64, s->cl.judge_part, s->cl.d_judge};
@@ -361,10 +363,8 @@ static int init_state(State* s, size_t maxp, float theta, const uint32_t* lvl_ca
     if (r != PSG_OK) return r;
     r = alloc_p2p(s, (uint32_t)(n < 4096 ? 4096 : n / 4));
     if (r != PSG_OK) return r;
-    r = alloc_dense(s, (uint32_t)(n / 4 + 1024));
+    r = alloc_dense(s, (uint32_t)(n / 2 + 1024), (uint32_t)(n / 8 + 4096));
     if (r != PSG_OK) return r;
-    s->dense_part_warps = (uint32_t)dense_grid(s, n) * kDenseWarpsPerBlock;
-    PSG_ALLOC(s->dense_part, (size_t)s->dense_part_warps * kDensePartCap * sizeof(uint2));
     // shallow leaves: a frontier holds at most one level's nodes plus the
     // parent's near list
     s->heavy_slots = 64;
@@ -462,7 +462,7 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
     PSG_CHECK(cudaMemsetAsync(&s->d_status->ns_used[0], 0, sizeof(s->d_status->ns_used),
                               s->stream));
     PSG_CHECK(cudaMemsetAsync(&s->d_status->p2p_chunks, 0, 4, s->stream));
-    PSG_CHECK(cudaMemsetAsync(&s->d_status->dense_count, 0, 8, s->stream));
+    PSG_CHECK(cudaMemsetAsync(&s->d_status->dense_count, 0, 12, s->stream));
     PSG_CHECK(cudaMemsetAsync(&s->d_status->heavy_work, 0, 4, s->stream));
     PSG_CHECK(cudaMemsetAsync(&s->d_status->ns_fail, 0, 4, s->stream));
     TravArgs A;
@@ -484,10 +484,7 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
     A.leaf_of = o ? s->cl.leaf_of : nullptr;
     A.tv.lg0 = o ? s->cl.lg0 : nullptr;
     A.tv.lg1 = o ? s->cl.lg1 : nullptr;
-    A.dense_rec = s->dense_rec;
-    A.dense_cap = s->dense_cap;
-    A.dense_part = s->dense_part;
-    A.dense_part_warps = s->dense_part_warps;
+    A.dense = s->dense;
     A.heavy_depth = heavy_depth_for(s);
     A.heavy_frontier = s->heavy_frontier;
     A.heavy_fcap = s->heavy_fcap;
@@ -620,10 +617,13 @@ static int regrow(State* s, uint32_t err) {
         if (r != PSG_OK) return r;
     }
     if (err & PSG_ERR_DENSE_OVERFLOW) {
-        unsigned long long need = s->h_status->dense_count;
-        need = need + need / 4 + 1024;
-        if (need > 0x7FFFFFFFull) need = 0x7FFFFFFFull;
-        int r = alloc_dense(s, (uint32_t)need);
+        auto room = [](uint32_t used, uint32_t cap) {
+            if (used <= cap) return cap;
+            const unsigned long long need = (unsigned long long)used + used / 4 + 1024;
+            return (uint32_t)std::min<unsigned long long>(need, 0x7FFFFFFFull);
+        };
+        int r = alloc_dense(s, room(s->h_status->dense_count, s->dense.rec_cap),
+                            room(s->h_status->dense_slots, s->dense.slot_cap));
         if (r != PSG_OK) return r;
     }
     if (err & PSG_ERR_P2P_OVERFLOW) {
@@ -1792,7 +1792,7 @@ int psg_set_option(void* mem, int key, double value) {
             PSG_CHECK(cudaStreamSynchronize(s->stream));
             int r = psg::alloc_ns(s, 1024);
             if (r == PSG_OK) r = psg::alloc_p2p(s, 64);
-            if (r == PSG_OK) r = psg::alloc_dense(s, 64);
+            if (r == PSG_OK) r = psg::alloc_dense(s, 64, 64);
             psg::reset_near_levels(s);
             return r;
         }
