@@ -168,30 +168,41 @@ __device__ __forceinline__ void cgp_put(float4 (*cgp)[2], const float4* cgeo, ui
     __syncwarp();
 }
 
+// the run of consecutive children that starts at the lowest bit of m (its
+// particles are contiguous): child mask, first particle, particles; taken off m
+__device__ __forceinline__ uint32_t next_run(const SmemLeaf& sm, uint32_t& m, uint32_t& first,
+                                             uint32_t& count) {
+    const uint32_t q0 = __ffs(m) - 1;
+    uint32_t q1 = q0;
+    first = sm.cpart[q0].x;
+    count = sm.cpart[q0].y;
+    while (q1 + 1 < 8 && ((m >> (q1 + 1)) & 1u)) count += sm.cpart[++q1].y;
+    m &= ~((2u << q1) - 1u);
+    return ((2u << q1) - 1u) & ~((1u << q0) - 1u);
+}
+
 // k_dense_p2p work records for the leaf children in mask of the group whose
 // children start at node fc, over the source chain phead: each run of
-// consecutive children (their particles are contiguous) is cut into records
-// of up to kDenseTargets particles.  A long source list is recorded in
-// segments of kSegChunks chunks (last: the group's last segment), so that the
-// records of a shallow leaf, whose list reaches most of the tree, are shared
-// out over many warps; the segments' sums meet in slots (DenseStore).  One
-// warp per whole list took 7.7 of a 131K closure tick's 9.9 ms, as segments
-// 0.9 ms; 32 chunks (at most 1,024 source leaves) keep a record to tens of
-// microseconds while most lists of a 1M tick stay whole.
-// Records: {fc, phead, first particle, count | run's child mask << 8},
-// {slot or kNone, the same targets' slot of the first segment, 0, 0}.
+// consecutive children is cut into records of up to kDenseTargets particles.
+// A long source list is recorded in segments of kSegChunks chunks (last: the
+// warp's last segment), so that the records of a shallow leaf, whose list
+// reaches most of the tree, are shared out over many warps; the segments'
+// sums meet in slots (DenseStore).  One warp per whole list took 7.7 of a
+// 131K closure tick's 9.9 ms, as segments 0.9 ms; 32 chunks (at most 1,024
+// source leaves) keep a record to tens of microseconds while most lists of a
+// 1M tick stay whole.  part: the list is one of several warps' (a split
+// group, whose last warp links the lists and fills in the items).
+// Record: {fc, phead, first particle, count | run's child mask << 8}, slot or
+// kNone.
 __device__ __noinline__ void record_dense(SmemLeaf& sm, const DenseStore& ds, uint32_t mask,
-                                          uint32_t fc, uint32_t phead, bool last,
+                                          uint32_t fc, uint32_t phead, bool last, bool part,
                                           Status* status) {
     const uint32_t lane = lane_id();
     const uint32_t segs = sm.seg_cnt;
-    const bool split = !last || segs != 0;
-    uint32_t nall = 0;
+    const bool split = !last || part || segs != 0;
+    uint32_t nall = 0, first, count;
     for (uint32_t m = mask; m;) {
-        const uint32_t q0 = __ffs(m) - 1;
-        uint32_t q1 = q0, count = sm.cpart[q0].y;
-        while (q1 + 1 < 8 && ((m >> (q1 + 1)) & 1u)) count += sm.cpart[++q1].y;
-        m &= ~((2u << q1) - 1u);
+        next_run(sm, m, first, count);
         nall += (count + kDenseTargets - 1) / kDenseTargets;
     }
     uint32_t r0 = 0, s0 = kNone;
@@ -201,32 +212,21 @@ __device__ __noinline__ void record_dense(SmemLeaf& sm, const DenseStore& ds, ui
     }
     r0 = __shfl_sync(0xFFFFFFFFu, r0, 0);
     s0 = __shfl_sync(0xFFFFFFFFu, s0, 0);
-    const uint32_t first_slot = segs ? sm.seg_first : s0;
     const uint32_t prev_slot = segs ? sm.seg_prev : kNone;
     uint32_t ord = 0;
     for (uint32_t m = mask; m;) {
-        const uint32_t q0 = __ffs(m) - 1;
-        uint32_t q1 = q0, count = sm.cpart[q0].y;
-        while (q1 + 1 < 8 && ((m >> (q1 + 1)) & 1u)) count += sm.cpart[++q1].y;
-        const uint32_t run = ((2u << q1) - 1u) & ~((1u << q0) - 1u);
-        m &= ~((2u << q1) - 1u);
-        const uint32_t first = sm.cpart[q0].x;
+        const uint32_t run = next_run(sm, m, first, count);
         const uint32_t nrec = (count + kDenseTargets - 1) / kDenseTargets;
         for (uint32_t k = lane; k < nrec; k += 32) {
-            const uint32_t r = r0 + ord + k, sl = s0 + ord + k, f = first_slot + ord + k;
+            const uint32_t r = r0 + ord + k, sl = s0 + ord + k, c0 = k * kDenseTargets;
             if (r < ds.rec_cap) {
-                const uint32_t c0 = k * kDenseTargets;
-                ds.rec[2 * (size_t)r] = make_uint4(fc, phead, first + c0,
-                                                   min(kDenseTargets, count - c0) | (run << 8));
-                ds.rec[2 * (size_t)r + 1] = make_uint4(split ? sl : kNone, f, 0u, 0u);
+                ds.rec[r] = make_uint4(fc, phead, first + c0,
+                                       min(kDenseTargets, count - c0) | (run << 8));
+                ds.rec_slot[r] = split ? sl : kNone;
             }
             if (split && sl < ds.slot_cap) {
-                ds.meta[sl] = make_uint4(prev_slot == kNone ? kNone : prev_slot + ord + k,
-                                         kNone, 0u, 0u);
-                if (last) {
-                    ds.meta[f].y = sl;
-                    ds.meta[f].z = segs + 1;
-                }
+                ds.prev[sl] = prev_slot == kNone ? kNone : prev_slot + ord + k;
+                if (last && !part) ds.item[first + c0] = make_uint4(sl, segs + 1, 0u, 0u);
             }
         }
         ord += nrec;
@@ -235,7 +235,7 @@ __device__ __noinline__ void record_dense(SmemLeaf& sm, const DenseStore& ds, ui
         set_err(status, PSG_ERR_DENSE_OVERFLOW);
     __syncwarp();
     if (lane == 0) {
-        sm.seg_first = first_slot;
+        if (segs == 0) sm.seg_first = s0;
         sm.seg_prev = s0;
         sm.seg_cnt = segs + 1;
         sm.seg_chunks = 0;
@@ -243,22 +243,59 @@ __device__ __noinline__ void record_dense(SmemLeaf& sm, const DenseStore& ds, ui
     __syncwarp();
 }
 
+// The last warp of a split group: the warps' source lists (SplitStore::list,
+// in warp order) become one list per target chunk -- each list's first slot
+// is linked to the list before it -- and the chunk's item holds its end.
+__device__ __noinline__ void link_split(SmemLeaf& sm, const TravArgs& A, uint32_t mask,
+                                        uint32_t fc, uint32_t sidx) {
+    const uint32_t lane = lane_id();
+    const DenseStore& ds = A.dense;
+    // lane w: warp w's list (first slot, last segment's slot, segments)
+    uint4 l = make_uint4(kNone, kNone, 0u, 0u);
+    if (lane < (uint32_t)kSplitParts) l = __ldcg(&A.split.list[(size_t)sidx * kSplitParts + lane]);
+    const uint32_t lists = __ballot_sync(0xFFFFFFFFu, l.z != 0u);
+    if (lists == 0) {  // no source at all: records that only add the field
+        if (lane == 0) sm.seg_chunks = sm.seg_cnt = 0;
+        __syncwarp();
+        record_dense(sm, ds, mask, fc, kNone, true, false, A.status);
+        return;
+    }
+    const uint32_t nseg = __reduce_add_sync(0xFFFFFFFFu, l.z);
+    uint32_t ord = 0, first, count;
+    for (uint32_t m = mask; m;) {
+        next_run(sm, m, first, count);
+        const uint32_t nrec = (count + kDenseTargets - 1) / kDenseTargets;
+        for (uint32_t k0 = 0; k0 < nrec; k0 += 32) {
+            const uint32_t k = k0 + lane;
+            uint32_t end = kNone;
+            for (uint32_t w = lists; w; w &= w - 1) {
+                const uint32_t fs = __shfl_sync(0xFFFFFFFFu, l.x, __ffs(w) - 1),
+                               ls = __shfl_sync(0xFFFFFFFFu, l.y, __ffs(w) - 1);
+                if (k < nrec && fs + ord + k < ds.slot_cap) ds.prev[fs + ord + k] = end;
+                end = ls + ord + k;
+            }
+            if (k < nrec && end < ds.slot_cap)
+                ds.item[first + k * kDenseTargets] = make_uint4(end, nseg, 0u, 0u);
+        }
+        ord += nrec;
+    }
+    __syncwarp();
+}
+
 // Spill the group's staged P2P sources [0, fill) to HBM chunks of
 // kP2PChunk (node, child mask) entries, chained to the group's earlier
 // chunks.  Warp-collective; chunk ids come from a per-warp pool.  Returns the
-// new chain head.  DENSE: a segment of kSegChunks chunks is recorded for
-// k_dense_p2p and the chain starts over.
-template <bool DENSE>
+// new chain head.  record: the list is for k_dense_p2p, so after kSegChunks
+// chunks a segment is recorded and the chain starts over.
 __device__ __noinline__ uint32_t spill_p2p(SmemLeaf& sm, uint32_t fill, uint32_t head,
-                                           const TravArgs& A, uint32_t tgt_mask, uint32_t fc) {
+                                           const TravArgs& A, uint32_t tgt_mask, uint32_t fc,
+                                           bool record) {
     const uint32_t lane = lane_id();
     const P2PStore& st = A.p2p;
     Status* status = A.status;
-    if constexpr (DENSE) {
-        if (sm.seg_chunks >= kSegChunks) {
-            record_dense(sm, A.dense, tgt_mask, fc, head, false, status);
-            head = kNone;
-        }
+    if (record && sm.seg_chunks >= kSegChunks) {
+        record_dense(sm, A.dense, tgt_mask, fc, head, false, false, status);
+        head = kNone;
     }
     for (uint32_t e0 = 0; e0 < fill; e0 += kP2PChunk) {
         if (sm.chunk_next >= sm.chunk_end) {
@@ -291,10 +328,9 @@ __device__ __noinline__ uint32_t spill_p2p(SmemLeaf& sm, uint32_t fill, uint32_t
         if (lane == 0) sm.chunk_next = c + 1;
         __syncwarp();
     }
-    if constexpr (DENSE) {
-        if (lane == 0) sm.seg_chunks += (fill + kP2PChunk - 1) / kP2PChunk;
-        __syncwarp();
-    }
+    __syncwarp();
+    if (lane == 0) sm.seg_chunks += (fill + kP2PChunk - 1) / kP2PChunk;
+    __syncwarp();
     return head;
 }
 
@@ -453,8 +489,8 @@ __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const TravArgs& o, u
     if constexpr (DENSE) {
         // the group's whole source list to HBM chunks, then k_dense_p2p work
         // records of up to kDenseTargets target particles
-        if (pfill) phead = spill_p2p<true>(sm, pfill, phead, o, tgt_mask, fc);
-        record_dense(sm, o.dense, tgt_mask, fc, phead, true, status);
+        if (pfill) phead = spill_p2p(sm, pfill, phead, o, tgt_mask, fc, true);
+        record_dense(sm, o.dense, tgt_mask, fc, phead, true, false, status);
         if (DEBUG && lane == 0) {
             for (uint32_t m = tgt_mask; m; m &= m - 1) {
                 const uint32_t q = __ffs(m) - 1;
@@ -541,10 +577,19 @@ __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const TravArgs& o, u
 // level or the P2P is streamed, so the other variants keep their registers.
 // The plain sparse leaf variant (the reference's tree and far field) keeps
 // 7 blocks per SM (72 registers), the order-1 leaf variants 4 (128).
-template <int MODE, bool DEBUG, bool GRAD, bool DENSE, bool XL>
+// SPLIT (leaf pass only): the groups of the depths < split_depth, whose leaves'
+// walks reach a large part of the tree, kSplitParts warps each (every warp
+// takes every kSplitParts-th candidate and what lies below it), on trees of
+// either kind; their P2P always goes to k_dense_p2p.  A launch of its own
+// beside the rest, so that the other variants keep their registers.
+enum { VAR_PLAIN = 0, VAR_XL = 1, VAR_SPLIT = 2 };
+
+template <int MODE, bool DEBUG, bool GRAD, bool DENSE, int VAR>
 __global__ void __launch_bounds__(
-    kTravThreads, (MODE == MODE_LEAF && !DEBUG && !XL) ? (GRAD ? 4 : (DENSE ? 1 : 7)) : 1)
+    kTravThreads,
+    (MODE == MODE_LEAF && !DEBUG && VAR != VAR_XL) ? (GRAD ? 4 : (DENSE ? 1 : 7)) : 1)
     k_trav(const __grid_constant__ TravArgs A) {
+    constexpr bool XL = VAR == VAR_XL, SPLIT = VAR == VAR_SPLIT;
     using Smem = typename SmemOf<MODE>::T;
     __shared__ Smem smem[kTravWarps];
     const uint32_t lane = lane_id();
@@ -559,31 +604,37 @@ __global__ void __launch_bounds__(
     if (MODE == MODE_LEAF && (status->err & PSG_ERR_NS_OVERFLOW)) return;
     // the variant for this tree (batched systems: each group takes its
     // system's variant, so a system sums exactly as it does alone)
-    if (MODE == MODE_LEAF && !tv.part_sys &&
+    if (MODE == MODE_LEAF && !SPLIT && !tv.part_sys &&
         ((status->max_leaf >= kDenseSwitch || A.leaf_cap >= kDenseCap) != DENSE))
         return;
     // a shallower level's near lists did not fit: this level's are void
     if (MODE == MODE_INTERNAL && (status->ns_fail & ((1u << A.level) - 1u))) return;
     const float theta2 = __fmul_rn(A.theta, A.theta);
 
-    // group index space: MODE_INTERNAL = the nodes at depth k-1; MODE_LEAF =
-    // the nodes at depths 0..9, level after level
+    // the closure's order-1 accumulators take a group's children 4 at a time:
+    // a work item is (group, half)
+    constexpr uint32_t SL = GRAD ? 4u : 8u;
+    constexpr uint32_t NH = 8u / SL;
+    // work items: MODE_INTERNAL = the (halves of the) nodes at depth k-1;
+    // MODE_LEAF = those of the nodes at depths shallow..9, level after level
+    // (SPLIT: at depths 0..shallow-1, each kSplitParts times)
     uint32_t cum[kMaxDepth + 1];
     uint32_t total = 0;
     uint32_t* work;
     if (MODE == MODE_INTERNAL) {
-        total = status->lvl_count[A.level - 1];
+        total = status->lvl_count[A.level - 1] * NH;
         work = &status->work[A.level];
     } else {
 #pragma unroll
         for (int d = 0; d < kMaxDepth; ++d) {
             cum[d] = total;
-            total += status->lvl_count[d];
+            if ((d < A.shallow) == SPLIT)
+                total += status->lvl_count[d] * NH * (SPLIT ? kSplitParts : 1u);
         }
         cum[kMaxDepth] = total;
         // batched systems run both variants over all groups, each with its
         // own counter (work[1] is no internal level's); one system: work[0]
-        work = &status->work[(tv.part_sys && DENSE) ? 1 : 0];
+        work = SPLIT ? &status->heavy_work : &status->work[(tv.part_sys && DENSE) ? 1 : 0];
     }
     if (lane == 0) {
         if constexpr (MODE == MODE_INTERNAL) {
@@ -598,11 +649,7 @@ __global__ void __launch_bounds__(
     // items taken per atomic: whole work queues are a few items per warp, so
     // the leaf pass takes them one by one (a batch would leave warps idle)
     const uint32_t batch = MODE == MODE_INTERNAL ? 4u : 1u;
-    // the closure's order-1 accumulators take a group's children 4 at a time:
-    // a work item is (group, half)
-    constexpr uint32_t SL = GRAD ? 4u : 8u;
-    constexpr uint32_t NH = 8u / SL;
-    const uint32_t items = total * NH;
+    const uint32_t items = total;
 
     for (;;) {
         uint32_t g0 = 0;
@@ -611,22 +658,31 @@ __global__ void __launch_bounds__(
         if (g0 >= items) break;
 #pragma unroll 1
         for (uint32_t gi = g0; gi < g0 + batch && gi < items; ++gi) {
-            const uint32_t g = gi / NH, base = (gi % NH) * SL;
-            uint32_t pid, dp;
+            uint32_t pid, dp, base;
+            // SPLIT: this is warp `part` of the group's `parts`
+            uint32_t parts = 1, part = 0;
             if (MODE == MODE_INTERNAL) {
                 dp = A.level - 1;
-                pid = tv.lvl_base[dp] + g;
+                pid = tv.lvl_base[dp] + gi / NH;
+                base = (gi % NH) * SL;
             } else {
                 dp = 0;
                 uint32_t off = 0;
 #pragma unroll
                 for (int d = 1; d < kMaxDepth; ++d) {
-                    if (g >= cum[d]) {
+                    if (gi >= cum[d]) {
                         dp = d;
                         off = cum[d];
                     }
                 }
-                pid = tv.lvl_base[dp] + (g - off);
+                uint32_t k = gi - off;
+                if constexpr (SPLIT) {
+                    parts = kSplitParts;
+                    part = k % kSplitParts;
+                    k /= kSplitParts;
+                }
+                pid = tv.lvl_base[dp] + k / NH;
+                base = (k % NH) * SL;
             }
             const long long t_group = DEBUG ? clock64() : 0;
             const uint32_t plink = tv.link[pid];
@@ -640,8 +696,9 @@ __global__ void __launch_bounds__(
             if (tv.part_sys) {
                 gsys = tv.part_sys[tv.info[pid].x];
                 th2 = tv.sys_theta2[gsys];
-                if (MODE == MODE_LEAF &&
-                    ((int)dp < tv.sys_heavy[gsys] ||
+                if (SPLIT && (int)dp >= tv.sys_shallow[gsys]) continue;
+                if (MODE == MODE_LEAF && !SPLIT &&
+                    ((int)dp < tv.sys_shallow[gsys] ||
                      ((tv.sys_maxleaf[gsys] >= kDenseSwitch || tv.sys_cap[gsys] >= kDenseCap) !=
                       DENSE)))
                     continue;
@@ -670,7 +727,7 @@ __global__ void __launch_bounds__(
                     sm.ns_cnt[lane] = 0;
                 } else {
                     if (DEBUG) sm.dbg_p2p[lane] = 0;
-                    if (DENSE && lane == 0) sm.seg_chunks = sm.seg_cnt = 0;
+                    if (lane == 0) sm.seg_chunks = sm.seg_cnt = 0;
                 }
             }
             // chain group (leaf pass, parent deeper than the near lists
@@ -702,12 +759,41 @@ __global__ void __launch_bounds__(
                 }
             }
             const float4 Lp = tv.lt[bnode];
-            const bool root_only = dp <= 1;
+            bool root_only = dp <= 1;
             const uint32_t* nsl = nullptr;
-            uint32_t nsn = 0;
+            uint32_t nsn = 0, nfirst = 0;
             if (!root_only) {
                 nsl = A.ns + tv.ns_off[bnode];
                 nsn = tv.ns_cnt[bnode];
+            }
+            if constexpr (SPLIT) {
+                if (root_only) {
+                    // the candidates of a group below the root are the root
+                    // alone: its warps start from the root's grandchildren,
+                    // unless a target is separated from the root or one of
+                    // its children (a tiny theta, or centres that rounding
+                    // has pulled together): then the first warp takes it whole
+                    const uint32_t rl = tv.link[gsys];
+                    const uint32_t rc = rl >> 28;
+                    bool far = false;
+                    if (lane <= rc) {
+                        const float4 sg = tv.geo[lane < rc ? (rl & kLinkMask) + lane : gsys];
+                        for (uint32_t m = tgt_mask; m; m &= m - 1) {
+                            const float4 c = sm.cgeo[__ffs(m) - 1];
+                            float dx, dy, dz, d2;
+                            far |= mac_separated(c.x, c.y, c.z, c.w, sg.x, sg.y, sg.z, sg.w, th2,
+                                                 dx, dy, dz, d2);
+                        }
+                    }
+                    if (__any_sync(0xFFFFFFFFu, far)) {
+                        if (part) continue;
+                        parts = 1;
+                    } else {
+                        root_only = false;
+                        nfirst = rl & kLinkMask;
+                        nsn = rc;
+                    }
+                }
             }
             // MODE_INTERNAL: reserve |cand| near-list entries per target child
             uint32_t cand_total = 1;
@@ -767,6 +853,7 @@ __global__ void __launch_bounds__(
             float cacc0 = 0.f, cacc1 = 0.f, cacc2 = 0.f;  // chain groups: ancestors' M2L
             bool flushed = false;                         // STREAM: a flush has run
             unsigned long long sinter = 0;                // ... its pairs (debug)
+            uint32_t crun = 0;                            // split: candidates passed
 
             for (;;) {
                 // ---- next batch of candidates into cand[0, tot) ----
@@ -782,18 +869,36 @@ __global__ void __launch_bounds__(
                 } else if (e0 < nsn &&
                            (MODE == MODE_INTERNAL ||
                             ssize <= (uint32_t)(kStackCap - kStackSlack - kCandBuf))) {
+                    // a split group's warp keeps every parts-th candidate, and
+                    // reads on until it has a warp's worth of them
+                    tot = 0;
+                    do {
                     const uint32_t e = e0 + lane;
                     uint32_t s0 = 0, c = 0, link = 0;
                     if (e < nsn) {
-                        s0 = nsl[e];
+                        s0 = (SPLIT && !nsl) ? nfirst + e : nsl[e];
                         link = tv.link[s0];
                         const uint32_t nch = link >> 28;
                         c = nch ? nch : 1u;
                     }
                     const uint32_t inc = warp_incl_scan(c);
-                    tot = __shfl_sync(0xFFFFFFFFu, inc, 31);
+                    const uint32_t all = __shfl_sync(0xFFFFFFFFu, inc, 31);
                     const uint32_t ex = inc - c;
                     const bool lf = (link >> 28) == 0;
+                    if (SPLIT && parts > 1u) {
+                        const uint32_t off = (part - crun) % kSplitParts;
+                        for (uint32_t i = 0; i < c; ++i) {
+                            const uint32_t k = ex + i - off;
+                            if (k % kSplitParts == 0) {
+                                sm.cand_node[tot + k / kSplitParts] =
+                                    lf ? s0 : (link & kLinkMask) + i;
+                                sm.cand_mask[tot + k / kSplitParts] = (uint8_t)tgt_mask;
+                            }
+                        }
+                        if (all > off) tot += (all - off + kSplitParts - 1) / kSplitParts;
+                        crun += all;
+                    } else {
+                    tot = all;
                     // a chain group's candidates are first tested against its
                     // ancestor a_{K+1} alone (level 1, no children)
                     const uint8_t cmk = (uint8_t)((XL && nchain) ? 0u : tgt_mask);
@@ -803,7 +908,9 @@ __global__ void __launch_bounds__(
                         if constexpr (MODE == MODE_LEAF && XL)
                             sm.cand_lvl[ex + i] = nchain ? 1 : 0;
                     }
+                    }
                     e0 += 32;
+                    } while (SPLIT && parts > 1u && tot < 32u && e0 < nsn);
                 } else if (MODE == MODE_LEAF && ssize > 0) {
                     // pop entries (bounded so the stack cannot overflow) and
                     // open them: an internal node's candidates are its
@@ -987,7 +1094,8 @@ __global__ void __launch_bounds__(
                                                             flushed, false, sinter);
                                     flushed = true;
                                 } else {
-                                    phead = spill_p2p<DENSE>(sm, pfill, phead, A, tgt_mask, fc);
+                                    phead = spill_p2p(sm, pfill, phead, A, tgt_mask, fc,
+                                                      DENSE);
                                 }
                                 pfill = 0;
                             }
@@ -1040,6 +1148,59 @@ __global__ void __launch_bounds__(
                 Lb.z = __fadd_rn(Lb.z, warp_sum(cacc1));
                 Lb.w = __fadd_rn(Lb.w, warp_sum(cacc2));
             }
+            // a split group: this warp's sums and source list are put down, and
+            // the warp that comes last adds them all up in warp order
+            const float* psum = nullptr;
+            if constexpr (SPLIT) {
+                if (parts > 1u) {
+                    const uint32_t sidx = gi / kSplitParts;
+                    float* own = A.split.sums + (size_t)gi * kSplitSums;
+#pragma unroll
+                    for (uint32_t k = 0; k < SL; ++k) {
+                        if (!((tgt_mask >> (base + k)) & 1u)) continue;
+#pragma unroll
+                        for (uint32_t c = 0; c < (GRAD ? 9u : 3u); ++c) {
+                            const float2 v2 = c < 3u ? acc[k >> 1][c]
+                                                     : gacc[GRAD ? (k >> 1) : 0][c < 3u ? 0 : c - 3u];
+                            const float v = warp_sum((k & 1) ? v2.y : v2.x);
+                            if (lane == 0) __stcg(own + k * (GRAD ? 9u : 3u) + c, v);
+                        }
+                        if (DEBUG && lane == 0) {
+                            const uint32_t q = base + k;
+                            atomicAdd(&tv.dbg_m2l[fc + q], sm.dbg_m2l[q]);
+                            atomicAdd(&tv.dbg_p2p[fc + q], sm.dbg_p2p[q]);
+                            atomicAdd(&status->stat[PSG_STAT_M2L],
+                                      (unsigned long long)sm.dbg_m2l[q]);
+                            atomicAdd(&status->stat[PSG_STAT_P2P_PAIRS],
+                                      (unsigned long long)sm.dbg_p2p[q]);
+                        }
+                    }
+                    if (pfill) phead = spill_p2p(sm, pfill, phead, A, tgt_mask, fc, true);
+                    if (phead != kNone)
+                        record_dense(sm, A.dense, tgt_mask, fc, phead, true, true, status);
+                    uint32_t done = 0;
+                    if (lane == 0) {
+                        __stcg(&A.split.list[gi],
+                               make_uint4(sm.seg_first, sm.seg_prev, sm.seg_cnt, 0u));
+                        __threadfence();
+                        done = atomicAdd(&A.split.count[sidx], 1u);
+                    }
+                    done = __shfl_sync(0xFFFFFFFFu, done, 0);
+                    if (done + 1u != parts) continue;
+                    __threadfence();
+                    link_split(sm, A, tgt_mask, fc, sidx);
+                    psum = A.split.sums + (size_t)sidx * kSplitParts * kSplitSums +
+                           lane * kSplitSums;
+                }
+            }
+            // the sum of a lane's value over the warp, or of the split group's
+            // warps' sums
+            auto total_of = [&](float v, uint32_t k, uint32_t c) {
+                if (SPLIT && psum)
+                    v = lane < (uint32_t)kSplitParts ? __ldcg(psum + k * (GRAD ? 9u : 3u) + c)
+                                                     : 0.f;
+                return warp_sum(v);
+            };
             float4 Gp0 = make_float4(0.f, 0.f, 0.f, 0.f), cp = Gp0;
             float2 Gp1 = make_float2(0.f, 0.f);
             if constexpr (GRAD) {
@@ -1054,9 +1215,9 @@ __global__ void __launch_bounds__(
                 const uint32_t q = base + k;
                 if (!((tgt_mask >> q) & 1u)) continue;
                 const float2* ak = acc[k >> 1];
-                const float ax = warp_sum((k & 1) ? ak[0].y : ak[0].x);
-                const float ay = warp_sum((k & 1) ? ak[1].y : ak[1].x);
-                const float az = warp_sum((k & 1) ? ak[2].y : ak[2].x);
+                const float ax = total_of((k & 1) ? ak[0].y : ak[0].x, k, 0);
+                const float ay = total_of((k & 1) ? ak[1].y : ak[1].x, k, 1);
+                const float az = total_of((k & 1) ? ak[2].y : ak[2].x, k, 2);
                 float4 L = make_float4(0.f, __fadd_rn(ax, Lb.y), __fadd_rn(ay, Lb.z),
                                        __fadd_rn(az, Lb.w));
                 float4 G0 = Gp0;
@@ -1068,12 +1229,12 @@ __global__ void __launch_bounds__(
                     L.z += sh.y;
                     L.w += sh.z;
                     const float2* gk = gacc[k >> 1];
-                    G0.x += warp_sum((k & 1) ? gk[0].y : gk[0].x);
-                    G0.y += warp_sum((k & 1) ? gk[1].y : gk[1].x);
-                    G0.z += warp_sum((k & 1) ? gk[2].y : gk[2].x);
-                    G0.w += warp_sum((k & 1) ? gk[3].y : gk[3].x);
-                    G1.x += warp_sum((k & 1) ? gk[4].y : gk[4].x);
-                    G1.y += warp_sum((k & 1) ? gk[5].y : gk[5].x);
+                    G0.x += total_of((k & 1) ? gk[0].y : gk[0].x, k, 3);
+                    G0.y += total_of((k & 1) ? gk[1].y : gk[1].x, k, 4);
+                    G0.z += total_of((k & 1) ? gk[2].y : gk[2].x, k, 5);
+                    G0.w += total_of((k & 1) ? gk[3].y : gk[3].x, k, 6);
+                    G1.x += total_of((k & 1) ? gk[4].y : gk[4].x, k, 7);
+                    G1.y += total_of((k & 1) ? gk[5].y : gk[5].x, k, 8);
                 }
                 if (lane == 0) {
                     const uint32_t u = fc + q;
@@ -1093,7 +1254,7 @@ __global__ void __launch_bounds__(
                         tv.ns_off[u] = (uint32_t)(ns_base + (unsigned long long)sub * cand_total);
                         tv.ns_cnt[u] = ns_ok ? sm.ns_cnt[q] : 0u;
                     }
-                    if (DEBUG) {
+                    if (DEBUG && !(SPLIT && parts > 1u)) {
                         tv.dbg_m2l[u] = sm.dbg_m2l[q];
                         atomicAdd(&status->stat[PSG_STAT_M2L], (unsigned long long)sm.dbg_m2l[q]);
                     }
@@ -1102,6 +1263,7 @@ __global__ void __launch_bounds__(
             __syncwarp();
 
             if constexpr (MODE == MODE_LEAF) {
+                if (SPLIT && parts > 1u) continue;  // (its P2P and L2P: k_dense_p2p)
                 leaf_epilogue<DEBUG, GRAD, DENSE>(sm, A, tgt_mask, fc, pfill, phead,
                                                   XL && A.stream != 0, flushed, sinter);
                 if (DEBUG && lane == 0) {
@@ -1236,7 +1398,7 @@ __device__ __forceinline__ void dense_step(DensePair<KAHAN> (&a)[kDensePairs],
 
 // one record
 template <bool KAHAN>
-__device__ __forceinline__ void dense_record(const TravArgs& A, DenseSmem& sm, uint4 rec, uint4 rec2,
+__device__ __forceinline__ void dense_record(const TravArgs& A, DenseSmem& sm, uint4 rec, uint32_t slot,
                                              unsigned long long& inter) {
     const TreeView& tv = A.tv;
     const float4* __restrict__ xyzm = A.xyzm;
@@ -1386,7 +1548,6 @@ __device__ __forceinline__ void dense_record(const TravArgs& A, DenseSmem& sm, u
     }
     // a segment of a longer list: its sums go to its slot, and the segment
     // that comes last adds them all, from the list's end
-    const uint32_t slot = rec2.x;
     if (slot != kNone) {
         const DenseStore& ds = A.dense;
         double* own = ds.sums + (size_t)slot * kDenseTargets * 3;
@@ -1397,14 +1558,14 @@ __device__ __forceinline__ void dense_record(const TravArgs& A, DenseSmem& sm, u
         }
         __threadfence();
         __syncwarp();
-        const uint32_t item = rec2.y;
+        uint4* item = ds.item + first;
         uint32_t done = 0;
-        if (lane == 0) done = atomicAdd(&ds.meta[item].w, 1u);
+        if (lane == 0) done = atomicAdd(&item->z, 1u);
         done = __shfl_sync(0xFFFFFFFFu, done, 0);
-        if (done + 1u != ds.meta[item].z) return;
+        if (done + 1u != item->y) return;
         __threadfence();
         bx = by = bz = 0.0;
-        for (uint32_t sl = ds.meta[item].y; sl != kNone; sl = ds.meta[sl].x) {
+        for (uint32_t sl = item->x; sl != kNone; sl = ds.prev[sl]) {
             if (lane < cnt) {
                 const double* v = ds.sums + (size_t)sl * kDenseTargets * 3 + 3 * lane;
                 bx += __ldcg(v);
@@ -1448,8 +1609,9 @@ __global__ void __launch_bounds__(kDenseThreads, KAHAN ? 2 : kDenseBlocksPerSm)
         if (lane == 0) r = atomicAdd(&status->dense_work, 1u);
         r = __shfl_sync(0xFFFFFFFFu, r, 0);
         if (r >= total) break;
-        const uint4 rec = A.dense.rec[2 * (size_t)r], rec2 = A.dense.rec[2 * (size_t)r + 1];
-        dense_record<KAHAN>(A, sm, rec, rec2, inter);
+        const uint4 rec = A.dense.rec[r];
+        const uint32_t slot = A.dense.rec_slot[r];
+        dense_record<KAHAN>(A, sm, rec, slot, inter);
         __syncwarp();
     }
     if (A.debug) {
@@ -1539,7 +1701,7 @@ __global__ void __launch_bounds__(kHeavyThreads, 2) k_heavy_leaf(const __grid_co
             if (tv.part_sys) {
                 // batched systems: only the groups shallow for their own system
                 gsys = tv.part_sys[tv.info[pid].x];
-                if ((int)dp >= tv.sys_heavy[gsys]) continue;
+                if ((int)dp >= tv.sys_shallow[gsys]) continue;
                 th2 = tv.sys_theta2[gsys];
             }
             const uint32_t plink = tv.link[pid];
@@ -1880,19 +2042,6 @@ __global__ void __launch_bounds__(kHeavyThreads, 2) k_heavy_leaf(const __grid_co
     }
 }
 
-// the leaf pass's work counter starts past the groups of depths 0 ..
-// heavy_depth-1, whose leaf children k_heavy_leaf takes
-__global__ void k_leaf_start(Status* status, int heavy_depth, uint32_t parts) {
-    uint32_t skip = 0;
-    for (int d = 0; d < heavy_depth && d < kMaxDepth; ++d) skip += status->lvl_count[d];
-    status->work[0] = skip * parts;
-}
-
-void launch_leaf_start(Status* status, int heavy_depth, int order, cudaStream_t st) {
-    // work items per group: 2 halves with the order-1 accumulators, else 1
-    k_leaf_start<<<1, 1, 0, st>>>(status, heavy_depth, order >= 1 ? 2u : 1u);
-}
-
 void launch_heavy_leaf(const TravArgs& A, int grid, cudaStream_t st) {
     if (A.order >= 1) {
         if (A.debug) k_heavy_leaf<true, true><<<grid, kHeavyThreads, 0, st>>>(A);
@@ -1908,14 +2057,14 @@ void launch_dense_p2p(const TravArgs& A, int grid, cudaStream_t st) {
     else k_dense_p2p<false><<<grid, kDenseThreads, 0, st>>>(A);
 }
 
-template <int MODE, bool DENSE, bool XL>
+template <int MODE, bool DENSE, int VAR>
 static void launch_mode(const TravArgs& A, int grid, cudaStream_t st) {
     if (A.order >= 1) {
-        if (A.debug) k_trav<MODE, true, true, DENSE, XL><<<grid, kTravThreads, 0, st>>>(A);
-        else k_trav<MODE, false, true, DENSE, XL><<<grid, kTravThreads, 0, st>>>(A);
+        if (A.debug) k_trav<MODE, true, true, DENSE, VAR><<<grid, kTravThreads, 0, st>>>(A);
+        else k_trav<MODE, false, true, DENSE, VAR><<<grid, kTravThreads, 0, st>>>(A);
     } else {
-        if (A.debug) k_trav<MODE, true, false, DENSE, XL><<<grid, kTravThreads, 0, st>>>(A);
-        else k_trav<MODE, false, false, DENSE, XL><<<grid, kTravThreads, 0, st>>>(A);
+        if (A.debug) k_trav<MODE, true, false, DENSE, VAR><<<grid, kTravThreads, 0, st>>>(A);
+        else k_trav<MODE, false, false, DENSE, VAR><<<grid, kTravThreads, 0, st>>>(A);
     }
 }
 
@@ -1924,39 +2073,43 @@ static bool leaf_xl(const TravArgs& A) { return A.ns_levels < kMaxDepth || A.str
 void launch_traverse_internal(const TravArgs& args, int level, int grid, cudaStream_t st) {
     TravArgs A = args;
     A.level = level;
-    launch_mode<MODE_INTERNAL, false, false>(A, grid, st);
+    launch_mode<MODE_INTERNAL, false, VAR_PLAIN>(A, grid, st);
 }
 
 void launch_traverse_leaves(const TravArgs& args, const int grid[2], cudaStream_t st) {
     if (leaf_xl(args)) {
-        launch_mode<MODE_LEAF, false, true>(args, grid[0], st);
-        launch_mode<MODE_LEAF, true, true>(args, grid[1], st);
+        launch_mode<MODE_LEAF, false, VAR_XL>(args, grid[0], st);
+        launch_mode<MODE_LEAF, true, VAR_XL>(args, grid[1], st);
     } else {
-        launch_mode<MODE_LEAF, false, false>(args, grid[0], st);
-        launch_mode<MODE_LEAF, true, false>(args, grid[1], st);
+        launch_mode<MODE_LEAF, false, VAR_PLAIN>(args, grid[0], st);
+        launch_mode<MODE_LEAF, true, VAR_PLAIN>(args, grid[1], st);
     }
+}
+
+void launch_traverse_split(const TravArgs& args, int grid, cudaStream_t st) {
+    launch_mode<MODE_LEAF, true, VAR_SPLIT>(args, grid, st);
 }
 
 int traverse_threads() { return kTravThreads; }
 const void* traverse_kernel_ptr(int order, int dense, int xl) {
     if (xl) {
         if (order) {
-            return dense ? (const void*)k_trav<MODE_LEAF, false, true, true, true>
-                         : (const void*)k_trav<MODE_LEAF, false, true, false, true>;
+            return dense ? (const void*)k_trav<MODE_LEAF, false, true, true, VAR_XL>
+                         : (const void*)k_trav<MODE_LEAF, false, true, false, VAR_XL>;
         }
-        return dense ? (const void*)k_trav<MODE_LEAF, false, false, true, true>
-                     : (const void*)k_trav<MODE_LEAF, false, false, false, true>;
+        return dense ? (const void*)k_trav<MODE_LEAF, false, false, true, VAR_XL>
+                     : (const void*)k_trav<MODE_LEAF, false, false, false, VAR_XL>;
     }
     if (order) {
-        return dense ? (const void*)k_trav<MODE_LEAF, false, true, true, false>
-                     : (const void*)k_trav<MODE_LEAF, false, true, false, false>;
+        return dense ? (const void*)k_trav<MODE_LEAF, false, true, true, VAR_PLAIN>
+                     : (const void*)k_trav<MODE_LEAF, false, true, false, VAR_PLAIN>;
     }
-    return dense ? (const void*)k_trav<MODE_LEAF, false, false, true, false>
-                 : (const void*)k_trav<MODE_LEAF, false, false, false, false>;
+    return dense ? (const void*)k_trav<MODE_LEAF, false, false, true, VAR_PLAIN>
+                 : (const void*)k_trav<MODE_LEAF, false, false, false, VAR_PLAIN>;
 }
 const void* traverse_internal_kernel_ptr(int order) {
-    return order ? (const void*)k_trav<MODE_INTERNAL, false, true, false, false>
-                 : (const void*)k_trav<MODE_INTERNAL, false, false, false, false>;
+    return order ? (const void*)k_trav<MODE_INTERNAL, false, true, false, VAR_PLAIN>
+                 : (const void*)k_trav<MODE_INTERNAL, false, false, false, VAR_PLAIN>;
 }
 
 }  // namespace psg

@@ -64,7 +64,8 @@ struct TreeView {
     const uint32_t* sys_cap;    // leaf capacity per system
     const float* sys_bbox;      // (min, max, range, 1023 / range) per system
     const float* sys_theta2;    // theta * theta (rounded) per system
-    const int32_t* sys_heavy;   // shallow-leaf depth per system
+    const int32_t* sys_shallow; // per system: depth above which its groups are split
+                                // over several warps, or k_heavy_leaf's
     uint32_t* sys_maxleaf;      // particles in each system's fullest leaf (this tick)
     uint32_t nsys;
     uint32_t lvl_base[kLevels + 1];

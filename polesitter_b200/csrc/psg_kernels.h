@@ -66,7 +66,7 @@ void launch_traverse_internal(const TravArgs& A, int level, int grid, cudaStream
 void launch_traverse_leaves(const TravArgs& A, const int grid[2], cudaStream_t st);
 void launch_dense_p2p(const TravArgs& A, int grid, cudaStream_t st);
 void launch_heavy_leaf(const TravArgs& A, int grid, cudaStream_t st);
-void launch_leaf_start(Status* status, int heavy_depth, int order, cudaStream_t st);
+void launch_traverse_split(const TravArgs& A, int grid, cudaStream_t st);
 
 
 // k_tick.cu -- the caller's tick loop on the device (README.md:65-111)
@@ -150,12 +150,24 @@ constexpr uint32_t kDenseTargets = 16;
 // work records of k_dense_p2p and, where a group's source list is recorded in
 // several segments, the slots their sums meet in
 struct DenseStore {
-    uint4* rec;         // two words per record (record_dense)
-    uint4* meta;        // per slot: the previous segment's slot; and in a target
-                        // chunk's first slot: its last slot, segments, segments done
-    double* sums;       // per slot: kDenseTargets x 3
+    uint4* rec;          // records (record_dense)
+    uint32_t* rec_slot;  // ... and their slots
+    uint32_t* prev;      // per slot: the previous segment's slot
+    double* sums;        // per slot: kDenseTargets x 3
+    uint4* item;         // per target chunk (by its first particle): its last
+                         // slot, segments, segments done
     uint32_t rec_cap;
     uint32_t slot_cap;
+};
+
+// Leaf pass, SPLIT: warps per group of the shallow depths.
+constexpr uint32_t kSplitParts = 16;
+constexpr uint32_t kSplitSums = 36;  // floats of a warp: 8 children x 3 or 4 x 9
+struct SplitStore {
+    float* sums;      // per group (half) and warp: kSplitSums
+    uint4* list;      // ... first slot, last segment's slot and segments of its P2P list
+    uint32_t* count;  // per group (half): warps done (0 at the run's start)
+    uint32_t cap;     // groups (halves)
 };
 }  // namespace psg
 
@@ -177,6 +189,10 @@ struct TravArgs {
     int order;          // closure: 0 = the reference's order-0 local, 1 = order-1
     uint32_t* leaf_of;  // closure: leaf node of each sorted particle (order 1)
     DenseStore dense;   // full-leaf P2P work records
+    SplitStore split;
+    int shallow;        // the groups of depths < this are not the leaf pass's but
+                        // split over several warps or k_heavy_leaf's (many
+                        // systems: SPLIT's; each group checks its system's depth)
     int heavy_depth;    // leaf children of nodes above this depth go to k_heavy_leaf
     uint32_t* heavy_frontier;  // per block: 2 x heavy_fcap candidate slots
     uint32_t heavy_fcap;

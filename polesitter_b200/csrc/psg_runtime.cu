@@ -105,6 +105,10 @@ struct State {
     unsigned long long ns_cap;
     P2PStore p2p;
     DenseStore dense;      // full-leaf P2P work records
+    SplitStore split;      // sums of the groups that several warps share
+    int forest_split;      // many systems: the deepest of their split depths
+    const int32_t* sys_heavy;  // ... and each one's shallow-leaf and split depth
+    const int32_t* sys_split;
     uint32_t* heavy_frontier;
     uint32_t heavy_fcap;
     int heavy_slots;       // blocks of k_heavy_leaf
@@ -193,15 +197,36 @@ static int alloc_p2p(State* s, uint32_t chunks) {
 
 static int alloc_dense(State* s, uint32_t recs, uint32_t slots) {
     DenseStore& d = s->dense;
-    void* ps[3] = {d.rec, d.meta, d.sums};
+    void* ps[4] = {d.rec, d.rec_slot, d.prev, d.sums};
     for (void* p : ps)
         if (p) cudaFree(p);
+    uint4* const item = d.item;  // (sized by the particles, not by the records)
     d = DenseStore{};
-    PSG_ALLOC(d.rec, (size_t)recs * 2 * sizeof(uint4));
-    PSG_ALLOC(d.meta, (size_t)slots * sizeof(uint4));
+    d.item = item;
+    PSG_ALLOC(d.rec, (size_t)recs * sizeof(uint4));
+    PSG_ALLOC(d.rec_slot, (size_t)recs * 4);
+    PSG_ALLOC(d.prev, (size_t)slots * 4);
     PSG_ALLOC(d.sums, (size_t)slots * kDenseTargets * 3 * sizeof(double));
     d.rec_cap = recs;
     d.slot_cap = slots;
+    return PSG_OK;
+}
+
+// sums and lists of the groups split over several warps: the groups (two
+// halves each) of the depths above `depth`
+static int ensure_split(State* s, int depth) {
+    uint32_t groups = 0;
+    for (int d = 0; d < depth; ++d) groups += 2 * s->tv.lvl_cap[d];
+    SplitStore& p = s->split;
+    if (p.cap >= groups) return PSG_OK;
+    void* ps[3] = {p.sums, p.list, p.count};
+    for (void* q : ps)
+        if (q) cudaFree(q);
+    p = SplitStore{};
+    PSG_ALLOC(p.sums, (size_t)groups * kSplitParts * kSplitSums * sizeof(float));
+    PSG_ALLOC(p.list, (size_t)groups * kSplitParts * sizeof(uint4));
+    PSG_ALLOC(p.count, (size_t)groups * 4);
+    p.cap = groups;
     return PSG_OK;
 }
 
@@ -273,7 +298,8 @@ static void free_state(State* s) {
                   s->tv.mp, s->tv.lt, s->tv.info, s->tv.parent, s->tv.arrive, s->tv.cbase,
                   s->tv.ns_off, s->tv.ns_cnt, s->tv.dbg_m2l, s->tv.dbg_p2p, s->tv.link,
                   s->tv.p2p_head, s->ns, s->p2p.src, s->p2p.mask, s->p2p.next, s->p2p.cnt,
-                  s->d_status, s->dense.rec, s->dense.meta, s->dense.sums, s->heavy_frontier, s->tk_partial, s->tk_bbox, s->tk_v[0], s->tk_v[1], s->tk_v[2],
+                  s->d_status, s->dense.rec, s->dense.rec_slot, s->dense.prev, s->dense.sums,
+                  s->dense.item, s->split.sums, s->split.list, s->split.count, s->heavy_frontier, s->tk_partial, s->tk_bbox, s->tk_v[0], s->tk_v[1], s->tk_v[2],
                   s->tk_vmir[0], s->tk_vmir[1], s->tk_vmir[2], s->cl.lg0, s->cl.lg1,
                   s->cl.leaf_of, s->cl.dF, s->cl.params, s->cl.packed, s->cl.judge_tg,
                   s->cl.judge_f64, s->cl.judge_part, s->cl.d_judge};
@@ -363,8 +389,9 @@ static int init_state(State* s, size_t maxp, float theta, const uint32_t* lvl_ca
     if (r != PSG_OK) return r;
     r = alloc_p2p(s, (uint32_t)(n < 4096 ? 4096 : n / 4));
     if (r != PSG_OK) return r;
-    r = alloc_dense(s, (uint32_t)(n / 2 + 1024), (uint32_t)(n / 8 + 4096));
+    r = alloc_dense(s, (uint32_t)(n / 2 + 1024), (uint32_t)(n / 8 + 8192));
     if (r != PSG_OK) return r;
+    PSG_ALLOC(s->dense.item, n * sizeof(uint4));
     // shallow leaves: a frontier holds at most one level's nodes plus the
     // parent's near list
     s->heavy_slots = 64;
@@ -420,12 +447,14 @@ static int closure_alloc(State* s) {
     return PSG_OK;
 }
 
-// Leaves at most this deep are walked block-parallel by k_heavy_leaf: a leaf
-// at depth d (half width H / 2^d of the root's H) stays unseparated from the
-// sources within about theta H / 2^(d-1), a large part of the tree once
-// 2^d <= 4 theta.  That only costs a warp long in a large system: below
-// kHeavyMinParticles, where a walk over the whole tree is still short (and
-// shallow leaves are most leaves), the leaf pass takes every leaf.
+// A leaf at depth d (half width H / 2^d of the root's H) stays unseparated
+// from the sources within about theta H / 2^(d-1), a large part of the tree
+// once 2^d <= 4 theta.  The leaf pass shares such groups out over kSplitParts
+// warps each (split_depth_of).  The leaf pass that walks ancestor chains or
+// streams its P2P takes each group in one warp; beside it such leaves are
+// walked block-parallel by k_heavy_leaf (also on demand:
+// PS_B200_OPT_HEAVY_DEPTH), but not below kHeavyMinParticles, where a walk
+// over the whole tree is still short and shallow leaves are most leaves.
 constexpr size_t kHeavyMinParticles = 131072;
 
 static int heavy_depth_of(float theta, size_t n) {
@@ -433,6 +462,24 @@ static int heavy_depth_of(float theta, size_t n) {
     int d = 0;
     while (d < 5 && (float)(2 << d) <= 4.0f * theta) ++d;
     return d < 2 ? 2 : d;
+}
+
+// Depth above which the leaf pass splits groups over kSplitParts warps: where
+// a leaf's walk is long (2^d <= 4 theta, at most depth 4), and only above the
+// depth at which n particles spread evenly would have their leaves (8^d * cap
+// < n), since groups that are the rule need no help.  Measured (leaf pass and
+// full-leaf P2P, one warp per group / split): 32K clumpy at theta 8 7.0 / 2.8
+// ms, 131K clumpy at theta 6.25 and leaf capacity 16 1.87 / 1.42 ms; theta 3
+// 32K clumpy 0.41 / 0.42 ms; without the second limit 32K cube at theta 10 and
+// leaf capacity 16 0.61 / 0.61 ms but 0.11 ms more a tick, 1K cube at theta 8
+// 0.21 / 0.41 ms.
+constexpr int kSplitBlocksPerSm = 4;
+
+static int split_depth_of(float theta, size_t n, uint32_t cap) {
+    if (theta < 3.0f) return 0;
+    int d = theta < 4.0f ? 3 : 4;
+    while (d > 0 && ((unsigned long long)cap << (3 * d)) >= n) --d;
+    return d;
 }
 
 static int heavy_depth_for(const State* s) {
@@ -485,7 +532,25 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
     A.tv.lg0 = o ? s->cl.lg0 : nullptr;
     A.tv.lg1 = o ? s->cl.lg1 : nullptr;
     A.dense = s->dense;
-    A.heavy_depth = heavy_depth_for(s);
+    const bool xl = near_levels(s) < kMaxDepth || s->stream_p2p || s->force_stream;
+    // the shallow groups: split over several warps, or (XL, or on demand)
+    // k_heavy_leaf's
+    const bool forest = s->tv.part_sys != nullptr;
+    const bool heavy = xl || s->heavy_depth >= 0;
+    const int depth = heavy    ? heavy_depth_for(s)
+                      : forest ? s->forest_split
+                               : split_depth_of(s->theta, s->trav_n, s->leaf_cap);
+    if (forest) A.tv.sys_shallow = heavy ? s->sys_heavy : s->sys_split;
+    A.shallow = forest ? 0 : depth;
+    if (!heavy) {
+        const int r = ensure_split(s, depth);
+        if (r != PSG_OK) return r;
+        // (not reset by the kernel: a void run may stop half way)
+        if (depth)
+            PSG_CHECK(cudaMemsetAsync(s->split.count, 0, (size_t)s->split.cap * 4, s->stream));
+    }
+    A.split = s->split;
+    A.heavy_depth = depth;
     A.heavy_frontier = s->heavy_frontier;
     A.heavy_fcap = s->heavy_fcap;
     A.ns_levels = near_levels(s);
@@ -496,46 +561,48 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
         const int v = (int)(g * gs);
         return v < 1 ? 1 : v;
     };
-    // Shallow leaves on the aux stream.  Their walk reads the near lists and
-    // fields of the groups above depth heavy_depth, final once the internal
-    // level of depth heavy_depth - 1 is done, so it starts there and runs
-    // beside the deeper levels and the leaf pass (which starts at the groups
-    // of depth heavy_depth).
-    bool heavy_started = false;
-    auto start_heavy = [&]() -> int {
+    // The shallow groups on the aux stream.  They read the near lists and
+    // fields of the nodes above `depth`, final once the internal level of
+    // depth - 1 is done, so they start there and run beside the deeper levels
+    // and the leaf pass (which starts at the groups of that depth).
+    bool started = depth == 0;
+    auto start_shallow = [&]() -> int {
         PSG_CHECK(cudaEventRecord(s->ev_levels, s->stream));
         PSG_CHECK(cudaStreamWaitEvent(s->aux, s->ev_levels, 0));
-        launch_heavy_leaf(A, scaled(s->heavy_slots), s->aux);
+        if (heavy) {
+            launch_heavy_leaf(A, scaled(s->heavy_slots), s->aux);
+        } else {
+            TravArgs S = A;
+            S.shallow = depth;
+            launch_traverse_split(S, scaled(s->sms * kSplitBlocksPerSm), s->aux);
+        }
         PSG_CHECK(cudaEventRecord(s->ev_heavy, s->aux));
-        heavy_started = true;
+        started = true;
         return PSG_OK;
     };
-    const int heavy_ready = A.heavy_depth - 1;
-    if (heavy_ready < 2) {
-        const int r = start_heavy();
+    if (!started && depth - 1 < 2) {
+        const int r = start_shallow();
         if (r != PSG_OK) return r;
     }
     for (int k = 2; k <= A.ns_levels; ++k) {
         launch_traverse_internal(A, k, scaled(s->trav_int_grid[o]), s->stream);
-        if (k == heavy_ready) {
-            const int r = start_heavy();
+        if (!started && k == depth - 1) {
+            const int r = start_shallow();
             if (r != PSG_OK) return r;
         }
     }
     record(s, PH_TRAV);
-    if (!heavy_started) {
-        const int r = start_heavy();
+    if (!started) {
+        const int r = start_shallow();
         if (r != PSG_OK) return r;
     }
-    // one system: the leaf pass starts past the shallow groups; many: each
-    // group checks its own system's depth
-    launch_leaf_start(s->d_status, s->tv.part_sys ? 0 : A.heavy_depth, o, s->stream);
-    const int xl = (A.ns_levels < kMaxDepth || A.stream) ? 1 : 0;
     const int lg[2] = {scaled(s->trav_grid[o][0][xl]), scaled(s->trav_grid[o][1][xl])};
     launch_traverse_leaves(A, lg, s->stream);
     record(s, PH_DENSE);
+    // (the split groups' records too; k_heavy_leaf leaves none)
+    if (depth && !heavy) PSG_CHECK(cudaStreamWaitEvent(s->stream, s->ev_heavy, 0));
     launch_dense_p2p(A, scaled((int)dense_grid(s, s->trav_n)), s->stream);
-    PSG_CHECK(cudaStreamWaitEvent(s->stream, s->ev_heavy, 0));
+    if (depth && heavy) PSG_CHECK(cudaStreamWaitEvent(s->stream, s->ev_heavy, 0));
     record(s, PH_END);
     return PSG_OK;
 }
@@ -660,6 +727,11 @@ static int run_traversal(State* s, const float4* xyzm, float* fx, float* fy, flo
         if (rg != PSG_OK) return rg;
         PSG_CHECK(cudaMemsetAsync(&s->d_status->err, 0, 4, s->stream));
         PSG_CHECK(cudaMemsetAsync(&s->d_status->stat[0], 0, sizeof(s->d_status->stat), s->stream));
+        if (s->debug) {
+            const size_t bytes = (size_t)s->tv.lvl_base[kLevels] * 4;
+            PSG_CHECK(cudaMemsetAsync(s->tv.dbg_m2l, 0, bytes, s->stream));
+            PSG_CHECK(cudaMemsetAsync(s->tv.dbg_p2p, 0, bytes, s->stream));
+        }
         if (s->timing) cudaEventRecord(s->ev[PH_UP], s->stream);
     }
     std::snprintf(g_err, sizeof(g_err), "traversal stores still too small after 6 runs");
@@ -1079,6 +1151,7 @@ struct Ensemble {
     uint32_t* sys_cap = nullptr;
     float* sys_theta2 = nullptr;
     int32_t* sys_heavy = nullptr;
+    int32_t* sys_split = nullptr;
     float* sys_bbox = nullptr;      // [nsys][4]
     uint32_t* sys_maxleaf = nullptr;
     uint32_t* sys_sort_offs = nullptr;  // digit starts of the system sort passes
@@ -1134,19 +1207,28 @@ static int set_order(State* s, int order) {
 // capacity of every system to the device tables
 static int upload_systems(Ensemble* e) {
     std::vector<float> th2(e->nsys);
-    std::vector<int32_t> hv(e->nsys);
-    int hmax = 0;
+    std::vector<int32_t> hv(e->nsys), sp(e->nsys);
+    int hmax = 0, smax = 0;
     for (size_t k = 0; k < e->nsys; ++k) {
         const float t = e->theta[k];
         th2[k] = t * t;
         hv[k] = heavy_depth_of(t, e->count[k]);
         hmax = std::max(hmax, (int)hv[k]);
+        sp[k] = split_depth_of(t, e->count[k], e->cap[k]);
+        smax = std::max(smax, (int)sp[k]);
     }
     PSG_CHECK(cudaMemcpy(e->sys_theta2, th2.data(), e->nsys * 4, cudaMemcpyHostToDevice));
     PSG_CHECK(cudaMemcpy(e->sys_heavy, hv.data(), e->nsys * 4, cudaMemcpyHostToDevice));
+    PSG_CHECK(cudaMemcpy(e->sys_split, sp.data(), e->nsys * 4, cudaMemcpyHostToDevice));
     PSG_CHECK(cudaMemcpy(e->sys_cap, e->cap.data(), e->nsys * 4, cudaMemcpyHostToDevice));
     if (hmax != e->fs->forest_heavy) e->dirty = true;  // a launch parameter changes
     e->fs->forest_heavy = hmax;
+    if (smax != e->fs->forest_split) e->dirty = true;
+    e->fs->forest_split = smax;
+    const SplitStore before = e->fs->split;  // (allocated here: not while capturing)
+    const int r = ensure_split(e->fs, smax);
+    if (r != PSG_OK) return r;
+    if (before.sums != e->fs->split.sums) e->dirty = true;
     // the stores' near-list depth and P2P mode start over with the settings
     // (both are launch parameters of the captured graphs)
     if (e->fs->ns_levels != kMaxDepth || e->fs->stream_p2p) e->dirty = true;
@@ -1305,7 +1387,7 @@ static void free_ensemble(Ensemble* e) {
         e->fs = nullptr;
     }
     void* ps[] = {e->part_sys, e->sys_off, e->sys_cap, e->sys_theta2, e->sys_heavy,
-                  e->sys_bbox, e->sys_maxleaf, e->sys_sort_offs, e->blk, e->sys_blk,
+                  e->sys_split, e->sys_bbox, e->sys_maxleaf, e->sys_sort_offs, e->blk, e->sys_blk,
                   e->partial, e->vtmp};
     for (void* p : ps)
         if (p) cudaFree(p);
@@ -1390,6 +1472,7 @@ static int ens_create(Ensemble* e, const size_t* counts, size_t nsys, const floa
     PSG_ALLOC(e->sys_cap, nsys * 4);
     PSG_ALLOC(e->sys_theta2, nsys * 4);
     PSG_ALLOC(e->sys_heavy, nsys * 4);
+    PSG_ALLOC(e->sys_split, nsys * 4);
     PSG_ALLOC(e->sys_bbox, nsys * 16);
     PSG_ALLOC(e->sys_maxleaf, nsys * 4);
     PSG_ALLOC(e->sys_sort_offs, so.size() * 4);
@@ -1408,7 +1491,8 @@ static int ens_create(Ensemble* e, const size_t* counts, size_t nsys, const floa
     tv.sys_cap = e->sys_cap;
     tv.sys_bbox = e->sys_bbox;
     tv.sys_theta2 = e->sys_theta2;
-    tv.sys_heavy = e->sys_heavy;
+    e->fs->sys_heavy = e->sys_heavy;
+    e->fs->sys_split = e->sys_split;
     tv.sys_maxleaf = e->sys_maxleaf;
     tv.nsys = (uint32_t)nsys;
     r = upload_systems(e);
