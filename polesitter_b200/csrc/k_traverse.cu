@@ -29,9 +29,12 @@
 // per-child register accumulators) for each of those children.  What is
 // not separated is dealt with once per chunk:
 //
-//  * MODE_INTERNAL, one launch per level k = 2..10, targets = the internal
-//    children of the depth-(k-1) nodes: near candidates form NS(u) in HBM for
-//    level k+1; L(u) = M2L(u) + L(p) is stored.
+//  * MODE_INTERNAL, levels k = 2..10, targets = the internal children of the
+//    depth-(k-1) nodes: near candidates form NS(u) in HBM for level k+1;
+//    L(u) = M2L(u) + L(p) is stored.  One launch runs a range of levels: the
+//    work queue is in level order, and a group waits (bounded) until its
+//    parent's list and field are marked final by the warp that made them,
+//    which took an earlier item, so some warp can always go on.
 //  * MODE_LEAF, one launch after all levels, targets = the leaf children of
 //    every node: a near leaf candidate is a P2P source, staged in shared
 //    memory with the set of children it serves (spilled to HBM chunks past
@@ -64,7 +67,6 @@ constexpr uint32_t kNsPool = 4096;        // near-list entries a warp reserves a
 constexpr uint32_t kChunkPool = 16;       // P2P spill chunks a warp reserves at once
 constexpr uint32_t kSegChunks = 32;       // chunks of source list per dense work record
 constexpr uint32_t kDenseSwitch = 32;     // fullest leaf from which the DENSE leaf pass runs
-constexpr uint32_t kDenseCap = 8;         // ... or leaf capacity (leaves of many particles)
 
 enum { MODE_INTERNAL = 0, MODE_LEAF = 1 };
 
@@ -207,8 +209,8 @@ __device__ __noinline__ void record_dense(SmemLeaf& sm, const DenseStore& ds, ui
     }
     uint32_t r0 = 0, s0 = kNone;
     if (lane == 0) {
-        r0 = atomicAdd(&status->dense_count, nall);
-        if (split) s0 = atomicAdd(&status->dense_slots, nall);
+        r0 = atomicAdd(&status->run.dense_count, nall);
+        if (split) s0 = atomicAdd(&status->run.dense_slots, nall);
     }
     r0 = __shfl_sync(0xFFFFFFFFu, r0, 0);
     s0 = __shfl_sync(0xFFFFFFFFu, s0, 0);
@@ -300,7 +302,7 @@ __device__ __noinline__ uint32_t spill_p2p(SmemLeaf& sm, uint32_t fill, uint32_t
     for (uint32_t e0 = 0; e0 < fill; e0 += kP2PChunk) {
         if (sm.chunk_next >= sm.chunk_end) {
             uint32_t c = 0;
-            if (lane == 0) c = atomicAdd(&status->p2p_chunks, kChunkPool);
+            if (lane == 0) c = atomicAdd(&status->run.p2p_chunks, kChunkPool);
             c = __shfl_sync(0xFFFFFFFFu, c, 0);
             __syncwarp();
             if (lane == 0) {
@@ -568,6 +570,27 @@ __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const TravArgs& o, u
     __syncwarp();
 }
 
+// Wait until a node's near list and field are final (ready set by the warp that
+// makes them, in this launch); false after kReadyPolls polls (~0.3 s) or once
+// another wait has given up.  Warp-collective.
+constexpr int kReadyPolls = 1 << 18;
+
+__device__ __noinline__ bool wait_ready(const uint32_t* flag, Status* status) {
+    uint32_t ok = 0;
+    if (lane_id() == 0) {
+        for (int i = 0; i < kReadyPolls; ++i) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(ok) : "l"(flag) : "memory");
+            if (ok) break;
+            if ((i & 255) == 255 && (*(volatile uint32_t*)&status->err & PSG_ERR_READY_SPIN)) break;
+            __nanosleep(64);
+        }
+        if (!ok) set_err(status, PSG_ERR_READY_SPIN);
+    }
+    ok = __shfl_sync(0xFFFFFFFFu, ok, 0);
+    __syncwarp();  // (orders the other lanes' reads after lane 0's acquire)
+    return ok != 0u;
+}
+
 // DENSE (leaf pass only): the variant for trees whose fullest leaf holds at
 // least kDenseSwitch particles or whose leaf capacity is kDenseCap or more,
 // which hands full leaves to k_dense_p2p.  Both
@@ -608,7 +631,9 @@ __global__ void __launch_bounds__(
         ((status->max_leaf >= kDenseSwitch || A.leaf_cap >= kDenseCap) != DENSE))
         return;
     // a shallower level's near lists did not fit: this level's are void
-    if (MODE == MODE_INTERNAL && (status->ns_fail & ((1u << A.level) - 1u))) return;
+    if (MODE == MODE_INTERNAL && A.level == A.level_end &&
+        (status->run.ns_fail & ((1u << A.level) - 1u)))
+        return;
     const float theta2 = __fmul_rn(A.theta, A.theta);
 
     // the closure's order-1 accumulators take a group's children 4 at a time:
@@ -622,8 +647,13 @@ __global__ void __launch_bounds__(
     uint32_t total = 0;
     uint32_t* work;
     if (MODE == MODE_INTERNAL) {
-        total = status->lvl_count[A.level - 1] * NH;
-        work = &status->work[A.level];
+#pragma unroll
+        for (int d = 0; d < kMaxDepth; ++d) {
+            cum[d] = total;
+            if (d + 1 >= A.level && d < A.level_end) total += status->lvl_count[d] * NH;
+        }
+        cum[kMaxDepth] = total;
+        work = &status->run.work[A.level];
     } else {
 #pragma unroll
         for (int d = 0; d < kMaxDepth; ++d) {
@@ -634,7 +664,7 @@ __global__ void __launch_bounds__(
         cum[kMaxDepth] = total;
         // batched systems run both variants over all groups, each with its
         // own counter (work[1] is no internal level's); one system: work[0]
-        work = SPLIT ? &status->heavy_work : &status->work[(tv.part_sys && DENSE) ? 1 : 0];
+        work = SPLIT ? &status->run.heavy_work : &status->run.work[(tv.part_sys && DENSE) ? 1 : 0];
     }
     if (lane == 0) {
         if constexpr (MODE == MODE_INTERNAL) {
@@ -661,16 +691,12 @@ __global__ void __launch_bounds__(
             uint32_t pid, dp, base;
             // SPLIT: this is warp `part` of the group's `parts`
             uint32_t parts = 1, part = 0;
-            if (MODE == MODE_INTERNAL) {
-                dp = A.level - 1;
-                pid = tv.lvl_base[dp] + gi / NH;
-                base = (gi % NH) * SL;
-            } else {
+            {
                 dp = 0;
                 uint32_t off = 0;
 #pragma unroll
                 for (int d = 1; d < kMaxDepth; ++d) {
-                    if (gi >= cum[d]) {
+                    if (gi >= cum[d] && cum[d + 1] > cum[d]) {
                         dp = d;
                         off = cum[d];
                     }
@@ -729,6 +755,10 @@ __global__ void __launch_bounds__(
                     if (DEBUG) sm.dbg_p2p[lane] = 0;
                     if (lane == 0) sm.seg_chunks = sm.seg_cnt = 0;
                 }
+            }
+            // a parent made in this launch: wait until it is final
+            if (MODE == MODE_INTERNAL && (int)dp >= A.level && dp >= 2u) {
+                if (!wait_ready(&tv.ready[pid], status)) continue;
             }
             // chain group (leaf pass, parent deeper than the near lists
             // reach, K = ns_levels): start from the near list of p's ancestor
@@ -814,7 +844,7 @@ __global__ void __launch_bounds__(
                 if (need && sm.ns_next + need > sm.ns_end) {
                     const unsigned long long take = need > kNsPool ? need : kNsPool;
                     unsigned long long b = 0;
-                    if (lane == 0) b = atomicAdd(&status->ns_used[0], take);
+                    if (lane == 0) b = atomicAdd(&status->run.ns_used, take);
                     b = __shfl_sync(0xFFFFFFFFu, b, 0);
                     __syncwarp();
                     if (lane == 0) {
@@ -827,7 +857,7 @@ __global__ void __launch_bounds__(
                 ns_ok = ns_base + need <= A.ns_cap;
                 if (!ns_ok && lane == 0) {
                     set_err(status, PSG_ERR_NS_OVERFLOW);
-                    atomicOr(&status->ns_fail, 1u << A.level);
+                    atomicOr(&status->run.ns_fail, 1u << (dp + 1));
                 }
                 __syncwarp();
                 if (lane == 0) sm.ns_next = ns_base + need;
@@ -1261,6 +1291,13 @@ __global__ void __launch_bounds__(
                 }
             }
             __syncwarp();
+            if constexpr (MODE == MODE_INTERNAL) {
+                // lists and fields of this group's children are final
+                if ((tgt_mask >> lane) & 1u) {
+                    __threadfence();
+                    __stcg(&tv.ready[fc + lane], 1u);
+                }
+            }
 
             if constexpr (MODE == MODE_LEAF) {
                 if (SPLIT && parts > 1u) continue;  // (its P2P and L2P: k_dense_p2p)
@@ -1602,11 +1639,11 @@ __global__ void __launch_bounds__(kDenseThreads, KAHAN ? 2 : kDenseBlocksPerSm)
     Status* status = A.status;
     if (status->err & (PSG_ERR_NODES | PSG_ERR_SORT_SPIN | PSG_ERR_DENSE_OVERFLOW)) return;
     const uint32_t lane = lane_id();
-    const uint32_t total = min(status->dense_count, A.dense.rec_cap);
+    const uint32_t total = min(status->run.dense_count, A.dense.rec_cap);
     unsigned long long inter = 0;
     for (;;) {
         uint32_t r = 0;
-        if (lane == 0) r = atomicAdd(&status->dense_work, 1u);
+        if (lane == 0) r = atomicAdd(&status->run.dense_work, 1u);
         r = __shfl_sync(0xFFFFFFFFu, r, 0);
         if (r >= total) break;
         const uint4 rec = A.dense.rec[r];
@@ -1689,7 +1726,7 @@ __global__ void __launch_bounds__(kHeavyThreads, 2) k_heavy_leaf(const __grid_co
     for (;;) {
         if (leaves == 0) {
             // next group with leaf children
-            if (tid == 0) s_rec = atomicAdd(&status->heavy_work, 1u);
+            if (tid == 0) s_rec = atomicAdd(&status->run.heavy_work, 1u);
             __syncthreads();
             const uint32_t g = s_rec;
             __syncthreads();
@@ -2070,19 +2107,23 @@ static void launch_mode(const TravArgs& A, int grid, cudaStream_t st) {
 
 static bool leaf_xl(const TravArgs& A) { return A.ns_levels < kMaxDepth || A.stream; }
 
-void launch_traverse_internal(const TravArgs& args, int level, int grid, cudaStream_t st) {
+void launch_traverse_internal(const TravArgs& args, int level, int level_end, int grid,
+                              cudaStream_t st) {
     TravArgs A = args;
     A.level = level;
+    A.level_end = level_end;
     launch_mode<MODE_INTERNAL, false, VAR_PLAIN>(A, grid, st);
 }
 
-void launch_traverse_leaves(const TravArgs& args, const int grid[2], cudaStream_t st) {
+// which: 1 the sparse variant, 2 the dense one, 3 both (each returns at once
+// unless the tree is its kind)
+void launch_traverse_leaves(const TravArgs& args, const int grid[2], int which, cudaStream_t st) {
     if (leaf_xl(args)) {
-        launch_mode<MODE_LEAF, false, VAR_XL>(args, grid[0], st);
-        launch_mode<MODE_LEAF, true, VAR_XL>(args, grid[1], st);
+        if (which & 1) launch_mode<MODE_LEAF, false, VAR_XL>(args, grid[0], st);
+        if (which & 2) launch_mode<MODE_LEAF, true, VAR_XL>(args, grid[1], st);
     } else {
-        launch_mode<MODE_LEAF, false, VAR_PLAIN>(args, grid[0], st);
-        launch_mode<MODE_LEAF, true, VAR_PLAIN>(args, grid[1], st);
+        if (which & 1) launch_mode<MODE_LEAF, false, VAR_PLAIN>(args, grid[0], st);
+        if (which & 2) launch_mode<MODE_LEAF, true, VAR_PLAIN>(args, grid[1], st);
     }
 }
 

@@ -385,6 +385,7 @@ __global__ void __launch_bounds__(256) k_tree_link(TreeView tv, const Status* st
         tv.info[id] = inf;
         tv.link[id] = nch ? ((inf.z & kLinkMask) | (nch << 28)) : 0u;
         tv.lt[id] = make_float4(0.f, 0.f, 0.f, 0.f);
+        tv.ready[id] = 0;
         if (nch == 0 && inf.y > max_leaf) max_leaf = inf.y;
         // batched systems: each system picks its own leaf-pass variant
         if (nch == 0 && tv.part_sys && inf.y >= 32u)
@@ -394,10 +395,49 @@ __global__ void __launch_bounds__(256) k_tree_link(TreeView tv, const Status* st
     if (lane_id() == 0 && max_leaf) atomicMax(&const_cast<Status*>(status)->max_leaf, max_leaf);
 }
 
-// Upward pass, one launch per level from the deepest up: a leaf sums P2M
-// over its particles, an internal node adds its children's multipoles (M2M).
+// Upward pass: P2M (a leaf's particles) and M2M (a node's children).
 // Operation order matches polesitter.h:978-1045 exactly (sequential sums over
-// the leaf's particles; children in octant order), every op rounded to nearest.
+// the leaf's particles; children in octant order), every op rounded to nearest,
+// whichever thread does it.
+// Bound: latency -- the sequential sum of the fullest leaf (its loads run
+// kP2mBatch ahead of the adds) and the way from the leaves to the root.
+constexpr int kP2mBatch = 8;
+
+__device__ __forceinline__ float4 p2m(const float4* __restrict__ xyzm, uint4 inf, float4 c) {
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&](const float4& p) {
+        o.x = __fadd_rn(o.x, p.w);
+        o.y = __fadd_rn(o.y, __fmul_rn(p.w, __fsub_rn(p.x, c.x)));
+        o.z = __fadd_rn(o.z, __fmul_rn(p.w, __fsub_rn(p.y, c.y)));
+        o.w = __fadd_rn(o.w, __fmul_rn(p.w, __fsub_rn(p.z, c.z)));
+    };
+    uint32_t k = 0;
+    for (; k + kP2mBatch <= inf.y; k += kP2mBatch) {
+        float4 p[kP2mBatch];
+#pragma unroll
+        for (int j = 0; j < kP2mBatch; ++j) p[j] = xyzm[inf.x + k + j];
+#pragma unroll
+        for (int j = 0; j < kP2mBatch; ++j) add(p[j]);
+    }
+    for (; k < inf.y; ++k) add(xyzm[inf.x + k]);
+    return o;
+}
+
+__device__ __forceinline__ float4 m2m(const TreeView& tv, uint32_t link, float4 c) {
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t fc = link & kLinkMask, nch = link >> 28;
+    for (uint32_t j = 0; j < nch; ++j) {
+        const float4 cm = __ldcg(&tv.mp[fc + j]);
+        const float4 cg = tv.geo[fc + j];
+        o.x = __fadd_rn(o.x, cm.x);
+        o.y = __fadd_rn(o.y, __fadd_rn(cm.y, __fmul_rn(cm.x, __fsub_rn(cg.x, c.x))));
+        o.z = __fadd_rn(o.z, __fadd_rn(cm.z, __fmul_rn(cm.x, __fsub_rn(cg.y, c.y))));
+        o.w = __fadd_rn(o.w, __fadd_rn(cm.w, __fmul_rn(cm.x, __fsub_rn(cg.z, c.z))));
+    }
+    return o;
+}
+
+// the nodes of one level (their children are done)
 __global__ void __launch_bounds__(256) k_upward_level(TreeView tv, const Status* status,
                                                       const float4* __restrict__ xyzm, int d) {
     if (status->err & (PSG_ERR_NODES | PSG_ERR_SORT_SPIN)) return;
@@ -406,28 +446,33 @@ __global__ void __launch_bounds__(256) k_upward_level(TreeView tv, const Status*
     const uint32_t id = tv.lvl_base[d] + r;
     const float4 c = tv.geo[id];
     const uint32_t link = tv.link[id];
-    float m0 = 0.f, mx = 0.f, my = 0.f, mz = 0.f;
-    if ((link >> 28) == 0) {
-        const uint4 inf = tv.info[id];
-        for (uint32_t k = 0; k < inf.y; ++k) {
-            const float4 p = xyzm[inf.x + k];
-            m0 = __fadd_rn(m0, p.w);
-            mx = __fadd_rn(mx, __fmul_rn(p.w, __fsub_rn(p.x, c.x)));
-            my = __fadd_rn(my, __fmul_rn(p.w, __fsub_rn(p.y, c.y)));
-            mz = __fadd_rn(mz, __fmul_rn(p.w, __fsub_rn(p.z, c.z)));
-        }
-    } else {
-        const uint32_t fc = link & kLinkMask, nch = link >> 28;
-        for (uint32_t j = 0; j < nch; ++j) {
-            const float4 cm = tv.mp[fc + j];
-            const float4 cg = tv.geo[fc + j];
-            m0 = __fadd_rn(m0, cm.x);
-            mx = __fadd_rn(mx, __fadd_rn(cm.y, __fmul_rn(cm.x, __fsub_rn(cg.x, c.x))));
-            my = __fadd_rn(my, __fadd_rn(cm.z, __fmul_rn(cm.x, __fsub_rn(cg.y, c.y))));
-            mz = __fadd_rn(mz, __fadd_rn(cm.w, __fmul_rn(cm.x, __fsub_rn(cg.z, c.z))));
-        }
+    tv.mp[id] = (link >> 28) == 0 ? p2m(xyzm, tv.info[id], c) : m2m(tv, link, c);
+}
+
+// the levels bottom .. 0 in one launch: a thread takes a node of the bottom
+// level (any deeper ones are done) or a leaf above it and climbs; of a node's
+// children the last to arrive (per-node counters, zeroed by k_tree_emit) adds
+// their multipoles and climbs on
+__global__ void __launch_bounds__(256) k_upward_climb(TreeView tv, const Status* status,
+                                                      const float4* __restrict__ xyzm,
+                                                      int bottom) {
+    if (status->err & (PSG_ERR_NODES | PSG_ERR_SORT_SPIN)) return;
+    const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= tv.lvl_base[bottom + 1]) return;
+    int d = 0;
+    while (d < bottom && id >= tv.lvl_base[d + 1]) ++d;
+    if (id - tv.lvl_base[d] >= status->lvl_count[d]) return;
+    uint32_t link = tv.link[id];
+    if ((link >> 28) != 0 && d < bottom) return;
+    const float4 c0 = tv.geo[id];
+    __stcg(&tv.mp[id], (link >> 28) == 0 ? p2m(xyzm, tv.info[id], c0) : m2m(tv, link, c0));
+    for (uint32_t cur = tv.parent[id]; cur != kNone; cur = tv.parent[cur]) {
+        link = tv.link[cur];
+        __threadfence();
+        if (atomicAdd(&tv.arrive[cur], 1u) + 1u != (link >> 28)) return;
+        __threadfence();
+        __stcg(&tv.mp[cur], m2m(tv, link, tv.geo[cur]));
     }
-    tv.mp[id] = make_float4(m0, mx, my, mz);
 }
 
 void launch_tree(const uint32_t* codes, size_t n, uint32_t* tile_buf, TreeView tv,
@@ -441,13 +486,21 @@ void launch_tree(const uint32_t* codes, size_t n, uint32_t* tile_buf, TreeView t
     k_tree_link<<<grid, 256, 0, st>>>(tv, status);
 }
 
-void launch_upward(TreeView tv, const Status* status, const float4* xyzm, int grid,
+constexpr size_t kClimbParticles = 262144;
+
+void launch_upward(TreeView tv, const Status* status, const float4* xyzm, size_t n,
                    cudaStream_t st) {
-    (void)grid;
-    for (int d = kMaxDepth; d >= 0; --d) {
-        const int g = (int)((tv.lvl_cap[d] + 255) / 256);
-        k_upward_level<<<g, 256, 0, st>>>(tv, status, xyzm, d);
-    }
+    // One climbing launch for a small system, where launches cost more than the
+    // climb; the three deepest (and widest) levels of a large one in launches of
+    // their own, since a fence and an atomic per leaf cost more than those.
+    // Measured (one launch / the 3 deepest levels apart): 33K Plummer 39 / 50 us,
+    // 262K 53 / 50, 1M 113 / 65, 4M 309 / 142; 262K clumpy at leaf capacity 16
+    // 51 / 69.  One launch per level: 65K 64 us, 1M 80 us.
+    const int bottom = n < kClimbParticles ? kMaxDepth : kMaxDepth - 3;
+    for (int d = kMaxDepth; d > bottom; --d)
+        k_upward_level<<<(tv.lvl_cap[d] + 255) / 256, 256, 0, st>>>(tv, status, xyzm, d);
+    k_upward_climb<<<(tv.lvl_base[bottom + 1] + 255) / 256, 256, 0, st>>>(tv, status, xyzm,
+                                                                         bottom);
 }
 
 }  // namespace psg

@@ -49,7 +49,7 @@ struct TreeView {
     uint32_t* arrive;      // upward-pass arrival counters
     uint32_t* cbase;       // first-child rank per node (tree link step)
     uint32_t* link;        // first child | nchild << 28
-    uint32_t* p2p_head;    // per leaf: last chunk of its P2P source list
+    uint32_t* ready;       // internal levels: the node's near list and field are final
     uint32_t* ns_off;      // per node: offset of its near-source list
     uint32_t* ns_cnt;      // per node: length of its near-source list
     uint32_t* dbg_m2l;     // per node M2L pair count (debug builds of a tick)
@@ -76,20 +76,21 @@ struct TreeView {
 struct Status {
     uint32_t err;                          // PSG_ERR_* bits
     uint32_t lvl_count[kLevels + 1];       // nodes per level
-    unsigned long long ns_used[kLevels + 1];  // near-list entries per level
-    unsigned long long ns_cap;             // capacity of one near-list region
-    uint32_t work[kLevels + 1];            // traversal work counters
     float bbox[4];                         // min, max, range, scale (prepare)
     unsigned long long stat[16];           // debug totals (see PSG_STAT_*)
     uint32_t max_stack;                    // deepest DFS stack seen (debug)
-    uint32_t p2p_chunks;                   // P2P chunks used this tick
     uint32_t sort_tiles[6];                // onesweep tile tickets (code + system passes)
-    uint32_t dense_count;                  // full-leaf P2P records written
-    uint32_t dense_work;                   // ... and taken by k_dense_p2p
-    uint32_t dense_slots;                  // slots taken by records of split source lists
     uint32_t max_leaf;                     // particles in the fullest leaf
-    uint32_t heavy_work;                   // groups taken by k_heavy_leaf
-    uint32_t ns_fail;                      // bit k: level k's near lists did not fit
+    struct Run {                           // one traversal run's counters
+        unsigned long long ns_used;        // near-list entries reserved
+        uint32_t work[kLevels + 1];        // work taken: internal levels, leaf pass
+        uint32_t p2p_chunks;               // P2P chunks used
+        uint32_t dense_count;              // full-leaf P2P records written
+        uint32_t dense_work;               // ... and taken by k_dense_p2p
+        uint32_t dense_slots;              // slots taken by records of split source lists
+        uint32_t heavy_work;               // shallow groups taken
+        uint32_t ns_fail;                  // bit k: level k's near lists did not fit
+    } run;
 };
 
 // P2P sources spilled from the traversal: chunk c holds cnt[c] source-leaf

@@ -53,7 +53,7 @@ int tree_tile_size();
 void launch_tree(const uint32_t* codes, size_t n, uint32_t* tile_buf, TreeView tv,
                  Status* status, float cx, float cy, float cz, float hw, int grid,
                  cudaStream_t st, const float* bbox = nullptr, uint32_t leaf_cap = 1);
-void launch_upward(TreeView tv, const Status* status, const float4* xyzm, int grid,
+void launch_upward(TreeView tv, const Status* status, const float4* xyzm, size_t n,
                    cudaStream_t st);
 
 // k_traverse.cu -- fused MAC / M2L / L2L, and L2P + P2P for the leaves
@@ -62,8 +62,9 @@ struct TravArgs;
 int traverse_threads();
 const void* traverse_kernel_ptr(int order, int dense, int xl);
 const void* traverse_internal_kernel_ptr(int order);
-void launch_traverse_internal(const TravArgs& A, int level, int grid, cudaStream_t st);
-void launch_traverse_leaves(const TravArgs& A, const int grid[2], cudaStream_t st);
+void launch_traverse_internal(const TravArgs& A, int level, int level_end, int grid,
+                              cudaStream_t st);
+void launch_traverse_leaves(const TravArgs& A, const int grid[2], int which, cudaStream_t st);
 void launch_dense_p2p(const TravArgs& A, int grid, cudaStream_t st);
 void launch_heavy_leaf(const TravArgs& A, int grid, cudaStream_t st);
 void launch_traverse_split(const TravArgs& A, int grid, cudaStream_t st);
@@ -146,6 +147,9 @@ constexpr int kDenseBlocksPerSm = 4;
 constexpr int kDenseWarpsPerBlock = 4;
 constexpr int kDenseThreads = 32 * kDenseWarpsPerBlock;
 constexpr uint32_t kDenseTargets = 16;
+// leaf capacity from which a tree takes the leaf pass's DENSE variant whatever
+// its fullest leaf
+constexpr uint32_t kDenseCap = 8;
 
 // work records of k_dense_p2p and, where a group's source list is recorded in
 // several segments, the slots their sums meet in
@@ -183,7 +187,8 @@ struct TravArgs {
     float* fz;
     Status* status;
     float theta;
-    int level;
+    int level;          // internal levels of this launch
+    int level_end;
     int debug;
     int kahan;          // compensated FP32 sums in P2P
     int order;          // closure: 0 = the reference's order-0 local, 1 = order-1

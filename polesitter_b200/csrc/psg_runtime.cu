@@ -106,6 +106,7 @@ struct State {
     P2PStore p2p;
     DenseStore dense;      // full-leaf P2P work records
     SplitStore split;      // sums of the groups that several warps share
+    bool dense_only;       // many systems: every one takes the dense leaf variant
     int forest_split;      // many systems: the deepest of their split depths
     const int32_t* sys_heavy;  // ... and each one's shallow-leaf and split depth
     const int32_t* sys_split;
@@ -129,6 +130,7 @@ struct State {
     int forest_heavy;      // many systems: the deepest of their shallow-leaf depths
     int ns_levels;         // near lists are stored for node depths <= this (kMaxDepth: all);
                            // lowered when they do not fit, deeper groups walk their chains
+    bool level_by_level;   // one launch per internal level: the lists once did not fit
     int stream_p2p;        // P2P summed in the leaf pass as found (no spill store)
     int force_ns_levels;   // option: store near lists for depths <= this at most
     int force_stream;      // option: always stream the P2P
@@ -153,6 +155,7 @@ struct State {
     ClosureState cl;
     int order;  // traversal's local expansion order: 0 (reference) or 1
     size_t last_n;  // particles of the last completed tick
+    bool trav_fresh;  // no traversal has run on the current tree yet
     size_t trav_n;  // particles of the tick whose traversal is being enqueued
     int attempts;   // traversal runs of the last tick (> 1: a capacity regrow)
 };
@@ -160,6 +163,7 @@ struct State {
 // the near-list levels and the P2P mode start over when what they depend
 // on (theta, leaf capacity, expansion order, store sizes) changes
 static void reset_near_levels(State* s) {
+    s->level_by_level = false;
     s->ns_levels = kMaxDepth;
     s->stream_p2p = 0;
 }
@@ -297,7 +301,7 @@ static void free_state(State* s) {
                   s->sort.hist, s->sort.offs, s->sort.lookback, s->tree_tiles, s->tv.geo,
                   s->tv.mp, s->tv.lt, s->tv.info, s->tv.parent, s->tv.arrive, s->tv.cbase,
                   s->tv.ns_off, s->tv.ns_cnt, s->tv.dbg_m2l, s->tv.dbg_p2p, s->tv.link,
-                  s->tv.p2p_head, s->ns, s->p2p.src, s->p2p.mask, s->p2p.next, s->p2p.cnt,
+                  s->tv.ready, s->ns, s->p2p.src, s->p2p.mask, s->p2p.next, s->p2p.cnt,
                   s->d_status, s->dense.rec, s->dense.rec_slot, s->dense.prev, s->dense.sums,
                   s->dense.item, s->split.sums, s->split.list, s->split.count, s->heavy_frontier, s->tk_partial, s->tk_bbox, s->tk_v[0], s->tk_v[1], s->tk_v[2],
                   s->tk_vmir[0], s->tk_vmir[1], s->tk_vmir[2], s->cl.lg0, s->cl.lg1,
@@ -381,7 +385,7 @@ static int init_state(State* s, size_t maxp, float theta, const uint32_t* lvl_ca
     PSG_ALLOC(s->tv.dbg_m2l, nodes * 4);
     PSG_ALLOC(s->tv.dbg_p2p, nodes * 4);
     PSG_ALLOC(s->tv.link, nodes * 4);
-    PSG_ALLOC(s->tv.p2p_head, nodes * 4);
+    PSG_ALLOC(s->tv.ready, nodes * 4);
     PSG_ALLOC(s->d_status, sizeof(Status));
     PSG_CHECK(cudaMallocHost((void**)&s->h_status, sizeof(Status)));
     std::memset(s->h_status, 0, sizeof(Status));
@@ -505,13 +509,13 @@ static void record(State* s, int ph) {
 // one traversal run (internal levels, leaf pass, shallow leaves, full
 // leaves) enqueued on s->stream; no host synchronisation
 static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy, float* fz) {
-    PSG_CHECK(cudaMemsetAsync(&s->d_status->work[0], 0, sizeof(s->d_status->work), s->stream));
-    PSG_CHECK(cudaMemsetAsync(&s->d_status->ns_used[0], 0, sizeof(s->d_status->ns_used),
-                              s->stream));
-    PSG_CHECK(cudaMemsetAsync(&s->d_status->p2p_chunks, 0, 4, s->stream));
-    PSG_CHECK(cudaMemsetAsync(&s->d_status->dense_count, 0, 12, s->stream));
-    PSG_CHECK(cudaMemsetAsync(&s->d_status->heavy_work, 0, 4, s->stream));
-    PSG_CHECK(cudaMemsetAsync(&s->d_status->ns_fail, 0, 4, s->stream));
+    if (!s->trav_fresh) {  // (a new tree comes with its counters and flags zeroed)
+        Status* const ds = s->d_status;
+        PSG_CHECK(cudaMemsetAsync(&ds->run, 0, sizeof(ds->run), s->stream));
+        PSG_CHECK(cudaMemsetAsync(s->tv.ready, 0, (size_t)s->tv.lvl_base[kLevels] * 4,
+                                  s->stream));
+    }
+    s->trav_fresh = false;
     TravArgs A;
     A.tv = s->tv;
     A.p2p = s->p2p;
@@ -584,12 +588,19 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
         const int r = start_shallow();
         if (r != PSG_OK) return r;
     }
-    for (int k = 2; k <= A.ns_levels; ++k) {
-        launch_traverse_internal(A, k, scaled(s->trav_int_grid[o]), s->stream);
-        if (!started && k == depth - 1) {
+    // the internal levels in one launch, two when the shallow groups start
+    // between them; one launch per level while the lists are short of memory
+    // (the first level that does not fit is then the same in every run)
+    for (int k = 2; k <= A.ns_levels;) {
+        int end = A.ns_levels;
+        if (s->level_by_level) end = k;
+        if (!started) end = std::min(end, std::max(k, depth - 1));
+        launch_traverse_internal(A, k, end, scaled(s->trav_int_grid[o]), s->stream);
+        if (!started && end >= depth - 1) {
             const int r = start_shallow();
             if (r != PSG_OK) return r;
         }
+        k = end + 1;
     }
     record(s, PH_TRAV);
     if (!started) {
@@ -597,7 +608,7 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
         if (r != PSG_OK) return r;
     }
     const int lg[2] = {scaled(s->trav_grid[o][0][xl]), scaled(s->trav_grid[o][1][xl])};
-    launch_traverse_leaves(A, lg, s->stream);
+    launch_traverse_leaves(A, lg, s->dense_only ? 2 : s->leaf_cap >= kDenseCap ? 2 : 3, s->stream);
     record(s, PH_DENSE);
     // (the split groups' records too; k_heavy_leaf leaves none)
     if (depth && !heavy) PSG_CHECK(cudaStreamWaitEvent(s->stream, s->ev_heavy, 0));
@@ -649,8 +660,8 @@ static bool try_alloc_p2p(State* s, uint32_t chunks) {
 // PSG_EOOM when nothing can give.
 static int regrow(State* s, uint32_t err) {
     if (err & PSG_ERR_NS_OVERFLOW) {
-        const unsigned long long used = s->h_status->ns_used[0];
-        const uint32_t fail = s->h_status->ns_fail;
+        const unsigned long long used = s->h_status->run.ns_used;
+        const uint32_t fail = s->h_status->run.ns_fail;
         const int kf = fail ? __builtin_ctz(fail) : kMaxDepth;
         const unsigned long long limit =
             std::min(0xFFFFFFF0ull, store_budget(s->ns_cap * 4) / 4);
@@ -663,6 +674,11 @@ static int regrow(State* s, uint32_t err) {
             // what the run reserved fits, twice that does not: the largest
             // store, and the levels below show whether it is enough
             done = try_alloc_ns(s, limit);
+        }
+        if (!done && s->order == 0 && !s->level_by_level) {
+            // which level is the first that does not fit: run level by level
+            s->level_by_level = true;
+            done = true;
         }
         if (!done && s->order == 0 && kf - 1 >= floor_k) {
             s->ns_levels = kf - 1;
@@ -689,13 +705,13 @@ static int regrow(State* s, uint32_t err) {
             const unsigned long long need = (unsigned long long)used + used / 4 + 1024;
             return (uint32_t)std::min<unsigned long long>(need, 0x7FFFFFFFull);
         };
-        int r = alloc_dense(s, room(s->h_status->dense_count, s->dense.rec_cap),
-                            room(s->h_status->dense_slots, s->dense.slot_cap));
+        int r = alloc_dense(s, room(s->h_status->run.dense_count, s->dense.rec_cap),
+                            room(s->h_status->run.dense_slots, s->dense.slot_cap));
         if (r != PSG_OK) return r;
     }
     if (err & PSG_ERR_P2P_OVERFLOW) {
         // the chunk counter is 32-bit: below the capacity it has wrapped
-        const unsigned long long used = s->h_status->p2p_chunks;
+        const unsigned long long used = s->h_status->run.p2p_chunks;
         const unsigned long long need = used < s->p2p.cap_chunks ? ~0ull : 2 * used + 1024;
         const unsigned long long per = kP2PChunk * 5 + 8;
         const unsigned long long limit =
@@ -709,7 +725,7 @@ static int regrow(State* s, uint32_t err) {
 // P2P chunk store and reruns when a capacity flag comes back
 static int run_traversal(State* s, const float4* xyzm, float* fx, float* fy, float* fz,
                          uint32_t* err_out) {
-    for (int attempt = 0; attempt < 6; ++attempt) {
+    for (int attempt = 0; attempt < 8; ++attempt) {
         s->attempts = attempt + 1;
         int r0 = enqueue_traversal(s, xyzm, fx, fy, fz);
         if (r0 != PSG_OK) return r0;
@@ -734,7 +750,7 @@ static int run_traversal(State* s, const float4* xyzm, float* fx, float* fy, flo
         }
         if (s->timing) cudaEventRecord(s->ev[PH_UP], s->stream);
     }
-    std::snprintf(g_err, sizeof(g_err), "traversal stores still too small after 6 runs");
+    std::snprintf(g_err, sizeof(g_err), "traversal stores still too small after 8 runs");
     return PSG_EOOM;
 }
 
@@ -836,7 +852,8 @@ static int tick_core(State* s, const DevArrays& d, size_t n, float cx, float cy,
     launch_tree(d.codes, n, s->tree_tiles, s->tv, s->d_status, cx, cy, cz, hw, gt, st, bbox,
                 s->leaf_cap);
     record(s, PH_TREE);
-    launch_upward(s->tv, s->d_status, s->xyzm, gt, st);
+    launch_upward(s->tv, s->d_status, s->xyzm, n, st);
+    s->trav_fresh = true;
     record(s, PH_UP);
     PSG_CHECK(cudaGetLastError());
     uint32_t err = 0;
@@ -862,11 +879,11 @@ static int tick_core(State* s, const DevArrays& d, size_t n, float cx, float cy,
         }
     }
     if (err & (PSG_ERR_SORT_SPIN | PSG_ERR_STACK | PSG_ERR_NODES | PSG_ERR_HEAVY_OVERFLOW |
-               PSG_ERR_CHAIN_ORDER)) {
+               PSG_ERR_CHAIN_ORDER | PSG_ERR_READY_SPIN)) {
         if (judge) cudaStreamSynchronize(cj.side);
         const bool nodes = (err & PSG_ERR_NODES) &&
                            !(err & (PSG_ERR_SORT_SPIN | PSG_ERR_STACK | PSG_ERR_HEAVY_OVERFLOW |
-                                    PSG_ERR_CHAIN_ORDER));
+                                    PSG_ERR_CHAIN_ORDER | PSG_ERR_READY_SPIN));
         std::snprintf(g_err, sizeof(g_err), nodes ? "morton codes not sorted/30-bit (0x%x)"
                                                   : "device status error 0x%x", err);
         return nodes ? PSG_EINVAL : PSG_EDEVICE;
@@ -919,10 +936,10 @@ static int tick_core(State* s, const DevArrays& d, size_t n, float cx, float cy,
     s->stats[8] = nodes;
     s->stats[9] = s->h_status->max_stack;
     for (int i = 8; i < 16; ++i) s->stats[i + 8] = s->h_status->stat[i];
-    s->stats[10] = s->h_status->p2p_chunks;
+    s->stats[10] = s->h_status->run.p2p_chunks;
     s->stats[11] = (unsigned long long)s->attempts;
     s->stats[12] = s->h_status->max_leaf;
-    s->stats[13] = s->h_status->dense_count;
+    s->stats[13] = s->h_status->run.dense_count;
     s->stats[14] = (unsigned long long)near_levels(s);
     s->stats[15] = (s->stream_p2p || s->force_stream) ? 1ull : 0ull;
     if (s->timing) {
@@ -1209,11 +1226,13 @@ static int upload_systems(Ensemble* e) {
     std::vector<float> th2(e->nsys);
     std::vector<int32_t> hv(e->nsys), sp(e->nsys);
     int hmax = 0, smax = 0;
+    bool dense_only = true;
     for (size_t k = 0; k < e->nsys; ++k) {
         const float t = e->theta[k];
         th2[k] = t * t;
         hv[k] = heavy_depth_of(t, e->count[k]);
         hmax = std::max(hmax, (int)hv[k]);
+        dense_only = dense_only && e->cap[k] >= kDenseCap;
         sp[k] = split_depth_of(t, e->count[k], e->cap[k]);
         smax = std::max(smax, (int)sp[k]);
     }
@@ -1223,7 +1242,8 @@ static int upload_systems(Ensemble* e) {
     PSG_CHECK(cudaMemcpy(e->sys_cap, e->cap.data(), e->nsys * 4, cudaMemcpyHostToDevice));
     if (hmax != e->fs->forest_heavy) e->dirty = true;  // a launch parameter changes
     e->fs->forest_heavy = hmax;
-    if (smax != e->fs->forest_split) e->dirty = true;
+    if (smax != e->fs->forest_split || dense_only != e->fs->dense_only) e->dirty = true;
+    e->fs->dense_only = dense_only;
     e->fs->forest_split = smax;
     const SplitStore before = e->fs->split;  // (allocated here: not while capturing)
     const int r = ensure_split(e->fs, smax);
@@ -1231,9 +1251,9 @@ static int upload_systems(Ensemble* e) {
     if (before.sums != e->fs->split.sums) e->dirty = true;
     // the stores' near-list depth and P2P mode start over with the settings
     // (both are launch parameters of the captured graphs)
-    if (e->fs->ns_levels != kMaxDepth || e->fs->stream_p2p) e->dirty = true;
-    e->fs->ns_levels = kMaxDepth;
-    e->fs->stream_p2p = 0;
+    if (e->fs->ns_levels != kMaxDepth || e->fs->stream_p2p || e->fs->level_by_level)
+        e->dirty = true;
+    reset_near_levels(e->fs);
     return PSG_OK;
 }
 
@@ -1263,7 +1283,8 @@ static int enqueue_forest_forces(Ensemble* e, const DevArrays& d) {
     const int gt = (int)((s->tv.lvl_base[kLevels] + 255) / 256);
     launch_tree(d.codes, n, s->tree_tiles, s->tv, s->d_status, 0.f, 0.f, 0.f, 0.f, gt, st,
                 nullptr, 1);
-    launch_upward(s->tv, s->d_status, s->xyzm, gt, st);
+    launch_upward(s->tv, s->d_status, s->xyzm, n, st);
+    s->trav_fresh = true;
     s->trav_n = n;
     int r = enqueue_traversal(s, s->xyzm, d.fx, d.fy, d.fz);
     if (r != PSG_OK) return r;
@@ -1337,7 +1358,7 @@ static int ensure_graphs(Ensemble* e, const DevArrays& a, float* const v[3], flo
 static int check_forest(Ensemble* e, const DevArrays& a) {
     State* s = e->fs;
     const uint32_t err = s->h_status->err;
-    if (err & (PSG_ERR_SORT_SPIN | PSG_ERR_STACK | PSG_ERR_NODES | PSG_ERR_CHAIN_ORDER)) {
+    if (err & (PSG_ERR_SORT_SPIN | PSG_ERR_STACK | PSG_ERR_NODES | PSG_ERR_CHAIN_ORDER | PSG_ERR_READY_SPIN)) {
         std::snprintf(g_err, sizeof(g_err), "ensemble: device status 0x%x", err);
         return (err & PSG_ERR_NODES) ? PSG_EINVAL : PSG_EDEVICE;
     }
