@@ -33,7 +33,11 @@ constexpr int kTreeThreads = 256;
 constexpr int kTreePer = 4;
 constexpr int kTreeTile = kTreeThreads * kTreePer;  // 1024 positions
 
-int tree_tile_size() { return kTreeTile; }
+// bytes of the build's scratch: counts per tile and depth, flags per position
+size_t tree_scratch_bytes(size_t n) {
+    const size_t tiles = (n + kTreeTile - 1) / kTreeTile;
+    return tiles * (kMaxDepth * sizeof(uint32_t) + kTreeTile * sizeof(unsigned short));
+}
 
 __device__ __forceinline__ int cpl2(uint32_t a, uint32_t b) {
     // common octal prefix length of two codes (0 .. 10)
@@ -42,9 +46,10 @@ __device__ __forceinline__ int cpl2(uint32_t a, uint32_t b) {
     return (__clz(x) - 2) / 3;
 }
 
-__device__ __forceinline__ int cpl_at(const uint32_t* __restrict__ c, size_t i, size_t n) {
-    // common octal prefix length of codes[i-1], codes[i]; -1 outside [1, n)
-    if (i == 0 || i >= n) return -1;
+__device__ __forceinline__ int cpl_at(const uint32_t* __restrict__ c, size_t i, size_t lo,
+                                      size_t hi) {
+    // common octal prefix length of codes[i-1], codes[i]; -1 outside (lo, hi)
+    if (i <= lo || i >= hi) return -1;
     return cpl2(c[i - 1], c[i]);
 }
 
@@ -76,28 +81,30 @@ __device__ __forceinline__ uint32_t get_cnt(unsigned long long lo, unsigned long
                   : (uint32_t)((hi >> (12 * (d - 6))) & 0xFFFull);
 }
 
-__device__ __forceinline__ void thread_flags(const uint32_t* __restrict__ codes, size_t n,
-                                             size_t p0, uint32_t cap,
+// the flags of the positions p0 .. p0 + kTreePer - 1 of the system whose
+// particles are [lo, hi)
+__device__ __forceinline__ void thread_flags(const uint32_t* __restrict__ codes, size_t lo,
+                                             size_t hi, size_t p0, uint32_t cap,
                                              uint32_t (&f)[kTreePer]) {
-    int cprev = cpl_at(codes, p0, n);
+    int cprev = cpl_at(codes, p0, lo, hi);
     if (cap <= 1u) {
         // W(i) = max(cpl(i), cpl(i+1))
 #pragma unroll
         for (int q = 0; q < kTreePer; ++q) {
             size_t i = p0 + q;
-            int cnext = cpl_at(codes, i + 1, n);
-            f[q] = (i < n) ? node_flags(cprev, max(cprev, cnext), i == 0) : 0u;
+            int cnext = cpl_at(codes, i + 1, lo, hi);
+            f[q] = (i < hi) ? node_flags(cprev, max(cprev, cnext), i == lo) : 0u;
             cprev = cnext;
         }
         return;
     }
     // W over the windows [j, j + cap] with j in [p0 - cap, p0 + kTreePer - 1],
-    // 0 <= j and j + cap < n; at least 0 (the root is split) once n >= 2
+    // lo <= j and j + cap < hi; at least 0 (the root is split) once it holds 2
     int w[kTreePer];
 #pragma unroll
-    for (int q = 0; q < kTreePer; ++q) w[q] = n >= 2 ? 0 : -1;
-    const long long jlo = max(0ll, (long long)p0 - (long long)cap);
-    const long long jhi = min((long long)p0 + kTreePer - 1, (long long)n - 1 - (long long)cap);
+    for (int q = 0; q < kTreePer; ++q) w[q] = hi - lo >= 2 ? 0 : -1;
+    const long long jlo = max((long long)lo, (long long)p0 - (long long)cap);
+    const long long jhi = min((long long)p0 + kTreePer - 1, (long long)hi - 1 - (long long)cap);
 #pragma unroll 4
     for (long long j = jlo; j <= jhi; ++j) {
         const int c = cpl2(codes[j], codes[j + cap]);
@@ -110,8 +117,8 @@ __device__ __forceinline__ void thread_flags(const uint32_t* __restrict__ codes,
 #pragma unroll
     for (int q = 0; q < kTreePer; ++q) {
         size_t i = p0 + q;
-        f[q] = (i < n) ? node_flags(cprev, w[q], i == 0) : 0u;
-        cprev = cpl_at(codes, i + 1, n);
+        f[q] = (i < hi) ? node_flags(cprev, w[q], i == lo) : 0u;
+        cprev = cpl_at(codes, i + 1, lo, hi);
     }
 }
 
@@ -121,42 +128,38 @@ __device__ __forceinline__ void thread_flags(const uint32_t* __restrict__ codes,
 __device__ __forceinline__ void thread_flags_forest(const uint32_t* __restrict__ codes, size_t n,
                                                     size_t p0, const TreeView& tv,
                                                     uint32_t (&f)[kTreePer]) {
+    if (p0 + kTreePer <= n) {
+        const uint32_t k = tv.part_sys[p0];
+        if (tv.part_sys[p0 + kTreePer - 1] == k) {
+            thread_flags(codes, tv.sys_off[k], tv.sys_off[k + 1], p0, tv.sys_cap[k], f);
+            return;
+        }
+    }
 #pragma unroll 1
     for (int q = 0; q < kTreePer; ++q) {
         const size_t i = p0 + q;
-        if (i >= n) {
-            f[q] = 0u;
-            continue;
-        }
+        f[q] = 0u;
+        if (i >= n) continue;
         const uint32_t k = tv.part_sys[i];
-        const size_t lo = tv.sys_off[k], hi = tv.sys_off[k + 1];
-        const uint32_t cap = tv.sys_cap[k];
-        const bool first = i == lo;
-        const int cpl_i = first ? -1 : cpl2(codes[i - 1], codes[i]);
-        int w;
-        if (cap <= 1u) {
-            const int cnext = i + 1 < hi ? cpl2(codes[i], codes[i + 1]) : -1;
-            w = max(cpl_i, cnext);
-        } else {
-            w = hi - lo >= 2 ? 0 : -1;
-            const size_t jlo = i >= lo + cap ? i - cap : lo;
-            if (hi >= lo + cap + 1) {
-                const size_t jhi = min(i, hi - 1 - cap);
-                for (size_t j = jlo; j <= jhi; ++j) w = max(w, cpl2(codes[j], codes[j + cap]));
-            }
-        }
-        f[q] = node_flags(cpl_i, w, first);
+        uint32_t g[kTreePer];
+        thread_flags(codes, tv.sys_off[k], tv.sys_off[k + 1], i, tv.sys_cap[k], g);
+        f[q] = g[0];
     }
 }
 
+// The flags of every position, and per tile the nodes that start in it at
+// each depth.
 __global__ void __launch_bounds__(kTreeThreads) k_tree_count(const uint32_t* __restrict__ codes,
                                                             size_t n, uint32_t cap,
                                                             uint32_t* __restrict__ tile_cnt,
+                                                            ushort4* __restrict__ flags,
                                                             const TreeView tv) {
     const size_t p0 = (size_t)blockIdx.x * kTreeTile + (size_t)threadIdx.x * kTreePer;
     uint32_t f[kTreePer];
     if (tv.part_sys) thread_flags_forest(codes, n, p0, tv, f);
-    else thread_flags(codes, n, p0, cap, f);
+    else thread_flags(codes, 0, n, p0, cap, f);
+    flags[p0 / kTreePer] = make_ushort4((unsigned short)f[0], (unsigned short)f[1],
+                                        (unsigned short)f[2], (unsigned short)f[3]);
     unsigned long long lo = 0, hi = 0;
 #pragma unroll
     for (int q = 0; q < kTreePer; ++q) add_flags(lo, hi, f[q]);
@@ -176,64 +179,53 @@ __global__ void __launch_bounds__(kTreeThreads) k_tree_count(const uint32_t* __r
     }
 }
 
-// Exclusive scan of the tile counts per depth (one block of 1024 threads).
+// a level's node count, held to its capacity
+__device__ __forceinline__ uint32_t level_count(const TreeView& tv, Status* status, int d,
+                                                uint32_t total) {
+    if (total > tv.lvl_cap[d]) {
+        set_err(status, PSG_ERR_NODES);
+        total = tv.lvl_cap[d];
+    }
+    return total;
+}
+
+// Exclusive scan of the tile counts, one block of 1024 threads per depth (one
+// block for all depths took 12 us at 1M, where this takes 4).
 __global__ void __launch_bounds__(1024) k_tree_scan(uint32_t* __restrict__ tile_cnt, int tiles,
                                                     TreeView tv, Status* status) {
     __shared__ uint32_t wsum[32];
-    __shared__ uint32_t carry;
-    for (int d = 1; d <= kMaxDepth; ++d) {
-        if (threadIdx.x == 0) carry = 0;
+    const int d = blockIdx.x + 1;
+    const uint32_t w = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (int b0 = 0; b0 < tiles; b0 += 1024) {
+        const int b = b0 + threadIdx.x;
+        const uint32_t v = b < tiles ? tile_cnt[(size_t)b * kMaxDepth + d - 1] : 0u;
+        const uint32_t inc = warp_incl_scan(v);
+        if (lane_id() == 31) wsum[w] = inc;
         __syncthreads();
-        for (int b0 = 0; b0 < tiles; b0 += 1024) {
-            int b = b0 + threadIdx.x;
-            uint32_t v = b < tiles ? tile_cnt[(size_t)b * kMaxDepth + d - 1] : 0u;
-            uint32_t inc = warp_incl_scan(v);
-            if (lane_id() == 31) wsum[threadIdx.x >> 5] = inc;
-            __syncthreads();
-            uint32_t add = carry;
-            for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) add += wsum[w];
-            if (b < tiles) tile_cnt[(size_t)b * kMaxDepth + d - 1] = inc - v + add;
-            __syncthreads();
-            if (threadIdx.x == 1023) carry = add + inc;
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) {
-            uint32_t total = carry;
-            if (total > tv.lvl_cap[d]) {
-                set_err(status, PSG_ERR_NODES);
-                total = tv.lvl_cap[d];
-            }
-            status->lvl_count[d] = total;
-        }
+        const uint32_t ws = wsum[lane_id()];
+        const uint32_t wi = warp_incl_scan(ws);
+        const uint32_t add = carry + __shfl_sync(0xFFFFFFFFu, wi - ws, w);
+        if (b < tiles) tile_cnt[(size_t)b * kMaxDepth + d - 1] = inc - v + add;
+        carry += __shfl_sync(0xFFFFFFFFu, wi, 31);
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        status->lvl_count[0] = tv.part_sys ? tv.nsys : 1u;
-        status->lvl_count[kLevels] = 0;
+        status->lvl_count[d] = level_count(tv, status, d, carry);
+        if (d == 1) {
+            status->lvl_count[0] = tv.part_sys ? tv.nsys : 1u;
+            status->lvl_count[kLevels] = 0;
+        }
     }
 }
 
-// centre of the node whose first code is `code` at depth d: the reference's
-// chain of d rounded adds from the root centre
-__device__ __forceinline__ float4 node_centre(uint32_t code, int d, float cx, float cy, float cz,
-                                              float hw) {
-    for (int l = 1; l <= d; ++l) {
-        hw = __fmul_rn(hw, 0.5f);
-        uint32_t dig = (code >> (30 - 3 * l)) & 7u;
-        cx = __fadd_rn(cx, (dig & 1u) ? hw : -hw);
-        cy = __fadd_rn(cy, (dig & 2u) ? hw : -hw);
-        cz = __fadd_rn(cz, (dig & 4u) ? hw : -hw);
-    }
-    return make_float4(cx, cy, cz, hw);
-}
-
-// end of the run of codes sharing code[i]'s first d octal digits (gallop,
-// then binary search)
+// end of the run of codes sharing code[i]'s first d octal digits, at least
+// up to position `from` (gallop, then binary search)
 __device__ __forceinline__ size_t run_end(const uint32_t* __restrict__ c, size_t n, size_t i,
-                                          int d) {
+                                          size_t from, int d) {
     const int sh = 30 - 3 * d;
     const uint32_t key = (c[i] & 0x3FFFFFFFu) >> sh;
-    size_t lo = i, step = 1;  // invariant: prefix(c[lo]) == key
+    size_t lo = from, step = 1;  // invariant: prefix(c[lo]) == key
     while (lo + step < n && ((c[lo + step] & 0x3FFFFFFFu) >> sh) == key) {
         lo += step;
         step <<= 1;
@@ -246,14 +238,23 @@ __device__ __forceinline__ size_t run_end(const uint32_t* __restrict__ c, size_t
     return hi;
 }
 
+// Nodes.  A depth-d node that starts at i ends where the next node of depth <= d
+// starts (or its system ends), which the block looks up in its tile's flags; only
+// a node that runs past the tile searches the codes.  Up to kSelfScanTiles tiles
+// every block adds up the tile counts before it itself (no k_tree_scan).
+// Measured (whole build; flags computed twice, a scan of all depths in one block
+// and a search of the codes per node / now): 1K 48 / 34 us, 33K 56 / 44 us, 1M
+// 144 / 130 us, 4M 379 / 317 us.
+constexpr int kSelfScanTiles = 64;
+
 __global__ void __launch_bounds__(kTreeThreads) k_tree_emit(const uint32_t* __restrict__ codes,
-                                                           size_t n,
+                                                           size_t n, int tiles,
                                                            const uint32_t* __restrict__ tile_off,
-                                                           TreeView tv, const Status* status,
+                                                           const ushort4* __restrict__ flags,
+                                                           TreeView tv, Status* status,
                                                            float cx, float cy, float cz,
                                                            float hw,
-                                                           const float* __restrict__ bbox,
-                                                           uint32_t cap) {
+                                                           const float* __restrict__ bbox) {
     if (bbox) {
         // root from a device-side bounding box (min, max, range), as the
         // caller's loop derives it: c = min + range / 2, hw = range / 2
@@ -264,11 +265,31 @@ __global__ void __launch_bounds__(kTreeThreads) k_tree_emit(const uint32_t* __re
     const size_t p0 = (size_t)blockIdx.x * kTreeTile + (size_t)threadIdx.x * kTreePer;
     uint32_t f[kTreePer];
     const bool forest = tv.part_sys != nullptr;
-    if (forest) thread_flags_forest(codes, n, p0, tv, f);
-    else thread_flags(codes, n, p0, cap, f);
+    {
+        const ushort4 v = flags[p0 / kTreePer];
+        f[0] = v.x;
+        f[1] = v.y;
+        f[2] = v.z;
+        f[3] = v.w;
+    }
     unsigned long long lo = 0, hi = 0;
 #pragma unroll
     for (int q = 0; q < kTreePer; ++q) add_flags(lo, hi, f[q]);
+    // the shallowest depth that starts at each position (11: none), and its
+    // minimum over a thread's and a warp's positions
+    __shared__ uint8_t s_md[kTreeTile], s_tmd[kTreeThreads], s_wmd[kTreeThreads / 32];
+    {
+        uint32_t m = kMaxDepth + 1;
+#pragma unroll
+        for (int q = 0; q < kTreePer; ++q) {
+            const uint32_t md = f[q] ? __ffs(f[q]) : kMaxDepth + 1;
+            s_md[threadIdx.x * kTreePer + q] = (uint8_t)md;
+            m = min(m, md);
+        }
+        s_tmd[threadIdx.x] = (uint8_t)m;
+        m = __reduce_min_sync(0xFFFFFFFFu, m);
+        if (lane_id() == 0) s_wmd[threadIdx.x >> 5] = (uint8_t)m;
+    }
     // block exclusive scan of the packed counters
     unsigned long long ilo = lo, ihi = hi;
     const uint32_t l = lane_id(), w = threadIdx.x >> 5;
@@ -282,14 +303,65 @@ __global__ void __launch_bounds__(kTreeThreads) k_tree_emit(const uint32_t* __re
         }
     }
     __shared__ unsigned long long s[2][kTreeThreads / 32];
-    __shared__ uint32_t s_off[kMaxDepth + 1];
+    __shared__ uint32_t s_off[kMaxDepth + 1], s_lvl[kMaxDepth + 1];
+    const bool self = tiles <= kSelfScanTiles;
+    if (threadIdx.x <= kMaxDepth) s_off[threadIdx.x] = s_lvl[threadIdx.x] = 0;
     if (l == 31) {
         s[0][w] = ilo;
         s[1][w] = ihi;
     }
-    if (threadIdx.x < kMaxDepth)
-        s_off[threadIdx.x + 1] = tile_off[(size_t)blockIdx.x * kMaxDepth + threadIdx.x];
     __syncthreads();
+    if (self) {
+        constexpr int kParts = kTreeThreads / kMaxDepth;  // 25 threads per depth
+        const int d = threadIdx.x % kMaxDepth, part = threadIdx.x / kMaxDepth;
+        uint32_t before = 0, all = 0;
+        if (part < kParts) {
+            for (int b = part; b < tiles; b += kParts) {
+                const uint32_t v = tile_off[(size_t)b * kMaxDepth + d];
+                all += v;
+                if (b < (int)blockIdx.x) before += v;
+            }
+            if (before) atomicAdd(&s_off[d + 1], before);
+            if (all) atomicAdd(&s_lvl[d + 1], all);
+        }
+        __syncthreads();
+        if (threadIdx.x < kMaxDepth) {
+            const int dd = threadIdx.x + 1;
+            const uint32_t c = min(s_lvl[dd], tv.lvl_cap[dd]);
+            if (blockIdx.x == 0) status->lvl_count[dd] = level_count(tv, status, dd, s_lvl[dd]);
+            s_lvl[dd] = c;
+        }
+        if (blockIdx.x == 0 && threadIdx.x == kMaxDepth) {
+            status->lvl_count[0] = forest ? tv.nsys : 1u;
+            status->lvl_count[kLevels] = 0;
+        }
+    } else if (threadIdx.x < kMaxDepth) {
+        s_off[threadIdx.x + 1] = tile_off[(size_t)blockIdx.x * kMaxDepth + threadIdx.x];
+        s_lvl[threadIdx.x + 1] = status->lvl_count[threadIdx.x + 1];
+    }
+    __syncthreads();
+    // the tile position after li at which a node of depth <= d starts
+    // (kTreeTile: none), position by position to the thread's end, thread by
+    // thread to the warp's, and down again
+    auto next_start = [&](int li, int d) -> int {
+        int j = li + 1;
+        for (; j & (kTreePer - 1); ++j)
+            if (s_md[j] <= d) return j;
+        int t = j / kTreePer;
+        for (; t < kTreeThreads && (t & 31) && s_tmd[t] > d; ++t) {
+        }
+        if (t < kTreeThreads && !(t & 31)) {
+            int w2 = t >> 5;
+            while (w2 < kTreeThreads / 32 && s_wmd[w2] > d) ++w2;
+            if (w2 == kTreeThreads / 32) return kTreeTile;
+            for (t = w2 * 32; s_tmd[t] > d; ++t) {
+            }
+        }
+        if (t >= kTreeThreads) return kTreeTile;
+        for (j = t * kTreePer; s_md[j] > d; ++j) {
+        }
+        return j;
+    };
     unsigned long long elo = ilo - lo, ehi = ihi - hi;
     for (uint32_t j = 0; j < w; ++j) {
         elo += s[0][j];
@@ -335,19 +407,31 @@ __global__ void __launch_bounds__(kTreeThreads) k_tree_emit(const uint32_t* __re
         if (fq) {
             const uint32_t code = codes[i];
             const size_t run_n = forest ? tv.sys_off[sys + 1] : n;
+            // centre and half width down the code's digits: the reference's
+            // chain of rounded adds from the root centre
+            float4 g = make_float4(cx, cy, cz, hw);
 #pragma unroll 1
             for (int d = 1; d <= kMaxDepth; ++d) {
+                const uint32_t dig = (code >> (30 - 3 * d)) & 7u;
+                g.w = __fmul_rn(g.w, 0.5f);
+                g.x = __fadd_rn(g.x, (dig & 1u) ? g.w : -g.w);
+                g.y = __fadd_rn(g.y, (dig & 2u) ? g.w : -g.w);
+                g.z = __fadd_rn(g.z, (dig & 4u) ? g.w : -g.w);
                 if (!((fq >> (d - 1)) & 1u)) continue;
                 const uint32_t id = rank[d];
-                if (id - tv.lvl_base[d] >= status->lvl_count[d]) continue;  // capacity guard
-                const size_t end = run_end(codes, run_n, i, d);
+                if (id - tv.lvl_base[d] >= s_lvl[d]) continue;  // capacity guard
+                const int ne = next_start((int)threadIdx.x * kTreePer + q, d);
+                const size_t tile_end = (size_t)blockIdx.x * kTreeTile + (size_t)ne;
+                size_t end = tile_end < run_n ? tile_end : run_n;
+                if (ne == kTreeTile && tile_end < run_n)
+                    end = run_end(codes, run_n, i, tile_end - 1, d);
                 const uint32_t cnt = (uint32_t)(end - i);
                 uint32_t par = forest ? sys : 0u;
                 if (d > 1) par = rank[d - 1] + ((fq >> (d - 2)) & 1u) - 1u;
                 const uint32_t cb = d < kMaxDepth ? rank[d + 1] : 0u;
-                tv.geo[id] = node_centre(code, d, cx, cy, cz, hw);
+                tv.geo[id] = g;
                 tv.info[id] = make_uint4((uint32_t)i, cnt, cb,
-                                         pack_flags(0, d, (code >> (30 - 3 * d)) & 7u));
+                                         pack_flags(0, d, dig));
                 tv.parent[id] = par;
                 tv.cbase[id] = cb;
                 tv.arrive[id] = 0;
@@ -479,10 +563,12 @@ void launch_tree(const uint32_t* codes, size_t n, uint32_t* tile_buf, TreeView t
                  Status* status, float cx, float cy, float cz, float hw, int grid,
                  cudaStream_t st, const float* bbox, uint32_t leaf_cap) {
     const int tiles = (int)((n + kTreeTile - 1) / kTreeTile);
-    k_tree_count<<<tiles, kTreeThreads, 0, st>>>(codes, n, leaf_cap, tile_buf, tv);
-    k_tree_scan<<<1, 1024, 0, st>>>(tile_buf, tiles, tv, status);
-    k_tree_emit<<<tiles, kTreeThreads, 0, st>>>(codes, n, tile_buf, tv, status, cx, cy, cz, hw,
-                                                bbox, leaf_cap);
+    ushort4* const flags = (ushort4*)(tile_buf + (size_t)tiles * kMaxDepth);
+    k_tree_count<<<tiles, kTreeThreads, 0, st>>>(codes, n, leaf_cap, tile_buf, flags, tv);
+    if (tiles > kSelfScanTiles)
+        k_tree_scan<<<kMaxDepth, 1024, 0, st>>>(tile_buf, tiles, tv, status);
+    k_tree_emit<<<tiles, kTreeThreads, 0, st>>>(codes, n, tiles, tile_buf, flags, tv, status, cx,
+                                                cy, cz, hw, bbox);
     k_tree_link<<<grid, 256, 0, st>>>(tv, status);
 }
 

@@ -29,8 +29,7 @@ struct SortBuffers {
     uint32_t* val_a;
     uint32_t* val_b;
     uint32_t* hist;      // [4][256]
-    uint32_t* offs;      // [4][256]
-    uint32_t* lookback;  // [4][tiles][256]
+    uint32_t* lookback;  // [passes][tiles][256], right after hist
     uint32_t* perm;      // output: val_a after the last pass
 };
 int sort_tile_size();
@@ -41,7 +40,12 @@ void launch_sort(SortBuffers& b, uint32_t* codes, size_t n, int grid, Status* st
 // sys_passes passes)
 void launch_sort_forest(SortBuffers& b, uint32_t* codes, size_t n, int grid, Status* status,
                         cudaStream_t st, const uint32_t* part_sys, int sys_passes,
-                        const uint32_t* sys_offs);
+                        const uint32_t* sys_hist);
+// the sort, gather and write-back of a small system in one block
+cudaError_t prepare_sort_small();
+bool sort_small_fits(size_t n);
+void launch_sort_small(uint32_t* codes, size_t n, float* x, float* y, float* z, float* m,
+                       uint32_t* id, float4* xyzm, uint32_t* ids, cudaStream_t st);
 void launch_gather(const uint32_t* perm, const float* x, const float* y, const float* z,
                    const float* m, const uint32_t* id, size_t n, float4* xyzm, uint32_t* ids,
                    int grid, cudaStream_t st);
@@ -49,7 +53,7 @@ void launch_writeback(const float4* xyzm, const uint32_t* ids, size_t n, float* 
                       float* z, float* m, uint32_t* id, int grid, cudaStream_t st);
 
 // k_tree.cu -- octree build (polesitter.h:906-967) + upward pass (:971-1046)
-int tree_tile_size();
+size_t tree_scratch_bytes(size_t n);
 void launch_tree(const uint32_t* codes, size_t n, uint32_t* tile_buf, TreeView tv,
                  Status* status, float cx, float cy, float cz, float hw, int grid,
                  cudaStream_t st, const float* bbox = nullptr, uint32_t leaf_cap = 1);

@@ -51,10 +51,15 @@ constexpr int kPhases = 9;  // timing events
 enum Phase { PH_SORT = 0, PH_GATHER, PH_TREE, PH_UP, PH_TRAV, PH_END, PH_BEGIN, PH_CLOSURE,
              PH_DENSE };
 
+// device mirrors of host arrays: one block of 9 rows of cap elements, in the
+// order x y z m id codes fx fy fz; stage: pinned rows that a small call's
+// pageable arrays pass through
 struct Mirror {
     float *x, *y, *z, *m, *fx, *fy, *fz;
     uint32_t *id, *codes;
     size_t cap;
+    uint32_t* stage;
+    size_t stage_cap;
 };
 
 // the learned closure's device buffers (allocated when it is first enabled)
@@ -125,7 +130,7 @@ struct State {
     size_t early_bytes = 0;
     bool early_issued = false;
     cudaStream_t copy_out = nullptr;
-    cudaEvent_t ev_written = nullptr, ev_copied = nullptr;
+    cudaEvent_t ev_written = nullptr;
     int heavy_depth;       // option; < 0: derived from theta
     int forest_heavy;      // many systems: the deepest of their shallow-leaf depths
     int ns_levels;         // near lists are stored for node depths <= this (kMaxDepth: all);
@@ -251,54 +256,74 @@ static int alloc_heavy(State* s, uint32_t cap) {
     return PSG_OK;
 }
 
-static int ensure_mirror(Mirror& mi, size_t n) {
-    if (mi.cap >= n) return PSG_OK;
-    void** ps[9] = {(void**)&mi.x, (void**)&mi.y, (void**)&mi.z, (void**)&mi.m, (void**)&mi.fx,
-                    (void**)&mi.fy, (void**)&mi.fz, (void**)&mi.id, (void**)&mi.codes};
-    for (auto p : ps) {
-        if (*p) cudaFree(*p);
-        *p = nullptr;
-    }
-    for (auto p : ps) {
-        cudaError_t e = cudaMalloc(p, n * 4 ? n * 4 : 16);
-        if (e != cudaSuccess) {
-            note("cudaMalloc mirror", e);
-            return PSG_EALLOC;
-        }
-    }
-    mi.cap = n;
-    return PSG_OK;
-}
-
 static void free_mirror(Mirror& mi) {
-    void* ps[9] = {mi.x, mi.y, mi.z, mi.m, mi.fx, mi.fy, mi.fz, mi.id, mi.codes};
-    for (auto p : ps)
-        if (p) cudaFree(p);
+    if (mi.x) cudaFree(mi.x);
+    if (mi.stage) cudaFreeHost(mi.stage);
     std::memset(&mi, 0, sizeof(mi));
 }
 
-// true when the GPU can dereference p (device or managed memory)
-static bool pinned_host(const void* p) {
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
+static int ensure_mirror(Mirror& mi, size_t n) {
+    if (mi.cap >= n && mi.x) return PSG_OK;
+    free_mirror(mi);
+    const size_t cap = n ? n : 4;
+    float* base = nullptr;
+    const cudaError_t e = cudaMalloc((void**)&base, 9 * cap * 4);
+    if (e != cudaSuccess) {
+        note("cudaMalloc mirror", e);
+        return PSG_EALLOC;
     }
-    return a.type == cudaMemoryTypeHost;
+    mi.x = base;
+    mi.y = base + cap;
+    mi.z = base + 2 * cap;
+    mi.m = base + 3 * cap;
+    mi.id = (uint32_t*)(base + 4 * cap);
+    mi.codes = (uint32_t*)(base + 5 * cap);
+    mi.fx = base + 6 * cap;
+    mi.fy = base + 7 * cap;
+    mi.fz = base + 8 * cap;
+    mi.cap = cap;
+    return PSG_OK;
 }
 
-static bool on_device(const void* p) {
+// Up to this many particles, pageable arrays go through pinned rows in one copy
+// each way: with a pageable copy per array (19 a tick, the ones back each
+// waiting for the GPU) a 1K tick took 390 us, so it takes 245.  Above it the
+// copies themselves are the cost, and the driver's staging does them.
+constexpr size_t kStageMax = 32768;
+
+static int ensure_stage(Mirror& mi, size_t n) {
+    if (mi.stage_cap >= n) return PSG_OK;
+    if (mi.stage) cudaFreeHost(mi.stage);
+    mi.stage = nullptr;
+    mi.stage_cap = 0;
+    const cudaError_t e = cudaMallocHost((void**)&mi.stage, 9 * n * 4);
+    if (e != cudaSuccess) {
+        note("cudaMallocHost stage", e);
+        return PSG_EALLOC;
+    }
+    mi.stage_cap = n;
+    return PSG_OK;
+}
+
+// where p lives: device (or managed) memory, pinned or pageable host memory
+enum Place { PAGEABLE = 0, PINNED, DEVICE };
+
+static Place place_of(const void* p) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return PAGEABLE;
     }
-    return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+    if (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged) return DEVICE;
+    return a.type == cudaMemoryTypeHost ? PINNED : PAGEABLE;
 }
+
+// true when the GPU can dereference p (device or managed memory)
+static bool on_device(const void* p) { return place_of(p) == DEVICE; }
 
 static void free_state(State* s) {
     void* ps[] = {s->xyzm, s->ids, s->sort.key_a, s->sort.key_b, s->sort.val_a, s->sort.val_b,
-                  s->sort.hist, s->sort.offs, s->sort.lookback, s->tree_tiles, s->tv.geo,
+                  s->sort.hist, s->tree_tiles, s->tv.geo,
                   s->tv.mp, s->tv.lt, s->tv.info, s->tv.parent, s->tv.arrive, s->tv.cbase,
                   s->tv.ns_off, s->tv.ns_cnt, s->tv.dbg_m2l, s->tv.dbg_p2p, s->tv.link,
                   s->tv.ready, s->ns, s->p2p.src, s->p2p.mask, s->p2p.next, s->p2p.cnt,
@@ -329,7 +354,6 @@ static void free_state(State* s) {
         cudaStreamDestroy(s->copy_out);
     }
     if (s->ev_written) cudaEventDestroy(s->ev_written);
-    if (s->ev_copied) cudaEventDestroy(s->ev_copied);
     if (s->stream) cudaStreamDestroy(s->stream);
     s->magic = 0;
 }
@@ -353,12 +377,11 @@ static int init_state(State* s, size_t maxp, float theta, const uint32_t* lvl_ca
     PSG_ALLOC(s->sort.key_b, n * 4);
     PSG_ALLOC(s->sort.val_a, n * 4);
     PSG_ALLOC(s->sort.val_b, n * 4);
-    PSG_ALLOC(s->sort.hist, 4 * 256 * 4);
-    PSG_ALLOC(s->sort.offs, 4 * 256 * 4);
     const size_t stiles = (n + sort_tile_size() - 1) / sort_tile_size();
-    PSG_ALLOC(s->sort.lookback, (size_t)sort_passes * stiles * 256 * 4);
-    const size_t ttiles = (n + tree_tile_size() - 1) / tree_tile_size();
-    PSG_ALLOC(s->tree_tiles, ttiles * kMaxDepth * 4);
+    PSG_ALLOC(s->sort.hist, ((size_t)sort_passes * stiles + 4) * 256 * 4);
+    s->sort.lookback = s->sort.hist + 4 * 256;
+    PSG_CHECK(prepare_sort_small());
+    PSG_ALLOC(s->tree_tiles, tree_scratch_bytes(n));
     // level capacities: min(8^d, n) nodes at depth d
     uint32_t base = 0;
     for (int d = 0; d <= kMaxDepth; ++d) {
@@ -759,51 +782,72 @@ static int run_traversal(State* s, const float4* xyzm, float* fx, float* fy, flo
 struct DevArrays {
     float *x, *y, *z, *m, *fx, *fy, *fz;
     uint32_t *id, *codes;
-    bool dev[9];
+    bool dev[9];      // (rows as in Mirror) no copy back is due
+    bool pinned[9];
     bool any_host;
+    bool staged;      // all through the mirror's pinned rows
 };
 
 static int map_arrays(State* s, const psg_arrays_t* a, DevArrays& d, bool upload_codes) {
     const size_t n = a->n;
     d.x = a->x; d.y = a->y; d.z = a->z; d.m = a->mass;
     d.fx = a->fx; d.fy = a->fy; d.fz = a->fz; d.id = a->id; d.codes = a->codes;
-    void* ps[9] = {d.x, d.y, d.z, d.m, d.fx, d.fy, d.fz, d.id, d.codes};
+    void* const ps[9] = {d.x, d.y, d.z, d.m, d.id, d.codes, d.fx, d.fy, d.fz};
     d.any_host = false;
+    d.staged = n <= kStageMax;
     for (int i = 0; i < 9; ++i) {
-        d.dev[i] = on_device(ps[i]);
-        d.any_host |= !d.dev[i];
+        const Place p = place_of(ps[i]);
+        d.dev[i] = p == DEVICE;
+        d.pinned[i] = p == PINNED;
+        d.any_host |= p != DEVICE;
+        d.staged &= p == PAGEABLE;
     }
     if (!d.any_host) return PSG_OK;
-    int r = ensure_mirror(s->mir, s->max_particles);
+    Mirror& mi = s->mir;
+    int r = ensure_mirror(mi, s->max_particles);
+    if (r == PSG_OK && d.staged) r = ensure_stage(mi, std::min(s->max_particles, kStageMax));
     if (r != PSG_OK) return r;
-    struct { void* h; void* dv; bool in; } io[9] = {
-        {a->x, s->mir.x, true}, {a->y, s->mir.y, true}, {a->z, s->mir.z, true},
-        {a->mass, s->mir.m, true}, {a->fx, s->mir.fx, false}, {a->fy, s->mir.fy, false},
-        {a->fz, s->mir.fz, false}, {a->id, s->mir.id, true}, {a->codes, s->mir.codes, upload_codes}};
-    for (int i = 0; i < 9; ++i)
-        if (!d.dev[i] && io[i].in)
-            PSG_CHECK(cudaMemcpyAsync(io[i].dv, io[i].h, n * 4, cudaMemcpyHostToDevice, s->stream));
-    if (!d.dev[0]) d.x = s->mir.x;
-    if (!d.dev[1]) d.y = s->mir.y;
-    if (!d.dev[2]) d.z = s->mir.z;
-    if (!d.dev[3]) d.m = s->mir.m;
-    if (!d.dev[4]) d.fx = s->mir.fx;
-    if (!d.dev[5]) d.fy = s->mir.fy;
-    if (!d.dev[6]) d.fz = s->mir.fz;
-    if (!d.dev[7]) d.id = s->mir.id;
-    if (!d.dev[8]) d.codes = s->mir.codes;
+    void* const rows[9] = {mi.x, mi.y, mi.z, mi.m, mi.id, mi.codes, mi.fx, mi.fy, mi.fz};
+    const int in = upload_codes ? 6 : 5;
+    if (d.staged) {
+        for (int i = 0; i < in; ++i) std::memcpy(mi.stage + (size_t)i * n, ps[i], n * 4);
+        PSG_CHECK(cudaMemcpy2DAsync(mi.x, mi.cap * 4, mi.stage, n * 4, n * 4, in,
+                                    cudaMemcpyHostToDevice, s->stream));
+    } else {
+        for (int i = 0; i < in; ++i)
+            if (!d.dev[i])
+                PSG_CHECK(cudaMemcpyAsync(rows[i], ps[i], n * 4, cudaMemcpyHostToDevice,
+                                          s->stream));
+    }
+    if (!d.dev[0]) d.x = mi.x;
+    if (!d.dev[1]) d.y = mi.y;
+    if (!d.dev[2]) d.z = mi.z;
+    if (!d.dev[3]) d.m = mi.m;
+    if (!d.dev[4]) d.id = mi.id;
+    if (!d.dev[5]) d.codes = mi.codes;
+    if (!d.dev[6]) d.fx = mi.fx;
+    if (!d.dev[7]) d.fy = mi.fy;
+    if (!d.dev[8]) d.fz = mi.fz;
     return PSG_OK;
 }
 
+// the results back into the caller's host arrays, final when this returns
 static int unmap_arrays(State* s, const psg_arrays_t* a, const DevArrays& d) {
-    if (!d.any_host) return PSG_OK;
-    struct { void* h; void* dv; } out[9] = {
-        {a->x, d.x}, {a->y, d.y}, {a->z, d.z}, {a->mass, d.m}, {a->fx, d.fx},
-        {a->fy, d.fy}, {a->fz, d.fz}, {a->id, d.id}, {a->codes, d.codes}};
-    for (int i = 0; i < 9; ++i)
+    const size_t n = a->n;
+    Mirror& mi = s->mir;
+    void* const hs[9] = {a->x, a->y, a->z, a->mass, a->id, a->codes, a->fx, a->fy, a->fz};
+    if (d.staged && d.any_host) {
+        PSG_CHECK(cudaMemcpy2DAsync(mi.stage, n * 4, mi.x, mi.cap * 4, n * 4, 9,
+                                    cudaMemcpyDeviceToHost, s->stream));
+        PSG_CHECK(cudaStreamSynchronize(s->stream));
+        for (int i = 0; i < 9; ++i) std::memcpy(hs[i], mi.stage + (size_t)i * n, n * 4);
+        return PSG_OK;
+    }
+    const void* const ds[9] = {d.x, d.y, d.z, d.m, d.id, d.codes, d.fx, d.fy, d.fz};
+    for (int i = 0; d.any_host && i < 9; ++i)
         if (!d.dev[i])
-            PSG_CHECK(cudaMemcpyAsync(out[i].h, out[i].dv, a->n * 4, cudaMemcpyDeviceToHost,
-                                      s->stream));
+            PSG_CHECK(cudaMemcpyAsync(hs[i], ds[i], n * 4, cudaMemcpyDeviceToHost, s->stream));
+    PSG_CHECK(cudaStreamSynchronize(s->stream));
     return PSG_OK;
 }
 
@@ -816,17 +860,21 @@ static int tick_core(State* s, const DevArrays& d, size_t n, float cx, float cy,
     record(s, PH_BEGIN);
     PSG_CHECK(cudaMemsetAsync(s->d_status, 0, sizeof(Status), st));
     const int g = grid_for(s, n, 1024);
-    launch_sort(s->sort, d.codes, n, g, s->d_status, st, s->sort_spin_limit);
-    record(s, PH_SORT);
-    launch_gather(s->sort.perm, d.x, d.y, d.z, d.m, d.id, n, s->xyzm, s->ids, g, st);
-    launch_writeback(s->xyzm, s->ids, n, d.x, d.y, d.z, d.m, d.id, g, st);
+    if (sort_small_fits(n) && s->sort_spin_limit == 0) {
+        launch_sort_small(d.codes, n, d.x, d.y, d.z, d.m, d.id, s->xyzm, s->ids, st);
+        record(s, PH_SORT);
+    } else {
+        launch_sort(s->sort, d.codes, n, g, s->d_status, st, s->sort_spin_limit);
+        record(s, PH_SORT);
+        launch_gather(s->sort.perm, d.x, d.y, d.z, d.m, d.id, n, s->xyzm, s->ids, g, st);
+        launch_writeback(s->xyzm, s->ids, n, d.x, d.y, d.z, d.m, d.id, g, st);
+    }
     if (s->n_early && !s->early_issued) {
         PSG_CHECK(cudaEventRecord(s->ev_written, st));
         PSG_CHECK(cudaStreamWaitEvent(s->copy_out, s->ev_written, 0));
         for (int k = 0; k < s->n_early; ++k)
             PSG_CHECK(cudaMemcpyAsync(s->early[k].h, s->early[k].dv, s->early_bytes,
                                       cudaMemcpyDeviceToHost, s->copy_out));
-        PSG_CHECK(cudaEventRecord(s->ev_copied, s->copy_out));
         s->early_issued = true;
     }
     record(s, PH_GATHER);
@@ -971,34 +1019,29 @@ static int calc(State* s, const psg_arrays_t* a, float cx, float cy, float cz, f
     if (d.any_host) {
         void* const hs[6] = {a->x, a->y, a->z, a->mass, a->id, a->codes};
         const void* const ds[6] = {d.x, d.y, d.z, d.m, d.id, d.codes};
-        const int which[6] = {0, 1, 2, 3, 7, 8};
         for (int k = 0; k < 6; ++k) {
-            if (d.dev[which[k]] || !pinned_host(hs[k])) continue;
+            if (d.dev[k] || !d.pinned[k]) continue;
             s->early[s->n_early++] = State::EarlyCopy{hs[k], ds[k]};
-            d.dev[which[k]] = true;  // (unmap_arrays skips it)
+            d.dev[k] = true;  // (unmap_arrays skips it)
         }
         if (s->n_early && !s->copy_out) {
             PSG_CHECK(cudaStreamCreateWithFlags(&s->copy_out, cudaStreamNonBlocking));
             PSG_CHECK(cudaEventCreateWithFlags(&s->ev_written, cudaEventDisableTiming));
-            PSG_CHECK(cudaEventCreateWithFlags(&s->ev_copied, cudaEventDisableTiming));
         }
     }
     r = tick_core(s, d, n, cx, cy, cz, hw, nullptr);
     if (r == PSG_OK) r = unmap_arrays(s, a, d);
     if (s->early_issued) {
-        // the forces' copies and the tick's end wait for the early copies too
-        const cudaError_t e = cudaStreamWaitEvent(s->stream, s->ev_copied, 0);
+        // the early copies are done too when the call returns
+        const cudaError_t e = cudaStreamSynchronize(s->copy_out);
         if (e != cudaSuccess && r == PSG_OK) {
-            note("cudaStreamWaitEvent", e);
+            note("cudaStreamSynchronize copy_out", e);
             r = PSG_EDEVICE;
         }
-        cudaStreamSynchronize(s->copy_out);
     }
     s->n_early = 0;
     s->early_issued = false;
-    if (r != PSG_OK) return r;
-    PSG_CHECK(cudaStreamSynchronize(s->stream));
-    return PSG_OK;
+    return r;
 }
 
 // `ticks` iterations of the caller's loop (README.md:65-111) without leaving
@@ -1063,10 +1106,7 @@ static int run_ticks(State* s, const psg_arrays_t* a, float* vx, float* vy, floa
         if (vdst[c] != vh[c])
             PSG_CHECK(cudaMemcpyAsync(vh[c], vdst[c], n * 4, cudaMemcpyDeviceToHost, st));
     }
-    r = unmap_arrays(s, a, d);
-    if (r != PSG_OK) return r;
-    PSG_CHECK(cudaStreamSynchronize(st));
-    return PSG_OK;
+    return unmap_arrays(s, a, d);  // (and all before it)
 }
 
 // ---- process-wide workspace of ps_prepare_particles (it takes no context) ----
@@ -1110,23 +1150,43 @@ static int prepare(const psg_arrays_t* a, float* out_min, float* out_max, float*
     cudaStream_t st = g_prep.stream;
     const float* x = a->x; const float* y = a->y; const float* z = a->z;
     uint32_t* codes = a->codes;
-    const bool dx = on_device(x), dy = on_device(y), dz = on_device(z), dc = on_device(codes);
-    if (!(dx && dy && dz && dc)) {
-        int r = ensure_mirror(g_prep.mir, n);
+    Mirror& mi = g_prep.mir;
+    const void* const hs[3] = {x, y, z};
+    const Place at[4] = {place_of(x), place_of(y), place_of(z), place_of(codes)};
+    const bool dc = at[3] == DEVICE;
+    // (pageable arrays of a small call: as in map_arrays)
+    const bool staged = n <= kStageMax && at[0] == PAGEABLE && at[1] == PAGEABLE &&
+                        at[2] == PAGEABLE && at[3] == PAGEABLE;
+    if (!(at[0] == DEVICE && at[1] == DEVICE && at[2] == DEVICE && dc)) {
+        int r = ensure_mirror(mi, n);
+        if (r == PSG_OK && staged) r = ensure_stage(mi, n);
         if (r != PSG_OK) return r;
-        if (!dx) { PSG_CHECK(cudaMemcpyAsync(g_prep.mir.x, x, n * 4, cudaMemcpyHostToDevice, st)); x = g_prep.mir.x; }
-        if (!dy) { PSG_CHECK(cudaMemcpyAsync(g_prep.mir.y, y, n * 4, cudaMemcpyHostToDevice, st)); y = g_prep.mir.y; }
-        if (!dz) { PSG_CHECK(cudaMemcpyAsync(g_prep.mir.z, z, n * 4, cudaMemcpyHostToDevice, st)); z = g_prep.mir.z; }
-        if (!dc) codes = g_prep.mir.codes;
+        float* const rows[3] = {mi.x, mi.y, mi.z};
+        if (staged) {
+            for (int i = 0; i < 3; ++i) std::memcpy(mi.stage + (size_t)i * n, hs[i], n * 4);
+            PSG_CHECK(cudaMemcpy2DAsync(mi.x, mi.cap * 4, mi.stage, n * 4, n * 4, 3,
+                                        cudaMemcpyHostToDevice, st));
+        } else {
+            for (int i = 0; i < 3; ++i)
+                if (at[i] != DEVICE)
+                    PSG_CHECK(cudaMemcpyAsync(rows[i], hs[i], n * 4, cudaMemcpyHostToDevice, st));
+        }
+        if (at[0] != DEVICE) x = mi.x;
+        if (at[1] != DEVICE) y = mi.y;
+        if (at[2] != DEVICE) z = mi.z;
+        if (!dc) codes = mi.codes;
     }
     int grid = (int)((n + 1023) / 1024);
     if (grid > g_prep.grid) grid = g_prep.grid;
     if (grid < 1) grid = 1;
     launch_prepare(x, y, z, n, g_prep.partial, grid, codes, g_prep.bbox, variant, st);
     PSG_CHECK(cudaGetLastError());
-    if (!dc) PSG_CHECK(cudaMemcpyAsync(a->codes, codes, n * 4, cudaMemcpyDeviceToHost, st));
+    if (!dc)
+        PSG_CHECK(cudaMemcpyAsync(staged ? mi.stage : a->codes, codes, n * 4,
+                                  cudaMemcpyDeviceToHost, st));
     PSG_CHECK(cudaMemcpyAsync(g_prep.h_bbox, g_prep.bbox, 4 * sizeof(float), cudaMemcpyDeviceToHost, st));
     PSG_CHECK(cudaStreamSynchronize(st));
+    if (staged) std::memcpy(a->codes, mi.stage, n * 4);
     if (out_min) *out_min = g_prep.h_bbox[0];
     if (out_max) *out_max = g_prep.h_bbox[1];
     if (out_range) *out_range = g_prep.h_bbox[2];
@@ -1171,7 +1231,7 @@ struct Ensemble {
     int32_t* sys_split = nullptr;
     float* sys_bbox = nullptr;      // [nsys][4]
     uint32_t* sys_maxleaf = nullptr;
-    uint32_t* sys_sort_offs = nullptr;  // digit starts of the system sort passes
+    uint32_t* sys_sort_hist = nullptr;  // digit counts of the system sort passes
     int sys_passes = 1;
     uint4* blk = nullptr;           // prepare blocks: (system, first, end)
     uint32_t* sys_blk = nullptr;    // [nsys + 1]
@@ -1277,7 +1337,7 @@ static int enqueue_forest_forces(Ensemble* e, const DevArrays& d) {
     PSG_CHECK(cudaMemsetAsync(s->d_status, 0, sizeof(Status), st));
     PSG_CHECK(cudaMemsetAsync(e->sys_maxleaf, 0, e->nsys * 4, st));
     launch_sort_forest(s->sort, d.codes, n, g, s->d_status, st, e->part_sys, e->sys_passes,
-                       e->sys_sort_offs);
+                       e->sys_sort_hist);
     launch_gather(s->sort.perm, d.x, d.y, d.z, d.m, d.id, n, s->xyzm, s->ids, g, st);
     launch_writeback(s->xyzm, s->ids, n, d.x, d.y, d.z, d.m, d.id, g, st);
     const int gt = (int)((s->tv.lvl_base[kLevels] + 255) / 256);
@@ -1408,7 +1468,7 @@ static void free_ensemble(Ensemble* e) {
         e->fs = nullptr;
     }
     void* ps[] = {e->part_sys, e->sys_off, e->sys_cap, e->sys_theta2, e->sys_heavy,
-                  e->sys_split, e->sys_bbox, e->sys_maxleaf, e->sys_sort_offs, e->blk, e->sys_blk,
+                  e->sys_split, e->sys_bbox, e->sys_maxleaf, e->sys_sort_hist, e->blk, e->sys_blk,
                   e->partial, e->vtmp};
     for (void* p : ps)
         if (p) cudaFree(p);
@@ -1475,19 +1535,11 @@ static int ens_create(Ensemble* e, const size_t* counts, size_t nsys, const floa
     soff[nsys] = (uint32_t)e->total;
     sblk[nsys] = (uint32_t)blk.size();
     e->nblk = (int)blk.size();
-    // digit starts of the system passes: the systems are contiguous, so a
-    // digit's start is where its first system starts (low byte pass: systems
-    // grouped by their low byte)
+    // digit counts of the system passes, from the system sizes
     std::vector<uint32_t> so(256 * e->sys_passes, 0u);
-    for (int q = 0; q < e->sys_passes; ++q) {
-        std::vector<unsigned long long> hist(256, 0ull);
-        for (size_t k = 0; k < nsys; ++k) hist[(k >> (8 * q)) & 0xFFu] += counts[k];
-        unsigned long long run = 0;
-        for (int dgt = 0; dgt < 256; ++dgt) {
-            so[256 * q + dgt] = (uint32_t)run;
-            run += hist[dgt];
-        }
-    }
+    for (int q = 0; q < e->sys_passes; ++q)
+        for (size_t k = 0; k < nsys; ++k)
+            so[256 * q + ((k >> (8 * q)) & 0xFFu)] += (uint32_t)counts[k];
     PSG_ALLOC(e->part_sys, e->total * 4);
     PSG_ALLOC(e->sys_off, (nsys + 1) * 4);
     PSG_ALLOC(e->sys_cap, nsys * 4);
@@ -1496,14 +1548,14 @@ static int ens_create(Ensemble* e, const size_t* counts, size_t nsys, const floa
     PSG_ALLOC(e->sys_split, nsys * 4);
     PSG_ALLOC(e->sys_bbox, nsys * 16);
     PSG_ALLOC(e->sys_maxleaf, nsys * 4);
-    PSG_ALLOC(e->sys_sort_offs, so.size() * 4);
+    PSG_ALLOC(e->sys_sort_hist, so.size() * 4);
     PSG_ALLOC(e->blk, blk.size() * sizeof(uint4));
     PSG_ALLOC(e->sys_blk, (nsys + 1) * 4);
     PSG_ALLOC(e->partial, blk.size() * sizeof(float2));
     PSG_ALLOC(e->vtmp, 3 * e->total * sizeof(float));
     PSG_CHECK(cudaMemcpy(e->part_sys, psys.data(), e->total * 4, cudaMemcpyHostToDevice));
     PSG_CHECK(cudaMemcpy(e->sys_off, soff.data(), (nsys + 1) * 4, cudaMemcpyHostToDevice));
-    PSG_CHECK(cudaMemcpy(e->sys_sort_offs, so.data(), so.size() * 4, cudaMemcpyHostToDevice));
+    PSG_CHECK(cudaMemcpy(e->sys_sort_hist, so.data(), so.size() * 4, cudaMemcpyHostToDevice));
     PSG_CHECK(cudaMemcpy(e->blk, blk.data(), blk.size() * sizeof(uint4), cudaMemcpyHostToDevice));
     PSG_CHECK(cudaMemcpy(e->sys_blk, sblk.data(), (nsys + 1) * 4, cudaMemcpyHostToDevice));
     TreeView& tv = e->fs->tv;
@@ -1524,7 +1576,7 @@ static int ens_create(Ensemble* e, const size_t* counts, size_t nsys, const floa
 
 static int ens_run(Ensemble* e, const psg_arrays_t* a, float* const v[3], float dt,
                    uint32_t ticks) {
-    DevArrays d;
+    DevArrays d{};
     int r = ens_map(e, a, d);
     if (r != PSG_OK) return r;
     for (int c = 0; c < 3; ++c) {
@@ -1559,7 +1611,7 @@ static int ens_run(Ensemble* e, const psg_arrays_t* a, float* const v[3], float 
 // the caller's arrays are left as they are.
 static int ens_autotune(Ensemble* e, const psg_arrays_t* a, float target, float* theta_out,
                         double* scale_out) {
-    DevArrays d;
+    DevArrays d{};
     int r = ens_map(e, a, d);
     if (r != PSG_OK) return r;
     PSG_CHECK(cudaSetDevice(e->device));
@@ -1567,7 +1619,7 @@ static int ens_autotune(Ensemble* e, const psg_arrays_t* a, float target, float*
     const size_t T = e->total;
     float* buf = nullptr;  // scratch copy: x y z m fx fy fz (7 T floats), id, codes
     PSG_ALLOC(buf, (size_t)9 * T * 4 + 16);
-    DevArrays c;
+    DevArrays c{};
     c.x = buf; c.y = buf + T; c.z = buf + 2 * T; c.m = buf + 3 * T;
     c.fx = buf + 4 * T; c.fy = buf + 5 * T; c.fz = buf + 6 * T;
     c.id = (uint32_t*)(buf + 7 * T); c.codes = (uint32_t*)(buf + 8 * T);
