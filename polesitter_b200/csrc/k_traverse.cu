@@ -71,8 +71,9 @@ constexpr uint32_t kDenseSwitch = 32;     // fullest leaf from which the DENSE l
 enum { MODE_INTERNAL = 0, MODE_LEAF = 1 };
 
 struct SmemInternal {
-    float4 cgeo[8];  // the group's children: centre + half width
+    float4 cgeo[8];  // the targets: centre + half width
     float4 cgp[4][2];  // ... pair-packed for the MAC (cgp_put)
+    uint8_t tq[8];     // ... and which of the group's children each is
     uint32_t cand_node[kCandBuf];
     uint32_t ns_cnt[8];
     uint32_t dbg_m2l[8];
@@ -83,6 +84,7 @@ struct SmemInternal {
 struct SmemLeaf {
     float4 cgeo[8];
     float4 cgp[4][2];
+    uint8_t tq[8];
     float4 chain_geo[8];    // chain groups: the ancestors a_{K+1} .. p under test
     float4 sL[8];           // the children's local fields
     float4 sG0[8];          // closure order 1: the children's field gradients
@@ -368,20 +370,21 @@ __device__ __forceinline__ void p2p_range(const float4* __restrict__ xyzm, uint2
     }
 }
 
-// STREAM: the P2P sums of the staged sources [0, pfill) for every target
-// particle of the work item's leaf children (tgt_mask), computed where they
-// are found instead of spilled to HBM, so that no store grows with the size
-// of a source list.  The children's particles are enumerated flat (children
-// in mask order), 32 at a time; T lanes own targets (T the smallest power of
-// two >= their count) and the 32 / T slices of lanes split the staged source
-// leaves.  The slices' sums are added in a fixed order and kept in the force
-// arrays between flushes (accum: add to what an earlier flush of this item
-// left there).  fin: the item's last flush, which also applies L2P,
-// F = m (L + all P2P sums), with order 1's shift to the particle.
+// The P2P sums of the staged sources [0, pfill), and of the chain phead of
+// spilled ones, for every target particle of the work item's leaf children
+// (tgt_mask).  The children's particles are enumerated flat (children in mask
+// order), 32 at a time; T lanes own targets (T the smallest power of two >=
+// their count) and the 32 / T slices of lanes split the source leaves; the
+// slices' sums are added in a fixed order.  fin: also L2P, F = m (L + all P2P
+// sums), with order 1's shift to the particle.
+// STREAM: the sums are taken when the stage is full instead of spilling it to
+// HBM, so that no store grows with the size of a source list; they are kept in
+// the force arrays between flushes (accum: add to what an earlier flush of
+// this item left there; fin: the item's last flush).
 template <bool DEBUG, bool GRAD>
 __device__ __noinline__ void stream_p2p(SmemLeaf& sm, const TravArgs& o, uint32_t tgt_mask,
-                                        uint32_t fc, uint32_t pfill, bool accum, bool fin,
-                                        unsigned long long& inter) {
+                                        uint32_t fc, uint32_t pfill, uint32_t phead, bool accum,
+                                        bool fin, unsigned long long& inter) {
     const uint32_t lane = lane_id();
     for (uint32_t e = lane; e < pfill; e += 32) {
         const uint4 si = o.tv.info[sm.p2p_node[e]];
@@ -417,6 +420,16 @@ __device__ __noinline__ void stream_p2p(SmemLeaf& sm, const TravArgs& o, uint32_
                 used += r.y;
             }
         }
+        for (uint32_t c = phead; c != kNone; c = o.p2p.next[c]) {
+            const uint32_t n = o.p2p.cnt[c];
+            for (uint32_t e = slice; e < n; e += S) {
+                if ((o.p2p.mask[(size_t)c * kP2PChunk + e] >> q) & 1u) {
+                    const uint4 si = o.tv.info[o.p2p.src[(size_t)c * kP2PChunk + e]];
+                    p2p_range(o.xyzm, make_uint2(si.x, si.y), t, o.kahan, bx, by, bz, cx, cy, cz);
+                    used += si.y;
+                }
+            }
+        }
         bx -= cx;
         by -= cy;
         bz -= cz;
@@ -446,7 +459,7 @@ __device__ __noinline__ void stream_p2p(SmemLeaf& sm, const TravArgs& o, uint32_
                     lx += sh.x;
                     ly += sh.y;
                     lz += sh.z;
-                    if (o.leaf_of) o.leaf_of[i] = fc + q;
+                    if (o.leaf_of) o.leaf_of[i] = fc + sm.tq[q];
                 }
                 const double mm = (double)t.w;
                 o.fx[i] = (float)(mm * ((double)lx + (double)bx));
@@ -460,112 +473,32 @@ __device__ __noinline__ void stream_p2p(SmemLeaf& sm, const TravArgs& o, uint32_
 
 // L2P + P2P of a group's leaf children once its candidates are done: with
 // DENSE, every group is handed to k_dense_p2p (which adds L and the P2P sum);
-// otherwise F = m (L + P2P sum) here, one target particle at a time with the
-// lanes over its sources.
+// otherwise, and where the P2P is streamed, F = m (L + P2P sum) here.
 template <bool DEBUG, bool GRAD, bool DENSE>
 __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const TravArgs& o, uint32_t tgt_mask,
                                            uint32_t fc, uint32_t pfill, uint32_t phead,
                                            bool stream, bool flushed,
-                                           unsigned long long inter0) {
+                                           unsigned long long inter) {
     const uint32_t lane = lane_id();
     Status* status = o.status;
-    if (stream) {
-        // the staged remainder, then L2P, in the warp (no spill, no records)
-        unsigned long long inter = inter0;
-        stream_p2p<DEBUG, GRAD>(sm, o, tgt_mask, fc, pfill, flushed, true, inter);
+    if (!DENSE || stream) {
+        stream_p2p<DEBUG, GRAD>(sm, o, tgt_mask, fc, pfill, phead, flushed, true, inter);
         if (DEBUG) {
-            if (lane == 0) {
-                for (uint32_t m = tgt_mask; m; m &= m - 1) {
-                    const uint32_t q = __ffs(m) - 1;
-                    o.tv.dbg_p2p[fc + q] = sm.dbg_p2p[q];
-                    atomicAdd(&status->stat[PSG_STAT_P2P_PAIRS],
-                              (unsigned long long)sm.dbg_p2p[q]);
-                }
-            }
             inter = warp_sum(inter);
             if (lane == 0) atomicAdd(&status->stat[PSG_STAT_P2P_INTER], inter);
         }
-        __syncwarp();
-        return;
-    }
-    if constexpr (DENSE) {
+    } else {
         // the group's whole source list to HBM chunks, then k_dense_p2p work
         // records of up to kDenseTargets target particles
         if (pfill) phead = spill_p2p(sm, pfill, phead, o, tgt_mask, fc, true);
         record_dense(sm, o.dense, tgt_mask, fc, phead, true, false, status);
-        if (DEBUG && lane == 0) {
-            for (uint32_t m = tgt_mask; m; m &= m - 1) {
-                const uint32_t q = __ffs(m) - 1;
-                o.tv.dbg_p2p[fc + q] = sm.dbg_p2p[q];
-                atomicAdd(&status->stat[PSG_STAT_P2P_PAIRS], (unsigned long long)sm.dbg_p2p[q]);
-            }
-        }
-        __syncwarp();
-        return;
     }
-    // ---- L2P + P2P: F = m * (L(u) + sum of u's P2P sources) ----
-    for (uint32_t e = lane; e < pfill; e += 32) {
-        const uint4 si = o.tv.info[sm.p2p_node[e]];
-        sm.p2p_range[e] = make_uint2(si.x, si.y);
-    }
-    __syncwarp();
-    unsigned long long inter = 0;
-#pragma unroll 1
-    for (uint32_t m = tgt_mask; m; m &= m - 1) {
-        const uint32_t q = __ffs(m) - 1;
-        const uint2 up = sm.cpart[q];
-        const float4 L = sm.sL[q];
-        for (uint32_t ti = 0; ti < up.y; ++ti) {
-            const float4 t = o.xyzm[up.x + ti];
-            float bx = 0.f, by = 0.f, bz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-            for (uint32_t e = lane; e < pfill; e += 32) {
-                if ((sm.p2p_mask[e] >> q) & 1u) {
-                    const uint2 r = sm.p2p_range[e];
-                    p2p_range(o.xyzm, r, t, o.kahan, bx, by, bz, cx, cy, cz);
-                    if (DEBUG) inter += r.y;
-                }
-            }
-            for (uint32_t c = phead; c != kNone; c = o.p2p.next[c]) {
-                if (lane < o.p2p.cnt[c] &&
-                    ((o.p2p.mask[(size_t)c * kP2PChunk + lane] >> q) & 1u)) {
-                    const uint4 si = o.tv.info[o.p2p.src[(size_t)c * kP2PChunk + lane]];
-                    p2p_range(o.xyzm, make_uint2(si.x, si.y), t, o.kahan, bx, by, bz,
-                              cx, cy, cz);
-                    if (DEBUG) inter += si.y;
-                }
-            }
-            const float sx = warp_sum(bx - cx);
-            const float sy = warp_sum(by - cy);
-            const float sz = warp_sum(bz - cz);
-            if (lane == 0) {
-                // final per-particle accumulation in FP64
-                const size_t gi = (size_t)up.x + ti;
-                const double mm = (double)t.w;
-                float lx = L.y, ly = L.z, lz = L.w;
-                if constexpr (GRAD) {
-                    // order-1 L2P: the field at the particle
-                    const float4 cu = sm.cgeo[q];
-                    const float3 sh = grad_apply(sm.sG0[q], sm.sG1[q], t.x - cu.x,
-                                                 t.y - cu.y, t.z - cu.z);
-                    lx += sh.x;
-                    ly += sh.y;
-                    lz += sh.z;
-                    if (o.leaf_of) o.leaf_of[gi] = fc + q;
-                }
-                o.fx[gi] = (float)(mm * ((double)lx + (double)sx));
-                o.fy[gi] = (float)(mm * ((double)ly + (double)sy));
-                o.fz[gi] = (float)(mm * ((double)lz + (double)sz));
-            }
+    if (DEBUG && lane == 0) {
+        for (uint32_t m = tgt_mask; m; m &= m - 1) {
+            const uint32_t q = __ffs(m) - 1;
+            o.tv.dbg_p2p[fc + sm.tq[q]] = sm.dbg_p2p[q];
+            atomicAdd(&status->stat[PSG_STAT_P2P_PAIRS], (unsigned long long)sm.dbg_p2p[q]);
         }
-        if (DEBUG && lane == 0) {
-            o.tv.dbg_p2p[fc + q] = sm.dbg_p2p[q];
-            atomicAdd(&status->stat[PSG_STAT_P2P_PAIRS],
-                      (unsigned long long)sm.dbg_p2p[q]);
-        }
-    }
-    if (DEBUG) {
-        inter = warp_sum(inter);
-        if (lane == 0) atomicAdd(&status->stat[PSG_STAT_P2P_INTER], inter);
     }
     __syncwarp();
 }
@@ -598,8 +531,12 @@ __device__ __noinline__ bool wait_ready(const uint32_t* flag, Status* status) {
 // XL (leaf pass only): the variant that also serves chain groups and
 // streamed P2P, launched only when the near lists stop short of the deepest
 // level or the P2P is streamed, so the other variants keep their registers.
-// The plain sparse leaf variant (the reference's tree and far field) keeps
-// 7 blocks per SM (72 registers), the order-1 leaf variants 4 (128).
+// Blocks per SM, measured: the plain sparse leaf variant (the reference's tree
+// and far field) 7 (72 registers; 5, 6 and 8 took a 1M tick's leaf pass from
+// 1.43 to 1.62, 1.48 and 1.70 ms), the order-1 leaf variants 4 (128; 3 and 5 took
+// a 1M closure tick's from 4.35 to 4.70 and 5.14 ms), the internal levels 5, with
+// order 1 4 (3, 4, 5 blocks: 0.49, 0.50, 0.45 ms of a 1M plain tick, 0.24, 0.26,
+// 0.30 of a 131K closure tick).
 // SPLIT (leaf pass only): the groups of the depths < split_depth, whose leaves'
 // walks reach a large part of the tree, kSplitParts warps each (every warp
 // takes every kSplitParts-th candidate and what lies below it), on trees of
@@ -610,9 +547,12 @@ enum { VAR_PLAIN = 0, VAR_XL = 1, VAR_SPLIT = 2 };
 template <int MODE, bool DEBUG, bool GRAD, bool DENSE, int VAR>
 __global__ void __launch_bounds__(
     kTravThreads,
-    (MODE == MODE_LEAF && !DEBUG && VAR != VAR_XL) ? (GRAD ? 4 : (DENSE ? 1 : 7)) : 1)
+    (DEBUG || VAR == VAR_XL) ? 1
+    : MODE == MODE_INTERNAL  ? (GRAD ? 4 : 5)
+                             : (GRAD ? 4 : (DENSE ? 1 : 7)))
     k_trav(const __grid_constant__ TravArgs A) {
     constexpr bool XL = VAR == VAR_XL, SPLIT = VAR == VAR_SPLIT;
+    constexpr bool COMPACT = MODE == MODE_INTERNAL || !DENSE;
     using Smem = typename SmemOf<MODE>::T;
     __shared__ Smem smem[kTravWarps];
     const uint32_t lane = lane_id();
@@ -640,9 +580,9 @@ __global__ void __launch_bounds__(
     // a work item is (group, half)
     constexpr uint32_t SL = GRAD ? 4u : 8u;
     constexpr uint32_t NH = 8u / SL;
-    // work items: MODE_INTERNAL = the (halves of the) nodes at depth k-1;
-    // MODE_LEAF = those of the nodes at depths shallow..9, level after level
-    // (SPLIT: at depths 0..shallow-1, each kSplitParts times)
+    // work items: MODE_INTERNAL = the (halves of the) internal nodes at depth
+    // k-1; MODE_LEAF = those at depths shallow..9, level after level (SPLIT: at
+    // depths 0..shallow-1, each kSplitParts times)
     uint32_t cum[kMaxDepth + 1];
     uint32_t total = 0;
     uint32_t* work;
@@ -650,7 +590,7 @@ __global__ void __launch_bounds__(
 #pragma unroll
         for (int d = 0; d < kMaxDepth; ++d) {
             cum[d] = total;
-            if (d + 1 >= A.level && d < A.level_end) total += status->lvl_count[d] * NH;
+            if (d + 1 >= A.level && d < A.level_end) total += status->group_count[d] * NH;
         }
         cum[kMaxDepth] = total;
         work = &status->run.work[A.level];
@@ -659,7 +599,7 @@ __global__ void __launch_bounds__(
         for (int d = 0; d < kMaxDepth; ++d) {
             cum[d] = total;
             if ((d < A.shallow) == SPLIT)
-                total += status->lvl_count[d] * NH * (SPLIT ? kSplitParts : 1u);
+                total += status->group_count[d] * NH * (SPLIT ? kSplitParts : 1u);
         }
         cum[kMaxDepth] = total;
         // batched systems run both variants over all groups, each with its
@@ -676,9 +616,9 @@ __global__ void __launch_bounds__(
         }
     }
     __syncwarp();
-    // items taken per atomic: whole work queues are a few items per warp, so
-    // the leaf pass takes them one by one (a batch would leave warps idle)
-    const uint32_t batch = MODE == MODE_INTERNAL ? 4u : 1u;
+    // items taken per atomic: one, since whole work queues are a few items per
+    // warp (4 at a time cost the internal levels of a 65K tick 70 of 104 us)
+    constexpr uint32_t batch = 1u;
     const uint32_t items = total;
 
     for (;;) {
@@ -707,13 +647,12 @@ __global__ void __launch_bounds__(
                     part = k % kSplitParts;
                     k /= kSplitParts;
                 }
-                pid = tv.lvl_base[dp] + k / NH;
+                pid = tv.groups[tv.lvl_base[dp] + k / NH];
                 base = (k % NH) * SL;
             }
             const long long t_group = DEBUG ? clock64() : 0;
             const uint32_t plink = tv.link[pid];
             const uint32_t nc = plink >> 28;
-            if (nc == 0) continue;
             const uint32_t fc = plink & kLinkMask;
             // batched systems: the group's own system, theta and root; its
             // shallow leaves belong to k_heavy_leaf
@@ -730,23 +669,40 @@ __global__ void __launch_bounds__(
                     continue;
             }
             uint32_t cl = 0;
+            float4 cg = make_float4(0.f, 0.f, 0.f, 0.f);
             if (lane < nc) {
-                sm.cgeo[lane] = tv.geo[fc + lane];
+                cg = tv.geo[fc + lane];
                 cl = tv.link[fc + lane];
             }
-            cgp_put(sm.cgp, sm.cgeo, nc);
             const uint32_t leaf_mask =
                 __ballot_sync(0xFFFFFFFFu, lane < nc && (cl >> 28) == 0) & 0xFFu;
-            const uint32_t tgt_mask =
-                (MODE == MODE_INTERNAL ? (((1u << nc) - 1u) & ~leaf_mask) : leaf_mask) &
-                (((1u << SL) - 1u) << base);
+            uint32_t tgt_mask = MODE == MODE_INTERNAL ? (((1u << nc) - 1u) & ~leaf_mask)
+                                                      : leaf_mask;
+            // The targets are numbered without gaps, so that the pairs (and
+            // order 1's halves) run full; where k_dense_p2p takes the P2P they
+            // keep their child numbers, which its source masks refer to.
+            uint32_t slot = lane;
+            bool tgt = lane < nc;
+            if constexpr (COMPACT) {
+                slot = __popc(tgt_mask & lt_mask);
+                tgt = (tgt_mask >> lane) & 1u;
+                tgt_mask = (1u << __popc(tgt_mask)) - 1u;
+            }
+            const uint32_t nt = COMPACT ? __popc(tgt_mask) : nc;
+            tgt_mask &= ((1u << SL) - 1u) << base;
             if (tgt_mask == 0) continue;
+            if (tgt) {
+                sm.cgeo[slot] = cg;
+                sm.tq[slot] = (uint8_t)lane;
+            }
+            cgp_put(sm.cgp, sm.cgeo, nt);
             if constexpr (MODE == MODE_LEAF) {
                 if ((tgt_mask >> lane) & 1u) {
-                    const uint4 ci = tv.info[fc + lane];
+                    const uint4 ci = tv.info[fc + sm.tq[lane]];
                     sm.cpart[lane] = make_uint2(ci.x, ci.y);
                 }
             }
+            const float thw = sm.cgeo[base].w;  // (siblings are equally wide)
             if (lane < 8) {
                 if (DEBUG) sm.dbg_m2l[lane] = 0;
                 if constexpr (MODE == MODE_INTERNAL) {
@@ -833,7 +789,7 @@ __global__ void __launch_bounds__(
                 if (!root_only) {
                     uint32_t c = 0;
                     for (uint32_t e = lane; e < nsn; e += 32) {
-                        const uint32_t nch = tv.link[nsl[e]] >> 28;
+                        const uint32_t nch = nsl[e] >> 28;
                         c += nch ? nch : 1u;
                     }
                     cand_total = warp_sum(c);
@@ -904,10 +860,15 @@ __global__ void __launch_bounds__(
                     tot = 0;
                     do {
                     const uint32_t e = e0 + lane;
+                    // an entry is an internal source's link or a leaf's id
                     uint32_t s0 = 0, c = 0, link = 0;
                     if (e < nsn) {
-                        s0 = (SPLIT && !nsl) ? nfirst + e : nsl[e];
-                        link = tv.link[s0];
+                        if (SPLIT && !nsl) {
+                            s0 = nfirst + e;
+                            link = tv.link[s0];
+                        } else {
+                            s0 = link = nsl[e];
+                        }
                         const uint32_t nch = link >> 28;
                         c = nch ? nch : 1u;
                     }
@@ -957,7 +918,7 @@ __global__ void __launch_bounds__(
                     }
                     __syncwarp();
                     ssize -= kp;
-                    const uint32_t link = lane < kp ? tv.link[node] : 0u;
+                    const uint32_t link = node;  // (a leaf's id in chain groups)
                     const uint32_t nch = link >> 28;
                     const uint32_t c = lane < kp ? (XL && nch == 0 ? 1u : nch) : 0u;
                     const uint32_t inc = warp_incl_scan(c);
@@ -1003,7 +964,9 @@ __global__ void __launch_bounds__(
                         }
                     }
                     const uint32_t chunk_mask = __reduce_or_sync(0xFFFFFFFFu, smask);
-                    uint32_t near_bits = 0;
+                    uint32_t sep = 0;  // targets the candidate is separated from
+                    const float hs = __fadd_rn(thw, sg.w);
+                    const float mac = __fmul_rn(th2, __fmul_rn(hs, hs));
                     // children two at a time: the MAC per child (mac_separated,
                     // scalar, so its decisions are the reference's), then the
                     // M2L of m2l_field(_grad) for both children in paired FP32
@@ -1013,20 +976,19 @@ __global__ void __launch_bounds__(
                         const uint32_t q = base + 2 * k;  // children q and q + 1
                         if (!((chunk_mask >> q) & 3u)) continue;
                         const float4 ga = sm.cgp[q >> 1][0], gb = sm.cgp[q >> 1][1];
-                        float dx0, dy0, dz0, e0, dx1, dy1, dz1, e1;
-                        const bool m0 = mac_separated(ga.x, ga.z, gb.x, gb.z, sg.x, sg.y, sg.z,
-                                                      sg.w, th2, dx0, dy0, dz0, e0);
-                        const bool m1 = mac_separated(ga.y, ga.w, gb.y, gb.w, sg.x, sg.y, sg.z,
-                                                      sg.w, th2, dx1, dy1, dz1, e1);
+                        float dx0, dy0, dz0, d20, dx1, dy1, dz1, d21;
+                        const bool m0 = mac_far(ga.x, ga.z, gb.x, sg, mac, dx0, dy0, dz0, d20);
+                        const bool m1 = mac_far(ga.y, ga.w, gb.y, sg, mac, dx1, dy1, dz1, d21);
+                        sep |= (m0 ? 1u << q : 0u) | (m1 ? 2u << q : 0u);
                         const float2 dx = make_float2(dx0, dx1), dy = make_float2(dy0, dy1),
-                                     dz = make_float2(dz0, dz1), d2 = make_float2(e0, e1);
-                        const bool a0 = (smask >> q) & 1u, a1 = (smask >> (q + 1)) & 1u;
-                        const bool s0 = m0 && a0, s1 = m1 && a1;
-                        // branch-free: every lane evaluates, only separated
-                        // pairs add (x * 1 + acc = x + acc, x * 0 + acc = acc)
-                        const float2 on = make_float2(s0 ? 1.f : 0.f, s1 ? 1.f : 0.f);
+                                     dz = make_float2(dz0, dz1), d2 = make_float2(d20, d21);
+                        const bool s0 = m0 && ((smask >> q) & 1u),
+                                   s1 = m1 && ((smask >> (q + 1)) & 1u);
+                        // branch-free: every lane evaluates; a pair that is not
+                        // separated has its 1/r zeroed and adds zeros
                         const float2 soft = __fadd2_rn(d2, make_float2(0.1f, 0.1f));
-                        const float2 inv = make_float2(rsqrt_soft(soft.x), rsqrt_soft(soft.y));
+                        const float2 inv = make_float2(s0 ? rsqrt_soft(soft.x) : 0.f,
+                                                       s1 ? rsqrt_soft(soft.y) : 0.f);
                         const float2 inv2 = __fmul2_rn(inv, inv);
                         const float2 ir3 = __fmul2_rn(inv2, inv);
                         const float2 ir5 = __fmul2_rn(ir3, inv2);
@@ -1038,18 +1000,14 @@ __global__ void __launch_bounds__(
                             __ffma2_rn(my, dx, __ffma2_rn(mz, dy, __fmul2_rn(mw, dz)));
                         const float2 a = __ffma2_rn(
                             mx, ir3, __fmul2_rn(__fmul2_rn(make_float2(-3.f, -3.f), mdr), ir5));
-                        const float2 fx = __ffma2_rn(dx, a, __fmul2_rn(my, ir3));
-                        const float2 fy = __ffma2_rn(dy, a, __fmul2_rn(mz, ir3));
-                        const float2 fz = __ffma2_rn(dz, a, __fmul2_rn(mw, ir3));
-                        acc[k][0] = __ffma2_rn(fx, on, acc[k][0]);
-                        acc[k][1] = __ffma2_rn(fy, on, acc[k][1]);
-                        acc[k][2] = __ffma2_rn(fz, on, acc[k][2]);
+                        acc[k][0] = __ffma2_rn(dx, a, __ffma2_rn(my, ir3, acc[k][0]));
+                        acc[k][1] = __ffma2_rn(dy, a, __ffma2_rn(mz, ir3, acc[k][1]));
+                        acc[k][2] = __ffma2_rn(dz, a, __ffma2_rn(mw, ir3, acc[k][2]));
                         if constexpr (GRAD) {
                             // g3 d d^T - gi I, g3 = 3 m0 / r^5, gi = m0 / r^3
-                            const float2 g3 = __fmul2_rn(
-                                __fmul2_rn(__fmul2_rn(make_float2(3.f, 3.f), mx), ir5), on);
-                            const float2 gi = __fmul2_rn(__fmul2_rn(mx, ir3), on);
-                            const float2 ngi = make_float2(-gi.x, -gi.y);
+                            const float2 g3 =
+                                __fmul2_rn(__fmul2_rn(make_float2(3.f, 3.f), mx), ir5);
+                            const float2 ngi = __fmul2_rn(make_float2(-mx.x, -mx.y), ir3);
                             const float2 gx = __fmul2_rn(g3, dx), gy = __fmul2_rn(g3, dy);
                             gacc[k][0] = __fadd2_rn(gacc[k][0], __ffma2_rn(gx, dx, ngi));
                             gacc[k][1] = __fadd2_rn(gacc[k][1], __ffma2_rn(gy, dy, ngi));
@@ -1059,8 +1017,6 @@ __global__ void __launch_bounds__(
                             gacc[k][4] = __ffma2_rn(gx, dz, gacc[k][4]);
                             gacc[k][5] = __ffma2_rn(gy, dz, gacc[k][5]);
                         }
-                        if (a0 && !s0) near_bits |= 1u << q;
-                        if (a1 && !s1) near_bits |= 2u << q;
                         if (DEBUG) {
                             const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, s0);
                             const uint32_t b1 = __ballot_sync(0xFFFFFFFFu, s1);
@@ -1070,6 +1026,7 @@ __global__ void __launch_bounds__(
                             }
                         }
                     }
+                    const uint32_t near_bits = smask & ~sep;
                     if constexpr (MODE == MODE_INTERNAL) {
                         // near candidates of internal children: their near lists
                         const uint32_t near_any = __reduce_or_sync(0xFFFFFFFFu, near_bits);
@@ -1078,14 +1035,14 @@ __global__ void __launch_bounds__(
                             const uint32_t q = __ffs(m) - 1;
                             const bool nr = (near_bits >> q) & 1u;
                             const uint32_t nm = __ballot_sync(0xFFFFFFFFu, nr);
-                            const uint32_t base = sm.ns_cnt[q];
+                            const uint32_t have = sm.ns_cnt[q];
                             if (ns_ok && nr) {
-                                const uint32_t sub = __popc(tgt_mask & ((1u << q) - 1u));
-                                A.ns[ns_base + (unsigned long long)sub * cand_total + base +
-                                     __popc(nm & lt_mask)] = s;
+                                const uint32_t sub = q - base;
+                                A.ns[ns_base + (unsigned long long)sub * cand_total + have +
+                                     __popc(nm & lt_mask)] = (slink >> 28) ? slink : s;
                             }
                             __syncwarp();
-                            if (lane == 0) sm.ns_cnt[q] = base + __popc(nm);
+                            if (lane == 0) sm.ns_cnt[q] = have + __popc(nm);
                             __syncwarp();
                         }
                     } else {
@@ -1120,7 +1077,7 @@ __global__ void __launch_bounds__(
                         if (pb) {
                             if (pfill + __popc(pb) > (uint32_t)kP2PCap) {
                                 if (XL && A.stream) {
-                                    stream_p2p<DEBUG, GRAD>(sm, A, tgt_mask, fc, pfill,
+                                    stream_p2p<DEBUG, GRAD>(sm, A, tgt_mask, fc, pfill, kNone,
                                                             flushed, false, sinter);
                                     flushed = true;
                                 } else {
@@ -1152,7 +1109,7 @@ __global__ void __launch_bounds__(
                         if (qb) {
                             const uint32_t pos = ssize + __popc(qb & lt_mask);
                             if (push && pos < (uint32_t)kStackCap) {
-                                sm.stk_node[pos] = s;
+                                sm.stk_node[pos] = (XL && sleaf) ? s : slink;
                                 sm.stk_mask[pos] = (uint8_t)(cpush ? cmask : qbits);
                                 if constexpr (XL) sm.stk_lvl[pos] = (uint8_t)(cpush ? clvl : 0u);
                             }
@@ -1267,7 +1224,7 @@ __global__ void __launch_bounds__(
                     G1.y += total_of((k & 1) ? gk[5].y : gk[5].x, k, 8);
                 }
                 if (lane == 0) {
-                    const uint32_t u = fc + q;
+                    const uint32_t u = fc + sm.tq[q];
                     tv.lt[u] = L;
                     if constexpr (GRAD) {
                         tv.lg0[u] = G0;
@@ -1280,7 +1237,7 @@ __global__ void __launch_bounds__(
                             sm.sG1[q] = G1;
                         }
                     } else {
-                        const uint32_t sub = __popc(tgt_mask & ((1u << q) - 1u));
+                        const uint32_t sub = q - base;
                         tv.ns_off[u] = (uint32_t)(ns_base + (unsigned long long)sub * cand_total);
                         tv.ns_cnt[u] = ns_ok ? sm.ns_cnt[q] : 0u;
                     }
@@ -1295,7 +1252,7 @@ __global__ void __launch_bounds__(
                 // lists and fields of this group's children are final
                 if ((tgt_mask >> lane) & 1u) {
                     __threadfence();
-                    __stcg(&tv.ready[fc + lane], 1u);
+                    __stcg(&tv.ready[fc + sm.tq[lane]], 1u);
                 }
             }
 
@@ -1766,8 +1723,7 @@ __global__ void __launch_bounds__(kHeavyThreads, 2) k_heavy_leaf(const __grid_co
                 const uint32_t e = e0 + tid;
                 uint32_t s0 = 0, link = 0, c = 0;
                 if (e < nsn) {
-                    s0 = nsl[e];
-                    link = tv.link[s0];
+                    s0 = link = nsl[e];  // an internal source's link or a leaf's id
                     c = (link >> 28) ? (link >> 28) : 1u;
                 }
                 uint32_t ex;

@@ -442,25 +442,28 @@ __global__ void __launch_bounds__(kTreeThreads) k_tree_emit(const uint32_t* __re
     }
 }
 
-// child count = next node's first-child rank - this node's (same level);
-// also the particle count of the fullest leaf
-__global__ void __launch_bounds__(256) k_tree_link(TreeView tv, const Status* status) {
+// child count = next node's first-child rank - this node's (same level); also
+// the particle count of the fullest leaf, and the list of each level's
+// internal nodes (the traversal's groups: without the leaves, 3 of 4 nodes,
+// its work queues hold no empty items), in Morton order but for the order in
+// which warps append
+__global__ void __launch_bounds__(256) k_tree_link(TreeView tv, Status* status) {
     const uint32_t total = tv.lvl_base[kLevels];
-    const uint32_t stride = gridDim.x * blockDim.x;
-    uint32_t max_leaf = 0;
-    for (uint32_t id = blockIdx.x * blockDim.x + threadIdx.x; id < total; id += stride) {
-        int d = 0;
-        while (d < kMaxDepth && id >= tv.lvl_base[d + 1]) ++d;
-        const uint32_t r = id - tv.lvl_base[d];
-        const uint32_t cnt_d = status->lvl_count[d];
-        if (r >= cnt_d) continue;
-        uint32_t nch = 0;
+    const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
+    int d = 0;
+    while (d < kMaxDepth && id >= tv.lvl_base[d + 1]) ++d;
+    const uint32_t r = id - tv.lvl_base[d];
+    const uint32_t cnt_d = status->lvl_count[d];
+    const bool node = id < total && r < cnt_d;
+    if (!__any_sync(0xFFFFFFFFu, node)) return;
+    uint32_t nch = 0, max_leaf = 0;
+    if (node) {
         if (d < kMaxDepth) {
             const uint32_t next = (r + 1 < cnt_d) ? tv.cbase[id + 1]
                                                   : tv.lvl_base[d + 1] + status->lvl_count[d + 1];
             nch = next - tv.cbase[id];
             if (nch > 8u) {  // codes not sorted by their 30-bit prefix
-                set_err(const_cast<Status*>(status), PSG_ERR_NODES);
+                set_err(status, PSG_ERR_NODES);
                 nch = 0;
             }
         }
@@ -470,13 +473,21 @@ __global__ void __launch_bounds__(256) k_tree_link(TreeView tv, const Status* st
         tv.link[id] = nch ? ((inf.z & kLinkMask) | (nch << 28)) : 0u;
         tv.lt[id] = make_float4(0.f, 0.f, 0.f, 0.f);
         tv.ready[id] = 0;
-        if (nch == 0 && inf.y > max_leaf) max_leaf = inf.y;
+        if (nch == 0) max_leaf = inf.y;
         // batched systems: each system picks its own leaf-pass variant
         if (nch == 0 && tv.part_sys && inf.y >= 32u)
             atomicMax(&tv.sys_maxleaf[tv.part_sys[inf.x]], inf.y);
     }
+    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, nch ? (uint32_t)d : kNone);
+    if (nch) {
+        const int leader = __ffs(peers) - 1;
+        uint32_t base = 0;
+        if ((int)lane_id() == leader) base = atomicAdd(&status->group_count[d], __popc(peers));
+        base = __shfl_sync(peers, base, leader);
+        tv.groups[tv.lvl_base[d] + base + __popc(peers & lanemask_lt())] = id;
+    }
     max_leaf = __reduce_max_sync(0xFFFFFFFFu, max_leaf);
-    if (lane_id() == 0 && max_leaf) atomicMax(&const_cast<Status*>(status)->max_leaf, max_leaf);
+    if (lane_id() == 0 && max_leaf) atomicMax(&status->max_leaf, max_leaf);
 }
 
 // Upward pass: P2M (a leaf's particles) and M2M (a node's children).

@@ -49,6 +49,7 @@ struct TreeView {
     uint32_t* arrive;      // upward-pass arrival counters
     uint32_t* cbase;       // first-child rank per node (tree link step)
     uint32_t* link;        // first child | nchild << 28
+    uint32_t* groups;      // the internal nodes of level d at lvl_base[d] .. + group_count[d]
     uint32_t* ready;       // internal levels: the node's near list and field are final
     uint32_t* ns_off;      // per node: offset of its near-source list
     uint32_t* ns_cnt;      // per node: length of its near-source list
@@ -76,6 +77,7 @@ struct TreeView {
 struct Status {
     uint32_t err;                          // PSG_ERR_* bits
     uint32_t lvl_count[kLevels + 1];       // nodes per level
+    uint32_t group_count[kLevels];         // ... of them internal
     float bbox[4];                         // min, max, range, scale (prepare)
     unsigned long long stat[16];           // debug totals (see PSG_STAT_*)
     uint32_t max_stack;                    // deepest DFS stack seen (debug)
@@ -117,6 +119,17 @@ __device__ __forceinline__ bool mac_separated(float tx, float ty, float tz, floa
     d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
     float hs = __fadd_rn(thw, shw);
     return d2 > __fmul_rn(theta2, __fmul_rn(hs, hs));
+}
+
+// mac_separated with the right side, theta^2 * hw_sum^2, given (the same for all
+// children of a node: they are equally wide)
+__device__ __forceinline__ bool mac_far(float tx, float ty, float tz, float4 s, float limit,
+                                        float& dx, float& dy, float& dz, float& d2) {
+    dx = __fsub_rn(s.x, tx);
+    dy = __fsub_rn(s.y, ty);
+    dz = __fsub_rn(s.z, tz);
+    d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+    return d2 > limit;
 }
 
 // 1/sqrt of a softened squared distance (x >= 0.1f, inf or NaN).  The same

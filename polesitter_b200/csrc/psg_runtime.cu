@@ -326,7 +326,7 @@ static void free_state(State* s) {
                   s->sort.hist, s->tree_tiles, s->tv.geo,
                   s->tv.mp, s->tv.lt, s->tv.info, s->tv.parent, s->tv.arrive, s->tv.cbase,
                   s->tv.ns_off, s->tv.ns_cnt, s->tv.dbg_m2l, s->tv.dbg_p2p, s->tv.link,
-                  s->tv.ready, s->ns, s->p2p.src, s->p2p.mask, s->p2p.next, s->p2p.cnt,
+                  s->tv.ready, s->tv.groups, s->ns, s->p2p.src, s->p2p.mask, s->p2p.next, s->p2p.cnt,
                   s->d_status, s->dense.rec, s->dense.rec_slot, s->dense.prev, s->dense.sums,
                   s->dense.item, s->split.sums, s->split.list, s->split.count, s->heavy_frontier, s->tk_partial, s->tk_bbox, s->tk_v[0], s->tk_v[1], s->tk_v[2],
                   s->tk_vmir[0], s->tk_vmir[1], s->tk_vmir[2], s->cl.lg0, s->cl.lg1,
@@ -409,6 +409,7 @@ static int init_state(State* s, size_t maxp, float theta, const uint32_t* lvl_ca
     PSG_ALLOC(s->tv.dbg_p2p, nodes * 4);
     PSG_ALLOC(s->tv.link, nodes * 4);
     PSG_ALLOC(s->tv.ready, nodes * 4);
+    PSG_ALLOC(s->tv.groups, nodes * 4);
     PSG_ALLOC(s->d_status, sizeof(Status));
     PSG_CHECK(cudaMallocHost((void**)&s->h_status, sizeof(Status)));
     std::memset(s->h_status, 0, sizeof(Status));
