@@ -47,98 +47,15 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// GELU, tanh form: 0.5 x (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3)))
-__device__ __forceinline__ float gelu(float x) {
-    const float u = 0.7978845608028654f * fmaf(0.044715f * x, x * x, x);
-    return 0.5f * x * (1.0f + tanhf(u));
-}
-
-__device__ __forceinline__ float gelu_grad(float x) {
+// GELU, tanh form: 0.5 x (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3))), and its
+// derivative
+__device__ __forceinline__ float gelu(float x, float& grad) {
     const float x2 = x * x;
     const float u = 0.7978845608028654f * fmaf(0.044715f * x, x2, x);
     const float th = tanhf(u);
-    return fmaf(0.5f * x * (1.0f - th * th) * 0.7978845608028654f, fmaf(0.134145f, x2, 1.0f),
+    grad = fmaf(0.5f * x * (1.0f - th * th) * 0.7978845608028654f, fmaf(0.134145f, x2, 1.0f),
                 0.5f * (1.0f + th));
-}
-
-// One warp, 16 rows: C[16 x 8 NT] = A[16 x 16 KC] . W, A as m16n8k16
-// A-fragments, W as Wt[out][in] (row stride LD) in shared memory.
-template <int KC, int NT, int LD>
-__device__ __forceinline__ void warp_layer(const uint32_t (&a)[KC][4], const uint16_t* wt,
-                                           float (&c)[NT][4]) {
-    const uint32_t lane = lane_id(), g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-        c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.f;
-        const uint16_t* row = wt + (nt * 8 + g) * LD + 2 * t;
-#pragma unroll
-        for (int kc = 0; kc < KC; ++kc) {
-            const uint32_t b0 = *reinterpret_cast<const uint32_t*>(row + kc * 16);
-            const uint32_t b1 = *reinterpret_cast<const uint32_t*>(row + kc * 16 + 8);
-            mma_bf16(c[nt], a[kc], b0, b1);
-        }
-    }
-}
-
-// z = c + b; h = GELU(z) rounded to BF16 and repacked as the next layer's
-// A-fragments (k-chunk kc = n-tiles 2kc and 2kc+1).  With STORE, z (FP32) and
-// h (BF16 bits) also go to shared memory rows [16][64] for the backward pass.
-template <bool STORE>
-__device__ __forceinline__ void act_to_frag(float (&c)[8][4], const float* bias,
-                                            uint32_t (&a)[4][4], float* zrow, uint16_t* hrow) {
-    const uint32_t lane = lane_id(), g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-        const int col = nt * 8 + 2 * t;
-        const float z0 = c[nt][0] + bias[col], z1 = c[nt][1] + bias[col + 1];
-        const float z2 = c[nt][2] + bias[col], z3 = c[nt][3] + bias[col + 1];
-        const uint32_t lo = pack_bf16x2(gelu(z0), gelu(z1));
-        const uint32_t hi = pack_bf16x2(gelu(z2), gelu(z3));
-        const int kc = nt >> 1, half = nt & 1;
-        a[kc][half ? 2 : 0] = lo;
-        a[kc][half ? 3 : 1] = hi;
-        if constexpr (STORE) {
-            zrow[g * kMlpHid + col] = z0;
-            zrow[g * kMlpHid + col + 1] = z1;
-            zrow[(g + 8) * kMlpHid + col] = z2;
-            zrow[(g + 8) * kMlpHid + col + 1] = z3;
-            *reinterpret_cast<uint32_t*>(hrow + g * kMlpHid + col) = lo;
-            *reinterpret_cast<uint32_t*>(hrow + (g + 8) * kMlpHid + col) = hi;
-        }
-    }
-}
-
-// input fragments from feat[16][17] (FP32), rounded to BF16
-__device__ __forceinline__ void input_frag(const float (*feat)[17], uint32_t (&a)[1][4]) {
-    const uint32_t lane = lane_id(), g = lane >> 2, t = lane & 3;
-    a[0][0] = pack_bf16x2(feat[g][2 * t], feat[g][2 * t + 1]);
-    a[0][1] = pack_bf16x2(feat[g + 8][2 * t], feat[g + 8][2 * t + 1]);
-    a[0][2] = pack_bf16x2(feat[g][2 * t + 8], feat[g][2 * t + 9]);
-    a[0][3] = pack_bf16x2(feat[g + 8][2 * t + 8], feat[g + 8][2 * t + 9]);
-}
-
-// the whole network on 16 rows; y[16][9] receives the 8 outputs
-template <bool STORE>
-__device__ __forceinline__ void warp_mlp(const MlpPacked& w, const float (*feat)[17],
-                                         float (*y)[9], float* z1, float* z2, float* z3,
-                                         uint16_t* h1, uint16_t* h2, uint16_t* h3) {
-    const uint32_t lane = lane_id(), g = lane >> 2, t = lane & 3;
-    uint32_t a0[1][4];
-    input_frag(feat, a0);
-    float c[8][4];
-    uint32_t a[4][4];
-    warp_layer<1, 8, kLd1>(a0, w.wt1, c);
-    act_to_frag<STORE>(c, w.b1, a, z1, h1);
-    warp_layer<4, 8, kLdH>(a, w.wt2, c);
-    act_to_frag<STORE>(c, w.b2, a, z2, h2);
-    warp_layer<4, 8, kLdH>(a, w.wt3, c);
-    act_to_frag<STORE>(c, w.b3, a, z3, h3);
-    float o[1][4];
-    warp_layer<4, 1, kLdH>(a, w.wt4, o);
-    y[g][2 * t] = o[0][0] + w.b4[2 * t];
-    y[g][2 * t + 1] = o[0][1] + w.b4[2 * t + 1];
-    y[g + 8][2 * t] = o[0][2] + w.b4[2 * t];
-    y[g + 8][2 * t + 1] = o[0][3] + w.b4[2 * t + 1];
+    return 0.5f * x * (1.0f + th);
 }
 
 // features of sorted particle i; returns m_i s kMlpOutScale
@@ -590,56 +507,158 @@ __global__ void k_mlp_pack(const float* __restrict__ p, MlpPacked* __restrict__ 
 }
 
 // ---- training ---------------------------------------------------------------
-constexpr int kTrainRows = 64;  // samples per block (4 warps x 16)
+constexpr int kTrainRows = 32;      // samples per block: 128 blocks a batch of 4096
+constexpr int kTrainThreads = 256;  // 8 warps: 2 row tiles of 16 x 4 column groups of 16
+constexpr int kTrLd0 = kLd1;        // row strides in shared memory, padded against
+constexpr int kTrLdH = kLdH;        // bank conflicts
+constexpr int kTrLdF = kMlpHid + 4;
 
 struct TrainSmem {
     MlpPacked w;
-    uint16_t h0[kTrainRows * kMlpIn];   // BF16 inputs
-    uint16_t h1[kTrainRows * kMlpHid];  // BF16 activations
-    uint16_t h2[kTrainRows * kMlpHid];
-    uint16_t h3[kTrainRows * kMlpHid];
-    float z1[kTrainRows * kMlpHid];     // FP32 pre-activations
-    float z2[kTrainRows * kMlpHid];
-    float z3[kTrainRows * kMlpHid];
-    float da[kTrainRows * kMlpHid];     // gradients, ping-pong
-    float db[kTrainRows * kMlpHid];
+    uint16_t h0[kTrainRows * kTrLd0];  // BF16 inputs
+    uint16_t h[3][kTrainRows * kTrLdH];  // BF16 activations
+    float dact[3][kTrainRows * kTrLdF];  // GELU' at the pre-activations
+    float da[kTrainRows * kTrLdF];       // gradients, ping-pong
+    float db[kTrainRows * kTrLdF];
     float dy[kTrainRows * kMlpOut];
-    float feat[4][16][17];
-    float y[4][16][9];
 };
 
 size_t mlp_train_smem_bytes() { return sizeof(TrainSmem); }
 
-// dW[k][n] += sum_b h[b][k] d[b][n]  and  db[n] += sum_b d[b][n]
-__device__ __forceinline__ void accum_dw(const uint16_t* h, int K, const float* d, int N,
-                                         float* gW, float* gB) {
-    for (int e = threadIdx.x; e < K * N; e += blockDim.x) {
-        const int n = e / K, k = e % K;
-        float sum = 0.f;
-        for (int b = 0; b < kTrainRows; ++b) sum = fmaf(bf16_bits_to_float(h[b * K + k]), d[b * N + n], sum);
-        atomicAdd(&gW[k * N + n], sum);
+// this warp's tiles of C[32 x 8 NT] = A[32 x 16 KC] . W: row tile rt, the NT
+// n-tiles from nt0, A as BF16 rows (stride LDA), W as Wt[out][in] (stride LDW)
+template <int KC, int NT, int LDA, int LDW>
+__device__ __forceinline__ void train_layer(const uint16_t* a, const uint16_t* wt, int rt, int nt0,
+                                            float (&c)[NT][4]) {
+    const uint32_t lane = lane_id(), g = lane >> 2, t = lane & 3;
+    uint32_t f[KC][4];
+    const uint16_t* row = a + (rt * 16 + g) * LDA + 2 * t;
+#pragma unroll
+    for (int kc = 0; kc < KC; ++kc) {
+        f[kc][0] = *reinterpret_cast<const uint32_t*>(row + kc * 16);
+        f[kc][1] = *reinterpret_cast<const uint32_t*>(row + 8 * LDA + kc * 16);
+        f[kc][2] = *reinterpret_cast<const uint32_t*>(row + kc * 16 + 8);
+        f[kc][3] = *reinterpret_cast<const uint32_t*>(row + 8 * LDA + kc * 16 + 8);
     }
-    for (int e = threadIdx.x; e < N; e += blockDim.x) {
-        float sum = 0.f;
-        for (int b = 0; b < kTrainRows; ++b) sum += d[b * N + e];
-        atomicAdd(&gB[e], sum);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+        c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
+        const uint16_t* wr = wt + ((nt0 + j) * 8 + g) * LDW + 2 * t;
+#pragma unroll
+        for (int kc = 0; kc < KC; ++kc) {
+            const uint32_t b0 = *reinterpret_cast<const uint32_t*>(wr + kc * 16);
+            const uint32_t b1 = *reinterpret_cast<const uint32_t*>(wr + kc * 16 + 8);
+            mma_bf16(c[j], f[kc], b0, b1);
+        }
     }
 }
 
-// dnext[b][k] = (sum_n d[b][n] W[k][n]) * GELU'(z[b][k]), W[k][n] = Wt[n][k]
-__device__ __forceinline__ void back_act(const float* d, int N, const uint16_t* wt, int ld,
-                                         const float* z, float* dnext) {
-    for (int e = threadIdx.x; e < kTrainRows * kMlpHid; e += blockDim.x) {
-        const int b = e / kMlpHid, k = e % kMlpHid;
+// z = c + b; GELU(z) rounded to BF16 and GELU'(z) to shared memory
+__device__ __forceinline__ void train_act(const float (&c)[2][4], const float* bias, int rt,
+                                          int nt0, uint16_t* h, float* dact) {
+    const uint32_t lane = lane_id(), g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int col = (nt0 + j) * 8 + 2 * t;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int r = rt * 16 + half * 8 + g;
+            float g0, g1;
+            const float a0 = gelu(c[j][2 * half] + bias[col], g0);
+            const float a1 = gelu(c[j][2 * half + 1] + bias[col + 1], g1);
+            *reinterpret_cast<uint32_t*>(h + r * kTrLdH + col) = pack_bf16x2(a0, a1);
+            *reinterpret_cast<float2*>(dact + r * kTrLdF + col) = make_float2(g0, g1);
+        }
+    }
+}
+
+__device__ __forceinline__ float4 bf16x4_to_float4(uint2 v) {
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xFFFF0000u),
+                       __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xFFFF0000u));
+}
+
+// dW[k][n] += sum_b h[b][k] d[b][n] over 64 columns n and K = 64 or 16 rows k:
+// each thread a tile of K / 16 x 4
+template <int K, int LDH>
+__device__ __forceinline__ void accum_dw(const uint16_t* h, const float* d, float* gW) {
+    constexpr int R = K / 16;
+    const int k0 = (threadIdx.x >> 4) * R, n0 = (threadIdx.x & 15) * 4;
+    float4 acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int b = 0; b < kTrainRows; ++b) {
+        const float4 v = *reinterpret_cast<const float4*>(d + b * kTrLdF + n0);
+        float hk[R];
+        if constexpr (R == 4) {
+            const float4 q =
+                bf16x4_to_float4(*reinterpret_cast<const uint2*>(h + b * LDH + k0));
+            hk[0] = q.x;
+            hk[1] = q.y;
+            hk[2] = q.z;
+            hk[3] = q.w;
+        } else {
+            hk[0] = bf16_bits_to_float(h[b * LDH + k0]);
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            acc[r].x = fmaf(hk[r], v.x, acc[r].x);
+            acc[r].y = fmaf(hk[r], v.y, acc[r].y);
+            acc[r].z = fmaf(hk[r], v.z, acc[r].z);
+            acc[r].w = fmaf(hk[r], v.w, acc[r].w);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        atomicAdd(reinterpret_cast<float4*>(gW + (k0 + r) * kMlpHid + n0), acc[r]);
+}
+
+// db[n] += sum_b d[b][n] over 64 columns
+__device__ __forceinline__ void accum_db(const float* d, float* gB) {
+    if (threadIdx.x < (unsigned)kMlpHid) {
         float sum = 0.f;
-        for (int n = 0; n < N; ++n) sum = fmaf(d[b * N + n], bf16_bits_to_float(wt[n * ld + k]), sum);
-        dnext[e] = sum * gelu_grad(z[e]);
+#pragma unroll 8
+        for (int b = 0; b < kTrainRows; ++b) sum += d[b * kTrLdF + threadIdx.x];
+        atomicAdd(gB + threadIdx.x, sum);
+    }
+}
+
+// dnext[b][k] = (sum_n d[b][n] W[k][n]) * GELU'(z[b][k]), W[k][n] = Wt[n][k]:
+// each thread 2 rows x 4 columns
+template <int N, int LDD>
+__device__ __forceinline__ void back_act(const float* d, const uint16_t* wt, const float* dact,
+                                         float* dnext) {
+    const int b0 = (threadIdx.x >> 4) * 2, k0 = (threadIdx.x & 15) * 4;
+    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int n = 0; n < N; ++n) {
+        const float4 w = bf16x4_to_float4(*reinterpret_cast<const uint2*>(wt + n * kLdH + k0));
+        const float d0 = d[b0 * LDD + n], d1 = d[(b0 + 1) * LDD + n];
+        s0[0] = fmaf(d0, w.x, s0[0]);
+        s0[1] = fmaf(d0, w.y, s0[1]);
+        s0[2] = fmaf(d0, w.z, s0[2]);
+        s0[3] = fmaf(d0, w.w, s0[3]);
+        s1[0] = fmaf(d1, w.x, s1[0]);
+        s1[1] = fmaf(d1, w.y, s1[1]);
+        s1[2] = fmaf(d1, w.z, s1[2]);
+        s1[3] = fmaf(d1, w.w, s1[3]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        dnext[b0 * kTrLdF + k0 + j] = s0[j] * dact[b0 * kTrLdF + k0 + j];
+        dnext[(b0 + 1) * kTrLdF + k0 + j] = s1[j] * dact[(b0 + 1) * kTrLdF + k0 + j];
     }
 }
 
 // Loss sum_{samples, outputs 0..2} (y - t)^2 and its gradient, scaled by
 // inv_norm, accumulated into grad (FP32 parameter layout) and loss_sum.
-__global__ void __launch_bounds__(128) k_mlp_grad(const float* __restrict__ X,
+// Forward on the tensor cores (mma.sync, BF16 with FP32 accumulation), backward
+// in FP32 with register tiles: a batch of 4096 is 164 MFLOP of FP32, so the
+// kernel is bound by the chain of small phases and their barriers, not by a
+// pipe; 32 rows a block spread a batch over 128 SMs.  Measured: a batch of 4096
+// 62 us (64 rows a block, one thread per output, one shared-memory load per
+// FMA) -> 17 us.
+__global__ void __launch_bounds__(kTrainThreads) k_mlp_grad(const float* __restrict__ X,
                                                   const float* __restrict__ T,
                                                   const uint32_t* __restrict__ perm, size_t b0,
                                                   size_t count, const MlpPacked* __restrict__ wts,
@@ -647,72 +666,114 @@ __global__ void __launch_bounds__(128) k_mlp_grad(const float* __restrict__ X,
                                                   float* __restrict__ loss_sum) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(smem_raw);
-    load_packed(S.w, wts);
     const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+    const int rt = (int)w >> 2, nt0 = ((int)w & 3) * 2;
     const size_t r_blk = (size_t)blockIdx.x * kTrainRows;
-    // inputs of this warp's 16 rows
-    if (lane < 16) {
-        const size_t r = r_blk + w * 16 + lane;
-        const bool valid = r < count;
-        const size_t src = valid ? (perm ? perm[b0 + r] : b0 + r) : 0;
-        for (int k = 0; k < kMlpIn; ++k) {
-            const float v = valid ? X[src * kMlpIn + k] : 0.f;
-            S.feat[w][lane][k] = v;
-            S.h0[(w * 16 + lane) * kMlpIn + k] = float_to_bf16_bits(v);
-        }
+    load_packed(S.w, wts);
+    // inputs, rounded to BF16 (zeros past the batch)
+    for (int e = threadIdx.x; e < kTrainRows * kMlpIn; e += kTrainThreads) {
+        const int r = e / kMlpIn, k = e % kMlpIn;
+        const bool valid = r_blk + r < count;
+        const size_t src = valid ? (perm ? perm[b0 + r_blk + r] : b0 + r_blk + r) : 0;
+        S.h0[r * kTrLd0 + k] = float_to_bf16_bits(valid ? X[src * kMlpIn + k] : 0.f);
     }
     __syncthreads();
-    const int row0 = w * 16;
-    warp_mlp<true>(S.w, S.feat[w], S.y[w], S.z1 + row0 * kMlpHid, S.z2 + row0 * kMlpHid,
-                   S.z3 + row0 * kMlpHid, S.h1 + row0 * kMlpHid, S.h2 + row0 * kMlpHid,
-                   S.h3 + row0 * kMlpHid);
-    __syncwarp();
-    float lsum = 0.f;
-    if (lane < 16) {
-        const size_t r = r_blk + row0 + lane;
-        const bool valid = r < count;
-        const size_t src = valid ? (perm ? perm[b0 + r] : b0 + r) : 0;
-        for (int o = 0; o < kMlpOut; ++o) {
+    float c[2][4];
+    train_layer<1, 2, kTrLd0, kLd1>(S.h0, S.w.wt1, rt, nt0, c);
+    train_act(c, S.w.b1, rt, nt0, S.h[0], S.dact[0]);
+    __syncthreads();
+    train_layer<4, 2, kTrLdH, kLdH>(S.h[0], S.w.wt2, rt, nt0, c);
+    train_act(c, S.w.b2, rt, nt0, S.h[1], S.dact[1]);
+    __syncthreads();
+    train_layer<4, 2, kTrLdH, kLdH>(S.h[1], S.w.wt3, rt, nt0, c);
+    train_act(c, S.w.b3, rt, nt0, S.h[2], S.dact[2]);
+    __syncthreads();
+    if (nt0 == 0) {  // the output layer: one warp per row tile
+        float o[1][4];
+        train_layer<4, 1, kTrLdH, kLdH>(S.h[2], S.w.wt4, rt, 0, o);
+        const uint32_t g = lane >> 2, t = lane & 3;
+        float lsum = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = rt * 16 + (j >> 1) * 8 + (int)g, col = 2 * (int)t + (j & 1);
+            const bool valid = r_blk + r < count;
             float d = 0.f;
-            if (valid && o < kMlpOutUsed) {
-                const float e = S.y[w][lane][o] - T[src * kMlpOutUsed + o];
+            if (valid && col < kMlpOutUsed) {
+                const size_t src = perm ? perm[b0 + r_blk + r] : b0 + r_blk + r;
+                const float e = o[0][j] + S.w.b4[col] - T[src * kMlpOutUsed + col];
                 lsum = fmaf(e, e, lsum);
                 d = 2.0f * e * inv_norm;
             }
-            S.dy[(row0 + lane) * kMlpOut + o] = d;
+            S.dy[r * kMlpOut + col] = d;
         }
+        lsum = warp_sum(lsum);
+        if (lane == 0 && lsum != 0.f) atomicAdd(loss_sum, lsum);
     }
-    lsum = warp_sum(lsum);
-    if (lane == 0 && lsum != 0.f) atomicAdd(loss_sum, lsum);
     __syncthreads();
-    // layer 4
-    accum_dw(S.h3, kMlpHid, S.dy, kMlpOut, grad + kOffW4, grad + kOffB4);
-    back_act(S.dy, kMlpOut, S.w.wt4, kLdH, S.z3, S.da);
+    // layer 4: 64 x 8 weights, 2 per thread
+    {
+        const int k = threadIdx.x >> 2, n = (threadIdx.x & 3) * 2;
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll 8
+        for (int b = 0; b < kTrainRows; ++b) {
+            const float hk = bf16_bits_to_float(S.h[2][b * kTrLdH + k]);
+            const float2 v = *reinterpret_cast<const float2*>(S.dy + b * kMlpOut + n);
+            s0 = fmaf(hk, v.x, s0);
+            s1 = fmaf(hk, v.y, s1);
+        }
+        atomicAdd(reinterpret_cast<float2*>(grad + kOffW4 + k * kMlpOut + n), make_float2(s0, s1));
+    }
+    if (threadIdx.x < (unsigned)kMlpOut) {
+        float sum = 0.f;
+        for (int b = 0; b < kTrainRows; ++b) sum += S.dy[b * kMlpOut + threadIdx.x];
+        atomicAdd(grad + kOffB4 + threadIdx.x, sum);
+    }
+    back_act<kMlpOut, kMlpOut>(S.dy, S.w.wt4, S.dact[2], S.da);
     __syncthreads();
     // layer 3
-    accum_dw(S.h2, kMlpHid, S.da, kMlpHid, grad + kOffW3, grad + kOffB3);
-    back_act(S.da, kMlpHid, S.w.wt3, kLdH, S.z2, S.db);
+    accum_dw<kMlpHid, kTrLdH>(S.h[1], S.da, grad + kOffW3);
+    accum_db(S.da, grad + kOffB3);
+    back_act<kMlpHid, kTrLdF>(S.da, S.w.wt3, S.dact[1], S.db);
     __syncthreads();
     // layer 2
-    accum_dw(S.h1, kMlpHid, S.db, kMlpHid, grad + kOffW2, grad + kOffB2);
-    back_act(S.db, kMlpHid, S.w.wt2, kLdH, S.z1, S.da);
+    accum_dw<kMlpHid, kTrLdH>(S.h[0], S.db, grad + kOffW2);
+    accum_db(S.db, grad + kOffB2);
+    back_act<kMlpHid, kTrLdF>(S.db, S.w.wt2, S.dact[0], S.da);
     __syncthreads();
     // layer 1
-    accum_dw(S.h0, kMlpIn, S.da, kMlpHid, grad + kOffW1, grad + kOffB1);
+    accum_dw<kMlpIn, kTrLd0>(S.h0, S.da, grad + kOffW1);
+    accum_db(S.da, grad + kOffB1);
 }
 
-// Adam (Kingma & Ba 2015) on the FP32 master parameters
+// the BF16 weight or FP32 bias of parameter i in the kernels' packed copy
+__device__ __forceinline__ void pack_param(MlpPacked* out, int i, float p) {
+    const uint16_t w = float_to_bf16_bits(p);
+    if (i < kOffB1) out->wt1[(i % kMlpHid) * kLd1 + i / kMlpHid] = w;
+    else if (i < kOffW2) out->b1[i - kOffB1] = p;
+    else if (i < kOffB2) out->wt2[((i - kOffW2) % kMlpHid) * kLdH + (i - kOffW2) / kMlpHid] = w;
+    else if (i < kOffW3) out->b2[i - kOffB2] = p;
+    else if (i < kOffB3) out->wt3[((i - kOffW3) % kMlpHid) * kLdH + (i - kOffW3) / kMlpHid] = w;
+    else if (i < kOffW4) out->b3[i - kOffB3] = p;
+    else if (i < kOffB4) out->wt4[((i - kOffW4) % kMlpOut) * kLdH + (i - kOffW4) / kMlpOut] = w;
+    else out->b4[i - kOffB4] = p;
+}
+
+// Adam (Kingma & Ba 2015) on the FP32 master parameters; the next step's packed
+// weights and zeroed gradient too (launches of their own took 5 us each)
 __global__ void k_mlp_adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
-                           const float* __restrict__ g, int n, float lr, float beta1, float beta2,
-                           float eps, float bc1, float bc2) {
+                           float* __restrict__ g, MlpPacked* __restrict__ packed, int n, float lr,
+                           float beta1, float beta2, float eps, float bc1, float bc2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gi = g[i];
+    g[i] = 0.f;
     const float mi = fmaf(beta1, m[i], (1.0f - beta1) * gi);
     const float vi = fmaf(beta2, v[i], (1.0f - beta2) * gi * gi);
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+    const float pi = p[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+    p[i] = pi;
+    pack_param(packed, i, pi);
 }
 
 // ---- launchers ------------------------------------------------------------------
@@ -778,13 +839,14 @@ void launch_mlp_grad(const float* X, const float* T, const uint32_t* perm, size_
                      float* loss_sum, cudaStream_t st) {
     if (count == 0) return;
     const unsigned grid = (unsigned)((count + kTrainRows - 1) / kTrainRows);
-    k_mlp_grad<<<grid, 128, sizeof(TrainSmem), st>>>(X, T, perm, b0, count, w, inv_norm, grad,
+    k_mlp_grad<<<grid, kTrainThreads, sizeof(TrainSmem), st>>>(X, T, perm, b0, count, w, inv_norm, grad,
                                                      loss_sum);
 }
 
-void launch_mlp_adam(float* p, float* m, float* v, const float* g, int n, float lr, float beta1,
-                     float beta2, float eps, float bc1, float bc2, cudaStream_t st) {
-    k_mlp_adam<<<(n + 255) / 256, 256, 0, st>>>(p, m, v, g, n, lr, beta1, beta2, eps, bc1, bc2);
+void launch_mlp_adam(float* p, float* m, float* v, float* g, MlpPacked* packed, int n, float lr,
+                     float beta1, float beta2, float eps, float bc1, float bc2, cudaStream_t st) {
+    k_mlp_adam<<<(n + 127) / 128, 128, 0, st>>>(p, m, v, g, packed, n, lr, beta1, beta2, eps, bc1,
+                                                bc2);
 }
 
 }  // namespace psg

@@ -129,8 +129,9 @@ size_t mlp_train_smem_bytes();
 void launch_mlp_grad(const float* X, const float* T, const uint32_t* perm, size_t b0,
                      size_t count, const MlpPacked* w, float inv_norm, float* grad,
                      float* loss_sum, cudaStream_t st);
-void launch_mlp_adam(float* p, float* m, float* v, const float* g, int n, float lr, float beta1,
-                     float beta2, float eps, float bc1, float bc2, cudaStream_t st);
+// the step also packs the new parameters and zeroes g
+void launch_mlp_adam(float* p, float* m, float* v, float* g, MlpPacked* packed, int n, float lr,
+                     float beta1, float beta2, float eps, float bc1, float bc2, cudaStream_t st);
 
 // k_direct.cu -- FP64 direct-sum forces for sampled targets (tests/accuracy.c:42-72)
 // part: partial sums of the source splits (summed in split order, so the

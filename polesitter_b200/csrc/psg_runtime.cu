@@ -2259,6 +2259,8 @@ int psg_closure_train(void* mem, const float* x, const float* t, size_t n, float
     PSG_CHECK(cudaMemcpyAsync(d_p, params, P * 4, cudaMemcpyHostToDevice, st));
     PSG_CHECK(cudaMemsetAsync(d_m, 0, P * 4, st));
     PSG_CHECK(cudaMemsetAsync(d_v, 0, P * 4, st));
+    PSG_CHECK(cudaMemsetAsync(d_g, 0, P * 4, st));
+    psg::launch_mlp_pack(d_p, d_w, st);
     PSG_CHECK(cudaMemsetAsync(d_loss, 0, (epochs ? epochs : 1) * 4, st));
     uint32_t* perm = nullptr;
     PSG_CHECK(cudaMallocHost((void**)&perm, n * 4));
@@ -2287,14 +2289,13 @@ int psg_closure_train(void* mem, const float* x, const float* t, size_t n, float
             lr * (0.05f + 0.95f * 0.5f * (1.0f + cosf(3.14159265f * (float)ep / (float)epochs)));
         for (size_t b0 = 0; b0 < n; b0 += batch) {
             const size_t cnt = n - b0 < batch ? n - b0 : batch;
-            PSG_CHECK(cudaMemsetAsync(d_g, 0, P * 4, st));
-            psg::launch_mlp_pack(d_p, d_w, st);
             psg::launch_mlp_grad(d_x, d_t, d_perm, b0, cnt, d_w, 1.0f / (3.0f * (float)cnt), d_g,
                                  d_loss + ep, st);
             ++step;
             const float bc1 = 1.0f - powf(beta1, (float)step);
             const float bc2 = 1.0f - powf(beta2, (float)step);
-            psg::launch_mlp_adam(d_p, d_m, d_v, d_g, P, lr_ep, beta1, beta2, eps, bc1, bc2, st);
+            psg::launch_mlp_adam(d_p, d_m, d_v, d_g, d_w, P, lr_ep, beta1, beta2, eps, bc1, bc2,
+                                 st);
         }
         if (cudaGetLastError() != cudaSuccess) r = PSG_EDEVICE;
     }
