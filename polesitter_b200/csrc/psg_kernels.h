@@ -138,6 +138,8 @@ void launch_mlp_adam(float* p, float* m, float* v, float* g, MlpPacked* packed, 
 // result does not depend on scheduling); as many splits as part_doubles
 // holds, at most those that fill about `blocks` blocks
 size_t direct_f64_part_doubles(size_t n, size_t n_targets, int blocks);
+void launch_direct_pack(const float* x, const float* y, const float* z, const float* m, size_t n,
+                        float4* out, cudaStream_t st);
 void launch_direct_f64(const float4* xyzm, size_t n, const uint32_t* targets, size_t n_targets,
                        double* out /*[n_targets][3]*/, int blocks, cudaStream_t st,
                        double* part, size_t part_doubles);

@@ -151,6 +151,9 @@ struct State {
     unsigned long long stats[24];
     uint32_t last_nodes;
     uint32_t lvl_count[kLevels];  // node counts of the last completed tick
+    // workspace of ps_b200_direct_f64 (grown by its calls)
+    double* direct_ws;
+    size_t direct_bytes;
     // device tick loop scratch (allocated by its first call)
     int tk_grid;
     float2* tk_partial;
@@ -328,7 +331,7 @@ static void free_state(State* s) {
                   s->tv.ns_off, s->tv.ns_cnt, s->tv.dbg_m2l, s->tv.dbg_p2p, s->tv.link,
                   s->tv.ready, s->tv.groups, s->ns, s->p2p.src, s->p2p.mask, s->p2p.next, s->p2p.cnt,
                   s->d_status, s->dense.rec, s->dense.rec_slot, s->dense.prev, s->dense.sums,
-                  s->dense.item, s->split.sums, s->split.list, s->split.count, s->heavy_frontier, s->tk_partial, s->tk_bbox, s->tk_v[0], s->tk_v[1], s->tk_v[2],
+                  s->direct_ws, s->dense.item, s->split.sums, s->split.list, s->split.count, s->heavy_frontier, s->tk_partial, s->tk_bbox, s->tk_v[0], s->tk_v[1], s->tk_v[2],
                   s->tk_vmir[0], s->tk_vmir[1], s->tk_vmir[2], s->cl.lg0, s->cl.lg1,
                   s->cl.leaf_of, s->cl.dF, s->cl.params, s->cl.packed, s->cl.judge_tg,
                   s->cl.judge_f64, s->cl.judge_part, s->cl.d_judge};
@@ -2035,39 +2038,40 @@ int psg_direct_f64(void* mem, const psg_arrays_t* a, const uint32_t* targets, si
     if (n == 0 || n > s->max_particles) return PSG_EINVAL;
     PSG_CHECK(cudaSetDevice(s->device));
     cudaStream_t st = s->stream;
+    // host arrays come in through the context's mirrors
     const float* src[4] = {a->x, a->y, a->z, a->mass};
-    float* tmp = nullptr;
-    PSG_ALLOC(tmp, n * 4);
-    // pack (x, y, z, m) into the context's particle scratch
     for (int c = 0; c < 4; ++c) {
-        const float* p = src[c];
-        if (!psg::on_device(p)) {
-            PSG_CHECK(cudaMemcpyAsync(tmp, p, n * 4, cudaMemcpyHostToDevice, st));
-            p = tmp;
-        }
-        PSG_CHECK(cudaMemcpy2DAsync((char*)s->xyzm + 4 * c, 16, p, 4, 4, n,
-                                    cudaMemcpyDeviceToDevice, st));
-        PSG_CHECK(cudaStreamSynchronize(st));
+        if (psg::on_device(src[c])) continue;
+        const int r = psg::ensure_mirror(s->mir, s->max_particles);
+        if (r != PSG_OK) return r;
+        float* const rows[4] = {s->mir.x, s->mir.y, s->mir.z, s->mir.m};
+        PSG_CHECK(cudaMemcpyAsync(rows[c], src[c], n * 4, cudaMemcpyHostToDevice, st));
+        src[c] = rows[c];
     }
-    cudaFree(tmp);
-    uint32_t* dt = const_cast<uint32_t*>(targets);
-    double* dout = out;
+    // workspace, kept with the context: targets, forces, partial sums
     const bool ht = !psg::on_device(targets), ho = !psg::on_device(out);
-    if (ht) {
-        PSG_ALLOC(dt, n_t * 4);
-        PSG_CHECK(cudaMemcpyAsync(dt, targets, n_t * 4, cudaMemcpyHostToDevice, st));
-    }
-    if (ho) PSG_ALLOC(dout, n_t * 3 * sizeof(double));
     const size_t part_n = psg::direct_f64_part_doubles(n, n_t, s->sms * 8);
-    double* part = nullptr;
-    PSG_ALLOC(part, part_n * sizeof(double));
+    const size_t need = (part_n + n_t * 3) * sizeof(double) + n_t * 4;
+    if (s->direct_bytes < need) {
+        if (s->direct_ws) cudaFree(s->direct_ws);
+        s->direct_ws = nullptr;
+        s->direct_bytes = 0;
+        PSG_ALLOC(s->direct_ws, need);
+        s->direct_bytes = need;
+    }
+    double* const part = s->direct_ws;
+    double* const dout = ho ? part + part_n : out;
+    const uint32_t* dt = targets;
+    if (ht) {
+        uint32_t* const d = (uint32_t*)(part + part_n + n_t * 3);
+        PSG_CHECK(cudaMemcpyAsync(d, targets, n_t * 4, cudaMemcpyHostToDevice, st));
+        dt = d;
+    }
+    psg::launch_direct_pack(src[0], src[1], src[2], src[3], n, s->xyzm, st);
     psg::launch_direct_f64(s->xyzm, n, dt, n_t, dout, s->sms * 8, st, part, part_n);
     PSG_CHECK(cudaGetLastError());
     if (ho) PSG_CHECK(cudaMemcpyAsync(out, dout, n_t * 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
     PSG_CHECK(cudaStreamSynchronize(st));
-    cudaFree(part);
-    if (ht) cudaFree(dt);
-    if (ho) cudaFree(dout);
     return PSG_OK;
 }
 
