@@ -90,10 +90,12 @@ struct SmemLeaf {
     float4 sG0[8];          // closure order 1: the children's field gradients
     float2 sG1[8];
     uint2 cpart[8];         // the children's particle ranges
+    // staged P2P sources: leaves (p2p_node), or, where neighbours are merged and
+    // in stream_p2p, their first particle and count (p2p_range)
     uint2 p2p_range[kP2PCap];
+    uint32_t p2p_node[kP2PCap];
     uint32_t cand_node[kCandBuf];
     uint32_t stk_node[kStackCap];
-    uint32_t p2p_node[kP2PCap];
     uint32_t chunk_next, chunk_end;
     // DENSE: the group's source list so far -- chunks in the open segment,
     // segments recorded, the first and the latest recorded segment's slots
@@ -192,9 +194,9 @@ __device__ __forceinline__ uint32_t next_run(const SmemLeaf& sm, uint32_t& m, ui
 // warp's last segment), so that the records of a shallow leaf, whose list
 // reaches most of the tree, are shared out over many warps; the segments'
 // sums meet in slots (DenseStore).  One warp per whole list took 7.7 of a
-// 131K closure tick's 9.9 ms, as segments 0.9 ms; 32 chunks (at most 1,024
-// source leaves) keep a record to tens of microseconds while most lists of a
-// 1M tick stay whole.  part: the list is one of several warps' (a split
+// 131K closure tick's 9.9 ms, as segments 0.8 ms; 32 chunks (at most 1,024
+// sources) keep a record to tens of microseconds while most lists of a 1M tick
+// stay whole (16 chunks: 3 % faster at 131K, 2 % slower at 1M).  part: the list is one of several warps' (a split
 // group, whose last warp links the lists and fills in the items).
 // Record: {fc, phead, first particle, count | run's child mask << 8}, slot or
 // kNone.
@@ -286,14 +288,21 @@ __device__ __noinline__ void link_split(SmemLeaf& sm, const TravArgs& A, uint32_
     __syncwarp();
 }
 
+// a listed P2P source's particles: first, count
+__device__ __forceinline__ uint2 source_range(const TreeView& tv, uint2 r) {
+    if (r.y != kNone) return r;
+    const uint4 si = tv.info[r.x];
+    return make_uint2(si.x, si.y);
+}
+
 // Spill the group's staged P2P sources [0, fill) to HBM chunks of
-// kP2PChunk (node, child mask) entries, chained to the group's earlier
+// kP2PChunk (particle range, child mask) entries, chained to the group's earlier
 // chunks.  Warp-collective; chunk ids come from a per-warp pool.  Returns the
 // new chain head.  record: the list is for k_dense_p2p, so after kSegChunks
 // chunks a segment is recorded and the chain starts over.
 __device__ __noinline__ uint32_t spill_p2p(SmemLeaf& sm, uint32_t fill, uint32_t head,
                                            const TravArgs& A, uint32_t tgt_mask, uint32_t fc,
-                                           bool record) {
+                                           bool record, bool merged) {
     const uint32_t lane = lane_id();
     const P2PStore& st = A.p2p;
     Status* status = A.status;
@@ -317,7 +326,8 @@ __device__ __noinline__ uint32_t spill_p2p(SmemLeaf& sm, uint32_t fill, uint32_t
         const uint32_t cnt = min((uint32_t)kP2PChunk, fill - e0);
         if (c < st.cap_chunks) {
             if (lane < cnt) {
-                st.src[(size_t)c * kP2PChunk + lane] = sm.p2p_node[e0 + lane];
+                st.src[(size_t)c * kP2PChunk + lane] =
+                    merged ? sm.p2p_range[e0 + lane] : make_uint2(sm.p2p_node[e0 + lane], kNone);
                 st.mask[(size_t)c * kP2PChunk + lane] = sm.p2p_mask[e0 + lane];
             }
             if (lane == 0) {
@@ -386,10 +396,8 @@ __device__ __noinline__ void stream_p2p(SmemLeaf& sm, const TravArgs& o, uint32_
                                         uint32_t fc, uint32_t pfill, uint32_t phead, bool accum,
                                         bool fin, unsigned long long& inter) {
     const uint32_t lane = lane_id();
-    for (uint32_t e = lane; e < pfill; e += 32) {
-        const uint4 si = o.tv.info[sm.p2p_node[e]];
-        sm.p2p_range[e] = make_uint2(si.x, si.y);
-    }
+    for (uint32_t e = lane; e < pfill; e += 32)
+        sm.p2p_range[e] = source_range(o.tv, make_uint2(sm.p2p_node[e], kNone));
     __syncwarp();
     uint32_t total = 0;
     for (uint32_t m = tgt_mask; m; m &= m - 1) total += sm.cpart[__ffs(m) - 1].y;
@@ -424,9 +432,9 @@ __device__ __noinline__ void stream_p2p(SmemLeaf& sm, const TravArgs& o, uint32_
             const uint32_t n = o.p2p.cnt[c];
             for (uint32_t e = slice; e < n; e += S) {
                 if ((o.p2p.mask[(size_t)c * kP2PChunk + e] >> q) & 1u) {
-                    const uint4 si = o.tv.info[o.p2p.src[(size_t)c * kP2PChunk + e]];
-                    p2p_range(o.xyzm, make_uint2(si.x, si.y), t, o.kahan, bx, by, bz, cx, cy, cz);
-                    used += si.y;
+                    const uint2 r = source_range(o.tv, o.p2p.src[(size_t)c * kP2PChunk + e]);
+                    p2p_range(o.xyzm, r, t, o.kahan, bx, by, bz, cx, cy, cz);
+                    used += r.y;
                 }
             }
         }
@@ -477,7 +485,7 @@ __device__ __noinline__ void stream_p2p(SmemLeaf& sm, const TravArgs& o, uint32_
 template <bool DEBUG, bool GRAD, bool DENSE>
 __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const TravArgs& o, uint32_t tgt_mask,
                                            uint32_t fc, uint32_t pfill, uint32_t phead,
-                                           bool stream, bool flushed,
+                                           bool merged, bool stream, bool flushed,
                                            unsigned long long inter) {
     const uint32_t lane = lane_id();
     Status* status = o.status;
@@ -490,7 +498,7 @@ __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const TravArgs& o, u
     } else {
         // the group's whole source list to HBM chunks, then k_dense_p2p work
         // records of up to kDenseTargets target particles
-        if (pfill) phead = spill_p2p(sm, pfill, phead, o, tgt_mask, fc, true);
+        if (pfill) phead = spill_p2p(sm, pfill, phead, o, tgt_mask, fc, true, merged);
         record_dense(sm, o.dense, tgt_mask, fc, phead, true, false, status);
     }
     if (DEBUG && lane == 0) {
@@ -542,16 +550,25 @@ __device__ __noinline__ bool wait_ready(const uint32_t* flag, Status* status) {
 // takes every kSplitParts-th candidate and what lies below it), on trees of
 // either kind; their P2P always goes to k_dense_p2p.  A launch of its own
 // beside the rest, so that the other variants keep their registers.
-enum { VAR_PLAIN = 0, VAR_XL = 1, VAR_SPLIT = 2 };
+// MERGE (leaf pass only): the dense variant for leaf capacities of kDenseCap and
+// more (SPLIT_MERGE: of the split groups), which lists neighbouring source
+// leaves as one range, so that k_dense_p2p walks fewer entries (5.51 against 6.17 ms of
+// P2P in a 1M closure tick, 5.36 against 6.10 in a 250K one at theta 10, for
+// 0.18 and 0.08 ms of leaf pass).  One-particle leaves are listed singly:
+// merging cost a 100K tick at theta 8 and leaf capacity 1 0.45 ms of leaf pass.
+// The dense variants run 4 blocks per SM (128 registers; 3 blocks: 3.48 against
+// 2.88 ms of leaf pass in that tick, 6: 3.42).
+enum { VAR_PLAIN = 0, VAR_XL = 1, VAR_SPLIT = 2, VAR_MERGE = 3, VAR_SPLIT_MERGE = 4 };
 
 template <int MODE, bool DEBUG, bool GRAD, bool DENSE, int VAR>
 __global__ void __launch_bounds__(
     kTravThreads,
     (DEBUG || VAR == VAR_XL) ? 1
     : MODE == MODE_INTERNAL  ? (GRAD ? 4 : 5)
-                             : (GRAD ? 4 : (DENSE ? 1 : 7)))
+                             : (GRAD ? 4 : (DENSE ? 4 : 7)))
     k_trav(const __grid_constant__ TravArgs A) {
-    constexpr bool XL = VAR == VAR_XL, SPLIT = VAR == VAR_SPLIT;
+    constexpr bool XL = VAR == VAR_XL, SPLIT = VAR == VAR_SPLIT || VAR == VAR_SPLIT_MERGE;
+    constexpr bool MERGE = VAR == VAR_MERGE || VAR == VAR_SPLIT_MERGE;
     constexpr bool COMPACT = MODE == MODE_INTERNAL || !DENSE;
     using Smem = typename SmemOf<MODE>::T;
     __shared__ Smem smem[kTravWarps];
@@ -567,7 +584,7 @@ __global__ void __launch_bounds__(
     if (MODE == MODE_LEAF && (status->err & PSG_ERR_NS_OVERFLOW)) return;
     // the variant for this tree (batched systems: each group takes its
     // system's variant, so a system sums exactly as it does alone)
-    if (MODE == MODE_LEAF && !SPLIT && !tv.part_sys &&
+    if (MODE == MODE_LEAF && !SPLIT && !MERGE && !tv.part_sys &&
         ((status->max_leaf >= kDenseSwitch || A.leaf_cap >= kDenseCap) != DENSE))
         return;
     // a shallower level's near lists did not fit: this level's are void
@@ -604,7 +621,9 @@ __global__ void __launch_bounds__(
         cum[kMaxDepth] = total;
         // batched systems run both variants over all groups, each with its
         // own counter (work[1] is no internal level's); one system: work[0]
-        work = SPLIT ? &status->run.heavy_work : &status->run.work[(tv.part_sys && DENSE) ? 1 : 0];
+        work = SPLIT   ? (MERGE ? &status->run.split_work : &status->run.heavy_work)
+               : MERGE ? &status->run.work[kLevels]
+                       : &status->run.work[(tv.part_sys && DENSE) ? 1 : 0];
     }
     if (lane == 0) {
         if constexpr (MODE == MODE_INTERNAL) {
@@ -661,12 +680,14 @@ __global__ void __launch_bounds__(
             if (tv.part_sys) {
                 gsys = tv.part_sys[tv.info[pid].x];
                 th2 = tv.sys_theta2[gsys];
-                if (SPLIT && (int)dp >= tv.sys_shallow[gsys]) continue;
-                if (MODE == MODE_LEAF && !SPLIT &&
-                    ((int)dp < tv.sys_shallow[gsys] ||
-                     ((tv.sys_maxleaf[gsys] >= kDenseSwitch || tv.sys_cap[gsys] >= kDenseCap) !=
-                      DENSE)))
-                    continue;
+                const bool many = tv.sys_cap[gsys] >= kDenseCap;
+                if (SPLIT && ((int)dp >= tv.sys_shallow[gsys] || many != MERGE)) continue;
+                if (MODE == MODE_LEAF && !SPLIT) {
+                    const bool dense = many || tv.sys_maxleaf[gsys] >= kDenseSwitch;
+                    if ((int)dp < tv.sys_shallow[gsys] ||
+                        (MERGE ? !many : (DENSE && !XL) ? !dense || many : dense != DENSE))
+                        continue;
+                }
             }
             uint32_t cl = 0;
             float4 cg = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1075,23 +1096,50 @@ __global__ void __launch_bounds__(
                         const uint32_t pbits = sleaf ? near_bits : 0u;
                         const uint32_t pb = __ballot_sync(0xFFFFFFFFu, pbits != 0);
                         if (pb) {
-                            if (pfill + __popc(pb) > (uint32_t)kP2PCap) {
+                            // neighbouring leaves that follow one another in
+                            // memory and serve the same children (siblings, as
+                            // a rule) make one source range, which ends with the
+                            // last source before the next one's
+                            uint32_t hb = pb;
+                            uint2 r = make_uint2(0u, 0u);
+                            if (MERGE) {
+                                uint32_t end = 0;
+                                if (pbits) {
+                                    const uint4 si = tv.info[s];
+                                    r.x = si.x;
+                                    end = si.x + si.y;
+                                }
+                                const uint32_t below = pb & lt_mask;
+                                const int prev = below ? 31 - __clz(below) : (int)lane;
+                                const uint32_t pe = __shfl_sync(0xFFFFFFFFu, end, prev),
+                                               pm = __shfl_sync(0xFFFFFFFFu, pbits, prev);
+                                hb = __ballot_sync(0xFFFFFFFFu,
+                                                   pbits && !(below && pm == pbits && pe == r.x));
+                                const uint32_t after = hb & ~(lt_mask | (1u << lane));
+                                const uint32_t upto =
+                                    after ? pb & ((after & (0u - after)) - 1u) : pb;
+                                r.y = __shfl_sync(0xFFFFFFFFu, end, 31 - __clz(upto)) - r.x;
+                            }
+                            if (pfill + __popc(hb) > (uint32_t)kP2PCap) {
                                 if (XL && A.stream) {
                                     stream_p2p<DEBUG, GRAD>(sm, A, tgt_mask, fc, pfill, kNone,
                                                             flushed, false, sinter);
                                     flushed = true;
                                 } else {
-                                    phead = spill_p2p(sm, pfill, phead, A, tgt_mask, fc,
-                                                      DENSE);
+                                    phead = spill_p2p(sm, pfill, phead, A, tgt_mask, fc, DENSE,
+                                                      MERGE);
                                 }
                                 pfill = 0;
                             }
-                            if (pbits) {
-                                const uint32_t pos = pfill + __popc(pb & lt_mask);
-                                sm.p2p_node[pos] = s;
+                            if (MERGE ? ((hb >> lane) & 1u) : pbits) {
+                                const uint32_t pos = pfill + __popc(hb & lt_mask);
+                                if (MERGE)
+                                    sm.p2p_range[pos] = r;
+                                else
+                                    sm.p2p_node[pos] = s;
                                 sm.p2p_mask[pos] = (uint8_t)pbits;
                             }
-                            pfill += __popc(pb);
+                            pfill += __popc(hb);
                             if (DEBUG) {
                                 const uint32_t pany = __reduce_or_sync(0xFFFFFFFFu, pbits);
                                 for (uint32_t m = pany; m; m &= m - 1) {
@@ -1162,7 +1210,7 @@ __global__ void __launch_bounds__(
                                       (unsigned long long)sm.dbg_p2p[q]);
                         }
                     }
-                    if (pfill) phead = spill_p2p(sm, pfill, phead, A, tgt_mask, fc, true);
+                    if (pfill) phead = spill_p2p(sm, pfill, phead, A, tgt_mask, fc, true, MERGE);
                     if (phead != kNone)
                         record_dense(sm, A.dense, tgt_mask, fc, phead, true, true, status);
                     uint32_t done = 0;
@@ -1259,6 +1307,7 @@ __global__ void __launch_bounds__(
             if constexpr (MODE == MODE_LEAF) {
                 if (SPLIT && parts > 1u) continue;  // (its P2P and L2P: k_dense_p2p)
                 leaf_epilogue<DEBUG, GRAD, DENSE>(sm, A, tgt_mask, fc, pfill, phead,
+                                                  MERGE,
                                                   XL && A.stream != 0, flushed, sinter);
                 if (DEBUG && lane == 0) {
                     const unsigned long long cyc = (unsigned long long)(clock64() - t_group);
@@ -1281,8 +1330,10 @@ __global__ void __launch_bounds__(
 // So targets are padded to the pair only, sources not at all, a source's
 // load and lookup serve all targets, and no source passes through shared
 // memory.  A source that serves only some leaves of the record (its child
-// mask) has its mass zeroed for the other targets; steps whose sources serve
-// all of them skip that.
+// mask) has its mass zeroed for the other targets; such sources are set aside
+// and summed 32 or more at a time, so that every other step skips the masks
+// (one mixed stream, masked wherever a lane needed it: 6.48 against 6.17 ms in
+// the 1M tick below).
 //
 // Bound: the FP32 pipe.  A step on a pair of targets is 12 paired FP32
 // instructions of two cycles and 2 MUFU; alone in a loop that takes 32 cycles
@@ -1292,20 +1343,22 @@ __global__ void __launch_bounds__(
 // hide the chain's latency.  Measured at 1M clumpy, theta 6.25, leaf capacity
 // 16 (8.2 G pairs): closure tick 14.2 -> 13.0 ms against lanes that owned
 // targets, with sources staged in shared-memory tiles and a second walk per
-// leaf for partly wanted sources.
+// leaf for partly wanted sources; with the masked sources apart and merged
+// source leaves this kernel takes 5.5 ms of it (1.5e12 pairs/s).
 //
 // Sums are taken in chain order, the lanes and the segments added in a fixed
 // order, so the result does not depend on scheduling.
 
 // a spilled chunk as one lane sees it: the chunk's entry count and link,
-// and the lane's entry (its source leaf and child mask; slots past the count
-// hold stale values and are not used)
+// and the lane's entry (its source and child mask; slots past the count hold
+// stale values and are not used)
 struct ChunkHead {
-    uint32_t cnt, next, src, mask;
+    uint32_t cnt, next, mask;
+    uint2 src;
 };
 
 __device__ __forceinline__ ChunkHead load_chunk(const P2PStore& st, uint32_t c, uint32_t lane) {
-    ChunkHead h{0u, kNone, 0u, 0u};
+    ChunkHead h{0u, kNone, 0u, make_uint2(0u, 0u)};
     if (c != kNone) {
         h.cnt = st.cnt[c];
         h.next = st.next[c];
@@ -1328,6 +1381,8 @@ struct DensePair<true> {
 
 struct DenseSmem {
     uint2 ent[32];
+    uint2 part[64];   // partly wanted entries: first particle, particles
+    uint16_t ptm[64]; // ... and the targets that want them
     float4 txy[kDenseTargets / 2];  // a pair's targets, negated: x, x', y, y'
     float2 tz[kDenseTargets / 2];
 };
@@ -1372,23 +1427,43 @@ __device__ __forceinline__ void dense_pair(DensePair<KAHAN>& a, const DenseSmem&
 }
 
 constexpr int kDensePairs = (int)kDenseTargets / 2;
-constexpr int kDenseBlock = 4;
+constexpr int kDenseBlock = 2;
 
 // one step: a lane's source p on the record's np target pairs, kDenseBlock
-// pairs at a time (their chains of dependent instructions overlap)
+// pairs at a time (their chains of dependent instructions overlap; 1 or 4 at a
+// time: 6.87 and 6.48 against 6.17 ms in the 1M tick below).  MASKED: tm
+// are the targets that want p, want those that any lane's source is wanted by.
 template <bool KAHAN, bool MASKED>
 __device__ __forceinline__ void dense_step(DensePair<KAHAN> (&a)[kDensePairs],
                                            const DenseSmem& sm, float4 p, uint32_t tm,
-                                           uint32_t np) {
+                                           uint32_t want, uint32_t np) {
 #pragma unroll
     for (int k = 0; k < kDensePairs; k += kDenseBlock) {
-        if (k == 0 || np > (uint32_t)k) {
+        constexpr uint32_t block = (1u << (2 * kDenseBlock)) - 1u;
+        if (MASKED ? ((want >> (2 * k)) & block) != 0u : (k == 0 || np > (uint32_t)k)) {
 #pragma unroll
             for (int j = 0; j < kDenseBlock; ++j)
                 dense_pair<KAHAN, MASKED>(a[k + j], sm, p, tm, k + j);
         }
     }
 }
+
+// Entries of source leaves held one per lane (en particles, 0: none), laid end
+// to end from position start; ent holds each one's first particle less its
+// start (and its targets), compacted past empty entries.
+struct DenseRun {
+    uint32_t en, start, before, b;
+    // the entry (in ent) of this lane's position b + lane: the last to start at
+    // or before it; warp-collective, for successive b
+    __device__ __forceinline__ uint32_t entry(uint32_t le_mask) {
+        const uint32_t d = start - b;
+        const uint32_t bits =
+            __reduce_or_sync(0xFFFFFFFFu, (en != 0u && d < 32u) ? 1u << d : 0u);
+        const uint32_t e = before + __popc(bits & le_mask);
+        before += __popc(bits);
+        return e ? e - 1u : 0u;
+    }
+};
 
 // one record
 template <bool KAHAN>
@@ -1433,89 +1508,109 @@ __device__ __forceinline__ void dense_record(const TravArgs& A, DenseSmem& sm, u
     // chunks one ahead: the next chunk's source ranges and the header after
     // it are in flight while a chunk is summed
     auto src_range = [&](const ChunkHead& hh) -> uint2 {
-        if (lane < hh.cnt && (hh.mask & leaves) != 0u) {
-            const uint4 si = tv.info[hh.src];
-            return make_uint2(si.x, si.y);
-        }
+        if (lane < hh.cnt && (hh.mask & leaves) != 0u) return source_range(tv, hh.src);
         return make_uint2(0u, 0u);
     };
     ChunkHead h = load_chunk(A.p2p, rec.y, lane);
     uint2 hr = src_range(h);
     ChunkHead hn = load_chunk(A.p2p, h.next, lane);
     uint32_t c = rec.y;
-    // positions left over from a chunk (fewer than 32) are carried into the
-    // next, and the particle loaded in one step is summed in the next one
-    uint32_t carry = 0, carry_idx = 0, carry_tm = 0;
-    const uint32_t all = (1u << cnt) - 1u;
+    // wholly wanted sources: positions left over from a chunk (fewer than 32)
+    // are carried into the next, and the particle loaded in one step is summed
+    // in the next one
+    uint32_t carry = 0, carry_idx = 0, npart = 0;
     float4 p = none;
-    uint32_t ptm = all;
     for (bool more = true; more;) {
-        uint32_t en = 0, tm = 0, es = 0;
+        uint32_t em = 0, en_all = 0, es = 0;
         more = c != kNone;
         if (more) {
-            const uint32_t em = lane < h.cnt ? (h.mask & leaves) : 0u;
+            em = lane < h.cnt ? (h.mask & leaves) : 0u;
             es = hr.x;
-            en = hr.y;
-            for (uint32_t m = leaves; m; m &= m - 1) {
-                const uint32_t qq = __ffs(m) - 1;
-                const uint32_t v = __shfl_sync(0xFFFFFFFFu, tset, qq);
-                tm |= ((em >> qq) & 1u) ? v : 0u;
-            }
+            en_all = hr.y;
             c = h.next;
             h = hn;
             hr = src_range(h);
             hn = load_chunk(A.p2p, h.next, lane);
         }
-        // the entries' particles laid end to end after the carried ones: entry
-        // e starts at position start; its (particle - position, targets) in
-        // ent, compacted past empty entries
-        const uint32_t incl = warp_incl_scan(en);
-        const uint32_t ptot = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        const uint32_t start = carry + incl - en;
-        const uint32_t full = __ballot_sync(0xFFFFFFFFu, en != 0u);
+        DenseRun w;
+        w.en = em == leaves ? en_all : 0u;
+        w.before = w.b = 0;
+        const uint32_t incl = warp_incl_scan(w.en);
+        const uint32_t total = carry + __shfl_sync(0xFFFFFFFFu, incl, 31);
+        w.start = carry + incl - w.en;
+        const uint32_t full = __ballot_sync(0xFFFFFFFFu, w.en != 0u);
+        // partly wanted entries: collected, and summed when 32 are in
+        const bool partial = em != 0u && em != leaves;
+        const uint32_t pb = __ballot_sync(0xFFFFFFFFu, partial);
         __syncwarp();
-        if (en) sm.ent[__popc(full & lanemask_lt())] = make_uint2(es - start, tm);
+        if (w.en) sm.ent[__popc(full & lanemask_lt())].x = es - w.start;
+        if (pb) {
+            uint32_t tm = 0;
+            for (uint32_t m = leaves; m; m &= m - 1) {
+                const uint32_t qq = __ffs(m) - 1;
+                const uint32_t v = __shfl_sync(0xFFFFFFFFu, tset, qq);
+                tm |= ((em >> qq) & 1u) ? v : 0u;
+            }
+            if (partial) {
+                const uint32_t pos = npart + __popc(pb & lanemask_lt());
+                sm.part[pos] = make_uint2(es, en_all);
+                sm.ptm[pos] = (uint16_t)tm;
+            }
+            npart += __popc(pb);
+            if (A.debug) inter += partial ? (unsigned long long)en_all * __popc(tm) : 0ull;
+        }
         __syncwarp();
-        if (A.debug) inter += (unsigned long long)en * __popc(tm);
-        const uint32_t total = carry + ptot;
+        if (A.debug) inter += (unsigned long long)w.en * cnt;
         // at the chain's end: the remainder, and the step that sums it
         const uint32_t steps = more ? total >> 5 : ((total + 31u) >> 5) + 1u;
-        uint32_t before = 0;  // entries that start before the step's positions
-        uint32_t b = 0;
-        // lane's source at position b + lane: its entry is the last to start
-        // at or before it
-        auto locate = [&](uint32_t& idx, uint32_t& mask) {
-            const uint32_t d = start - b;
-            const uint32_t bits =
-                __reduce_or_sync(0xFFFFFFFFu, (en != 0u && d < 32u) ? 1u << d : 0u);
-            const uint32_t f = b + lane;
-            const uint32_t e = before + __popc(bits & le_mask);
-            const uint2 v = sm.ent[e ? e - 1u : 0u];
-            before += __popc(bits);
-            idx = f < carry ? carry_idx : v.x + f;
-            mask = f < carry ? carry_tm : v.y;
-        };
 #pragma unroll 1
-        for (uint32_t st = 0; st < steps; ++st, b += 32) {
-            uint32_t idx, mask;
-            locate(idx, mask);
-            const bool in = b + lane < total;
-            const float4 pn = in ? xyzm[idx] : none;
-            // most steps' sources serve every leaf of the record
-            if (__all_sync(0xFFFFFFFFu, ptm == all))
-                dense_step<KAHAN, false>(a, sm, p, ptm, np);
-            else
-                dense_step<KAHAN, true>(a, sm, p, ptm, np);
+        for (uint32_t st = 0; st < steps; ++st, w.b += 32) {
+            const uint32_t f = w.b + lane;
+            const uint32_t at = sm.ent[w.entry(le_mask)].x + f;
+            const float4 pn = f < total ? xyzm[f < carry ? carry_idx : at] : none;
+            dense_step<KAHAN, false>(a, sm, p, 0u, 0u, np);
             p = pn;
-            ptm = in ? mask : all;  // (no source: no mass)
         }
-        if (more && b < total) {
-            uint32_t idx, mask;
-            locate(idx, mask);  // (lanes past the remainder are not used)
-            carry_idx = idx;
-            carry_tm = mask;
+        if (more && w.b < total) {
+            const uint32_t f = w.b + lane;
+            const uint32_t at = sm.ent[w.entry(le_mask)].x + f;
+            if (f >= carry) carry_idx = at;  // (lanes past the remainder are not used)
         }
-        carry = more ? total - b : 0u;
+        carry = more ? total - w.b : 0u;
+        while (npart >= 32u || (!more && npart)) {
+            const uint32_t take = min(npart, 32u);
+            __syncwarp();
+            const uint2 e0 = lane < take ? sm.part[lane] : make_uint2(0u, 0u);
+            const uint32_t t0 = sm.ptm[lane];
+            const uint2 e1 = sm.part[32 + lane];
+            const uint16_t t1 = sm.ptm[32 + lane];
+            __syncwarp();
+            sm.part[lane] = e1;
+            sm.ptm[lane] = t1;
+            npart -= take;
+            DenseRun v;
+            v.en = e0.y;
+            v.before = v.b = 0;
+            const uint32_t pincl = warp_incl_scan(v.en);
+            const uint32_t ptot = __shfl_sync(0xFFFFFFFFu, pincl, 31);
+            v.start = pincl - v.en;
+            const uint32_t pfull = __ballot_sync(0xFFFFFFFFu, v.en != 0u);
+            if (v.en) sm.ent[__popc(pfull & lanemask_lt())] = make_uint2(e0.x - v.start, t0);
+            __syncwarp();
+            float4 pp = none;
+            uint32_t tm = 0;
+#pragma unroll 1
+            for (; v.b < ptot + 32u; v.b += 32) {
+                const uint32_t f = v.b + lane;
+                const uint2 at = sm.ent[v.entry(le_mask)];
+                const bool in = f < ptot;
+                const float4 pn = in ? xyzm[at.x + f] : none;
+                const uint32_t want = __reduce_or_sync(0xFFFFFFFFu, tm);
+                dense_step<KAHAN, true>(a, sm, pp, tm, want, np);
+                pp = pn;
+                tm = in ? at.y : 0u;
+            }
+        }
     }
     // the lanes' sums; lane k keeps target k's
     double bx = 0.0, by = 0.0, bz = 0.0;
@@ -2071,20 +2166,22 @@ void launch_traverse_internal(const TravArgs& args, int level, int level_end, in
     launch_mode<MODE_INTERNAL, false, VAR_PLAIN>(A, grid, st);
 }
 
-// which: 1 the sparse variant, 2 the dense one, 3 both (each returns at once
-// unless the tree is its kind)
+// which: 1 the variants for leaf capacities below kDenseCap (sparse and dense:
+// each returns at once unless the tree is its kind), 2 the one for the others
 void launch_traverse_leaves(const TravArgs& args, const int grid[2], int which, cudaStream_t st) {
     if (leaf_xl(args)) {
         if (which & 1) launch_mode<MODE_LEAF, false, VAR_XL>(args, grid[0], st);
-        if (which & 2) launch_mode<MODE_LEAF, true, VAR_XL>(args, grid[1], st);
+        launch_mode<MODE_LEAF, true, VAR_XL>(args, grid[1], st);
     } else {
         if (which & 1) launch_mode<MODE_LEAF, false, VAR_PLAIN>(args, grid[0], st);
-        if (which & 2) launch_mode<MODE_LEAF, true, VAR_PLAIN>(args, grid[1], st);
+        if (which & 1) launch_mode<MODE_LEAF, true, VAR_PLAIN>(args, grid[1], st);
+        if (which & 2) launch_mode<MODE_LEAF, true, VAR_MERGE>(args, grid[1], st);
     }
 }
 
-void launch_traverse_split(const TravArgs& args, int grid, cudaStream_t st) {
-    launch_mode<MODE_LEAF, true, VAR_SPLIT>(args, grid, st);
+void launch_traverse_split(const TravArgs& args, int grid, int which, cudaStream_t st) {
+    if (which & 1) launch_mode<MODE_LEAF, true, VAR_SPLIT>(args, grid, st);
+    if (which & 2) launch_mode<MODE_LEAF, true, VAR_SPLIT_MERGE>(args, grid, st);
 }
 
 int traverse_threads() { return kTravThreads; }

@@ -91,15 +91,17 @@ struct Status {
         uint32_t dense_work;               // ... and taken by k_dense_p2p
         uint32_t dense_slots;              // slots taken by records of split source lists
         uint32_t heavy_work;               // shallow groups taken
+        uint32_t split_work;               // ... by the variant that merges leaves
         uint32_t ns_fail;                  // bit k: level k's near lists did not fit
     } run;
 };
 
-// P2P sources spilled from the traversal: chunk c holds cnt[c] source-leaf
-// ids in src[c * kP2PChunk ...], each with the set of the group's children it
-// serves in mask[...], and links to the group's previous chunk via next[c].
+// P2P sources spilled from the traversal: chunk c holds cnt[c] sources in
+// src[c * kP2PChunk ...] (a leaf and kNone, or the first particle and count of
+// merged leaves), each with the set of the group's children it serves in
+// mask[...], and links to the group's previous chunk via next[c].
 struct P2PStore {
-    uint32_t* src;
+    uint2* src;
     uint8_t* mask;
     uint32_t* next;
     uint32_t* cnt;

@@ -71,7 +71,7 @@ void launch_traverse_internal(const TravArgs& A, int level, int level_end, int g
 void launch_traverse_leaves(const TravArgs& A, const int grid[2], int which, cudaStream_t st);
 void launch_dense_p2p(const TravArgs& A, int grid, cudaStream_t st);
 void launch_heavy_leaf(const TravArgs& A, int grid, cudaStream_t st);
-void launch_traverse_split(const TravArgs& A, int grid, cudaStream_t st);
+void launch_traverse_split(const TravArgs& A, int grid, int which, cudaStream_t st);
 
 
 // k_tick.cu -- the caller's tick loop on the device (README.md:65-111)

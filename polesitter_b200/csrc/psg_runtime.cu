@@ -111,7 +111,7 @@ struct State {
     P2PStore p2p;
     DenseStore dense;      // full-leaf P2P work records
     SplitStore split;      // sums of the groups that several warps share
-    bool dense_only;       // many systems: every one takes the dense leaf variant
+    int forest_caps;       // many systems: leaf capacities below kDenseCap (1), others (2)
     int forest_split;      // many systems: the deepest of their split depths
     const int32_t* sys_heavy;  // ... and each one's shallow-leaf and split depth
     const int32_t* sys_split;
@@ -196,10 +196,11 @@ static int alloc_p2p(State* s, uint32_t chunks) {
     void* ps[4] = {s->p2p.src, s->p2p.mask, s->p2p.next, s->p2p.cnt};
     for (void* p : ps)
         if (p) cudaFree(p);
-    s->p2p.src = s->p2p.next = s->p2p.cnt = nullptr;
+    s->p2p.src = nullptr;
+    s->p2p.next = s->p2p.cnt = nullptr;
     s->p2p.mask = nullptr;
     s->p2p.cap_chunks = 0;
-    PSG_ALLOC(s->p2p.src, (size_t)chunks * kP2PChunk * 4);
+    PSG_ALLOC(s->p2p.src, (size_t)chunks * kP2PChunk * sizeof(uint2));
     PSG_ALLOC(s->p2p.mask, (size_t)chunks * kP2PChunk);
     PSG_ALLOC(s->p2p.next, (size_t)chunks * 4);
     PSG_ALLOC(s->p2p.cnt, (size_t)chunks * 4);
@@ -592,6 +593,8 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
         const int v = (int)(g * gs);
         return v < 1 ? 1 : v;
     };
+    // leaf capacities below kDenseCap (1), others (2), systems of both kinds (3)
+    const int caps = forest ? s->forest_caps : s->leaf_cap >= kDenseCap ? 2 : 1;
     // The shallow groups on the aux stream.  They read the near lists and
     // fields of the nodes above `depth`, final once the internal level of
     // depth - 1 is done, so they start there and run beside the deeper levels
@@ -605,7 +608,7 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
         } else {
             TravArgs S = A;
             S.shallow = depth;
-            launch_traverse_split(S, scaled(s->sms * kSplitBlocksPerSm), s->aux);
+            launch_traverse_split(S, scaled(s->sms * kSplitBlocksPerSm), caps, s->aux);
         }
         PSG_CHECK(cudaEventRecord(s->ev_heavy, s->aux));
         started = true;
@@ -635,7 +638,7 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
         if (r != PSG_OK) return r;
     }
     const int lg[2] = {scaled(s->trav_grid[o][0][xl]), scaled(s->trav_grid[o][1][xl])};
-    launch_traverse_leaves(A, lg, s->dense_only ? 2 : s->leaf_cap >= kDenseCap ? 2 : 3, s->stream);
+    launch_traverse_leaves(A, lg, caps, s->stream);
     record(s, PH_DENSE);
     // (the split groups' records too; k_heavy_leaf leaves none)
     if (depth && !heavy) PSG_CHECK(cudaStreamWaitEvent(s->stream, s->ev_heavy, 0));
@@ -740,7 +743,7 @@ static int regrow(State* s, uint32_t err) {
         // the chunk counter is 32-bit: below the capacity it has wrapped
         const unsigned long long used = s->h_status->run.p2p_chunks;
         const unsigned long long need = used < s->p2p.cap_chunks ? ~0ull : 2 * used + 1024;
-        const unsigned long long per = kP2PChunk * 5 + 8;
+        const unsigned long long per = kP2PChunk * 9 + 8;
         const unsigned long long limit =
             std::min(0x7FFFFFFFull, store_budget(s->p2p.cap_chunks * per) / per);
         if (!(need <= limit && try_alloc_p2p(s, (uint32_t)need))) s->stream_p2p = 1;
@@ -1290,13 +1293,13 @@ static int upload_systems(Ensemble* e) {
     std::vector<float> th2(e->nsys);
     std::vector<int32_t> hv(e->nsys), sp(e->nsys);
     int hmax = 0, smax = 0;
-    bool dense_only = true;
+    int caps = 0;
     for (size_t k = 0; k < e->nsys; ++k) {
         const float t = e->theta[k];
         th2[k] = t * t;
         hv[k] = heavy_depth_of(t, e->count[k]);
         hmax = std::max(hmax, (int)hv[k]);
-        dense_only = dense_only && e->cap[k] >= kDenseCap;
+        caps |= e->cap[k] >= kDenseCap ? 2 : 1;
         sp[k] = split_depth_of(t, e->count[k], e->cap[k]);
         smax = std::max(smax, (int)sp[k]);
     }
@@ -1306,8 +1309,8 @@ static int upload_systems(Ensemble* e) {
     PSG_CHECK(cudaMemcpy(e->sys_cap, e->cap.data(), e->nsys * 4, cudaMemcpyHostToDevice));
     if (hmax != e->fs->forest_heavy) e->dirty = true;  // a launch parameter changes
     e->fs->forest_heavy = hmax;
-    if (smax != e->fs->forest_split || dense_only != e->fs->dense_only) e->dirty = true;
-    e->fs->dense_only = dense_only;
+    if (smax != e->fs->forest_split || caps != e->fs->forest_caps) e->dirty = true;
+    e->fs->forest_caps = caps;
     e->fs->forest_split = smax;
     const SplitStore before = e->fs->split;  // (allocated here: not while capturing)
     const int r = ensure_split(e->fs, smax);
