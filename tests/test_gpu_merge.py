@@ -55,3 +55,26 @@ def test_merged_source_leaves_match_oracle(oracle, make, theta, cap, order, kaha
     F = np.stack([b.fx, b.fy, b.fz], 1).astype(np.float64)
     G = np.stack([a.fx, a.fy, a.fz], 1).astype(np.float64)
     assert rel_l2(F, G) < FORCE_REL_L2
+
+
+def test_many_short_records_match_streamed_sums():
+    """So many full-leaf P2P records that they are loaded ahead: against the
+    sums taken in the leaf pass itself."""
+    n = 1 << 20
+    p = W.clumpy_plummer(n, 24)
+    for k in ("x", "y", "z"):
+        a = getattr(p, k)
+        a[1000:1040] = a[1000]  # one leaf of 40: every group takes the recorded path
+    out = []
+    for stream in (0, 1):
+        b = p.copy()
+        with P.Context(n, theta=1.0) as ctx:
+            ctx.set_option(P.OPT_DEBUG, 1)
+            ctx.set_option(P.OPT_STREAM, stream)
+            ctx.tick(b, np.zeros(n, np.uint32))
+            out.append((np.stack([b.fx, b.fy, b.fz], 1).astype(np.float64), b.id, ctx.stats()))
+    (F, fi, fs), (G, gi, gs) = out
+    assert fs["dense_records"] >= 64 * 148 * 16  # from here on they are loaded ahead
+    assert fs["p2p_interactions"] == gs["p2p_interactions"]
+    assert np.array_equal(fi, gi)
+    assert rel_l2(F, G) < FORCE_REL_L2
