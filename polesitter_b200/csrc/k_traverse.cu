@@ -63,8 +63,6 @@ constexpr int kCandBuf = 256;             // children of 32 opened entries
 constexpr int kStackCap = 384;            // DFS stack (node, child mask)
 constexpr int kStackSlack = 72;           // 9 levels x 7: growth of a single-entry descent
 constexpr int kP2PCap = 128;              // staged P2P sources of a group
-constexpr uint32_t kNsPool = 4096;        // near-list entries a warp reserves at once
-constexpr uint32_t kChunkPool = 16;       // P2P spill chunks a warp reserves at once
 constexpr uint32_t kSegChunks = 32;       // chunks of source list per dense work record
 constexpr uint32_t kDenseSwitch = 32;     // fullest leaf from which the DENSE leaf pass runs
 

@@ -152,6 +152,8 @@ namespace psg {
 // k_dense_p2p: blocks per SM, warps per block, target particles of a record
 constexpr int kDenseBlocksPerSm = 4;
 constexpr int kDenseWarpsPerBlock = 4;
+constexpr uint32_t kNsPool = 4096;   // near-list entries a warp reserves at once
+constexpr uint32_t kChunkPool = 16;  // P2P spill chunks a warp reserves at once
 constexpr int kDenseThreads = 32 * kDenseWarpsPerBlock;
 constexpr uint32_t kDenseTargets = 16;
 // leaf capacity from which a tree takes the leaf pass's DENSE variant whatever
