@@ -672,7 +672,7 @@ __global__ void __launch_bounds__(
             const uint32_t nc = plink >> 28;
             const uint32_t fc = plink & kLinkMask;
             // batched systems: the group's own system, theta and root; its
-            // shallow leaves belong to k_heavy_leaf
+            // shallow leaves belong to the split groups or k_heavy_leaf
             uint32_t gsys = 0;
             float th2 = theta2;
             if (tv.part_sys) {
@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(
                     (unsigned long long)__popc(tgt_mask) * cand_total;
                 __syncwarp();
                 if (need && sm.ns_next + need > sm.ns_end) {
-                    const unsigned long long take = need > kNsPool ? need : kNsPool;
+                    const unsigned long long take = need > A.ns_pool ? need : A.ns_pool;
                     unsigned long long b = 0;
                     if (lane == 0) b = atomicAdd(&status->run.ns_used, take);
                     b = __shfl_sync(0xFFFFFFFFu, b, 0);

@@ -190,6 +190,7 @@ struct TravArgs {
     P2PStore p2p;       // spill chunks of P2P source lists longer than a chunk
     uint32_t* ns;       // near lists of all levels
     unsigned long long ns_cap;
+    uint32_t ns_pool;   // near-list entries a warp reserves at once
     const float4* xyzm;  // sorted particles
     float* fx;          // output forces, sorted order
     float* fy;

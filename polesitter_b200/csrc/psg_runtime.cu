@@ -118,7 +118,7 @@ struct State {
     uint32_t* heavy_frontier;
     uint32_t heavy_fcap;
     int heavy_slots;       // blocks of k_heavy_leaf
-    cudaStream_t aux;      // k_heavy_leaf, beside the leaf pass
+    cudaStream_t aux;      // split groups or k_heavy_leaf, beside the leaf pass
     cudaEvent_t ev_levels, ev_heavy;
     // host-array calls: the sorted arrays (final after the gather) go back to
     // pinned host buffers on their own stream while the traversal runs
@@ -183,6 +183,10 @@ static int grid_for(const State* s, size_t n, int per_block_items) {
     return (int)(want < cap ? want : cap);
 }
 
+// near-list entries a warp reserves at once: a warp of a small system takes few
+// groups, and pools for all warps would dwarf its lists
+static uint32_t ns_pool(size_t n) { return n < 262144 ? kNsPool / 8 : kNsPool; }
+
 static int alloc_ns(State* s, unsigned long long cap) {
     if (s->ns) cudaFree(s->ns);
     s->ns = nullptr;
@@ -192,34 +196,52 @@ static int alloc_ns(State* s, unsigned long long cap) {
     return PSG_OK;
 }
 
+// one allocation for several arrays, the first of which is its address: a
+// cudaMalloc takes some 50-100 us whatever its size (ps_init and ps_destroy of a
+// 64K context together: 17 -> 12 ms)
+struct Carve {
+    size_t total = 0;
+    size_t add(size_t bytes) {
+        const size_t at = total;
+        total += (bytes + 255) & ~(size_t)255;
+        return at;
+    }
+};
+template <typename T>
+static T* carved(void* base, size_t at) {
+    return reinterpret_cast<T*>(static_cast<char*>(base) + at);
+}
+
 static int alloc_p2p(State* s, uint32_t chunks) {
-    void* ps[4] = {s->p2p.src, s->p2p.mask, s->p2p.next, s->p2p.cnt};
-    for (void* p : ps)
-        if (p) cudaFree(p);
-    s->p2p.src = nullptr;
-    s->p2p.next = s->p2p.cnt = nullptr;
-    s->p2p.mask = nullptr;
-    s->p2p.cap_chunks = 0;
-    PSG_ALLOC(s->p2p.src, (size_t)chunks * kP2PChunk * sizeof(uint2));
-    PSG_ALLOC(s->p2p.mask, (size_t)chunks * kP2PChunk);
-    PSG_ALLOC(s->p2p.next, (size_t)chunks * 4);
-    PSG_ALLOC(s->p2p.cnt, (size_t)chunks * 4);
-    s->p2p.cap_chunks = chunks;
+    P2PStore& p = s->p2p;
+    if (p.src) cudaFree(p.src);
+    p = P2PStore{};
+    Carve c;
+    c.add((size_t)chunks * kP2PChunk * sizeof(uint2));
+    const size_t next = c.add((size_t)chunks * 4), cnt = c.add((size_t)chunks * 4),
+                 mask = c.add((size_t)chunks * kP2PChunk);
+    PSG_ALLOC(p.src, c.total);
+    p.next = carved<uint32_t>(p.src, next);
+    p.cnt = carved<uint32_t>(p.src, cnt);
+    p.mask = carved<uint8_t>(p.src, mask);
+    p.cap_chunks = chunks;
     return PSG_OK;
 }
 
 static int alloc_dense(State* s, uint32_t recs, uint32_t slots) {
     DenseStore& d = s->dense;
-    void* ps[4] = {d.rec, d.rec_slot, d.prev, d.sums};
-    for (void* p : ps)
-        if (p) cudaFree(p);
+    if (d.rec) cudaFree(d.rec);
     uint4* const item = d.item;  // (sized by the particles, not by the records)
     d = DenseStore{};
     d.item = item;
-    PSG_ALLOC(d.rec, (size_t)recs * sizeof(uint4));
-    PSG_ALLOC(d.rec_slot, (size_t)recs * 4);
-    PSG_ALLOC(d.prev, (size_t)slots * 4);
-    PSG_ALLOC(d.sums, (size_t)slots * kDenseTargets * 3 * sizeof(double));
+    Carve c;
+    c.add((size_t)recs * sizeof(uint4));
+    const size_t rec_slot = c.add((size_t)recs * 4), prev = c.add((size_t)slots * 4),
+                 sums = c.add((size_t)slots * kDenseTargets * 3 * sizeof(double));
+    PSG_ALLOC(d.rec, c.total);
+    d.rec_slot = carved<uint32_t>(d.rec, rec_slot);
+    d.prev = carved<uint32_t>(d.rec, prev);
+    d.sums = carved<double>(d.rec, sums);
     d.rec_cap = recs;
     d.slot_cap = slots;
     return PSG_OK;
@@ -232,13 +254,15 @@ static int ensure_split(State* s, int depth) {
     for (int d = 0; d < depth; ++d) groups += 2 * s->tv.lvl_cap[d];
     SplitStore& p = s->split;
     if (p.cap >= groups) return PSG_OK;
-    void* ps[3] = {p.sums, p.list, p.count};
-    for (void* q : ps)
-        if (q) cudaFree(q);
+    if (p.sums) cudaFree(p.sums);
     p = SplitStore{};
-    PSG_ALLOC(p.sums, (size_t)groups * kSplitParts * kSplitSums * sizeof(float));
-    PSG_ALLOC(p.list, (size_t)groups * kSplitParts * sizeof(uint4));
-    PSG_ALLOC(p.count, (size_t)groups * 4);
+    Carve c;
+    c.add((size_t)groups * kSplitParts * kSplitSums * sizeof(float));
+    const size_t list = c.add((size_t)groups * kSplitParts * sizeof(uint4)),
+                 count = c.add((size_t)groups * 4);
+    PSG_ALLOC(p.sums, c.total);
+    p.list = carved<uint4>(p.sums, list);
+    p.count = carved<uint32_t>(p.sums, count);
     p.cap = groups;
     return PSG_OK;
 }
@@ -328,11 +352,9 @@ static bool on_device(const void* p) { return place_of(p) == DEVICE; }
 static void free_state(State* s) {
     void* ps[] = {s->xyzm, s->ids, s->sort.key_a, s->sort.key_b, s->sort.val_a, s->sort.val_b,
                   s->sort.hist, s->tree_tiles, s->tv.geo,
-                  s->tv.mp, s->tv.lt, s->tv.info, s->tv.parent, s->tv.arrive, s->tv.cbase,
-                  s->tv.ns_off, s->tv.ns_cnt, s->tv.dbg_m2l, s->tv.dbg_p2p, s->tv.link,
-                  s->tv.ready, s->tv.groups, s->ns, s->p2p.src, s->p2p.mask, s->p2p.next, s->p2p.cnt,
-                  s->d_status, s->dense.rec, s->dense.rec_slot, s->dense.prev, s->dense.sums,
-                  s->direct_ws, s->dense.item, s->split.sums, s->split.list, s->split.count, s->heavy_frontier, s->tk_partial, s->tk_bbox, s->tk_v[0], s->tk_v[1], s->tk_v[2],
+                  s->tv.mp, s->tv.lt, s->tv.info, s->tv.parent, s->tv.arrive, s->ns, s->p2p.src,
+                  s->d_status, s->dense.rec, s->direct_ws, s->dense.item, s->split.sums,
+                  s->heavy_frontier, s->tk_partial, s->tk_bbox, s->tk_v[0], s->tk_v[1], s->tk_v[2],
                   s->tk_vmir[0], s->tk_vmir[1], s->tk_vmir[2], s->cl.lg0, s->cl.lg1,
                   s->cl.leaf_of, s->cl.dF, s->cl.params, s->cl.packed, s->cl.judge_tg,
                   s->cl.judge_f64, s->cl.judge_part, s->cl.d_judge};
@@ -405,15 +427,17 @@ static int init_state(State* s, size_t maxp, float theta, const uint32_t* lvl_ca
     PSG_ALLOC(s->tv.lt, nodes * 16);
     PSG_ALLOC(s->tv.info, nodes * 16);
     PSG_ALLOC(s->tv.parent, nodes * 4);
-    PSG_ALLOC(s->tv.arrive, nodes * 4);
-    PSG_ALLOC(s->tv.cbase, nodes * 4);
-    PSG_ALLOC(s->tv.ns_off, nodes * 4);
-    PSG_ALLOC(s->tv.ns_cnt, nodes * 4);
-    PSG_ALLOC(s->tv.dbg_m2l, nodes * 4);
-    PSG_ALLOC(s->tv.dbg_p2p, nodes * 4);
-    PSG_ALLOC(s->tv.link, nodes * 4);
-    PSG_ALLOC(s->tv.ready, nodes * 4);
-    PSG_ALLOC(s->tv.groups, nodes * 4);
+    {
+        TreeView& t = s->tv;
+        uint32_t** const per_node[] = {&t.arrive,  &t.cbase, &t.ns_off, &t.ns_cnt, &t.dbg_m2l,
+                                       &t.dbg_p2p, &t.link,  &t.ready,  &t.groups};
+        Carve c;
+        for (auto q : per_node) (void)q, c.add(nodes * 4);
+        PSG_ALLOC(t.arrive, c.total);
+        uint32_t* const base = t.arrive;
+        Carve at;
+        for (auto q : per_node) *q = carved<uint32_t>(base, at.add(nodes * 4));
+    }
     PSG_ALLOC(s->d_status, sizeof(Status));
     PSG_CHECK(cudaMallocHost((void**)&s->h_status, sizeof(Status)));
     std::memset(s->h_status, 0, sizeof(Status));
@@ -422,7 +446,7 @@ static int init_state(State* s, size_t maxp, float theta, const uint32_t* lvl_ca
     // first tick of a system of up to some 100K particles was run twice: 1.33
     // against 0.49 ms at 65K, 4.0 against 0.64 at 8K with leaves of 16)
     const unsigned long long warps = std::min<unsigned long long>(n / 4 + 1, s->sms * 20ull);
-    int r = alloc_ns(s, (unsigned long long)(n < 1024 ? 1024 : n) * 48ull + warps * kNsPool);
+    int r = alloc_ns(s, (unsigned long long)(n < 1024 ? 1024 : n) * 48ull + warps * ns_pool(n));
     if (r != PSG_OK) return r;
     r = alloc_p2p(s, (uint32_t)((n < 4096 ? 4096 : n / 4) + warps * kChunkPool));
     if (r != PSG_OK) return r;
@@ -554,6 +578,7 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
     A.p2p = s->p2p;
     A.ns = s->ns;
     A.ns_cap = s->ns_cap;
+    A.ns_pool = ns_pool(s->max_particles);
     A.status = s->d_status;
     A.theta = s->theta;
     A.level = 0;
