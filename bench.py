@@ -86,12 +86,13 @@ WORKLOADS = {
     "plain": ("plain FMM tick (ps_prepare_particles + ps_calc_forces), Plummer sphere "
               "N=1,048,576, a=1, r<=10a, equal mass 1/N, theta=2, float32 SoA"),
 }
-# kernels of this library launched per tick: 2 prepare + 6 sort + gather +
-# write-back + 4 tree + 11 upward + 9 internal levels + leaf-pass start +
-# 2 leaf-pass variants + shallow leaves + full leaves; the closure adds the
-# judge (sample, FP64 direct sum over source splits, their fixed-order sum,
+# kernels of this library launched per 1M tick: 2 prepare + 5 sort + gather +
+# write-back + 4 tree + 4 upward + the internal levels + 2 leaf-pass variants +
+# full leaves; the closure runs one leaf-pass variant, the internal levels in
+# two launches with the split shallow groups between, and adds the judge
+# (sample, FP64 direct sum over source splits, their fixed-order sum,
 # decision), the MLP and the apply kernel
-KERNELS_PER_TICK = {"plain": 39, "closure": 45}
+KERNELS_PER_TICK = {"plain": 21, "closure": 28}
 # DRAM bytes (read + write) of one launch of the dominant kernel, from the
 # ncu captures summarised under profiles/ (None: not captured for this
 # configuration)
@@ -419,7 +420,7 @@ def run_b200(args):
     peaks, peak_src = measured_peaks()
     props = torch.cuda.get_device_properties(dev)
     fp32_peak = props.multi_processor_count * 128 * 2 * float(peaks.get("sm_max_mhz", 1965.0)) * 1e6
-    # the dominant phase: the leaf pass (k_trav leaf + k_heavy_leaf: M2L of
+    # the dominant phase: the leaf pass (k_trav leaf and split groups: M2L of
     # the leaf targets, P2P outside full leaves) or the full-leaf P2P
     # (k_dense_p2p: P2P + L2P of the records)
     m2l_flop = FLOP_M2L_ORDER1 if closure else FLOP_M2L
@@ -430,7 +431,7 @@ def run_b200(args):
                                   ph["full_leaves"], flops_full)
         counts = {"p2p_particle_pairs": p2p_full, "flop_per_p2p": FLOP_P2P}
     else:
-        kern, launch_ms, flops = ("leaf pass: k_trav<MODE_LEAF> + k_heavy_leaf "
+        kern, launch_ms, flops = ("leaf pass: k_trav<MODE_LEAF> "
                                   "(MAC+M2L+L2L+P2P+L2P)", ph["leaves"], flops_leaf)
         counts = {"m2l_pairs_leaf_targets": m2l_leaf,
                   "p2p_particle_pairs": p2p_inter - p2p_full,

@@ -23,8 +23,11 @@ size_t ps_b200_context_size(void);
 #define PS_B200_OPT_CLOSURE 7        /* learned far-field closure, see below */
 #define PS_B200_OPT_JUDGE 8          /* 1: run the closure's judge in mode 1 too */
 #define PS_B200_OPT_HEAVY_DEPTH 9    /* leaves at most this deep (0..5) are walked by a whole
-                                        block each; -1 (default): the largest d with
-                                        2^d <= 4 theta */
+                                        block each; -1 (default): shallow leaves share
+                                        16 warps a group instead, and are walked by
+                                        blocks (to the largest d with 2^d <= 4 theta)
+                                        only where the leaf pass walks ancestor chains
+                                        or streams its P2P */
 #define PS_B200_OPT_LEAF_CAP 10      /* leaf capacity B (1..256): a node below the root
                                         holding more than B particles is split (the
                                         reference: 1, polesitter.h:911); the root is split
