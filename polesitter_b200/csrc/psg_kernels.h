@@ -152,7 +152,7 @@ namespace psg {
 // k_dense_p2p: blocks per SM, warps per block, target particles of a record
 constexpr int kDenseBlocksPerSm = 4;
 constexpr int kDenseWarpsPerBlock = 4;
-constexpr uint32_t kNsPool = 4096;   // near-list entries a warp reserves at once
+constexpr uint32_t kNsPool = 4096;   // near-list entries a warp reserves at once (large systems)
 constexpr uint32_t kChunkPool = 16;  // P2P spill chunks a warp reserves at once
 constexpr int kDenseThreads = 32 * kDenseWarpsPerBlock;
 constexpr uint32_t kDenseTargets = 16;
