@@ -57,6 +57,11 @@ size_t ps_b200_context_size(void);
                                         default 1024).  Its FP64 direct sum costs samples x N
                                         pair terms a tick; the median it decides on has a
                                         relative standard error of ~1/sqrt(samples) */
+#define PS_B200_OPT_READY_SPIN 17    /* test of the traversal's bounded wait: > 0 lets a group
+                                        poll for its parent's near list only this many
+                                        times while the first level publishes its own
+                                        ~200 us late; the tick then returns PS_EDEVICE; 0
+                                        (default) restores the normal limit */
 ps_result_t ps_b200_set_option(ps_context_t* ctx, int key, double value);
 
 /* Morton quantisation of ps_prepare_particles, process-wide (it takes no

@@ -22,13 +22,6 @@ constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagInc = 2u << 30;
 constexpr uint32_t kValMask = (1u << 30) - 1;
 constexpr int kSpinLimit = 1 << 22;
-constexpr unsigned long long kLateNs = 200000;  // the late tile of the wait test: 200 us
-
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
 
 int sort_tile_size() { return kSortTile; }
 
@@ -121,12 +114,9 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_sort_pass(
     uint32_t prefix = 0;
     if (tile == 0) {
         if (late) {
-            // test of the bounded wait: this tile publishes ~200 us late, so
-            // a successor polling fewer times gives up (bounded: at most
-            // 2^20 reads of the clock)
-            const unsigned long long t0 = global_ns();
-            for (int i = 0; i < (1 << 20) && global_ns() - t0 < kLateNs; ++i) {
-            }
+            // test of the bounded wait: this tile publishes late, so a
+            // successor polling fewer times gives up
+            publish_late();
         }
         atomicExch(my, kFlagInc | total);
     } else {

@@ -510,14 +510,19 @@ __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const TravArgs& o, u
 }
 
 // Wait until a node's near list and field are final (ready set by the warp that
-// makes them, in this launch); false after kReadyPolls polls (~0.3 s) or once
-// another wait has given up.  Warp-collective.
-constexpr int kReadyPolls = 1 << 18;
+// makes them, in this launch); false after kReadyPolls polls (a poll takes 0.26 us
+// alone and up to 0.65 us on a full GPU: 0.27 to 0.7 s) or once another wait has
+// given up.  The longest waits are for groups whose candidates are most of a
+// level's nodes: 3,000 polls measured (100K particles, theta 16), 114 at 1M and
+// theta 2.  A group that gives up leaves its children's lists and offsets as an
+// earlier run left them, or never written: every later kernel of the run returns at
+// once (PSG_ERR_VOID).  Warp-collective.
+constexpr int kReadyPolls = 1 << 20;
 
-__device__ __noinline__ bool wait_ready(const uint32_t* flag, Status* status) {
+__device__ __noinline__ bool wait_ready(const uint32_t* flag, int polls, Status* status) {
     uint32_t ok = 0;
     if (lane_id() == 0) {
-        for (int i = 0; i < kReadyPolls; ++i) {
+        for (int i = 0; i < polls; ++i) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(ok) : "l"(flag) : "memory");
             if (ok) break;
             if ((i & 255) == 255 && (*(volatile uint32_t*)&status->err & PSG_ERR_READY_SPIN)) break;
@@ -575,7 +580,7 @@ __global__ void __launch_bounds__(
     Smem& sm = smem[threadIdx.x >> 5];
     const TreeView& tv = A.tv;
     Status* status = A.status;
-    if (status->err & (PSG_ERR_NODES | PSG_ERR_SORT_SPIN)) return;
+    if (status->err & PSG_ERR_VOID) return;
     // a run whose near lists ran out is void (the host grows them and runs
     // again): the internal levels below the one that failed did not run, so
     // their lists must not be read
@@ -733,7 +738,8 @@ __global__ void __launch_bounds__(
             }
             // a parent made in this launch: wait until it is final
             if (MODE == MODE_INTERNAL && (int)dp >= A.level && dp >= 2u) {
-                if (!wait_ready(&tv.ready[pid], status)) continue;
+                const int polls = A.ready_spin > 0 ? A.ready_spin : kReadyPolls;
+                if (!wait_ready(&tv.ready[pid], polls, status)) continue;
             }
             // chain group (leaf pass, parent deeper than the near lists
             // reach, K = ns_levels): start from the near list of p's ancestor
@@ -1296,6 +1302,7 @@ __global__ void __launch_bounds__(
             __syncwarp();
             if constexpr (MODE == MODE_INTERNAL) {
                 // lists and fields of this group's children are final
+                if (A.ready_spin > 0 && (int)dp + 1 == A.level) publish_late();
                 if ((tgt_mask >> lane) & 1u) {
                     __threadfence();
                     __stcg(&tv.ready[fc + sm.tq[lane]], 1u);
@@ -1688,7 +1695,7 @@ __global__ void __launch_bounds__(kDenseThreads, KAHAN ? 2 : kDenseBlocksPerSm)
     __shared__ DenseSmem smem[kDenseWarpsPerBlock];
     DenseSmem& sm = smem[threadIdx.x >> 5];
     Status* status = A.status;
-    if (status->err & (PSG_ERR_NODES | PSG_ERR_SORT_SPIN | PSG_ERR_DENSE_OVERFLOW)) return;
+    if (status->err & (PSG_ERR_VOID | PSG_ERR_DENSE_OVERFLOW)) return;
     const uint32_t lane = lane_id();
     const uint32_t total = min(status->run.dense_count, A.dense.rec_cap);
     unsigned long long inter = 0;
@@ -1779,9 +1786,7 @@ __global__ void __launch_bounds__(kHeavyThreads, 2) k_heavy_leaf(const __grid_co
     __shared__ float s_redt[kHeavyWarps][3 * kHeavyTargets];
     Status* status = A.status;
     // (a run whose near lists ran out is void: see k_trav)
-    if (status->err & (PSG_ERR_NODES | PSG_ERR_SORT_SPIN | PSG_ERR_HEAVY_OVERFLOW |
-                       PSG_ERR_NS_OVERFLOW))
-        return;
+    if (status->err & (PSG_ERR_VOID | PSG_ERR_HEAVY_OVERFLOW | PSG_ERR_NS_OVERFLOW)) return;
     const TreeView& tv = A.tv;
     // work items: the leaf children of the nodes at depths 0 .. heavy_depth-1
     uint32_t cum[kMaxDepth + 1];

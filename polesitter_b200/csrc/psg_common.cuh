@@ -150,6 +150,20 @@ __device__ __forceinline__ uint32_t lane_id() {
     return l;
 }
 
+// the tests of the bounded waits: a publisher that comes ~200 us late (at most
+// 2^20 reads of the clock)
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+inline __device__ __noinline__ void publish_late() {
+    const unsigned long long t0 = global_ns();
+    for (int i = 0; i < (1 << 20) && global_ns() - t0 < 200000ull; ++i) {
+    }
+}
+
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
     asm volatile("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

@@ -33,6 +33,10 @@ extern "C" {
 #define PSG_ERR_TC_TIMEOUT 0x100u   /* a tensor-core MMA did not complete in time */
 #define PSG_ERR_READY_SPIN 0x200u   /* a wait for a parent's near list ran out of polls */
 
+/* the run is void, and what it has left of the tree, the near lists or their
+ * offsets must not be followed: the kernels after it return at once */
+#define PSG_ERR_VOID (PSG_ERR_NODES | PSG_ERR_SORT_SPIN | PSG_ERR_READY_SPIN)
+
 /* debug statistics slots (Status.stat) */
 #define PSG_STAT_MAC 0
 #define PSG_STAT_M2L 1
@@ -134,6 +138,7 @@ int psg_prepare_noalloc(const float* x, const float* y, const float* z, size_t n
 #define PSG_OPT_SORT_SPIN 14     /* > 0: sort look-back polls, first tile publishing late */
 #define PSG_OPT_JUDGE_BLOCKS 15  /* blocks per SM of the closure judge's FP64 sum (1..8) */
 #define PSG_OPT_JUDGE_SAMPLES 16 /* particles the closure judge samples (64..4096) */
+#define PSG_OPT_READY_SPIN 17    /* > 0: traversal waits poll this often, first level late */
 #define PSG_MAX_LEAF_CAP 256
 
 /* the learned far-field closure (k_closure.cu) */

@@ -199,6 +199,7 @@ struct TravArgs {
     float theta;
     int level;          // internal levels of this launch
     int level_end;
+    int ready_spin;     // test of their wait: > 0: polls, the first level publishing late
     int debug;
     int kahan;          // compensated FP32 sums in P2P
     int order;          // closure: 0 = the reference's order-0 local, 1 = order-1

@@ -140,6 +140,7 @@ struct State {
     int force_ns_levels;   // option: store near lists for depths <= this at most
     int force_stream;      // option: always stream the P2P
     int sort_spin_limit;   // look-back polls before the sort gives up (option; 0: default)
+    int ready_spin_limit;  // ... and a traversal group's polls for its parent
     uint32_t leaf_cap;     // option: nodes holding more particles are split (1: the reference)
     double grid_scale;     // traversal grids x this (ensemble autotuner); 0: 1
     int kahan;
@@ -582,6 +583,7 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
     A.status = s->d_status;
     A.theta = s->theta;
     A.level = 0;
+    A.ready_spin = s->ready_spin_limit;
     A.debug = s->debug;
     A.kahan = s->kahan;
     A.xyzm = xyzm;
@@ -1993,6 +1995,10 @@ int psg_set_option(void* mem, int key, double value) {
         case PSG_OPT_SORT_SPIN:
             if (value < 0 || value > (1 << 22) || (double)(int)value != value) return PSG_EINVAL;
             s->sort_spin_limit = (int)value;
+            return PSG_OK;
+        case PSG_OPT_READY_SPIN:
+            if (value < 0 || value > (1 << 22) || (double)(int)value != value) return PSG_EINVAL;
+            s->ready_spin_limit = (int)value;
             return PSG_OK;
         default: return PSG_EINVAL;
     }
