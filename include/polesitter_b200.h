@@ -253,6 +253,10 @@ ps_result_t ps_b200_ensemble_set_leaf_ladder(ps_b200_ensemble_t* ens, const uint
  * error, which ps_b200_ensemble_order then reads back */
 ps_result_t ps_b200_ensemble_set_order(ps_b200_ensemble_t* ens, int order);
 ps_result_t ps_b200_ensemble_order(ps_b200_ensemble_t* ens, int* order_out);
+/* options of an ensemble: PS_B200_OPT_READY_SPIN only (it takes effect when the
+ * next graph is captured, and at once in a traversal that is rerun because a
+ * store has grown) */
+ps_result_t ps_b200_ensemble_set_option(ps_b200_ensemble_t* ens, int key, double value);
 ps_result_t ps_b200_ensemble_destroy(ps_b200_ensemble_t* ens);
 
 /* message of the last CUDA-side failure on this thread */

@@ -43,7 +43,7 @@ EXPORTED = ("ps_init", "ps_prepare_particles", "ps_calc_forces", "ps_destroy",
             "ps_b200_ensemble_run", "ps_b200_ensemble_theta", "ps_b200_ensemble_destroy",
             "ps_b200_ensemble_leaf_caps", "ps_b200_ensemble_set_leaf_caps",
             "ps_b200_ensemble_set_leaf_ladder", "ps_b200_ensemble_set_order",
-            "ps_b200_ensemble_order")
+            "ps_b200_ensemble_order", "ps_b200_ensemble_set_option")
 
 
 class ParticleArrs(C.Structure):
@@ -133,11 +133,12 @@ def lib() -> C.CDLL:
     L.ps_b200_ensemble_set_leaf_ladder.argtypes = [vp, vp, sz]
     L.ps_b200_ensemble_set_order.argtypes = [vp, C.c_int]
     L.ps_b200_ensemble_order.argtypes = [vp, vp]
+    L.ps_b200_ensemble_set_option.argtypes = [vp, C.c_int, C.c_double]
     for name in ("ps_b200_ensemble_create", "ps_b200_ensemble_autotune", "ps_b200_ensemble_run",
                  "ps_b200_ensemble_theta", "ps_b200_ensemble_destroy",
                  "ps_b200_ensemble_leaf_caps", "ps_b200_ensemble_set_leaf_caps",
                  "ps_b200_ensemble_set_leaf_ladder", "ps_b200_ensemble_set_order",
-                 "ps_b200_ensemble_order"):
+                 "ps_b200_ensemble_order", "ps_b200_ensemble_set_option"):
         getattr(L, name).restype = C.c_int
     L.ps_b200_run_ticks.restype = C.c_int
     L.ps_b200_run_ticks.argtypes = [vp, C.POINTER(ParticleArrs), vp, vp, vp, vp, f32, C.c_uint32]
@@ -434,6 +435,10 @@ class Ensemble:
         o = C.c_int()
         _check("ps_b200_ensemble_order", lib().ps_b200_ensemble_order(self.ptr, C.byref(o)))
         return o.value
+
+    def set_option(self, key: int, value: float):
+        _check("ps_b200_ensemble_set_option",
+               lib().ps_b200_ensemble_set_option(self.ptr, key, value))
 
     def destroy(self):
         if self.ptr:

@@ -37,6 +37,10 @@ extern "C" {
  * offsets must not be followed: the kernels after it return at once */
 #define PSG_ERR_VOID (PSG_ERR_NODES | PSG_ERR_SORT_SPIN | PSG_ERR_READY_SPIN)
 
+/* the tick has failed, also on a rerun; the capacity bits (*_OVERFLOW) are
+ * regrown and rerun instead */
+#define PSG_ERR_FATAL (PSG_ERR_VOID | PSG_ERR_STACK | PSG_ERR_CHAIN_ORDER)
+
 /* debug statistics slots (Status.stat) */
 #define PSG_STAT_MAC 0
 #define PSG_STAT_M2L 1
@@ -115,6 +119,7 @@ int psg_ensemble_set_leaf_caps(void* ens, const uint32_t* caps, size_t n, int la
 /* local expansion order of all systems (0 or 1; < 0: the autotuner tries both) */
 int psg_ensemble_set_order(void* ens, int order);
 int psg_ensemble_order(void* ens, int* out);
+int psg_ensemble_set_option(void* ens, int key, double value);
 const char* psg_last_error(void);
 void psg_set_error(const char* msg);
 

@@ -965,12 +965,9 @@ static int tick_core(State* s, const DevArrays& d, size_t n, float cx, float cy,
             return r;
         }
     }
-    if (err & (PSG_ERR_SORT_SPIN | PSG_ERR_STACK | PSG_ERR_NODES | PSG_ERR_HEAVY_OVERFLOW |
-               PSG_ERR_CHAIN_ORDER | PSG_ERR_READY_SPIN)) {
+    if (err & PSG_ERR_FATAL) {
         if (judge) cudaStreamSynchronize(cj.side);
-        const bool nodes = (err & PSG_ERR_NODES) &&
-                           !(err & (PSG_ERR_SORT_SPIN | PSG_ERR_STACK | PSG_ERR_HEAVY_OVERFLOW |
-                                    PSG_ERR_CHAIN_ORDER | PSG_ERR_READY_SPIN));
+        const bool nodes = (err & PSG_ERR_FATAL) == PSG_ERR_NODES;
         std::snprintf(g_err, sizeof(g_err), nodes ? "morton codes not sorted/30-bit (0x%x)"
                                                   : "device status error 0x%x", err);
         return nodes ? PSG_EINVAL : PSG_EDEVICE;
@@ -1457,24 +1454,23 @@ static int ensure_graphs(Ensemble* e, const DevArrays& a, float* const v[3], flo
 static int check_forest(Ensemble* e, const DevArrays& a) {
     State* s = e->fs;
     const uint32_t err = s->h_status->err;
-    if (err & (PSG_ERR_SORT_SPIN | PSG_ERR_STACK | PSG_ERR_NODES | PSG_ERR_CHAIN_ORDER | PSG_ERR_READY_SPIN)) {
+    if (err & PSG_ERR_FATAL) {
         std::snprintf(g_err, sizeof(g_err), "ensemble: device status 0x%x", err);
         return (err & PSG_ERR_NODES) ? PSG_EINVAL : PSG_EDEVICE;
     }
     if (err & (PSG_ERR_NS_OVERFLOW | PSG_ERR_P2P_OVERFLOW | PSG_ERR_DENSE_OVERFLOW |
                PSG_ERR_HEAVY_OVERFLOW)) {
+        e->dirty = true;  // (the captured graphs hold the stores' old addresses)
         int r = regrow(s, err);
         if (r != PSG_OK) return r;
         PSG_CHECK(cudaMemsetAsync(&s->d_status->err, 0, 4, s->stream));
         uint32_t err2 = 0;
         r = run_traversal(s, s->xyzm, a.fx, a.fy, a.fz, &err2);
         if (r != PSG_OK) return r;
-        if (err2 & (PSG_ERR_SORT_SPIN | PSG_ERR_STACK | PSG_ERR_NODES | PSG_ERR_CHAIN_ORDER |
-                    PSG_ERR_HEAVY_OVERFLOW)) {
+        if (err2 & PSG_ERR_FATAL) {
             std::snprintf(g_err, sizeof(g_err), "ensemble: device status 0x%x", err2);
             return PSG_EDEVICE;
         }
-        e->dirty = true;
     }
     return PSG_OK;
 }
@@ -2206,6 +2202,13 @@ int psg_ensemble_order(void* h, int* out) {
     if (!e || e->magic != psg::kEnsMagic || !out) return PSG_EINVAL;
     *out = e->order;
     return PSG_OK;
+}
+
+// (no recapture: captured graphs keep the limit they have, reruns take the new one)
+int psg_ensemble_set_option(void* h, int key, double value) {
+    psg::Ensemble* e = static_cast<psg::Ensemble*>(h);
+    if (!e || e->magic != psg::kEnsMagic || key != PSG_OPT_READY_SPIN) return PSG_EINVAL;
+    return psg_set_option(e->fs, key, value);
 }
 
 // ---- learned closure ----------------------------------------------------------

@@ -367,6 +367,13 @@ ps_result_t ps_b200_ensemble_order(ps_b200_ensemble_t* ens, int* order_out) {
     return to_ps(psg_ensemble_order(ens, order_out));
 }
 
+ps_result_t ps_b200_ensemble_set_option(ps_b200_ensemble_t* ens, int key, double value) {
+    if (!ens) {
+        return PS_EINVAL;
+    }
+    return to_ps(psg_ensemble_set_option(ens, key, value));
+}
+
 ps_result_t ps_b200_ensemble_destroy(ps_b200_ensemble_t* ens) {
     if (!ens) {
         return PS_EINVAL;

@@ -76,3 +76,67 @@ def test_ready_spin_option_bounds():
             with pytest.raises(P.PolesitterError) as e:
                 ctx.set_option(P.OPT_READY_SPIN, bad)
             assert e.value.code == P.PS_EINVAL
+
+
+def test_ensemble_rerun_that_gives_up_is_an_error():
+    """A batch tick whose stores have to grow, and whose rerun then gives up: an
+    error, not void forces; the next tick is right."""
+    torch = pytest.importorskip("torch")
+    counts, theta = [20000, 3000], np.array([6.0, 2.0], np.float32)
+    heavy = [W.clumpy_plummer(counts[0], 34), W.plummer(counts[1], 35)]
+    keys = ("x", "y", "z", "mass")
+    n = sum(counts)
+
+    def light():
+        out = {k: np.concatenate([getattr(p, k) for p in heavy]) for k in keys}
+        for k in ("x", "y", "z"):  # near lists of a few entries
+            out[k] = np.zeros(n, np.float32)
+            out[k][[1, counts[0] + 1]] = 1.0
+        return out
+
+    def full():
+        return {k: np.concatenate([getattr(p, k) for p in heavy]) for k in keys}
+
+    class D:
+        pass
+
+    def arrays():
+        d = D()
+        for k in keys + ("fx", "fy", "fz"):
+            setattr(d, k, torch.zeros(n, device="cuda"))
+        d.id = torch.zeros(n, dtype=torch.int32, device="cuda")
+        return d, torch.zeros(n, dtype=torch.int32, device="cuda"), \
+            [torch.zeros(n, device="cuda") for _ in range(3)]
+
+    def load(d, v, src):
+        for k in keys:
+            getattr(d, k).copy_(torch.from_numpy(src[k]))
+        for a in v:
+            a.zero_()
+        torch.cuda.synchronize()
+
+    d, codes, v = arrays()
+    with P.Ensemble(counts, theta) as ens:
+        load(d, v, full())
+        ens.run(d, codes, *v, 1e-3, 1)
+        want = {k: getattr(d, k).clone() for k in ("x", "fx", "fy", "fz", "id")}
+    d, codes, v = arrays()
+    with P.Ensemble(counts, theta) as ens:
+        for _ in range(2):
+            load(d, v, light())
+            ens.run(d, codes, *v, 1e-3, 1)
+        ens.set_option(P.OPT_READY_SPIN, 4)
+        load(d, v, full())
+        with pytest.raises(P.PolesitterError) as e:
+            ens.run(d, codes, *v, 1e-3, 1)
+        assert e.value.code == P.PS_EDEVICE
+        m = re.search(r"device status 0x([0-9a-f]+)", str(e.value))
+        assert m and int(m.group(1), 16) & READY_SPIN, str(e.value)
+        ens.set_option(P.OPT_READY_SPIN, 0)
+        load(d, v, full())
+        ens.run(d, codes, *v, 1e-3, 1)
+        torch.cuda.synchronize()
+        for k, w in want.items():
+            assert torch.equal(getattr(d, k), w), k
+        with pytest.raises(P.PolesitterError):
+            ens.set_option(P.OPT_SORT_SPIN, 1)
