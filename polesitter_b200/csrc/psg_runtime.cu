@@ -710,6 +710,14 @@ static bool try_alloc_p2p(State* s, uint32_t chunks) {
     return false;
 }
 
+static bool try_alloc_dense(State* s, uint32_t recs, uint32_t slots) {
+    const uint32_t old_recs = s->dense.rec_cap, old_slots = s->dense.slot_cap;
+    if (alloc_dense(s, recs, slots) == PSG_OK) return true;
+    cudaGetLastError();
+    alloc_dense(s, old_recs, old_slots);
+    return false;
+}
+
 // After a traversal run read back its status, makes room for every store
 // that ran out, for the rerun and later ticks:
 //  * near lists: grown to twice what the run reserved while the device has
@@ -718,7 +726,9 @@ static bool try_alloc_p2p(State* s, uint32_t chunks) {
 //    their ancestor chains, and the P2P is streamed, so no store grows with
 //    theta any more;
 //  * P2P chunks: grown likewise, else the P2P is streamed;
-//  * full-leaf records and shallow-leaf frontiers: grown.
+//  * full-leaf records: grown (a segment of a source list takes a slot of 384
+//    bytes per record, so they too grow with theta), else the P2P is streamed;
+//  * shallow-leaf frontiers: grown.
 // PSG_EOOM when nothing can give.
 static int regrow(State* s, uint32_t err) {
     if (err & PSG_ERR_NS_OVERFLOW) {
@@ -761,16 +771,6 @@ static int regrow(State* s, uint32_t err) {
         int r = alloc_heavy(s, (uint32_t)(cap < most ? cap : most));
         if (r != PSG_OK) return r;
     }
-    if (err & PSG_ERR_DENSE_OVERFLOW) {
-        auto room = [](uint32_t used, uint32_t cap) {
-            if (used <= cap) return cap;
-            const unsigned long long need = (unsigned long long)used + used / 4 + 1024;
-            return (uint32_t)std::min<unsigned long long>(need, 0x7FFFFFFFull);
-        };
-        int r = alloc_dense(s, room(s->h_status->run.dense_count, s->dense.rec_cap),
-                            room(s->h_status->run.dense_slots, s->dense.slot_cap));
-        if (r != PSG_OK) return r;
-    }
     if (err & PSG_ERR_P2P_OVERFLOW) {
         // the chunk counter is 32-bit: below the capacity it has wrapped
         const unsigned long long used = s->h_status->run.p2p_chunks;
@@ -779,6 +779,18 @@ static int regrow(State* s, uint32_t err) {
         const unsigned long long limit =
             std::min(0x7FFFFFFFull, store_budget(s->p2p.cap_chunks * per) / per);
         if (!(need <= limit && try_alloc_p2p(s, (uint32_t)need))) s->stream_p2p = 1;
+    }
+    if ((err & PSG_ERR_DENSE_OVERFLOW) && !s->stream_p2p) {
+        auto room = [](uint32_t used, uint32_t cap) {
+            if (used <= cap) return cap;
+            const unsigned long long need = (unsigned long long)used + used / 4 + 1024;
+            return (uint32_t)std::min<unsigned long long>(need, 0x7FFFFFFFull);
+        };
+        const uint32_t recs = room(s->h_status->run.dense_count, s->dense.rec_cap),
+                       slots = room(s->h_status->run.dense_slots, s->dense.slot_cap);
+        // (both below their capacity: a 32-bit counter has wrapped)
+        const bool wrapped = recs == s->dense.rec_cap && slots == s->dense.slot_cap;
+        if (wrapped || !try_alloc_dense(s, recs, slots)) s->stream_p2p = 1;
     }
     return PSG_OK;
 }

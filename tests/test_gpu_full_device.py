@@ -1,0 +1,74 @@
+"""Ticks on a device whose memory is nearly full: a store that cannot be grown
+must cost speed, not the tick.  The rest of the memory is taken by one plain
+allocation; nothing is ever launched on it."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import polesitter_b200 as P
+from conftest import rel_l2
+from polesitter_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+# FP32 sums of a few thousand terms in another order; the parity tests' bar
+FORCE_REL_L2 = 1e-5
+MIB = 1 << 20
+
+
+def _fill(torch, leave):
+    """Tensors that take all device memory but `leave` bytes."""
+    held = []
+    torch.cuda.empty_cache()
+    while True:
+        free = torch.cuda.mem_get_info()[0] - leave
+        if free < 4 * MIB:
+            return held
+        try:
+            held.append(torch.empty(free // (2 * MIB) * 2 * MIB, dtype=torch.uint8,
+                                    device="cuda"))
+        except torch.cuda.OutOfMemoryError:
+            return held
+
+
+def _forces(p):
+    return np.stack([p.fx, p.fy, p.fz], 1).astype(np.float64)
+
+
+def test_p2p_is_streamed_when_its_records_do_not_fit():
+    torch = pytest.importorskip("torch")
+    n, theta, cap = 1 << 20, 12.0, 64
+    p0 = W.clumpy_plummer(n, 42)
+    want, streamed = p0.copy(), p0.copy()
+    with P.Context(n, theta=theta) as ctx:
+        ctx.set_option(P.OPT_LEAF_CAP, cap)
+        ctx.tick(want, np.zeros(n, np.uint32))
+        st = ctx.stats()
+        assert st["streamed"] == 0 and st["traversal_runs"] > 1  # (the records grew)
+        # (the streamed kernels are loaded while there is room)
+        ctx.set_option(P.OPT_STREAM, 1)
+        ctx.tick(streamed, np.zeros(n, np.uint32))
+    with P.Context(n, theta=2.99) as ctx:
+        # the near lists and the P2P chunks grow to what the next tick needs,
+        # the records do not: no source list is long enough to be segmented
+        ctx.tick(p0.copy(), np.zeros(n, np.uint32))
+        ctx.set_option(P.OPT_THETA, theta)
+        ctx.set_option(P.OPT_LEAF_CAP, cap)
+        held = _fill(torch, 24 * MIB)
+        got = p0.copy()
+        ctx.tick(got, np.zeros(n, np.uint32))
+        st = ctx.stats()
+        del held
+        torch.cuda.empty_cache()
+        assert st["near_levels"] == 10 and st["streamed"] == 1
+        # with room again, and the choice reset, the records come back
+        ctx.set_option(P.OPT_LEAF_CAP, cap)
+        again = p0.copy()
+        ctx.tick(again, np.zeros(n, np.uint32))
+        assert ctx.stats()["streamed"] == 0
+    assert np.array_equal(got.id, want.id)
+    assert rel_l2(_forces(got), _forces(want)) < FORCE_REL_L2
+    assert np.array_equal(_forces(got), _forces(streamed))
+    assert np.array_equal(_forces(again), _forces(want))
