@@ -248,13 +248,7 @@ static int alloc_dense(State* s, uint32_t recs, uint32_t slots) {
     return PSG_OK;
 }
 
-// sums and lists of the groups split over several warps: the groups (two
-// halves each) of the depths above `depth`
-static int ensure_split(State* s, int depth) {
-    uint32_t groups = 0;
-    for (int d = 0; d < depth; ++d) groups += 2 * s->tv.lvl_cap[d];
-    SplitStore& p = s->split;
-    if (p.cap >= groups) return PSG_OK;
+static int alloc_split(SplitStore& p, uint32_t groups) {
     if (p.sums) cudaFree(p.sums);
     p = SplitStore{};
     Carve c;
@@ -266,6 +260,18 @@ static int ensure_split(State* s, int depth) {
     p.count = carved<uint32_t>(p.sums, count);
     p.cap = groups;
     return PSG_OK;
+}
+
+// sums and lists of the groups split over several warps: the groups (two
+// halves each) of the depths above `depth`; false when the device cannot hold
+// them (many systems: 2.5 KB a group half, 3 MB a system at depth 4): the leaf
+// pass then takes every group in one warp
+static bool ensure_split(State* s, int depth) {
+    uint32_t groups = 0;
+    for (int d = 0; d < depth; ++d) groups += 2 * s->tv.lvl_cap[d];
+    if (s->split.cap >= groups || alloc_split(s->split, groups) == PSG_OK) return true;
+    cudaGetLastError();
+    return false;
 }
 
 // blocks of k_dense_p2p for n particles: the blocks that fit on the SMs,
@@ -601,18 +607,15 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
     // k_heavy_leaf's
     const bool forest = s->tv.part_sys != nullptr;
     const bool heavy = xl || s->heavy_depth >= 0;
-    const int depth = heavy    ? heavy_depth_for(s)
-                      : forest ? s->forest_split
-                               : split_depth_of(s->theta, s->trav_n, s->leaf_cap);
+    int depth = heavy    ? heavy_depth_for(s)
+                : forest ? s->forest_split
+                         : split_depth_of(s->theta, s->trav_n, s->leaf_cap);
+    if (!heavy && !ensure_split(s, depth)) depth = 0;
     if (forest) A.tv.sys_shallow = heavy ? s->sys_heavy : s->sys_split;
     A.shallow = forest ? 0 : depth;
-    if (!heavy) {
-        const int r = ensure_split(s, depth);
-        if (r != PSG_OK) return r;
-        // (not reset by the kernel: a void run may stop half way)
-        if (depth)
-            PSG_CHECK(cudaMemsetAsync(s->split.count, 0, (size_t)s->split.cap * 4, s->stream));
-    }
+    // (not reset by the kernel: a void run may stop half way)
+    if (!heavy && depth)
+        PSG_CHECK(cudaMemsetAsync(s->split.count, 0, (size_t)s->split.cap * 4, s->stream));
     A.split = s->split;
     A.heavy_depth = depth;
     A.heavy_frontier = s->heavy_frontier;
@@ -1344,6 +1347,12 @@ static int upload_systems(Ensemble* e) {
         sp[k] = split_depth_of(t, e->count[k], e->cap[k]);
         smax = std::max(smax, (int)sp[k]);
     }
+    const SplitStore before = e->fs->split;  // (allocated here: not while capturing)
+    if (!ensure_split(e->fs, smax)) {
+        std::fill(sp.begin(), sp.end(), 0);
+        smax = 0;
+    }
+    if (before.sums != e->fs->split.sums || before.cap != e->fs->split.cap) e->dirty = true;
     PSG_CHECK(cudaMemcpy(e->sys_theta2, th2.data(), e->nsys * 4, cudaMemcpyHostToDevice));
     PSG_CHECK(cudaMemcpy(e->sys_heavy, hv.data(), e->nsys * 4, cudaMemcpyHostToDevice));
     PSG_CHECK(cudaMemcpy(e->sys_split, sp.data(), e->nsys * 4, cudaMemcpyHostToDevice));
@@ -1353,10 +1362,6 @@ static int upload_systems(Ensemble* e) {
     if (smax != e->fs->forest_split || caps != e->fs->forest_caps) e->dirty = true;
     e->fs->forest_caps = caps;
     e->fs->forest_split = smax;
-    const SplitStore before = e->fs->split;  // (allocated here: not while capturing)
-    const int r = ensure_split(e->fs, smax);
-    if (r != PSG_OK) return r;
-    if (before.sums != e->fs->split.sums) e->dirty = true;
     // the stores' near-list depth and P2P mode start over with the settings
     // (both are launch parameters of the captured graphs)
     if (e->fs->ns_levels != kMaxDepth || e->fs->stream_p2p || e->fs->level_by_level)

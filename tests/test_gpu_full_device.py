@@ -72,3 +72,43 @@ def test_p2p_is_streamed_when_its_records_do_not_fit():
     assert rel_l2(_forces(got), _forces(want)) < FORCE_REL_L2
     assert np.array_equal(_forces(got), _forces(streamed))
     assert np.array_equal(_forces(again), _forces(want))
+
+
+def test_batch_runs_without_room_for_its_split_groups():
+    torch = pytest.importorskip("torch")
+    # theta 3 splits the groups above depth 3 of every system: 714 MiB in all
+    counts = [520] * 2000
+    n = sum(counts)
+    p0 = W.uniform_cube(n, 44)
+
+    class D:
+        pass
+
+    def run(ens):
+        d = D()
+        for k in ("x", "y", "z", "mass", "fx", "fy", "fz"):
+            setattr(d, k, torch.from_numpy(getattr(p0, k).copy()).cuda())
+        d.id = torch.from_numpy(p0.id.view(np.int32).copy()).cuda()
+        v = [torch.zeros(n, device="cuda") for _ in range(3)]
+        codes = torch.zeros(n, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        ens.run(d, codes, *v, 1e-3, 1)
+        torch.cuda.synchronize()
+        return d.id.cpu().numpy(), np.stack([a.cpu().numpy() for a in (d.fx, d.fy, d.fz)],
+                                            1).astype(np.float64)
+
+    with P.Ensemble(counts, np.full(2000, 3.0, np.float32)) as ens:
+        want_id, want = run(ens)
+    free = torch.cuda.mem_get_info()[0]
+    with P.Ensemble(counts, np.full(2000, 2.0, np.float32)):  # (no split groups)
+        need = free - torch.cuda.mem_get_info()[0]
+    held = _fill(torch, need + 320 * MIB)
+    with P.Ensemble(counts, np.full(2000, 3.0, np.float32)) as ens:
+        got_id, got = run(ens)
+        del held
+        torch.cuda.empty_cache()
+        ens.set_leaf_caps(np.full(2000, 1, np.uint32))  # (looks again)
+        again_id, again = run(ens)
+    assert np.array_equal(got_id, want_id)
+    assert rel_l2(got, want) < FORCE_REL_L2
+    assert np.array_equal(again_id, want_id) and np.array_equal(again, want)
