@@ -118,6 +118,7 @@ struct State {
     uint32_t* heavy_frontier;
     uint32_t heavy_fcap;
     int heavy_slots;       // blocks of k_heavy_leaf
+    bool heavy_off;        // its frontiers overflowed and could not be grown
     cudaStream_t aux;      // split groups or k_heavy_leaf, beside the leaf pass
     cudaEvent_t ev_levels, ev_heavy;
     // host-array calls: the sorted arrays (final after the gather) go back to
@@ -173,6 +174,7 @@ struct State {
 // on (theta, leaf capacity, expansion order, store sizes) changes
 static void reset_near_levels(State* s) {
     s->level_by_level = false;
+    s->heavy_off = false;
     s->ns_levels = kMaxDepth;
     s->stream_p2p = 0;
 }
@@ -285,10 +287,29 @@ static size_t dense_grid(const State* s, size_t n) {
 static int alloc_heavy(State* s, uint32_t cap) {
     if (s->heavy_frontier) cudaFree(s->heavy_frontier);
     s->heavy_frontier = nullptr;
+    s->heavy_fcap = 0;
     // per block: two frontiers and the P2P source list of a multi-particle leaf
     PSG_ALLOC(s->heavy_frontier, (size_t)s->heavy_slots * 3 * cap * 4);
     s->heavy_fcap = cap;
     return PSG_OK;
+}
+
+// ... allocated when that kernel first has work (most contexts never run it; 192
+// bytes a particle).  A frontier holds at most one level's nodes plus the parent's
+// near list.  On a full device they take the place of the P2P stores where the P2P
+// is streamed.  False when the device cannot hold them: the leaf pass then takes
+// the shallow leaves too.
+static bool ensure_heavy(State* s) {
+    if (s->heavy_frontier) return true;
+    if (s->heavy_off) return false;
+    const uint32_t cap = (uint32_t)(s->max_particles / 4 + 4096);
+    if (alloc_heavy(s, cap) == PSG_OK) return true;
+    cudaGetLastError();
+    if (s->stream_p2p && alloc_p2p(s, 64) == PSG_OK && alloc_dense(s, 64, 64) == PSG_OK &&
+        alloc_heavy(s, cap) == PSG_OK)
+        return true;
+    cudaGetLastError();
+    return false;
 }
 
 static void free_mirror(Mirror& mi) {
@@ -460,11 +481,7 @@ static int init_state(State* s, size_t maxp, float theta, const uint32_t* lvl_ca
     r = alloc_dense(s, (uint32_t)(n / 2 + 1024), (uint32_t)(n / 8 + 8192));
     if (r != PSG_OK) return r;
     PSG_ALLOC(s->dense.item, n * sizeof(uint4));
-    // shallow leaves: a frontier holds at most one level's nodes plus the
-    // parent's near list
     s->heavy_slots = 64;
-    r = alloc_heavy(s, (uint32_t)(n / 4 + 4096));
-    if (r != PSG_OK) return r;
     s->heavy_depth = -1;
     s->ns_levels = kMaxDepth;
     s->force_ns_levels = kMaxDepth;
@@ -582,7 +599,6 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
     s->trav_fresh = false;
     TravArgs A;
     A.tv = s->tv;
-    A.p2p = s->p2p;
     A.ns = s->ns;
     A.ns_cap = s->ns_cap;
     A.ns_pool = ns_pool(s->max_particles);
@@ -601,7 +617,6 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
     A.leaf_of = o ? s->cl.leaf_of : nullptr;
     A.tv.lg0 = o ? s->cl.lg0 : nullptr;
     A.tv.lg1 = o ? s->cl.lg1 : nullptr;
-    A.dense = s->dense;
     const bool xl = near_levels(s) < kMaxDepth || s->stream_p2p || s->force_stream;
     // the shallow groups: split over several warps, or (XL, or on demand)
     // k_heavy_leaf's
@@ -611,11 +626,17 @@ static int enqueue_traversal(State* s, const float4* xyzm, float* fx, float* fy,
                 : forest ? s->forest_split
                          : split_depth_of(s->theta, s->trav_n, s->leaf_cap);
     if (!heavy && !ensure_split(s, depth)) depth = 0;
+    if (heavy && depth && !ensure_heavy(s)) {
+        if (forest) return PSG_EALLOC;  // (its groups read their systems' depths)
+        depth = 0;
+    }
     if (forest) A.tv.sys_shallow = heavy ? s->sys_heavy : s->sys_split;
     A.shallow = forest ? 0 : depth;
     // (not reset by the kernel: a void run may stop half way)
     if (!heavy && depth)
         PSG_CHECK(cudaMemsetAsync(s->split.count, 0, (size_t)s->split.cap * 4, s->stream));
+    A.p2p = s->p2p;
+    A.dense = s->dense;
     A.split = s->split;
     A.heavy_depth = depth;
     A.heavy_frontier = s->heavy_frontier;
@@ -731,7 +752,8 @@ static bool try_alloc_dense(State* s, uint32_t recs, uint32_t slots) {
 //  * P2P chunks: grown likewise, else the P2P is streamed;
 //  * full-leaf records: grown (a segment of a source list takes a slot of 384
 //    bytes per record, so they too grow with theta), else the P2P is streamed;
-//  * shallow-leaf frontiers: grown.
+//  * shallow-leaf frontiers: grown, else (one system) the leaf pass takes the
+//    shallow leaves.
 // PSG_EOOM when nothing can give.
 static int regrow(State* s, uint32_t err) {
     if (err & PSG_ERR_NS_OVERFLOW) {
@@ -772,7 +794,11 @@ static int regrow(State* s, uint32_t err) {
         unsigned long long cap = 2ull * s->heavy_fcap;
         const unsigned long long most = 2ull * s->max_particles + 1024;
         int r = alloc_heavy(s, (uint32_t)(cap < most ? cap : most));
-        if (r != PSG_OK) return r;
+        if (r != PSG_OK && s->tv.part_sys) return r;
+        if (r != PSG_OK) {
+            cudaGetLastError();
+            s->heavy_off = true;
+        }
     }
     if (err & PSG_ERR_P2P_OVERFLOW) {
         // the chunk counter is 32-bit: below the capacity it has wrapped

@@ -112,3 +112,33 @@ def test_batch_runs_without_room_for_its_split_groups():
     assert np.array_equal(got_id, want_id)
     assert rel_l2(got, want) < FORCE_REL_L2
     assert np.array_equal(again_id, want_id) and np.array_equal(again, want)
+
+
+def test_shallow_leaf_frontiers_come_with_their_first_use():
+    torch = pytest.importorskip("torch")
+    n = 1 << 20
+    frontiers = 64 * 3 * (n // 4 + 4096) * 4
+    p0 = W.plummer(n, 45)
+
+    def tick(ctx):
+        p = p0.copy()
+        ctx.tick(p, np.zeros(n, np.uint32))
+        return _forces(p)
+
+    with P.Context(n, theta=2.0) as ctx:
+        plain = tick(ctx)
+        free = torch.cuda.mem_get_info()[0]
+        ctx.set_option(P.OPT_HEAVY_DEPTH, 3)
+        want = tick(ctx)
+        assert free - torch.cuda.mem_get_info()[0] >= frontiers
+    with P.Context(n, theta=2.0) as ctx:
+        tick(ctx)
+        ctx.set_option(P.OPT_HEAVY_DEPTH, 3)
+        held = _fill(torch, 24 * MIB)
+        got = tick(ctx)
+        del held
+        torch.cuda.empty_cache()
+        again = tick(ctx)
+    assert np.array_equal(got, plain)  # the leaf pass has taken them
+    assert rel_l2(got, want) < FORCE_REL_L2
+    assert np.array_equal(again, want)
