@@ -242,6 +242,7 @@ struct SmallSortSmem {
     uint32_t dstart[256];
     uint32_t wsum[8];
 };
+static_assert(sizeof(SmallSortSmem) <= 48 * 1024, "no opt-in needed");
 
 template <int ITEMS>
 __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
@@ -335,15 +336,6 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
             id[k] = rank[it];
         }
     }
-}
-
-cudaError_t prepare_sort_small() {
-    const cudaError_t e = cudaFuncSetAttribute(
-        k_sort_small<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmallSortSmem));
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_sort_small<kSmallItems>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(SmallSortSmem));
 }
 
 bool sort_small_fits(size_t n) { return n <= kSmallMax; }

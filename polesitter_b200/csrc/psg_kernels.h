@@ -42,7 +42,6 @@ void launch_sort_forest(SortBuffers& b, uint32_t* codes, size_t n, int grid, Sta
                         cudaStream_t st, const uint32_t* part_sys, int sys_passes,
                         const uint32_t* sys_hist);
 // the sort, gather and write-back of a small system in one block
-cudaError_t prepare_sort_small();
 bool sort_small_fits(size_t n);
 void launch_sort_small(uint32_t* codes, size_t n, float* x, float* y, float* z, float* m,
                        uint32_t* id, float4* xyzm, uint32_t* ids, cudaStream_t st);

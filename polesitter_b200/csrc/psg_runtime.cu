@@ -200,8 +200,10 @@ static int alloc_ns(State* s, unsigned long long cap) {
 }
 
 // one allocation for several arrays, the first of which is its address: a
-// cudaMalloc takes some 50-100 us whatever its size (ps_init and ps_destroy of a
-// 64K context together: 17 -> 12 ms)
+// cudaMalloc or cudaFree of more than some 100 KB takes 50-200 us whatever its size
+// (ps_init with the arrays that keep their size allocated one by one / together:
+// 1K particles 1.5 / 1.2 ms, 64K 3.9 / 1.6, 4M 6.7 / 1.9; ps_destroy of 64K
+// 4.0 / 1.7 ms)
 struct Carve {
     size_t total = 0;
     size_t add(size_t bytes) {
@@ -378,10 +380,7 @@ static Place place_of(const void* p) {
 static bool on_device(const void* p) { return place_of(p) == DEVICE; }
 
 static void free_state(State* s) {
-    void* ps[] = {s->xyzm, s->ids, s->sort.key_a, s->sort.key_b, s->sort.val_a, s->sort.val_b,
-                  s->sort.hist, s->tree_tiles, s->tv.geo,
-                  s->tv.mp, s->tv.lt, s->tv.info, s->tv.parent, s->tv.arrive, s->ns, s->p2p.src,
-                  s->d_status, s->dense.rec, s->direct_ws, s->dense.item, s->split.sums,
+    void* ps[] = {s->xyzm, s->ns, s->p2p.src, s->dense.rec, s->direct_ws, s->split.sums,
                   s->heavy_frontier, s->tk_partial, s->tk_bbox, s->tk_v[0], s->tk_v[1], s->tk_v[2],
                   s->tk_vmir[0], s->tk_vmir[1], s->tk_vmir[2], s->cl.lg0, s->cl.lg1,
                   s->cl.leaf_of, s->cl.dF, s->cl.params, s->cl.packed, s->cl.judge_tg,
@@ -425,17 +424,6 @@ static int init_state(State* s, size_t maxp, float theta, const uint32_t* lvl_ca
     s->theta = theta;
     s->morton_variant = PSG_MORTON_AVX2;
     const size_t n = maxp ? maxp : 1;
-    PSG_ALLOC(s->xyzm, n * sizeof(float4));
-    PSG_ALLOC(s->ids, n * 4);
-    PSG_ALLOC(s->sort.key_a, n * 4);
-    PSG_ALLOC(s->sort.key_b, n * 4);
-    PSG_ALLOC(s->sort.val_a, n * 4);
-    PSG_ALLOC(s->sort.val_b, n * 4);
-    const size_t stiles = (n + sort_tile_size() - 1) / sort_tile_size();
-    PSG_ALLOC(s->sort.hist, ((size_t)sort_passes * stiles + 4) * 256 * 4);
-    s->sort.lookback = s->sort.hist + 4 * 256;
-    PSG_CHECK(prepare_sort_small());
-    PSG_ALLOC(s->tree_tiles, tree_scratch_bytes(n));
     // level capacities: min(8^d, n) nodes at depth d
     uint32_t base = 0;
     for (int d = 0; d <= kMaxDepth; ++d) {
@@ -449,24 +437,32 @@ static int init_state(State* s, size_t maxp, float theta, const uint32_t* lvl_ca
     }
     s->tv.lvl_base[kLevels] = base;
     s->tv.lvl_cap[kLevels] = 0;
-    const size_t nodes = base;
-    PSG_ALLOC(s->tv.geo, nodes * 16);
-    PSG_ALLOC(s->tv.mp, nodes * 16);
-    PSG_ALLOC(s->tv.lt, nodes * 16);
-    PSG_ALLOC(s->tv.info, nodes * 16);
-    PSG_ALLOC(s->tv.parent, nodes * 4);
+    const size_t nodes = base, stiles = (n + sort_tile_size() - 1) / sort_tile_size();
     {
+        // everything that keeps its size, in one allocation (xyzm is its address)
         TreeView& t = s->tv;
-        uint32_t** const per_node[] = {&t.arrive,  &t.cbase, &t.ns_off, &t.ns_cnt, &t.dbg_m2l,
-                                       &t.dbg_p2p, &t.link,  &t.ready,  &t.groups};
-        Carve c;
-        for (auto q : per_node) (void)q, c.add(nodes * 4);
-        PSG_ALLOC(t.arrive, c.total);
-        uint32_t* const base = t.arrive;
-        Carve at;
-        for (auto q : per_node) *q = carved<uint32_t>(base, at.add(nodes * 4));
+        const struct { void* p; size_t bytes; } part[] = {
+            {&s->xyzm, n * sizeof(float4)}, {&s->ids, n * 4},
+            {&s->sort.key_a, n * 4}, {&s->sort.key_b, n * 4},
+            {&s->sort.val_a, n * 4}, {&s->sort.val_b, n * 4},
+            {&s->sort.hist, ((size_t)sort_passes * stiles + 4) * 256 * 4},
+            {&s->tree_tiles, tree_scratch_bytes(n)},
+            {&t.geo, nodes * 16}, {&t.mp, nodes * 16}, {&t.lt, nodes * 16},
+            {&t.info, nodes * 16}, {&t.parent, nodes * 4}, {&t.arrive, nodes * 4},
+            {&t.cbase, nodes * 4}, {&t.ns_off, nodes * 4}, {&t.ns_cnt, nodes * 4},
+            {&t.dbg_m2l, nodes * 4}, {&t.dbg_p2p, nodes * 4}, {&t.link, nodes * 4},
+            {&t.ready, nodes * 4}, {&t.groups, nodes * 4},
+            {&s->dense.item, n * sizeof(uint4)}, {&s->d_status, sizeof(Status)}};
+        Carve c, at;
+        for (const auto& q : part) c.add(q.bytes);
+        char* fixed = nullptr;
+        PSG_ALLOC(fixed, c.total);
+        for (const auto& q : part) {
+            void* const p = fixed + at.add(q.bytes);
+            std::memcpy(q.p, &p, sizeof(p));
+        }
+        s->sort.lookback = s->sort.hist + 4 * 256;
     }
-    PSG_ALLOC(s->d_status, sizeof(Status));
     PSG_CHECK(cudaMallocHost((void**)&s->h_status, sizeof(Status)));
     std::memset(s->h_status, 0, sizeof(Status));
     // first sizes of the stores that the warps take pools from: what the lists
@@ -480,7 +476,6 @@ static int init_state(State* s, size_t maxp, float theta, const uint32_t* lvl_ca
     if (r != PSG_OK) return r;
     r = alloc_dense(s, (uint32_t)(n / 2 + 1024), (uint32_t)(n / 8 + 8192));
     if (r != PSG_OK) return r;
-    PSG_ALLOC(s->dense.item, n * sizeof(uint4));
     s->heavy_slots = 64;
     s->heavy_depth = -1;
     s->ns_levels = kMaxDepth;
