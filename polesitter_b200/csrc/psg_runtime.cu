@@ -206,7 +206,8 @@ static int alloc_ns(State* s, unsigned long long cap) {
 // 4.0 / 1.7 ms)
 struct Carve {
     size_t total = 0;
-    size_t add(size_t bytes) {
+    size_t add(size_t bytes, size_t align = 256) {
+        total = (total + align - 1) & ~(align - 1);
         const size_t at = total;
         total += (bytes + 255) & ~(size_t)255;
         return at;
@@ -453,12 +454,15 @@ static int init_state(State* s, size_t maxp, float theta, const uint32_t* lvl_ca
             {&t.dbg_m2l, nodes * 4}, {&t.dbg_p2p, nodes * 4}, {&t.link, nodes * 4},
             {&t.ready, nodes * 4}, {&t.groups, nodes * 4},
             {&s->dense.item, n * sizeof(uint4)}, {&s->d_status, sizeof(Status)}};
+        // (large ones start at 2 MB, as an allocation of their own would: end to end
+        // a 1M tick took 2.29 instead of 2.28 ms)
+        auto align = [](size_t bytes) -> size_t { return bytes < (1u << 20) ? 256 : 2u << 20; };
         Carve c, at;
-        for (const auto& q : part) c.add(q.bytes);
+        for (const auto& q : part) c.add(q.bytes, align(q.bytes));
         char* fixed = nullptr;
         PSG_ALLOC(fixed, c.total);
         for (const auto& q : part) {
-            void* const p = fixed + at.add(q.bytes);
+            void* const p = fixed + at.add(q.bytes, align(q.bytes));
             std::memcpy(q.p, &p, sizeof(p));
         }
         s->sort.lookback = s->sort.hist + 4 * 256;
