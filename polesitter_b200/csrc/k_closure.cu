@@ -839,8 +839,8 @@ void launch_mlp_grad(const float* X, const float* T, const uint32_t* perm, size_
                      float* loss_sum, cudaStream_t st) {
     if (count == 0) return;
     const unsigned grid = (unsigned)((count + kTrainRows - 1) / kTrainRows);
-    k_mlp_grad<<<grid, kTrainThreads, sizeof(TrainSmem), st>>>(X, T, perm, b0, count, w, inv_norm, grad,
-                                                     loss_sum);
+    k_mlp_grad<<<grid, kTrainThreads, sizeof(TrainSmem), st>>>(X, T, perm, b0, count, w, inv_norm,
+                                                               grad, loss_sum);
 }
 
 void launch_mlp_adam(float* p, float* m, float* v, float* g, MlpPacked* packed, int n, float lr,

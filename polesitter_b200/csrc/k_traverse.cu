@@ -64,7 +64,6 @@ constexpr int kStackCap = 384;            // DFS stack (node, child mask)
 constexpr int kStackSlack = 72;           // 9 levels x 7: growth of a single-entry descent
 constexpr int kP2PCap = 128;              // staged P2P sources of a group
 constexpr uint32_t kSegChunks = 32;       // chunks of source list per dense work record
-constexpr uint32_t kDenseSwitch = 32;     // fullest leaf from which the DENSE leaf pass runs
 
 enum { MODE_INTERNAL = 0, MODE_LEAF = 1 };
 
@@ -194,8 +193,9 @@ __device__ __forceinline__ uint32_t next_run(const SmemLeaf& sm, uint32_t& m, ui
 // sums meet in slots (DenseStore).  One warp per whole list took 7.7 of a
 // 131K closure tick's 9.9 ms, as segments 0.8 ms; 32 chunks (at most 1,024
 // sources) keep a record to tens of microseconds while most lists of a 1M tick
-// stay whole (16 chunks: 3 % faster at 131K, 2 % slower at 1M).  part: the list is one of several warps' (a split
-// group, whose last warp links the lists and fills in the items).
+// stay whole (16 chunks: 3 % faster at 131K, 2 % slower at 1M).  part: the list is
+// one of several warps' (a split group, whose last warp links the lists and fills
+// in the items).
 // Record: {fc, phead, first particle, count | run's child mask << 8}, slot or
 // kNone.
 __device__ __noinline__ void record_dense(SmemLeaf& sm, const DenseStore& ds, uint32_t mask,
@@ -537,8 +537,9 @@ __device__ __noinline__ bool wait_ready(const uint32_t* flag, int polls, Status*
 
 // DENSE (leaf pass only): the variant for trees whose fullest leaf holds at
 // least kDenseSwitch particles or whose leaf capacity is kDenseCap or more,
-// which hands full leaves to k_dense_p2p.  Both
-// variants are launched; each returns at once unless the tree is its kind.
+// which hands every leaf's P2P to k_dense_p2p.  Below kDenseCap the host does not
+// know the fullest leaf: the sparse and the dense variant are both launched, and
+// each returns at once unless the tree is its kind.
 // XL (leaf pass only): the variant that also serves chain groups and
 // streamed P2P, launched only when the near lists stop short of the deepest
 // level or the P2P is streamed, so the other variants keep their registers.
@@ -548,7 +549,7 @@ __device__ __noinline__ bool wait_ready(const uint32_t* flag, int polls, Status*
 // a 1M closure tick's from 4.35 to 4.70 and 5.14 ms), the internal levels 5, with
 // order 1 4 (3, 4, 5 blocks: 0.49, 0.50, 0.45 ms of a 1M plain tick, 0.24, 0.26,
 // 0.30 of a 131K closure tick).
-// SPLIT (leaf pass only): the groups of the depths < split_depth, whose leaves'
+// SPLIT (leaf pass only): the groups of the depths < shallow, whose leaves'
 // walks reach a large part of the tree, kSplitParts warps each (every warp
 // takes every kSplitParts-th candidate and what lies below it), on trees of
 // either kind; their P2P always goes to k_dense_p2p.  A launch of its own
@@ -639,7 +640,9 @@ __global__ void __launch_bounds__(
     }
     __syncwarp();
     // items taken per atomic: one, since whole work queues are a few items per
-    // warp (4 at a time cost the internal levels of a 65K tick 70 of 104 us)
+    // warp (4 at a time cost the internal levels of a 65K tick 70 of 104 us; as a
+    // loop without the inner one the merging leaf variant spills more, for 0.5 % of
+    // a 131K closure tick)
     constexpr uint32_t batch = 1u;
     const uint32_t items = total;
 
@@ -884,48 +887,48 @@ __global__ void __launch_bounds__(
                     // reads on until it has a warp's worth of them
                     tot = 0;
                     do {
-                    const uint32_t e = e0 + lane;
-                    // an entry is an internal source's link or a leaf's id
-                    uint32_t s0 = 0, c = 0, link = 0;
-                    if (e < nsn) {
-                        if (SPLIT && !nsl) {
-                            s0 = nfirst + e;
-                            link = tv.link[s0];
-                        } else {
-                            s0 = link = nsl[e];
+                        const uint32_t e = e0 + lane;
+                        // an entry is an internal source's link or a leaf's id
+                        uint32_t s0 = 0, c = 0, link = 0;
+                        if (e < nsn) {
+                            if (SPLIT && !nsl) {
+                                s0 = nfirst + e;
+                                link = tv.link[s0];
+                            } else {
+                                s0 = link = nsl[e];
+                            }
+                            const uint32_t nch = link >> 28;
+                            c = nch ? nch : 1u;
                         }
-                        const uint32_t nch = link >> 28;
-                        c = nch ? nch : 1u;
-                    }
-                    const uint32_t inc = warp_incl_scan(c);
-                    const uint32_t all = __shfl_sync(0xFFFFFFFFu, inc, 31);
-                    const uint32_t ex = inc - c;
-                    const bool lf = (link >> 28) == 0;
-                    if (SPLIT && parts > 1u) {
-                        const uint32_t off = (part - crun) % kSplitParts;
-                        for (uint32_t i = 0; i < c; ++i) {
-                            const uint32_t k = ex + i - off;
-                            if (k % kSplitParts == 0) {
-                                sm.cand_node[tot + k / kSplitParts] =
-                                    lf ? s0 : (link & kLinkMask) + i;
-                                sm.cand_mask[tot + k / kSplitParts] = (uint8_t)tgt_mask;
+                        const uint32_t inc = warp_incl_scan(c);
+                        const uint32_t all = __shfl_sync(0xFFFFFFFFu, inc, 31);
+                        const uint32_t ex = inc - c;
+                        const bool lf = (link >> 28) == 0;
+                        if (SPLIT && parts > 1u) {
+                            const uint32_t off = (part - crun) % kSplitParts;
+                            for (uint32_t i = 0; i < c; ++i) {
+                                const uint32_t k = ex + i - off;
+                                if (k % kSplitParts == 0) {
+                                    sm.cand_node[tot + k / kSplitParts] =
+                                        lf ? s0 : (link & kLinkMask) + i;
+                                    sm.cand_mask[tot + k / kSplitParts] = (uint8_t)tgt_mask;
+                                }
+                            }
+                            if (all > off) tot += (all - off + kSplitParts - 1) / kSplitParts;
+                            crun += all;
+                        } else {
+                            tot = all;
+                            // a chain group's candidates are first tested against its
+                            // ancestor a_{K+1} alone (level 1, no children)
+                            const uint8_t cmk = (uint8_t)((XL && nchain) ? 0u : tgt_mask);
+                            for (uint32_t i = 0; i < c; ++i) {
+                                sm.cand_node[ex + i] = lf ? s0 : (link & kLinkMask) + i;
+                                sm.cand_mask[ex + i] = cmk;
+                                if constexpr (MODE == MODE_LEAF && XL)
+                                    sm.cand_lvl[ex + i] = nchain ? 1 : 0;
                             }
                         }
-                        if (all > off) tot += (all - off + kSplitParts - 1) / kSplitParts;
-                        crun += all;
-                    } else {
-                    tot = all;
-                    // a chain group's candidates are first tested against its
-                    // ancestor a_{K+1} alone (level 1, no children)
-                    const uint8_t cmk = (uint8_t)((XL && nchain) ? 0u : tgt_mask);
-                    for (uint32_t i = 0; i < c; ++i) {
-                        sm.cand_node[ex + i] = lf ? s0 : (link & kLinkMask) + i;
-                        sm.cand_mask[ex + i] = cmk;
-                        if constexpr (MODE == MODE_LEAF && XL)
-                            sm.cand_lvl[ex + i] = nchain ? 1 : 0;
-                    }
-                    }
-                    e0 += 32;
+                        e0 += 32;
                     } while (SPLIT && parts > 1u && tot < 32u && e0 < nsn);
                 } else if (MODE == MODE_LEAF && ssize > 0) {
                     // pop entries (bounded so the stack cannot overflow) and
@@ -1473,8 +1476,8 @@ struct DenseRun {
 
 // one record
 template <bool KAHAN>
-__device__ __forceinline__ void dense_record(const TravArgs& A, DenseSmem& sm, uint4 rec, uint32_t slot,
-                                             unsigned long long& inter) {
+__device__ __forceinline__ void dense_record(const TravArgs& A, DenseSmem& sm, uint4 rec,
+                                             uint32_t slot, unsigned long long& inter) {
     const TreeView& tv = A.tv;
     const float4* __restrict__ xyzm = A.xyzm;
     const uint32_t lane = lane_id(), le_mask = lanemask_lt() | (1u << lane);

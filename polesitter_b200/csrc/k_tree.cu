@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(256) k_tree_link(TreeView tv, Status* status) 
         tv.ready[id] = 0;
         if (nch == 0) max_leaf = inf.y;
         // batched systems: each system picks its own leaf-pass variant
-        if (nch == 0 && tv.part_sys && inf.y >= 32u)
+        if (nch == 0 && tv.part_sys && inf.y >= kDenseSwitch)
             atomicMax(&tv.sys_maxleaf[tv.part_sys[inf.x]], inf.y);
     }
     const uint32_t peers = __match_any_sync(0xFFFFFFFFu, nch ? (uint32_t)d : kNone);

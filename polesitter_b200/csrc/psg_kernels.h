@@ -158,6 +158,14 @@ constexpr uint32_t kDenseTargets = 16;
 // leaf capacity from which a tree takes the leaf pass's DENSE variant whatever
 // its fullest leaf
 constexpr uint32_t kDenseCap = 8;
+// ... and, below that capacity, the fullest leaf: the sparse variant sums a leaf's
+// P2P in its group's own warp, which one leaf of many particles (each of them a
+// walk over its group's whole list) holds up for long, while the dense variant's
+// records cost a tree of one-particle leaves more than they spread.  Measured
+// (ticks, sparse / dense): fullest leaf 1, 1K cube 0.238 / 0.263 ms; 3, 65K Plummer
+// 0.428 / 0.50; 10, 1M Plummer 2.28 / 3.16; 61, two spheres of 4M in all, two ticks
+// 13.0 / 12.7; 99, 100K clumpy at theta 8 7.59 / 4.56.
+constexpr uint32_t kDenseSwitch = 32;
 
 // work records of k_dense_p2p and, where a group's source list is recorded in
 // several segments, the slots their sums meet in

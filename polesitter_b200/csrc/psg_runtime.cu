@@ -548,10 +548,11 @@ static int heavy_depth_of(float theta, size_t n) {
     return d < 2 ? 2 : d;
 }
 
-// Depth above which the leaf pass splits groups over kSplitParts warps: where
-// a leaf's walk is long (2^d <= 4 theta, at most depth 4), and only above the
-// depth at which n particles spread evenly would have their leaves (8^d * cap
-// < n), since groups that are the rule need no help.  Measured (leaf pass and
+// Depth above which the leaf pass splits groups over kSplitParts warps: 3 from
+// theta 3 and 4 from theta 4 on, where a shallow leaf's walk is long, none below
+// theta 3, and only above the depth at which n particles spread evenly would have
+// their leaves (8^d * cap < n), since groups that are the rule need no help.
+// Measured (leaf pass and
 // full-leaf P2P, one warp per group / split): 32K clumpy at theta 8 7.0 / 2.8
 // ms, 131K clumpy at theta 6.25 and leaf capacity 16 1.87 / 1.42 ms; theta 3
 // 32K clumpy 0.41 / 0.42 ms; without the second limit 32K cube at theta 10 and
@@ -1277,9 +1278,9 @@ static int prepare(const psg_arrays_t* a, float* out_min, float* out_max, float*
 // box and Morton codes, the radix sort (four code passes, then stable passes
 // on the system index, so each system ends sorted within its range), the
 // tree build (a system's first position starts its root, node k of level 0;
-// no run crosses a system boundary), the level-synchronous upward pass, and
-// the persistent traversal kernels, whose work queues run over the groups of
-// every system with each group's own theta, root, leaf-pass variant and
+// no run crosses a system boundary), the upward pass, and the persistent
+// traversal kernels, whose work queues run over the groups of every system
+// with each group's own theta, root, leaf-pass variant, split depth and
 // shallow-leaf depth.  Per system the arithmetic is exactly that of its own
 // tick, so the results equal each system's ps_b200_run_ticks bit for bit.
 // One tick is two CUDA graphs captured once and replayed (forces; velocity
