@@ -513,10 +513,10 @@ __device__ __forceinline__ void leaf_epilogue(SmemLeaf& sm, const TravArgs& o, u
 // makes them, in this launch); false after kReadyPolls polls (a poll takes 0.26 us
 // alone and up to 0.65 us on a full GPU: 0.27 to 0.7 s) or once another wait has
 // given up.  The longest waits are for groups whose candidates are most of a
-// level's nodes: 3,000 polls measured (100K particles, theta 16), 114 at 1M and
-// theta 2.  A group that gives up leaves its children's lists and offsets as an
-// earlier run left them, or never written: every later kernel of the run returns at
-// once (PSG_ERR_VOID).  Warp-collective.
+// level's nodes: 9,100 polls measured (256K cube at theta 48; 5,700 for 1M clumpy
+// there, 114 for 1M Plummer at theta 2).  A group that gives up leaves its
+// children's lists and offsets as an earlier run left them, or never written: every
+// later kernel of the run returns at once (PSG_ERR_VOID).  Warp-collective.
 constexpr int kReadyPolls = 1 << 20;
 
 __device__ __noinline__ bool wait_ready(const uint32_t* flag, int polls, Status* status) {
@@ -648,7 +648,13 @@ __global__ void __launch_bounds__(
 
     for (;;) {
         uint32_t g0 = 0;
-        if (lane == 0) g0 = atomicAdd(work, batch);
+        if (lane == 0) {
+            g0 = atomicAdd(work, batch);
+            // once k_heavy_leaf, beside it, has run out of frontier the run is void
+            // (first tick of 1M clumpy at theta 48: 28.4 s when it was taken to its
+            // end and then done again, 13.8 so)
+            if (XL && (*(volatile uint32_t*)&status->err & PSG_ERR_HEAVY_OVERFLOW)) g0 = items;
+        }
         g0 = __shfl_sync(0xFFFFFFFFu, g0, 0);
         if (g0 >= items) break;
 #pragma unroll 1
