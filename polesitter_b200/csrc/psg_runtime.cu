@@ -153,9 +153,8 @@ struct State {
     unsigned long long stats[24];
     uint32_t last_nodes;
     uint32_t lvl_count[kLevels];  // node counts of the last completed tick
-    // workspace of ps_b200_direct_f64 (grown by its calls)
-    double* direct_ws;
-    size_t direct_bytes;
+    void* work;            // workspace of one call at a time (struct Work)
+    size_t work_bytes;
     // device tick loop scratch (allocated by its first call)
     int tk_grid;
     float2* tk_partial;
@@ -217,6 +216,39 @@ template <typename T>
 static T* carved(void* base, size_t at) {
     return reinterpret_cast<T*>(static_cast<char*>(base) + at);
 }
+
+// The device workspace of a call that brings data of its own (direct sums; the
+// closure's features, network, gradient and training), one call at a time.  It
+// stays with the context, so that repeated calls allocate nothing: with an
+// allocation per array a call paid 0.64 ms more whenever its small arrays needed
+// a page that the driver had just taken back (8192 samples trained 0.99 / 0.33 ms,
+// the network on 5000 0.78 / 0.14 ms).  Past kWorkKeep it is given back at the
+// call's end.
+constexpr size_t kWorkKeep = (size_t)64 << 20;
+
+struct Work {
+    State* s;
+    Carve c;
+    explicit Work(State* state) : s(state) {}
+    ~Work() {
+        if (s->work_bytes <= kWorkKeep) return;
+        cudaFree(s->work);
+        s->work = nullptr;
+        s->work_bytes = 0;
+    }
+    // (after every add)
+    int alloc() {
+        if (s->work_bytes >= c.total) return PSG_OK;
+        if (s->work) cudaFree(s->work);
+        s->work = nullptr;
+        s->work_bytes = 0;
+        PSG_ALLOC(s->work, c.total);
+        s->work_bytes = c.total;
+        return PSG_OK;
+    }
+    template <typename T>
+    T* at(size_t off) const { return carved<T>(s->work, off); }
+};
 
 static int alloc_p2p(State* s, uint32_t chunks) {
     P2PStore& p = s->p2p;
@@ -381,7 +413,7 @@ static Place place_of(const void* p) {
 static bool on_device(const void* p) { return place_of(p) == DEVICE; }
 
 static void free_state(State* s) {
-    void* ps[] = {s->xyzm, s->ns, s->p2p.src, s->dense.rec, s->direct_ws, s->split.sums,
+    void* ps[] = {s->xyzm, s->ns, s->p2p.src, s->dense.rec, s->work, s->split.sums,
                   s->heavy_frontier, s->tk_partial, s->tk_bbox, s->tk_v[0], s->tk_v[1], s->tk_v[2],
                   s->tk_vmir[0], s->tk_vmir[1], s->tk_vmir[2], s->cl.lg0, s->cl.lg1,
                   s->cl.leaf_of, s->cl.dF, s->cl.params, s->cl.packed, s->cl.judge_tg,
@@ -2126,22 +2158,18 @@ int psg_direct_f64(void* mem, const psg_arrays_t* a, const uint32_t* targets, si
         PSG_CHECK(cudaMemcpyAsync(rows[c], src[c], n * 4, cudaMemcpyHostToDevice, st));
         src[c] = rows[c];
     }
-    // workspace, kept with the context: targets, forces, partial sums
     const bool ht = !psg::on_device(targets), ho = !psg::on_device(out);
     const size_t part_n = psg::direct_f64_part_doubles(n, n_t, s->sms * 8);
-    const size_t need = (part_n + n_t * 3) * sizeof(double) + n_t * 4;
-    if (s->direct_bytes < need) {
-        if (s->direct_ws) cudaFree(s->direct_ws);
-        s->direct_ws = nullptr;
-        s->direct_bytes = 0;
-        PSG_ALLOC(s->direct_ws, need);
-        s->direct_bytes = need;
-    }
-    double* const part = s->direct_ws;
-    double* const dout = ho ? part + part_n : out;
+    psg::Work ws(s);
+    const size_t o_part = ws.c.add(part_n * sizeof(double)),
+                 o_out = ws.c.add(n_t * 3 * sizeof(double)), o_tg = ws.c.add(n_t * 4);
+    const int rw = ws.alloc();
+    if (rw != PSG_OK) return rw;
+    double* const part = ws.at<double>(o_part);
+    double* const dout = ho ? ws.at<double>(o_out) : out;
     const uint32_t* dt = targets;
     if (ht) {
-        uint32_t* const d = (uint32_t*)(part + part_n + n_t * 3);
+        uint32_t* const d = ws.at<uint32_t>(o_tg);
         PSG_CHECK(cudaMemcpyAsync(d, targets, n_t * 4, cudaMemcpyHostToDevice, st));
         dt = d;
     }
@@ -2299,10 +2327,12 @@ int psg_closure_features(void* mem, const uint32_t* idx, size_t k, float* x_out,
     if (k == 0) return PSG_OK;
     PSG_CHECK(cudaSetDevice(s->device));
     cudaStream_t st = s->stream;
-    uint32_t* d_idx = nullptr;
-    float* d_x = nullptr;
-    PSG_ALLOC(d_idx, k * 4);
-    PSG_ALLOC(d_x, k * 17 * 4);
+    psg::Work ws(s);
+    const size_t o_idx = ws.c.add(k * 4), o_x = ws.c.add(k * 17 * 4);
+    const int rw = ws.alloc();
+    if (rw != PSG_OK) return rw;
+    uint32_t* const d_idx = ws.at<uint32_t>(o_idx);
+    float* const d_x = ws.at<float>(o_x);
     PSG_CHECK(cudaMemcpyAsync(d_idx, idx, k * 4, cudaMemcpyHostToDevice, st));
     psg::TreeView tv = s->tv;
     tv.lg0 = s->cl.lg0;
@@ -2313,8 +2343,6 @@ int psg_closure_features(void* mem, const uint32_t* idx, size_t k, float* x_out,
     PSG_CHECK(cudaMemcpyAsync(x_out, d_x, k * 16 * 4, cudaMemcpyDeviceToHost, st));
     PSG_CHECK(cudaMemcpyAsync(scale_out, d_x + k * 16, k * 4, cudaMemcpyDeviceToHost, st));
     PSG_CHECK(cudaStreamSynchronize(st));
-    cudaFree(d_idx);
-    cudaFree(d_x);
     return PSG_OK;
 }
 
@@ -2330,19 +2358,19 @@ int psg_closure_train(void* mem, const float* x, const float* t, size_t n, float
     cudaStream_t st = s->stream;
     PSG_CHECK(psg::prepare_mlp_grad_kernel());
     const int P = psg::kMlpParams;
-    float *d_x = nullptr, *d_t = nullptr, *d_p = nullptr, *d_m = nullptr, *d_v = nullptr,
-          *d_g = nullptr, *d_loss = nullptr;
-    uint32_t* d_perm = nullptr;
-    psg::MlpPacked* d_w = nullptr;
-    PSG_ALLOC(d_x, n * 16 * 4);
-    PSG_ALLOC(d_t, n * 3 * 4);
-    PSG_ALLOC(d_perm, n * 4);
-    PSG_ALLOC(d_p, P * 4);
-    PSG_ALLOC(d_m, P * 4);
-    PSG_ALLOC(d_v, P * 4);
-    PSG_ALLOC(d_g, P * 4);
-    PSG_ALLOC(d_loss, (epochs ? epochs : 1) * 4);
-    PSG_ALLOC(d_w, sizeof(psg::MlpPacked));
+    psg::Work ws(s);
+    const size_t o_x = ws.c.add(n * 16 * 4), o_t = ws.c.add(n * 3 * 4), o_perm = ws.c.add(n * 4),
+                 o_p = ws.c.add(P * 4), o_m = ws.c.add(P * 4), o_v = ws.c.add(P * 4),
+                 o_g = ws.c.add(P * 4), o_loss = ws.c.add((size_t)(epochs ? epochs : 1) * 4),
+                 o_w = ws.c.add(sizeof(psg::MlpPacked));
+    const int rw = ws.alloc();
+    if (rw != PSG_OK) return rw;
+    float *const d_x = ws.at<float>(o_x), *const d_t = ws.at<float>(o_t),
+          *const d_p = ws.at<float>(o_p), *const d_m = ws.at<float>(o_m),
+          *const d_v = ws.at<float>(o_v), *const d_g = ws.at<float>(o_g),
+          *const d_loss = ws.at<float>(o_loss);
+    uint32_t* const d_perm = ws.at<uint32_t>(o_perm);
+    psg::MlpPacked* const d_w = ws.at<psg::MlpPacked>(o_w);
     PSG_CHECK(cudaMemcpyAsync(d_x, x, n * 16 * 4, cudaMemcpyHostToDevice, st));
     PSG_CHECK(cudaMemcpyAsync(d_t, t, n * 3 * 4, cudaMemcpyHostToDevice, st));
     PSG_CHECK(cudaMemcpyAsync(d_p, params, P * 4, cudaMemcpyHostToDevice, st));
@@ -2397,8 +2425,6 @@ int psg_closure_train(void* mem, const float* x, const float* t, size_t n, float
             for (uint32_t ep = 0; ep < epochs; ++ep) loss_out[ep] /= (float)(3 * n);
     }
     cudaFreeHost(perm);
-    void* bufs[] = {d_x, d_t, d_perm, d_p, d_m, d_v, d_g, d_loss, d_w};
-    for (void* b : bufs) cudaFree(b);
     if (r != PSG_OK) std::snprintf(psg::g_err, sizeof(psg::g_err), "closure training failed");
     return r;
 }
@@ -2414,14 +2440,16 @@ int psg_closure_grad(void* mem, const float* x, const float* t, size_t n, const 
     cudaStream_t st = s->stream;
     PSG_CHECK(psg::prepare_mlp_grad_kernel());
     const int P = psg::kMlpParams;
-    float *d_x = nullptr, *d_t = nullptr, *d_p = nullptr, *d_g = nullptr, *d_loss = nullptr;
-    psg::MlpPacked* d_w = nullptr;
-    PSG_ALLOC(d_x, n * 16 * 4);
-    PSG_ALLOC(d_t, n * 3 * 4);
-    PSG_ALLOC(d_p, P * 4);
-    PSG_ALLOC(d_g, P * 4);
-    PSG_ALLOC(d_loss, 4);
-    PSG_ALLOC(d_w, sizeof(psg::MlpPacked));
+    psg::Work ws(s);
+    const size_t o_x = ws.c.add(n * 16 * 4), o_t = ws.c.add(n * 3 * 4), o_p = ws.c.add(P * 4),
+                 o_g = ws.c.add(P * 4), o_loss = ws.c.add(4),
+                 o_w = ws.c.add(sizeof(psg::MlpPacked));
+    const int rw = ws.alloc();
+    if (rw != PSG_OK) return rw;
+    float *const d_x = ws.at<float>(o_x), *const d_t = ws.at<float>(o_t),
+          *const d_p = ws.at<float>(o_p), *const d_g = ws.at<float>(o_g),
+          *const d_loss = ws.at<float>(o_loss);
+    psg::MlpPacked* const d_w = ws.at<psg::MlpPacked>(o_w);
     PSG_CHECK(cudaMemcpyAsync(d_x, x, n * 16 * 4, cudaMemcpyHostToDevice, st));
     PSG_CHECK(cudaMemcpyAsync(d_t, t, n * 3 * 4, cudaMemcpyHostToDevice, st));
     PSG_CHECK(cudaMemcpyAsync(d_p, params, P * 4, cudaMemcpyHostToDevice, st));
@@ -2435,8 +2463,6 @@ int psg_closure_grad(void* mem, const float* x, const float* t, size_t n, const 
     PSG_CHECK(cudaMemcpyAsync(&loss, d_loss, 4, cudaMemcpyDeviceToHost, st));
     PSG_CHECK(cudaStreamSynchronize(st));
     if (loss_out) *loss_out = loss / (float)(3 * n);
-    void* bufs[] = {d_x, d_t, d_p, d_g, d_loss, d_w};
-    for (void* b : bufs) cudaFree(b);
     return PSG_OK;
 }
 
@@ -2447,12 +2473,14 @@ int psg_closure_forward(void* mem, const float* x, size_t n, const float* params
     if (!s || s->magic != psg::kMagic || !x || !params || !y_out || n == 0) return PSG_EINVAL;
     PSG_CHECK(cudaSetDevice(s->device));
     cudaStream_t st = s->stream;
-    float *d_x = nullptr, *d_p = nullptr, *d_y = nullptr;
-    psg::MlpPacked* d_w = nullptr;
-    PSG_ALLOC(d_x, n * 16 * 4);
-    PSG_ALLOC(d_p, psg::kMlpParams * 4);
-    PSG_ALLOC(d_y, n * 8 * 4);
-    PSG_ALLOC(d_w, sizeof(psg::MlpPacked));
+    psg::Work ws(s);
+    const size_t o_x = ws.c.add(n * 16 * 4), o_p = ws.c.add(psg::kMlpParams * 4),
+                 o_y = ws.c.add(n * 8 * 4), o_w = ws.c.add(sizeof(psg::MlpPacked));
+    const int rw = ws.alloc();
+    if (rw != PSG_OK) return rw;
+    float *const d_x = ws.at<float>(o_x), *const d_p = ws.at<float>(o_p),
+          *const d_y = ws.at<float>(o_y);
+    psg::MlpPacked* const d_w = ws.at<psg::MlpPacked>(o_w);
     PSG_CHECK(cudaMemcpyAsync(d_x, x, n * 16 * 4, cudaMemcpyHostToDevice, st));
     PSG_CHECK(cudaMemcpyAsync(d_p, params, psg::kMlpParams * 4, cudaMemcpyHostToDevice, st));
     psg::launch_mlp_pack(d_p, d_w, st);
@@ -2463,8 +2491,6 @@ int psg_closure_forward(void* mem, const float* x, size_t n, const float* params
     PSG_CHECK(cudaMemcpyAsync(&s->h_status->err, &s->d_status->err, 4, cudaMemcpyDeviceToHost,
                               st));
     PSG_CHECK(cudaStreamSynchronize(st));
-    void* bufs[] = {d_x, d_p, d_y, d_w};
-    for (void* b : bufs) cudaFree(b);
     if (s->h_status->err & PSG_ERR_TC_TIMEOUT) {
         std::snprintf(psg::g_err, sizeof(psg::g_err),
                       "closure network: a tensor-core MMA did not complete");
